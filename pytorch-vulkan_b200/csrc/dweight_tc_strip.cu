@@ -602,22 +602,64 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_strip_kernel(const DwStrip
   }
 }
 
-// Sum the split partials [split][cout][taps][cig] in ascending split order (run-to-run identical)
-// and write dW[cout][cig][taps].  Threads follow the partial layout, so the reads, which are
-// `splits` times the writes, are coalesced.
+// Sum the split partials [split][cout][taps][cig] in a fixed order (run-to-run identical) and write dW[cout][cig][taps].
+// A block owns 2^ch_log2 channels of one output channel with all their taps: it reads along the channels (16 bytes at a
+// time when VEC is 4) and writes along the taps, both coalesced, with the transposition in shared memory (written straight
+// from the reading order, each warp's stores touched 32 sectors).  `slices` threads share a value when a block has fewer
+// values than threads; four splits are in flight per thread.
+constexpr int FIN_SMEM = 48 << 10;
+template <int VEC>
 __global__ void __launch_bounds__(256) finalize_partials_kernel(const float* __restrict__ partial, float* __restrict__ dw,
-                                                               long long count, int splits, int cig, int taps) {
+                                                               long long count, int splits, int cig, int taps, int slices, int ch_log2,
+                                                               FastDiv div_chunks, FastDiv div_units) {
   // launched with programmatic stream serialisation behind the kernel that writes the partials: its blocks may be
   // resident before that kernel has finished, and wait here until it has (and its stores are visible)
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  const long long i = blockIdx.x * 256ll + threadIdx.x;
-  if (i >= count) return;
-  float sum = 0.f;
-  for (int s = 0; s < splits; ++s) sum += partial[(long long)s * count + i];
-  const int ci = (int)(i % cig);
-  const int tap = (int)((i / cig) % taps);
-  const long long co = i / ((long long)cig * taps);
-  dw[(co * cig + ci) * taps + tap] = sum;
+  extern __shared__ float part[];              // [slices][channel][tap]; not used by a block of one channel
+  const int co = (int)div_chunks.div(blockIdx.x), chunk = (int)blockIdx.x - co * (int)div_chunks.d;
+  const int ch = 1 << ch_log2, c0 = chunk << ch_log2, chans = min(ch, cig - c0), values = taps << ch_log2;
+  const int units = values / VEC, per_tap = ch / VEC, ptl = ch_log2 - (VEC == 4 ? 2 : 0);
+  const float* base = partial + (long long)co * taps * cig + c0;
+  float* dst = dw + ((long long)co * cig + c0) * taps;
+  for (int item = threadIdx.x; item < units * slices; item += 256) {
+    const int slice = (int)div_units.div((uint32_t)item), e = item - slice * units, tap = e >> ptl, c = (e & (per_tap - 1)) * VEC;
+    float sum[VEC];
+#pragma unroll
+    for (int k = 0; k < VEC; ++k) sum[k] = 0.f;
+    if (c < chans) {                           // chans is a multiple of VEC
+      const float* p = base + (long long)slice * count + tap * cig + c;
+      const long long step = (long long)slices * count;
+      for (int s = slice; s < splits; s += 4 * slices, p += 4 * step) {
+        float v[4][VEC];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const bool ok = s + u * slices < splits;
+          if (VEC == 4) {
+            const float4 f = ok ? *reinterpret_cast<const float4*>(p + u * step) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[u][0] = f.x; v[u][1 % VEC] = f.y; v[u][2 % VEC] = f.z; v[u][3 % VEC] = f.w;
+          } else {
+            v[u][0] = ok ? p[u * step] : 0.f;
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int k = 0; k < VEC; ++k) sum[k] += v[u][k];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < VEC; ++k) {
+      if (ch == 1) dst[tap] = sum[k];
+      else part[slice * values + (c + k) * taps + tap] = sum[k];
+    }
+  }
+  if (ch == 1) return;
+  __syncthreads();
+  for (int e = threadIdx.x; e < chans * taps; e += 256) {
+    float sum = part[e];
+    for (int k = 1; k < slices; ++k) sum += part[k * values + e];
+    dst[e] = sum;
+  }
 }
 
 struct DwStripPlan {
@@ -798,12 +840,28 @@ int dweight_strip(const ConvGeom& g, View4 x, View4 dy, float* dw, void* ws, siz
   if (plan.splits > 1) {
     const long long count = (long long)g.cout * g.cig * g.kh * g.kw;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)div_up64(count, 256)); cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = 0; cfg.stream = st;
+    const int taps = g.kh * g.kw;
+    const bool vec = g.cig % 4 == 0;
+    // channels per block: all of them if they fit the default shared memory, fewer while the blocks do not fill the SMs
+    // twice (down to 16: shorter runs waste the sectors at their ends); a single channel needs no shared memory
+    int ch_log2 = 0;
+    while (ch_log2 < 9 && (1 << ch_log2) < g.cig && ((size_t)taps << (ch_log2 + 1)) * sizeof(float) <= FIN_SMEM) ++ch_log2;
+    while (ch_log2 > 4 && (long long)g.cout * ((g.cig + (1 << ch_log2) - 1) >> ch_log2) < 2ll * sm_count()) --ch_log2;
+    const bool v4 = vec && ch_log2 >= 2;
+    const int chunks = (g.cig + (1 << ch_log2) - 1) >> ch_log2, units = (taps << ch_log2) / (v4 ? 4 : 1);
+    const long long blocks = (long long)g.cout * chunks;
+    const size_t values = ((size_t)taps << ch_log2) * sizeof(float);
+    int slices = 1;
+    while (ch_log2 > 0 && slices * 2 <= plan.splits && units * slices < 256 && 2 * slices * values <= FIN_SMEM) slices *= 2;
+    if (blocks > 2147483647ll) return fail(B200_ERANGE, "dWeight finalize: grid exceeds launch limits");
+    cfg.gridDim = dim3((unsigned)blocks); cfg.blockDim = dim3(256); cfg.stream = st;
+    cfg.dynamicSmemBytes = ch_log2 > 0 ? slices * values : 0;
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     if (!getenv("B200_DW_NO_PDL")) { cfg.attrs = &attr; cfg.numAttrs = 1; }
-    B200_CUDA(cudaLaunchKernelEx(&cfg, finalize_partials_kernel, (const float*)ws, dw, count, plan.splits, g.cig, g.kh * g.kw));
+    B200_CUDA(cudaLaunchKernelEx(&cfg, v4 ? finalize_partials_kernel<4> : finalize_partials_kernel<1>, (const float*)ws, dw, count, plan.splits,
+                                 g.cig, taps, slices, ch_log2, FastDiv((uint32_t)chunks), FastDiv((uint32_t)units)));
     count_launch();
     return launch_check("finalize_partials_kernel");
   }
