@@ -9,9 +9,9 @@
 // of ALL the group's output channels in registers, so an input value is loaded once for up to 3 x 8 multiply-adds.
 //   forward / dInput   one kernel; dInput runs it on dy with the filter rotated by 180 degrees and its channel roles
 //                      exchanged (prepared in shared memory while the tile loads)
-//   dWeight            each thread accumulates the (ci, 3, 3) block of one output channel over its pixel strips in registers; a block
-//                      reduces them with warp shuffles and writes one partial per block; a second kernel sums the
-//                      partials in ascending order (no atomics: results are identical from run to run)
+//   dWeight            each thread accumulates a 4 x 2 block of channel pairs with their nine taps over its pixel strips in
+//                      registers; a block reduces them with warp shuffles and writes one partial per block; a second kernel
+//                      sums the partials in a fixed order (no atomics: results are identical from run to run)
 // Inputs are read through their strides (NCHW: a warp reads consecutive pixels of a channel; channels-last: the
 // channels of a pixel first); results are contiguous NCHW.
 //
@@ -24,8 +24,6 @@
 namespace b200 {
 namespace gcs {
 
-constexpr int TH = 16;                   // rows of a dWeight tile (forward / dInput tiles come from the SX template parameter)
-constexpr int IH = TH + 2;               // its input rows with halo
 constexpr int THREADS = 256;
 
 struct GArgs {
@@ -157,121 +155,175 @@ __global__ void __launch_bounds__(THREADS) gconv_fwd_kernel(const GArgs a) {
 
 // ---- dWeight -------------------------------------------------------------------------------------------------------
 // dW[g*CPG + co][ci][ky][kx] = sum_{n, y, x} dy[n, g*CPG + co, y, x] * x[n, g*CPG + ci, y + ky - 1, x + kx - 1]
-// A thread owns a strip of 4 pixels and COT output channels of the group and keeps the COT x CPG x 9 sums of its
-// strips in registers over `tiles_per_block` tiles; the CPG / COT threads of a strip split the output channels.
+// Bound by the FP32 multiply-adds (CPG * 9 per dy value) and by the shared-memory reads that feed them.  A thread owns
+// strips of 8 pixels and a 4 x 2 block of (output, input) channels: its 72 sums stay in registers, and the ten x values of
+// a filter row feed 4 * 3 * 8 multiply-adds, so the reads take under half the time of the arithmetic (one output channel
+// and 4 pixels per thread read as much for an eighth of the work: 151 us at 256 channels, 32x32, batch 16; 14 us now).
+// Tiles of (128 / NQ / SX) rows x 8*SX columns arrive by 4-byte cp.async (any strides; zero fill outside the image), one or
+// two tiles ahead of the one being used.
 struct GdwArgs {
   View4 x, dy;
   float* partial;      // [blocks per group][cout][CPG][9]
   int n, c, h, w_, groups;
   int tiles_y, tiles_x, tiles_per_block, blocks_per_group;
 };
+constexpr int DW_THREADS = 128, DW_PITCH = 36;   // the pitch keeps 8-float strips of two rows on distinct banks
+template <int CPG> constexpr int dw_stages = CPG == 4 ? 2 : 3;   // within 48 KB
+template <int CPG> constexpr int dw_rows = DW_THREADS / (CPG * CPG / 8) / 4;   // tile rows (4 strips of 8 per row)
 
-template <int CPG, int COT>
-__global__ void __launch_bounds__(THREADS) gconv_dw_kernel(const GdwArgs a) {
-  constexpr int NQ = CPG / COT;                 // threads per strip
-  constexpr int STRIPS = THREADS / NQ;          // strips per tile
-  constexpr int SW = STRIPS / TH;               // strips per tile row
-  constexpr int DW_TW = SW * 4;                 // tile width in pixels
-  constexpr int XW = DW_TW + 4;                 // input row with halo, padded to a multiple of 4
-  __shared__ __align__(16) float s_x[CPG][IH][XW];
-  __shared__ __align__(16) float s_dy[CPG][TH][DW_TW];
-  const int tid = threadIdx.x;
+__device__ __forceinline__ void cp_async4(float* dst, const float* src, bool ok) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(ok ? 4 : 0) : "memory");
+}
+
+template <int CPG>
+__global__ void __launch_bounds__(DW_THREADS, 3) gconv_dw_kernel(const GdwArgs a) {
+  constexpr int NQ = CPG * CPG / 8;             // 4 x 2 channel blocks of a group
+  constexpr int STRIPS = DW_THREADS / NQ;       // strips per tile
+  constexpr int SX = 4, TR = STRIPS / SX, TW = 8 * SX;   // strips per row, rows, columns
+  constexpr int WARPS = DW_THREADS / 32, DW_STAGES = dw_stages<CPG>;
+  __shared__ __align__(16) float s_x[DW_STAGES][CPG][TR + 2][DW_PITCH];
+  __shared__ __align__(16) float s_dy[DW_STAGES][CPG][TR][DW_PITCH];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = blockIdx.x / a.blocks_per_group, pb = blockIdx.x % a.blocks_per_group;
   const long long chan0 = (long long)g * CPG;
-  const int q = tid / STRIPS, strip = tid % STRIPS;     // a warp holds one q (STRIPS >= 32)
-  const int ty = strip / SW, sx = strip % SW;
-  float acc[COT][CPG][9];
+  const int q = tid / STRIPS, strip = tid % STRIPS;
+  const int co0 = (q / (CPG / 2)) * 4, ci0 = (q % (CPG / 2)) * 2;
+  const int ty = strip / SX, sx = strip % SX;
+  float acc[72];       // [co 4][ci 2][tap 9]
 #pragma unroll
-  for (int co = 0; co < COT; ++co)
-#pragma unroll
-    for (int ci = 0; ci < CPG; ++ci)
-#pragma unroll
-      for (int k = 0; k < 9; ++k) acc[co][ci][k] = 0.f;
+  for (int i = 0; i < 72; ++i) acc[i] = 0.f;
   const int tiles_img = a.tiles_y * a.tiles_x, tiles_all = a.n * tiles_img;
-  for (int it = 0; it < a.tiles_per_block; ++it) {
-    const int t = pb * a.tiles_per_block + it;
-    if (t >= tiles_all) break;
-    const int n = t / tiles_img, rem = t % tiles_img;
-    const int y0 = (rem / a.tiles_x) * TH, x0 = (rem % a.tiles_x) * DW_TW;
-    __syncthreads();   // the previous tile has been consumed
+  const int t_begin = pb * a.tiles_per_block, t_end = min(tiles_all, t_begin + a.tiles_per_block);
+
+  auto load_tile = [&](int t, int stage) {
+    const int n = t / tiles_img, rem = t - n * tiles_img;
+    const int tyi = rem / a.tiles_x, y0 = tyi * TR, x0 = (rem - tyi * a.tiles_x) * TW;
     const float* px = a.x.ptr + n * a.x.s0 + chan0 * a.x.s1;
     const float* pd = a.dy.ptr + n * a.dy.s0 + chan0 * a.dy.s1;
-    if (a.x.s1 == 1) {
-#pragma unroll
-      for (int i = tid; i < CPG * IH * (DW_TW + 2); i += THREADS) {
-        const int ci = i % CPG, c = (i / CPG) % (DW_TW + 2), r = i / (CPG * (DW_TW + 2));
-        const int y = y0 - 1 + r, x = x0 - 1 + c;
-        s_x[ci][r][c] = (y >= 0 && y < a.h && x >= 0 && x < a.w_) ? __ldg(px + ci + (long long)y * a.x.s2 + (long long)x * a.x.s3) : 0.f;
+    if (a.x.s1 == 1) {   // channels-last: the channels of a pixel are adjacent
+      for (int i = tid; i < CPG * (TR + 2) * (TW + 2); i += DW_THREADS) {
+        const int ci = i % CPG, c = (i / CPG) % (TW + 2), r = i / (CPG * (TW + 2)), y = y0 - 1 + r, x = x0 - 1 + c;
+        const bool ok = y >= 0 && y < a.h && x >= 0 && x < a.w_;
+        cp_async4(&s_x[stage][ci][r][c], ok ? px + ci + (long long)y * a.x.s2 + (long long)x * a.x.s3 : a.x.ptr, ok);
       }
-    } else {
+    } else {             // a warp copies one row of 32 columns at a time, then the two last columns of all rows
+      const int x = x0 - 1 + lane;
+      const bool xok = x >= 0 && x < a.w_;
 #pragma unroll
-      for (int i = tid; i < CPG * IH * (DW_TW + 2); i += THREADS) {
-        const int c = i % (DW_TW + 2), r = (i / (DW_TW + 2)) % IH, ci = i / ((DW_TW + 2) * IH);
-        const int y = y0 - 1 + r, x = x0 - 1 + c;
-        s_x[ci][r][c] = (y >= 0 && y < a.h && x >= 0 && x < a.w_) ? __ldg(px + ci * a.x.s1 + (long long)y * a.x.s2 + (long long)x * a.x.s3) : 0.f;
+      for (int i = warp; i < CPG * (TR + 2); i += WARPS) {
+        const int ci = i / (TR + 2), r = i % (TR + 2), y = y0 - 1 + r;
+        const bool ok = xok && y >= 0 && y < a.h;
+        cp_async4(&s_x[stage][ci][r][lane], ok ? px + ci * a.x.s1 + (long long)y * a.x.s2 + (long long)x * a.x.s3 : a.x.ptr, ok);
+      }
+      for (int i = tid; i < CPG * (TR + 2) * 2; i += DW_THREADS) {
+        const int c = 32 + (i & 1), r = (i >> 1) % (TR + 2), ci = (i >> 1) / (TR + 2), y = y0 - 1 + r, xe = x0 - 1 + c;
+        const bool ok = xe < a.w_ && y >= 0 && y < a.h;
+        cp_async4(&s_x[stage][ci][r][c], ok ? px + ci * a.x.s1 + (long long)y * a.x.s2 + (long long)xe * a.x.s3 : a.x.ptr, ok);
       }
     }
     if (a.dy.s1 == 1) {
 #pragma unroll
-      for (int i = tid; i < CPG * TH * DW_TW; i += THREADS) {
-        const int co = i % CPG, c = (i / CPG) % DW_TW, r = i / (CPG * DW_TW);
-        const int y = y0 + r, x = x0 + c;
-        s_dy[co][r][c] = (y < a.h && x < a.w_) ? __ldg(pd + co + (long long)y * a.dy.s2 + (long long)x * a.dy.s3) : 0.f;
+      for (int i = tid; i < CPG * TR * TW; i += DW_THREADS) {
+        const int co = i % CPG, c = (i / CPG) % TW, r = i / (CPG * TW), y = y0 + r, x = x0 + c;
+        const bool ok = y < a.h && x < a.w_;
+        cp_async4(&s_dy[stage][co][r][c], ok ? pd + co + (long long)y * a.dy.s2 + (long long)x * a.dy.s3 : a.dy.ptr, ok);
       }
     } else {
+      const int x = x0 + lane;
 #pragma unroll
-      for (int i = tid; i < CPG * TH * DW_TW; i += THREADS) {
-        const int c = i % DW_TW, r = (i / DW_TW) % TH, co = i / (DW_TW * TH);
-        const int y = y0 + r, x = x0 + c;
-        s_dy[co][r][c] = (y < a.h && x < a.w_) ? __ldg(pd + co * a.dy.s1 + (long long)y * a.dy.s2 + (long long)x * a.dy.s3) : 0.f;
+      for (int i = warp; i < CPG * TR; i += WARPS) {
+        const int co = i / TR, r = i % TR, y = y0 + r;
+        const bool ok = x < a.w_ && y < a.h;
+        cp_async4(&s_dy[stage][co][r][lane], ok ? pd + co * a.dy.s1 + (long long)y * a.dy.s2 + (long long)x * a.dy.s3 : a.dy.ptr, ok);
       }
     }
-    __syncthreads();
-    float d[COT][4];
+  };
+
 #pragma unroll
-    for (int co = 0; co < COT; ++co) {
-      const float4 t4 = *reinterpret_cast<const float4*>(&s_dy[q * COT + co][ty][4 * sx]);
-      d[co][0] = t4.x; d[co][1] = t4.y; d[co][2] = t4.z; d[co][3] = t4.w;
+  for (int s = 0; s < DW_STAGES - 1; ++s) {
+    if (t_begin + s < t_end) load_tile(t_begin + s, s);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  int stage = 0;
+  for (int t = t_begin; t < t_end; ++t) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(DW_STAGES - 2) : "memory");
+    __syncthreads();   // tile t has landed for every thread, and the stage of tile t - 1 has been consumed
+    {
+      const int ahead = t + DW_STAGES - 1;
+      if (ahead < t_end) load_tile(ahead, stage == 0 ? DW_STAGES - 1 : stage - 1);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    float d[4][8];
+#pragma unroll
+    for (int co = 0; co < 4; ++co) {
+      const float4 lo = *reinterpret_cast<const float4*>(&s_dy[stage][co0 + co][ty][8 * sx]);
+      const float4 hi = *reinterpret_cast<const float4*>(&s_dy[stage][co0 + co][ty][8 * sx + 4]);
+      d[co][0] = lo.x; d[co][1] = lo.y; d[co][2] = lo.z; d[co][3] = lo.w;
+      d[co][4] = hi.x; d[co][5] = hi.y; d[co][6] = hi.z; d[co][7] = hi.w;
     }
 #pragma unroll
-    for (int ci = 0; ci < CPG; ++ci) {
+    for (int ci = 0; ci < 2; ++ci)
 #pragma unroll
       for (int ky = 0; ky < 3; ++ky) {
-        const float4 p0 = *reinterpret_cast<const float4*>(&s_x[ci][ty + ky][4 * sx]);
-        const float2 p1 = *reinterpret_cast<const float2*>(&s_x[ci][ty + ky][4 * sx + 4]);
-        const float v[6] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y};
+        const float* row = &s_x[stage][ci0 + ci][ty + ky][8 * sx];
+        const float4 p0 = *reinterpret_cast<const float4*>(row), p1 = *reinterpret_cast<const float4*>(row + 4);
+        const float2 p2 = *reinterpret_cast<const float2*>(row + 8);
+        const float v[10] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w, p2.x, p2.y};
 #pragma unroll
-        for (int kx = 0; kx < 3; ++kx)
+        for (int co = 0; co < 4; ++co)
 #pragma unroll
-          for (int co = 0; co < COT; ++co)
+          for (int kx = 0; kx < 3; ++kx)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[co][ci][ky * 3 + kx] = fmaf(d[co][j], v[j + kx], acc[co][ci][ky * 3 + kx]);
+            for (int j = 0; j < 8; ++j) acc[(co * 2 + ci) * 9 + ky * 3 + kx] = fmaf(d[co][j], v[j + kx], acc[(co * 2 + ci) * 9 + ky * 3 + kx]);
       }
+    if (++stage == DW_STAGES) stage = 0;
+  }
+  // Sum over the strips of a channel block: three halving exchanges over lane bits 3, 2, 1 (after each, a lane keeps half of the
+  // values, summed over the pair), then plain exchanges over the remaining lane bits, in a fixed order.
+  {
+    int keep = 36;
+#pragma unroll
+    for (int step = 0; step < 3; ++step, keep /= 2) {
+      const int o = 8 >> step;
+      const bool upper = (lane & o) != 0;
+#pragma unroll
+      for (int i = 0; i < 36; ++i)
+        if (i < keep) {
+          const float mine = upper ? acc[keep + i] : acc[i], theirs = upper ? acc[i] : acc[keep + i];
+          acc[i] = mine + __shfl_xor_sync(0xffffffffu, theirs, o);
+        }
     }
   }
-  // block reduction: shuffles inside a warp (one q per warp), then across the warps of a q in shared memory, in a
-  // fixed order, so that the partial of a block is the same from run to run
-  __shared__ float s_red[THREADS / 32][COT * CPG * 9];
-  const int warp = tid >> 5, lane = tid & 31;
 #pragma unroll
-  for (int co = 0; co < COT; ++co)
+  for (int i = 0; i < 9; ++i) {
+    acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], 1);
+    if (STRIPS >= 32) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], 16);
+  }
+  // lane bits 3..1 select nine adjacent values: piece = (co, ci) of the channel block
+  const int piece = ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1);
+  const int co = co0 + (piece >> 1), ci = ci0 + (piece & 1);
+  float* out = a.partial + ((long long)pb * a.c + chan0 + co) * (CPG * 9) + ci * 9;
+  if (STRIPS <= 32) {
+    if ((lane & 1) == 0 && (STRIPS < 32 || lane < 16)) {
 #pragma unroll
-    for (int ci = 0; ci < CPG; ++ci)
+      for (int i = 0; i < 9; ++i) out[i] = acc[i];
+    }
+  } else {               // several warps hold the same channel block (4 channels per group: two)
+    constexpr int WPQ = STRIPS / 32 > 0 ? STRIPS / 32 : 1;
+    __shared__ float s_red[WARPS][72];
+    if ((lane & 1) == 0 && lane < 16)
 #pragma unroll
-      for (int k = 0; k < 9; ++k) {
-        float v = acc[co][ci][k];
+      for (int i = 0; i < 9; ++i) s_red[warp][piece * 9 + i] = acc[i];
+    __syncthreads();
+    if (warp % WPQ == 0 && (lane & 1) == 0 && lane < 16) {
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-        if (lane == 0) s_red[warp][(co * CPG + ci) * 9 + k] = v;
+      for (int i = 0; i < 9; ++i) {
+        float v = acc[i];
+        for (int w = 1; w < WPQ; ++w) v += s_red[warp + w][piece * 9 + i];
+        out[i] = v;
       }
-  __syncthreads();
-  constexpr int WPQ = STRIPS / 32;   // warps per q
-  for (int i = tid; i < CPG * CPG * 9; i += THREADS) {
-    const int co = i / (CPG * 9), rest = i % (CPG * 9);
-    const int qq = co / COT, col = (co % COT) * CPG * 9 + rest;
-    float sum = 0.f;
-    for (int wq = 0; wq < WPQ; ++wq) sum += s_red[qq * WPQ + wq][col];
-    a.partial[((long long)pb * a.c + chan0 + co) * (CPG * 9) + rest] = sum;
+    }
   }
 }
 
@@ -284,12 +336,13 @@ bool group_small_supported(const ConvGeom& g) {
 }
 
 static void dw_tiling(const ConvGeom& g, int* tiles_y, int* tiles_x, int* tiles_per_block, int* blocks_per_group) {
-  const int tw = g.cig == 4 ? 16 : 8;   // one output channel per thread: 4 (8) threads share a strip, 64 (32) strips per tile
-  *tiles_y = (g.h + gcs::TH - 1) / gcs::TH;
-  *tiles_x = (g.w + tw - 1) / tw;
+  const int th = g.cig == 4 ? gcs::dw_rows<4> : gcs::dw_rows<8>;
+  *tiles_y = (g.h + th - 1) / th;
+  *tiles_x = (g.w + 31) / 32;
   const long long tiles_all = (long long)g.n * *tiles_y * *tiles_x;
-  // enough blocks for about six per SM, at least sixteen tiles per block (the block reduction costs about as much as two tiles)
-  long long bpg = std::max<long long>(1, std::min<long long>(tiles_all / 16, div_up64(6ll * sm_count(), g.groups)));
+  // three blocks per SM are resident (registers); at least four tiles per block, so that the pipeline and the block's reduction
+  // are a small part of it
+  const long long bpg = std::max<long long>(1, std::min<long long>(tiles_all / 4, 3ll * sm_count() / g.groups));
   *tiles_per_block = (int)div_up64(tiles_all, bpg);
   *blocks_per_group = (int)div_up64(tiles_all, *tiles_per_block);
 }
@@ -332,8 +385,8 @@ int group_small_dweight(const ConvGeom& g, View4 x, View4 dy, float* dw, float* 
     return fail(B200_EWORKSPACE, "grouped dWeight needs a workspace of %zu bytes (got %zu)", need, ws_bytes);
   a.partial = a.blocks_per_group > 1 ? ws : dw;   // one block per group writes dW directly ([cout][cig][9])
   const long long blocks = (long long)g.groups * a.blocks_per_group;
-  if (g.cig == 4) gcs::gconv_dw_kernel<4, 1><<<(unsigned)blocks, gcs::THREADS, 0, st>>>(a);
-  else gcs::gconv_dw_kernel<8, 1><<<(unsigned)blocks, gcs::THREADS, 0, st>>>(a);
+  if (g.cig == 4) gcs::gconv_dw_kernel<4><<<(unsigned)blocks, gcs::DW_THREADS, 0, st>>>(a);
+  else gcs::gconv_dw_kernel<8><<<(unsigned)blocks, gcs::DW_THREADS, 0, st>>>(a);
   count_launch();
   if (int rc = launch_check("gconv_dw_kernel")) return rc;
   if (a.blocks_per_group > 1) return finalize_splits(ws, dw, count, a.blocks_per_group, st);
