@@ -86,9 +86,11 @@ int simt_igemm_dinput(const ConvGeom& g, View4 dy, View4 w, float* dx, cudaStrea
 int simt_igemm_dweight(const ConvGeom& g, View4 x, View4 dy, float* dw, float* partial, int splits, int span,
                        cudaStream_t st);
 int finalize_splits(const float* partial, float* out, long long count, int splits, cudaStream_t st);
-int dbias_reduce(const ConvGeom& g, View4 dy, float* db, float* partial, int slabs, cudaStream_t st);
 int simt_gemm(long long M, long long N, long long K, const float* A, long long sa0, long long sa1, const float* B,
               long long sb0, long long sb1, const float* bias, float alpha, float beta, float* C, cudaStream_t st);
+
+// out[c] = sum of a [n][channels][h][w] view over everything but the channel, one launch (reduce.cu)
+int reduce_channels(View4 v, long long n, int channels, int h, int w, float* out, cudaStream_t st);
 
 // grouped 3x3 convolutions with 4 or 8 channels per group (conv_group_small.cu)
 bool group_small_supported(const ConvGeom& g);

@@ -48,18 +48,6 @@ static SplitPlan simt_dweight_plan(const ConvGeom& g, size_t budget) {
   return plan;
 }
 
-static int dbias_slabs(const ConvGeom& g, View4 dy, size_t budget) {
-  const bool channels_inner = dy.s1 == 1 && dy.s3 != 1;
-  const long long ctas = channels_inner ? div_up64(g.cout, 32) : g.cout;
-  long long slabs = div_up64(4ll * std::max(1, sm_count()), ctas);
-  // channels-last: a CTA pass covers 32 pixels, give every slab at least eight passes;
-  // planes: a warp takes an image, a CTA eight of them
-  const long long limit = channels_inner ? div_up64((long long)g.n * g.oh * g.ow, 256) : div_up64(g.n, 8);
-  slabs = std::max<long long>(1, std::min<long long>(slabs, limit));
-  slabs = std::min<long long>(slabs, (long long)(budget / (sizeof(float) * g.cout)));
-  return (int)std::max<long long>(1, slabs);
-}
-
 static int check_params(const b200_conv_params* p) {
   if (!p) return fail(B200_EINVAL, "null convolution parameters");
   if (!(p->n > 0 && p->cin > 0 && p->cout > 0 && p->h > 0 && p->w > 0 && p->kh > 0 && p->kw > 0 && p->oh > 0 &&
@@ -186,14 +174,7 @@ size_t b200_conv2d_workspace(const b200_conv_params* p, int phase, int algo, siz
   const ConvGeom g = to_geom(*p);
   const int chosen = select(g, phase, algo, budget_bytes);
   if (chosen < 0) return 0;
-  if (phase == B200_PHASE_DBIAS) {
-    const int slabs = dbias_slabs(g, contiguous_view(nullptr, g.cout, g.oh, g.ow), budget_bytes);
-    // channels-last gradients may want more slabs; reserve for the larger of the two layouts
-    View4 cl{nullptr, (long long)g.oh * g.ow * g.cout, 1, (long long)g.ow * g.cout, g.cout};
-    const int slabs_cl = dbias_slabs(g, cl, budget_bytes);
-    const int s = std::max(slabs, slabs_cl);
-    return s > 1 ? (size_t)s * g.cout * sizeof(float) : 0;
-  }
+  if (phase == B200_PHASE_DBIAS) return 0;
   if (chosen == B200_ALGO_TC) return tc_workspace(g, phase, budget_bytes, nullptr, nullptr);
   if (chosen == B200_ALGO_WINOGRAD) return winograd_workspace(g, phase, budget_bytes);
   if (chosen == B200_ALGO_TILED && phase == B200_PHASE_DWEIGHT) {
@@ -349,16 +330,14 @@ int b200_conv2d_dweight(const b200_conv_params* p, b200_view4 x, b200_view4 dy, 
   }
 }
 
-int b200_conv2d_dbias(const b200_conv_params* p, b200_view4 dy, float* db, void* workspace,
-                      size_t workspace_bytes, void* stream) {
+int b200_conv2d_dbias(const b200_conv_params* p, b200_view4 dy, float* db, void* /*workspace*/,
+                      size_t /*workspace_bytes*/, void* stream) {
   if (int rc = check_params(p)) return rc;
   if (int rc = ensure_init()) return rc;
   if (!dy.ptr || !db) return fail(B200_EINVAL, "convolution dBias: null tensor");
   const ConvGeom g = to_geom(*p);
-  if (!workspace) workspace_bytes = 0;
-  const int slabs = dbias_slabs(g, to_view(dy), workspace_bytes);
-  note_kernel(slabs > 1 ? "dbias_reduce+finalize" : "dbias_reduce");
-  return dbias_reduce(g, to_view(dy), db, (float*)workspace, slabs, (cudaStream_t)stream);
+  note_kernel("dbias_reduce");
+  return reduce_channels(to_view(dy), g.n, g.cout, g.oh, g.ow, db, (cudaStream_t)stream);
 }
 
 int b200_device_status(int* status, int clear) {
