@@ -174,7 +174,10 @@ size_t b200_conv2d_workspace(const b200_conv_params* p, int phase, int algo, siz
   const ConvGeom g = to_geom(*p);
   const int chosen = select(g, phase, algo, budget_bytes);
   if (chosen < 0) return 0;
-  if (phase == B200_PHASE_DBIAS) return 0;
+  if (phase == B200_PHASE_DBIAS) {
+    const size_t need = reduce_channels_workspace(g.n, g.cout, g.oh, g.ow);
+    return need <= budget_bytes ? need : 0;
+  }
   if (chosen == B200_ALGO_TC) return tc_workspace(g, phase, budget_bytes, nullptr, nullptr);
   if (chosen == B200_ALGO_WINOGRAD) return winograd_workspace(g, phase, budget_bytes);
   if (chosen == B200_ALGO_TILED && phase == B200_PHASE_DWEIGHT) {
@@ -330,14 +333,14 @@ int b200_conv2d_dweight(const b200_conv_params* p, b200_view4 x, b200_view4 dy, 
   }
 }
 
-int b200_conv2d_dbias(const b200_conv_params* p, b200_view4 dy, float* db, void* /*workspace*/,
-                      size_t /*workspace_bytes*/, void* stream) {
+int b200_conv2d_dbias(const b200_conv_params* p, b200_view4 dy, float* db, void* workspace,
+                      size_t workspace_bytes, void* stream) {
   if (int rc = check_params(p)) return rc;
   if (int rc = ensure_init()) return rc;
   if (!dy.ptr || !db) return fail(B200_EINVAL, "convolution dBias: null tensor");
   const ConvGeom g = to_geom(*p);
   note_kernel("dbias_reduce");
-  return reduce_channels(to_view(dy), g.n, g.cout, g.oh, g.ow, db, (cudaStream_t)stream);
+  return reduce_channels(to_view(dy), g.n, g.cout, g.oh, g.ow, db, (float*)workspace, workspace ? workspace_bytes : 0, (cudaStream_t)stream);
 }
 
 int b200_device_status(int* status, int clear) {

@@ -79,12 +79,14 @@ __global__ void __launch_bounds__(THREADS) reduce_planes_kernel(const float* __r
 }
 
 // out[c] = sum over rows of column c, columns adjacent in memory.  A CTA owns 4 * LPR columns (LPR lanes of 16 bytes per
-// row); blockIdx.x = column block, the cluster's ranks share the rows.
+// row); blockIdx.x = column block, the cluster's ranks share the rows; with gridDim.z > 1 clusters share them and write one
+// partial row each.
 template <int LPR, bool VEC, bool DENSE>
 __global__ void __launch_bounds__(COL_THREADS) reduce_columns_kernel(const float* __restrict__ src, Rows rows, uint32_t count, int cols,
                                                                  float* __restrict__ out, int accumulate) {
   cg::cluster_group cluster = cg::this_cluster();
-  const uint32_t ranks = cluster.num_blocks(), rank = cluster.block_rank();
+  const uint32_t cluster_ranks = cluster.num_blocks(), cluster_rank = cluster.block_rank();
+  const uint32_t ranks = cluster_ranks * gridDim.z, rank = blockIdx.z * cluster_ranks + cluster_rank;   // shares of the rows
   constexpr uint32_t ROWS = COL_THREADS / LPR;        // rows per CTA pass
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c0 = (int)blockIdx.x * 4 * LPR + (threadIdx.x % LPR) * 4;
@@ -127,22 +129,22 @@ __global__ void __launch_bounds__(COL_THREADS) reduce_columns_kernel(const float
     float v = 0.f;
 #pragma unroll
     for (int w = 0; w < COL_THREADS / 32; ++w) v += reinterpret_cast<const float*>(&warp_part[w][0])[threadIdx.x];
-    *cluster.map_shared_rank(&slab_part[rank][threadIdx.x], 0) = v;
+    *cluster.map_shared_rank(&slab_part[cluster_rank][threadIdx.x], 0) = v;
   }
   cluster.sync();
   const int c = (int)blockIdx.x * 4 * LPR + (int)threadIdx.x;
-  if (rank == 0 && threadIdx.x < 4 * LPR && c < cols) {
+  if (cluster_rank == 0 && threadIdx.x < 4 * LPR && c < cols) {
     float v = accumulate ? out[c] : 0.f;
-    for (uint32_t r = 0; r < ranks; ++r) v += slab_part[r][threadIdx.x];
-    out[c] = v;
+    for (uint32_t r = 0; r < cluster_ranks; ++r) v += slab_part[r][threadIdx.x];
+    out[(long long)blockIdx.z * cols + c] = v;
   }
 }
 
 template <int KERNEL_THREADS, typename... P, typename... A>
-static int launch_cluster(void (*kernel)(P...), unsigned blocks, int ranks, cudaStream_t st, A... args) {
+static int launch_cluster(void (*kernel)(P...), unsigned blocks, int ranks, int slabs, cudaStream_t st, A... args) {
   if (ranks > 8) B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(blocks, (unsigned)ranks); cfg.blockDim = dim3(KERNEL_THREADS); cfg.stream = st;
+  cfg.gridDim = dim3(blocks, (unsigned)ranks, (unsigned)slabs); cfg.blockDim = dim3(KERNEL_THREADS); cfg.stream = st;
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeClusterDimension;
   attr.val.clusterDim.x = 1; attr.val.clusterDim.y = (unsigned)ranks; attr.val.clusterDim.z = 1;
@@ -162,8 +164,17 @@ static int ranks_for(long long units_per_result, long long units_per_pass, long 
 
 }  // namespace red
 
+// Bytes of partial sums that reduce_channels can use for a channels-last view (few channels and many pixels: sixteen CTAs per
+// column block do not fill the machine, and a second small launch is then the cheaper way to add the clusters' sums).
+constexpr int MAX_SLABS = 8;
+constexpr long long SLAB_MIN_VALUES = 4ll << 20;   // below 16 MB one cluster per column block is as fast as two launches
+size_t reduce_channels_workspace(long long n, int channels, int h, int w) {
+  return (long long)n * h * w * channels >= SLAB_MIN_VALUES && div_up64(channels, 16) * red::MAX_CLUSTER < 2ll * sm_count()
+             ? (size_t)MAX_SLABS * channels * sizeof(float) : 0;
+}
+
 // Sums a [n][channels][h][w] view over everything but the channel.
-int reduce_channels(View4 v, long long n, int channels, int h, int w, float* out, cudaStream_t st) {
+int reduce_channels(View4 v, long long n, int channels, int h, int w, float* out, float* partial, size_t partial_bytes, cudaStream_t st) {
   using namespace red;
   const long long plane = (long long)h * w;
   const long long images_per_call = std::max<long long>(1, (1ll << 30) / plane);
@@ -188,11 +199,16 @@ int reduce_channels(View4 v, long long n, int channels, int h, int w, float* out
       const int lpr = wide ? 8 : 4;
       const unsigned blocks = (unsigned)div_up64(channels, 4 * lpr);
       const int ranks = ranks_for(count, COL_THREADS / lpr, blocks, MAX_CLUSTER);
-      auto go = [&](auto kernel) { return launch_cluster<COL_THREADS>(kernel, blocks, ranks, st, src, r, count, channels, out, acc); };
+      int slabs = 1;
+      if (partial && n <= images_per_call && reduce_channels_workspace(n, channels, h, w) > 0)
+        while (slabs < MAX_SLABS && blocks * (unsigned)(ranks * slabs) < 2u * (unsigned)sm_count() && 2 * slabs * sizeof(float) * channels <= partial_bytes) slabs *= 2;
+      float* dst = slabs > 1 ? partial : out;
+      auto go = [&](auto kernel) { return launch_cluster<COL_THREADS>(kernel, blocks, ranks, slabs, st, src, r, count, channels, dst, acc); };
       rc = wide ? (vec ? (dense ? go(reduce_columns_kernel<8, true, true>) : go(reduce_columns_kernel<8, true, false>))
                        : (dense ? go(reduce_columns_kernel<8, false, true>) : go(reduce_columns_kernel<8, false, false>)))
                 : (vec ? (dense ? go(reduce_columns_kernel<4, true, true>) : go(reduce_columns_kernel<4, true, false>))
                        : (dense ? go(reduce_columns_kernel<4, false, true>) : go(reduce_columns_kernel<4, false, false>)));
+      if (!rc && slabs > 1) rc = finalize_splits(partial, out, channels, slabs, st);
     } else {
       const bool vec = dense && v.s3 == 1 && aligned && plane % 4 == 0 && v.s0 % 4 == 0 && v.s1 % 4 == 0;
       uint32_t units = count;
@@ -201,7 +217,7 @@ int reduce_channels(View4 v, long long n, int channels, int h, int w, float* out
         units = count / 4;
       }
       const int ranks = ranks_for(units, THREADS, channels, 8);
-      auto go = [&](auto kernel) { return launch_cluster<THREADS>(kernel, (unsigned)channels, ranks, st, src, v.s1, r, units, out, acc); };
+      auto go = [&](auto kernel) { return launch_cluster<THREADS>(kernel, (unsigned)channels, ranks, 1, st, src, v.s1, r, units, out, acc); };
       rc = vec ? go(reduce_planes_kernel<true, true>) : dense ? go(reduce_planes_kernel<false, true>) : go(reduce_planes_kernel<false, false>);
     }
     if (rc) return rc;

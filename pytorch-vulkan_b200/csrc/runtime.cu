@@ -456,7 +456,7 @@ extern "C" int b200_sum_strided(float* dst, const float* src, int ndim, const in
   // own for 4 bytes of it (4096 x 2048: 120 us, 5.9 us this way).
   if (d.kept_dims == 1 && d.reduced_dims == 1 && d.kept_stride[0] == 1 && d.red_stride[0] != 1 && outputs < (1ll << 31) && d.red_total > 0 &&
       d.red_total < (1ll << 30))
-    return reduce_channels(View4{src, 0, 1, 0, d.red_stride[0]}, 1, (int)outputs, 1, (int)d.red_total, dst, (cudaStream_t)stream);
+    return reduce_channels(View4{src, 0, 1, 0, d.red_stride[0]}, 1, (int)outputs, 1, (int)d.red_total, dst, nullptr, 0, (cudaStream_t)stream);
   if (outputs > 8ll * 2147483647ll) return fail(B200_ERANGE, "strided sum: too many results");
   sum_strided_kernel<<<(unsigned)((outputs + 7) / 8), 256, 0, (cudaStream_t)stream>>>(dst, src, d, outputs);
   count_launch();

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 # (n, c, h, w): one value, scalar tails, one thread's batch, one pass of a cluster, whole planes off the vector width
 SHAPES = [(1, 1, 1, 1), (2, 3, 5, 7), (64, 512, 7, 7), (3, 5, 32, 32), (8, 64, 56, 56), (5, 33, 13, 16), (1, 2, 300, 301), (2, 1040, 4, 4),
-          (70, 4, 17, 9)]
+          (70, 4, 17, 9), (32, 20, 96, 96)]
 
 
 @pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "x".join(map(str, s)))
