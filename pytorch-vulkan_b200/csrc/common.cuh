@@ -89,8 +89,9 @@ int finalize_splits(const float* partial, float* out, long long count, int split
 int simt_gemm(long long M, long long N, long long K, const float* A, long long sa0, long long sa1, const float* B,
               long long sb0, long long sb1, const float* bias, float alpha, float beta, float* C, cudaStream_t st);
 
-// out[c] = sum of a [n][channels][h][w] view over everything but the channel, one launch (reduce.cu)
-int reduce_channels(View4 v, long long n, int channels, int h, int w, float* out, cudaStream_t st);
+// out[c] = sum of a [n][channels][h][w] view over everything but the channel (reduce.cu)
+int reduce_channels(View4 v, long long n, int channels, int h, int w, float* out, float* partial, size_t partial_bytes, cudaStream_t st);
+size_t reduce_channels_workspace(long long n, int channels, int h, int w);  // optional `partial` of reduce_channels
 
 // grouped 3x3 convolutions with 4 or 8 channels per group (conv_group_small.cu)
 bool group_small_supported(const ConvGeom& g);
@@ -140,6 +141,9 @@ bool tstrip_supported(const ConvGeom& g, int phase);
 size_t tstrip_workspace(const ConvGeom& g, int phase);
 int tstrip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* bias, long long bias_stride, float* out,
                 void* ws, size_t ws_bytes, cudaStream_t st);
+// row kernel (conv_tc_rows.cu): forward passes of layers with fewer than 16 input channels, no workspace
+bool rows_supported(const ConvGeom& g);
+int rows_conv(const ConvGeom& g, View4 x, View4 w, const float* bias, long long bias_stride, float* y, cudaStream_t st);
 int strip_column_tile(const ConvGeom& g, bool is_dx);   // column tile the plan picks, 0 if unsupported
 size_t strip_workspace(const ConvGeom& g, int phase);  // bytes of the weight stage images
 

@@ -577,7 +577,7 @@ static bool strip_allowed() {
 bool tc_supported(const ConvGeom& g, int phase) {
   // the gather kernels need the reduction channels in blocks of 32; the strip kernel pads a ragged block
   const bool strip = (phase == B200_PHASE_FORWARD || phase == B200_PHASE_DINPUT) && strip_allowed() && strip_supported(g, phase);
-  if (phase == B200_PHASE_FORWARD) return g.cog >= 16 && (g.cig % KBLK == 0 || strip);
+  if (phase == B200_PHASE_FORWARD) return g.cog >= 16 && (g.cig % KBLK == 0 || strip || rows_supported(g));
   if (phase == B200_PHASE_DINPUT) return g.cig >= 16 && (g.cog % KBLK == 0 || strip);
   if (phase == B200_PHASE_DWEIGHT) return g.cog >= 16 && g.cig * g.kh * g.kw >= 32;
   return false;
@@ -608,6 +608,7 @@ size_t tc_workspace(const ConvGeom& g, int phase, size_t budget, int* splits_out
   (void)budget;
   if (splits_out) *splits_out = 1;
   if (span_out) *span_out = 0;
+  if (phase == B200_PHASE_FORWARD && rows_supported(g)) return 0;   // the filter is split inside the kernel
   if (phase == B200_PHASE_FORWARD || phase == B200_PHASE_DINPUT) {
     const size_t planes = 2 * sizeof(float) * (size_t)g.cout * g.cig * g.kh * g.kw;  // hi + lo
     size_t need = strip_allowed() && strip_supported(g, phase) ? std::max(planes, strip_workspace(g, phase)) : planes;
@@ -721,6 +722,11 @@ int tc_route(const ConvGeom& g, bool is_dx, const View4& act) {
 
 int tc_forward(const ConvGeom& g, View4 x, View4 w, const float* bias, long long bias_stride, float* y, void* ws,
                size_t ws_bytes, cudaStream_t st) {
+  if (rows_supported(g)) {
+    note_kernel("tc_rows_forward");
+    const int rc = rows_conv(g, x, w, bias, bias_stride, y, st);
+    if (rc != B200_EUNSUPPORTED) return rc;   // falls through to the CUDA-core kernel
+  }
   int route = tc_route(g, false, x);
   if (route == 3) {
     note_kernel("tc_tstrip_forward");
