@@ -1,0 +1,15 @@
+// The pass behind both tcgen05 dWeight kernels, and the entry points of the tensor-memory one (dweight_tc_tmem.cu).
+#pragma once
+#include "common.cuh"
+
+namespace b200 {
+namespace tcdw {
+// dW = sum of `splits` partials [split][cout][kh*kw][cig] (dweight_tc_strip.cu)
+int finalize_partials(const float* partial, float* dw, const ConvGeom& g, int splits, cudaStream_t st);
+}  // namespace tcdw
+namespace tcdt {
+// Split count and scratch of the tensor-memory kernel for this budget; false where it does not take the geometry.
+bool plan_bytes(const ConvGeom& g, size_t budget, size_t* bytes);
+int run(const ConvGeom& g, View4 x, View4 dy, float* dw, void* ws, size_t ws_bytes, cudaStream_t st);
+}  // namespace tcdt
+}  // namespace b200

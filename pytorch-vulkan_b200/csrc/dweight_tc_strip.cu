@@ -1,5 +1,6 @@
 // tcgen05 dWeight kernel for filters up to eight taps wide (any stride, padding, dilation, groups;
-// at least 16 channels on both sides), FP32 via 3xTF32.
+// at least 16 channels on both sides), FP32 via 3xTF32, with both operands in shared memory: 1x1 filters, and what the
+// tensor-memory kernel (dweight_tc_tmem.cu), which is tried first, does not take.
 //
 //   dW[co][ci][ky][kx] = sum over grid pixels q of  dY[q][co] * X_phase(ky,kx)[q + shift(ky,kx)][ci]
 //
@@ -25,12 +26,15 @@
 // Replaces csrc/shaders/conv2d_backward_weight_tiled_body.glsl:42-70 and
 // conv2d_backward_weight_finalize.comp:9-18 of the reference for these geometries.
 #include "common.cuh"
+#include "dweight_plan.cuh"
+#include "dweight_stage.cuh"
 #include "tc_common.cuh"
 
 #include <algorithm>
 #include <mutex>
 #include <cstdio>
 #include <cstdlib>
+#include <cstring>
 
 namespace b200 {
 namespace tcdw {
@@ -101,157 +105,6 @@ struct Ctrl {
   uint32_t tmem_base;
   int abort_flag;
 };
-
-// byte offset of channel e (0..31) of row `row` in a plane using the 128B swizzle with 32-byte base
-__device__ __forceinline__ uint32_t sw32b_offset(int row, int e) {
-  return (uint32_t)(row * 128 + ((((e >> 3) ^ (row & 3)) << 5) | ((e & 7) << 2)));
-}
-// MN-major operand descriptor: blocks of 32 channels `lbo` bytes apart, 4-row groups 512 bytes apart
-__device__ __forceinline__ uint64_t make_mn_desc(uint32_t addr, uint32_t lbo) {
-  uint64_t d = 0;
-  d |= (uint64_t)((addr & 0x3FFFFu) >> 4);
-  d |= (uint64_t)(lbo >> 4) << 16;
-  d |= (uint64_t)(512u >> 4) << 32;
-  d |= (uint64_t)1 << 46;   // descriptor version of sm_100
-  d |= (uint64_t)1 << 61;   // SWIZZLE_128B with 32-byte base
-  return d;
-}
-
-// byte offset of channel e (0..31) of row `row` in a bf16 plane of 64-byte rows, SWIZZLE_64B
-__device__ __forceinline__ uint32_t sw64_offset(int row, int e) {
-  return (uint32_t)(row * 64 + ((((e >> 3) ^ ((row >> 1) & 3)) << 4) | ((e & 7) << 1)));
-}
-// MN-major descriptor of a bf16 plane (64-byte rows): blocks of 32 channels `lbo` bytes apart, 8-row
-// groups 512 bytes apart, SWIZZLE_64B
-__device__ __forceinline__ uint64_t make_mn_desc16(uint32_t addr, uint32_t lbo) {
-  uint64_t d = 0;
-  d |= (uint64_t)((addr & 0x3FFFFu) >> 4);
-  d |= (uint64_t)(lbo >> 4) << 16;
-  d |= (uint64_t)(512u >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)4 << 61;   // SWIZZLE_64B
-  return d;
-}
-
-// One warp stages `rows` (<= 32, lane = row) x 32 channels of a pixel-major block: gather from
-// the strided view, split into TF32 hi/lo, swizzled stores.  `q_first` is the padded pixel of row 0;
-// rows outside [q_lo, q_hi) or on padding are written as zeros.
-//
-// With the 32-byte-base swizzle rows r and r+4 put the same 16-byte chunk into the same banks, so
-// lanes 4-7 of every group of eight write the two chunks of a 32-byte pair in the opposite order
-// (every 8-lane store wavefront is then conflict-free).  To keep that free of per-value selects the
-// swapped lanes already LOAD their channels in swapped order: val[j] holds channel j ^ 4 there.
-__device__ __forceinline__ bool stage_block(const View4& v, long long chan0, int chans, int H, int W, int row_pitch,
-                                            int img_pitch, const FastDiv& img_div, const FastDiv& row_div, int q_first,
-                                            int q_lo, int q_hi, int rows, int lane, bool vec_ok, float (&val)[32],
-                                            int sph = 1, int spw = 1, int pa = 0, int pb = 0, int lim_h = 1 << 30,
-                                            int lim_w = 1 << 30) {
-  const int q = q_first + lane;
-  bool ok = lane < rows && q >= q_lo && q < q_hi;
-  const float* src = v.ptr;
-  if (ok) {
-    const int n = (int)img_div.div((uint32_t)q);
-    const int rem = q - n * img_pitch;
-    const int y = (int)row_div.div((uint32_t)rem), x = rem - y * row_pitch;
-    const int ty = y * sph + pa, tx = x * spw + pb;  // position in the tensor
-    ok = y < H && x < W && ty < lim_h && tx < lim_w;
-    src += n * v.s0 + chan0 * v.s1 + (long long)ty * v.s2 + (long long)tx * v.s3;
-  }
-  const int sw = (lane >> 2) & 1;
-  if (vec_ok && chans == 32) {
-    // Channels-last: eight lanes fetch the 128 contiguous bytes of one pixel, four pixels per load
-    // instruction; lane r computed the address of row r above and hands it to the lanes that fetch
-    // it.  val[4i..4i+3] is then the 16-byte chunk (lane & 7) of row 4i + (lane >> 3): see
-    // store_block_chunks.
-    const unsigned long long mine = ok ? reinterpret_cast<unsigned long long>(src) : 0ull;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float4* ps = reinterpret_cast<const float4*>(__shfl_sync(0xffffffffu, mine, 4 * i + (lane >> 3)));
-      const float4 f = ps ? __ldg(ps + (lane & 7)) : make_float4(0.f, 0.f, 0.f, 0.f);
-      val[4 * i] = f.x; val[4 * i + 1] = f.y; val[4 * i + 2] = f.z; val[4 * i + 3] = f.w;
-    }
-    return true;
-  } else if (chans == 32) {
-    // lane = pixel, one coalesced load per channel; 32-bit element offsets (the host checks that the
-    // tensor is addressable with them) keep this at two instructions per value
-    const int s1 = (int)v.s1;
-    const float* pa = src + 4 * sw * s1;  // for j with bit 2 clear
-    const float* pb = src - 4 * sw * s1;  // for j with bit 2 set
-    if (__all_sync(0xffffffffu, ok)) {  // the common case away from padding: no predication
-#pragma unroll
-      for (int j = 0; j < 32; ++j) val[j] = __ldg(((j & 4) ? pb : pa) + j * s1);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 32; ++j) val[j] = ok ? __ldg(((j & 4) ? pb : pa) + j * s1) : 0.f;
-    }
-  } else {
-    const int s1 = (int)v.s1;
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const int c = j ^ (sw << 2);
-      val[j] = (ok && c < chans) ? __ldg(src + c * s1) : 0.f;
-    }
-  }
-  return false;
-}
-// Where one staged block lives: the TF32 hi plane (128-byte rows) and either the FP32 lo plane or,
-// with BF16 cross terms, the two bf16 planes (64-byte rows) of bf16(hi) and bf16(lo).
-struct BlockPlanes {
-  uint32_t hi, lo, h16, l16;
-};
-// Store for the channels-last load pattern: eight lanes write the eight 16-byte chunks of one row
-// (a whole row per quarter warp: conflict-free in any swizzle).
-template <bool DW_CROSS>
-__device__ __forceinline__ void store_block_chunks(const float (&val)[32], int rows, int row0, const BlockPlanes& pl, int lane) {
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int r = 4 * i + (lane >> 3);
-    if (r < rows) {
-      float h[4], l[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) split_tf32_fast(val[4 * i + j], h[j], l[j]);
-      const int c4 = (lane & 7) * 4;
-      sts_f32x4(pl.hi + sw32b_offset(row0 + r, c4), h[0], h[1], h[2], h[3]);
-      if (DW_CROSS) {
-        const uint32_t o = sw64_offset(row0 + r, c4);
-        sts_b32x2(pl.h16 + o, pack_bf16x2(h[0], h[1]), pack_bf16x2(h[2], h[3]));
-        sts_b32x2(pl.l16 + o, pack_bf16x2(l[0], l[1]), pack_bf16x2(l[2], l[3]));
-      } else {
-        sts_f32x4(pl.lo + sw32b_offset(row0 + r, c4), l[0], l[1], l[2], l[3]);
-      }
-    }
-  }
-}
-// Store for the lane = row pattern; val[j] holds channel j ^ 4 in lanes 4-7 of every eight (see stage_block).
-template <bool DW_CROSS>
-__device__ __forceinline__ void store_block(const float (&val)[32], int rows, int row0, const BlockPlanes& pl, int lane) {
-  if (lane >= rows) return;
-  const uint32_t sw = (uint32_t)((lane >> 2) & 1);
-#pragma unroll
-  for (int m = 0; m < 4; ++m) {
-    float h0[4], l0[4], h1[4], l1[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      split_tf32_fast(val[m * 8 + j], h0[j], l0[j]);
-      split_tf32_fast(val[m * 8 + 4 + j], h1[j], l1[j]);
-    }
-    const uint32_t oa = sw32b_offset(row0 + lane, m * 8) ^ (sw << 4), ob = oa ^ 16u;
-    sts_f32x4(pl.hi + oa, h0[0], h0[1], h0[2], h0[3]);
-    sts_f32x4(pl.hi + ob, h1[0], h1[1], h1[2], h1[3]);
-    if (DW_CROSS) {
-      // the eight channels of this group are one 16-byte chunk of a bf16 row; its two 8-byte halves
-      // go where this lane's channel order puts them (64-byte rows need no bank-conflict swap)
-      const uint32_t qa = sw64_offset(row0 + lane, m * 8) ^ (sw << 3), qb = qa ^ 8u;
-      sts_b32x2(pl.h16 + qa, pack_bf16x2(h0[0], h0[1]), pack_bf16x2(h0[2], h0[3]));
-      sts_b32x2(pl.h16 + qb, pack_bf16x2(h1[0], h1[1]), pack_bf16x2(h1[2], h1[3]));
-      sts_b32x2(pl.l16 + qa, pack_bf16x2(l0[0], l0[1]), pack_bf16x2(l0[2], l0[3]));
-      sts_b32x2(pl.l16 + qb, pack_bf16x2(l1[0], l1[1]), pack_bf16x2(l1[2], l1[3]));
-    } else {
-      sts_f32x4(pl.lo + oa, l0[0], l0[1], l0[2], l0[3]);
-      sts_f32x4(pl.lo + ob, l1[0], l1[1], l1[2], l1[3]);
-    }
-  }
-}
 
 struct FoldArgs {
   float* out;            // this thread's first output element
@@ -662,6 +515,35 @@ __global__ void __launch_bounds__(256) finalize_partials_kernel(const float* __r
   }
 }
 
+int finalize_partials(const float* partial, float* dw, const ConvGeom& g, int splits, cudaStream_t st) {
+  const long long count = (long long)g.cout * g.cig * g.kh * g.kw;
+  cudaLaunchConfig_t cfg{};
+  const int taps = g.kh * g.kw;
+  const bool vec = g.cig % 4 == 0;
+  // channels per block: all of them if they fit the default shared memory, fewer while the blocks do not fill the SMs
+  // twice (down to 16: shorter runs waste the sectors at their ends); a single channel needs no shared memory
+  int ch_log2 = 0;
+  while (ch_log2 < 9 && (1 << ch_log2) < g.cig && ((size_t)taps << (ch_log2 + 1)) * sizeof(float) <= FIN_SMEM) ++ch_log2;
+  while (ch_log2 > 4 && (long long)g.cout * ((g.cig + (1 << ch_log2) - 1) >> ch_log2) < 2ll * sm_count()) --ch_log2;
+  const bool v4 = vec && ch_log2 >= 2;
+  const int chunks = (g.cig + (1 << ch_log2) - 1) >> ch_log2, units = (taps << ch_log2) / (v4 ? 4 : 1);
+  const long long blocks = (long long)g.cout * chunks;
+  const size_t values = ((size_t)taps << ch_log2) * sizeof(float);
+  int slices = 1;
+  while (ch_log2 > 0 && slices * 2 <= splits && units * slices < 256 && 2 * slices * values <= FIN_SMEM) slices *= 2;
+  if (blocks > 2147483647ll) return fail(B200_ERANGE, "dWeight finalize: grid exceeds launch limits");
+  cfg.gridDim = dim3((unsigned)blocks); cfg.blockDim = dim3(256); cfg.stream = st;
+  cfg.dynamicSmemBytes = ch_log2 > 0 ? slices * values : 0;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  if (!getenv("B200_DW_NO_PDL")) { cfg.attrs = &attr; cfg.numAttrs = 1; }
+  B200_CUDA(cudaLaunchKernelEx(&cfg, v4 ? finalize_partials_kernel<4> : finalize_partials_kernel<1>, partial, dw, count, splits,
+                               g.cig, taps, slices, ch_log2, FastDiv((uint32_t)chunks), FastDiv((uint32_t)units)));
+  count_launch();
+  return launch_check("finalize_partials_kernel");
+}
+
 struct DwStripPlan {
   bool ok = false;
   bool cross = false;  // BF16 cross terms (four accumulators)
@@ -761,7 +643,15 @@ static DwStripPlan plan_dw_strip(const ConvGeom& g, size_t budget) {
 }  // namespace tcdw
 
 bool dweight_strip_supported(const ConvGeom& g) { return tcdw::plan_dw_strip(g, 0).ok; }
-size_t dweight_strip_workspace(const ConvGeom& g, size_t budget) { return tcdw::plan_dw_strip(g, budget).bytes; }
+static bool tmem_allowed() {
+  const char* e = getenv("B200_DW_VARIANT");   // "strip" pins the kernel with both operands in shared memory (testing aid)
+  return !(e && !strcmp(e, "strip"));
+}
+size_t dweight_strip_workspace(const ConvGeom& g, size_t budget) {
+  size_t bytes = 0;
+  if (tmem_allowed() && tcdt::plan_bytes(g, budget, &bytes)) return bytes;
+  return tcdw::plan_dw_strip(g, budget).bytes;
+}
 
 template <int BN, bool CROSS>
 static int launch_dw_strip(const tcdw::DwStripArgs& a, dim3 grid, int smem, cudaStream_t st) {
@@ -785,6 +675,10 @@ int dweight_strip(const ConvGeom& g, View4 x, View4 dy, float* dw, void* ws, siz
   };
   if (span(x, g.n, g.cin, g.h, g.w) > 2147483647ll - 64 * std::llabs(x.s1) || span(dy, g.n, g.cout, g.oh, g.ow) > 2147483647ll - 64 * std::llabs(dy.s1))
     return fail(B200_EUNSUPPORTED, "dWeight strip kernel: tensor too large for 32-bit element offsets");
+  if (tmem_allowed()) {
+    const int rc = tcdt::run(g, x, dy, dw, ws, ws_bytes, st);
+    if (rc != B200_EUNSUPPORTED) return rc;
+  }
   DwStripArgs a{};
   a.g = g; a.x = x; a.dy = dy;
   a.H = plan.gh; a.W = plan.gw; a.pr = plan.pr; a.pc = plan.pc;
@@ -837,34 +731,7 @@ int dweight_strip(const ConvGeom& g, View4 x, View4 dy, float* dw, void* ws, siz
             "warp 0: jobs %llu load %llu wait_empty %llu store %llu | folds: %llu, cycles in them %llu (of which waiting for the accumulator %llu) | ns: last CTA start %llu, first start to last end %llu, CTA lifetime min %llu max %llu\n",
             plan.bn, plan.xblocks, plan.stages, gx, plan.splits, plan.span / KP, h[0], h[1], h[5], h[2], h[3], h[4], h[8], h[7], h[6], h[12] - h[11], h[13] - h[11], h[14], h[15]);
   }
-  if (plan.splits > 1) {
-    const long long count = (long long)g.cout * g.cig * g.kh * g.kw;
-    cudaLaunchConfig_t cfg{};
-    const int taps = g.kh * g.kw;
-    const bool vec = g.cig % 4 == 0;
-    // channels per block: all of them if they fit the default shared memory, fewer while the blocks do not fill the SMs
-    // twice (down to 16: shorter runs waste the sectors at their ends); a single channel needs no shared memory
-    int ch_log2 = 0;
-    while (ch_log2 < 9 && (1 << ch_log2) < g.cig && ((size_t)taps << (ch_log2 + 1)) * sizeof(float) <= FIN_SMEM) ++ch_log2;
-    while (ch_log2 > 4 && (long long)g.cout * ((g.cig + (1 << ch_log2) - 1) >> ch_log2) < 2ll * sm_count()) --ch_log2;
-    const bool v4 = vec && ch_log2 >= 2;
-    const int chunks = (g.cig + (1 << ch_log2) - 1) >> ch_log2, units = (taps << ch_log2) / (v4 ? 4 : 1);
-    const long long blocks = (long long)g.cout * chunks;
-    const size_t values = ((size_t)taps << ch_log2) * sizeof(float);
-    int slices = 1;
-    while (ch_log2 > 0 && slices * 2 <= plan.splits && units * slices < 256 && 2 * slices * values <= FIN_SMEM) slices *= 2;
-    if (blocks > 2147483647ll) return fail(B200_ERANGE, "dWeight finalize: grid exceeds launch limits");
-    cfg.gridDim = dim3((unsigned)blocks); cfg.blockDim = dim3(256); cfg.stream = st;
-    cfg.dynamicSmemBytes = ch_log2 > 0 ? slices * values : 0;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    if (!getenv("B200_DW_NO_PDL")) { cfg.attrs = &attr; cfg.numAttrs = 1; }
-    B200_CUDA(cudaLaunchKernelEx(&cfg, v4 ? finalize_partials_kernel<4> : finalize_partials_kernel<1>, (const float*)ws, dw, count, plan.splits,
-                                 g.cig, taps, slices, ch_log2, FastDiv((uint32_t)chunks), FastDiv((uint32_t)units)));
-    count_launch();
-    return launch_check("finalize_partials_kernel");
-  }
+  if (plan.splits > 1) return tcdw::finalize_partials((const float*)ws, dw, g, plan.splits, st);
   return B200_OK;
 }
 
