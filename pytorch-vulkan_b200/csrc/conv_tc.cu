@@ -579,7 +579,7 @@ bool tc_supported(const ConvGeom& g, int phase) {
   const bool strip = (phase == B200_PHASE_FORWARD || phase == B200_PHASE_DINPUT) && strip_allowed() && strip_supported(g, phase);
   if (phase == B200_PHASE_FORWARD) return g.cog >= 16 && (g.cig % KBLK == 0 || strip || rows_supported(g));
   if (phase == B200_PHASE_DINPUT) return g.cig >= 16 && (g.cog % KBLK == 0 || strip);
-  if (phase == B200_PHASE_DWEIGHT) return g.cog >= 16 && g.cig * g.kh * g.kw >= 32;
+  if (phase == B200_PHASE_DWEIGHT) return g.cog >= 16 && (g.cig * g.kh * g.kw >= 32 || (strip_allowed() && dweight_strip_supported(g)));
   return false;
 }
 
@@ -789,6 +789,10 @@ int tc_dweight(const ConvGeom& g, View4 x, View4 dy, float* dw, void* ws, size_t
     note_kernel("tc_strip_dweight");
     const int rc = dweight_strip(g, x, dy, dw, ws, ws_bytes, st);
     if (rc != B200_EUNSUPPORTED) return rc;  // tensors beyond 32-bit element offsets take the gather kernel
+    if (g.cig * g.kh * g.kw < 32) {        // too few rows for the gather kernel's tiles
+      note_kernel("simt_igemm_dweight");
+      return simt_igemm_dweight(g, x, dy, dw, nullptr, 1, 0, st);
+    }
     note_kernel("tc_igemm_dweight");
   }
   int splits, span;

@@ -642,10 +642,13 @@ static DwStripPlan plan_dw_strip(const ConvGeom& g, size_t budget) {
 
 }  // namespace tcdw
 
-bool dweight_strip_supported(const ConvGeom& g) { return tcdw::plan_dw_strip(g, 0).ok; }
 static bool tmem_allowed() {
   const char* e = getenv("B200_DW_VARIANT");   // "strip" pins the kernel with both operands in shared memory (testing aid)
   return !(e && !strcmp(e, "strip"));
+}
+bool dweight_strip_supported(const ConvGeom& g) {
+  size_t bytes;
+  return tcdw::plan_dw_strip(g, 0).ok || (tmem_allowed() && tcdt::plan_bytes(g, 0, &bytes));
 }
 size_t dweight_strip_workspace(const ConvGeom& g, size_t budget) {
   size_t bytes = 0;
@@ -667,6 +670,10 @@ static int launch_dw_strip(const tcdw::DwStripArgs& a, dim3 grid, int smem, cuda
 
 int dweight_strip(const ConvGeom& g, View4 x, View4 dy, float* dw, void* ws, size_t ws_bytes, cudaStream_t st) {
   using namespace tcdw;
+  if (tmem_allowed()) {
+    const int rc = tcdt::run(g, x, dy, dw, ws, ws_bytes, st);
+    if (rc != B200_EUNSUPPORTED) return rc;
+  }
   const DwStripPlan plan = plan_dw_strip(g, ws ? ws_bytes : 0);
   if (!plan.ok) return fail(B200_EUNSUPPORTED, "dWeight strip kernel does not take this geometry");
   // the kernel forms element offsets inside a tensor in 32 bits
@@ -675,10 +682,6 @@ int dweight_strip(const ConvGeom& g, View4 x, View4 dy, float* dw, void* ws, siz
   };
   if (span(x, g.n, g.cin, g.h, g.w) > 2147483647ll - 64 * std::llabs(x.s1) || span(dy, g.n, g.cout, g.oh, g.ow) > 2147483647ll - 64 * std::llabs(dy.s1))
     return fail(B200_EUNSUPPORTED, "dWeight strip kernel: tensor too large for 32-bit element offsets");
-  if (tmem_allowed()) {
-    const int rc = tcdt::run(g, x, dy, dw, ws, ws_bytes, st);
-    if (rc != B200_EUNSUPPORTED) return rc;
-  }
   DwStripArgs a{};
   a.g = g; a.x = x; a.dy = dy;
   a.H = plan.gh; a.W = plan.gw; a.pr = plan.pr; a.pc = plan.pc;

@@ -20,6 +20,10 @@
 // a descriptor (32 rows and up to eight rows of horizontal taps) never has to wrap.  Images too wide for that take one ky per
 // CTA.
 //
+// FOLD (fewer than sixteen input channels: a network's first layer): the (input channel, ky) pairs of a pixel take the place of the
+// channels of a strip, 21 of 32 for 3 channels and a 7x7 filter, and the taps kx stay row offsets.  dW is then that of a
+// one-row filter over cin * kh channels, whose layout it already has.
+//
 // The pixel grid, the split of the contraction over CTAs, the chunked accumulation (the tensor core truncates: CHUNK_KB) and
 // the partial layout [split][cout][kh*kw][cin/g] are those of dweight_tc_strip.cu.
 //
@@ -88,7 +92,12 @@ struct Args {
   Strip strips[MAX_STRIPS];
   Group groups[MAX_GROUPS];
   Slot slots[MAX_SLOTS];
+  int fold_kh, fold_sh, fold_dh, fold_ph, fold_h;   // FOLD: the real filter height and what places its rows (g describes the folded layer)
   int* status;
+};
+
+struct FoldEntry {
+  int offset, ky;            // elements from the window's first row; filter row
 };
 
 struct Ctrl {
@@ -111,7 +120,7 @@ __device__ __forceinline__ uint64_t desc64(uint32_t lo, uint32_t hi) {
 
 // NG groups of NB N-blocks each where the plan has that shape (0: as the arguments say): with the loop bounds and the step width
 // known, the issuing warp needs 175 clocks less per K block of a 3x3 filter.
-template <int NG, int NB>
+template <int NG, int NB, bool FOLD>
 __global__ void __launch_bounds__(THREADS, 1) dweight_tmem_kernel(const Args a) {
   constexpr int GROUPS = NG ? NG : MAX_GROUPS;
   extern __shared__ unsigned char smem_raw[];
@@ -123,6 +132,7 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_tmem_kernel(const Args a) 
   unsigned char* scratch_all = smem_raw + (base - raw) + a.n_strips * strip_bytes;
   const int dy_warps = 4 * a.dy_sets;
   Ctrl* ctrl = reinterpret_cast<Ctrl*>(scratch_all + dy_warps * SCRATCH);
+  FoldEntry* fold_tab = reinterpret_cast<FoldEntry*>(ctrl + 1);   // [cig]
   volatile int* abort_flag = &ctrl->abort_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -140,6 +150,11 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_tmem_kernel(const Args a) 
     ctrl->abort_flag = 0;
     fence_barrier_init();
   }
+  if (FOLD)
+    for (int c = threadIdx.x; c < g.cig; c += THREADS) {
+      const int ci = c / a.fold_kh, ky = c - ci * a.fold_kh;
+      fold_tab[c] = FoldEntry{(int)(ci * a.x.s1 + (long long)(ky * a.fold_dh) * a.x.s2), ky};
+    }
   if (warp == MMA_WARP) tmem_alloc(smem_u32(&ctrl->tmem_base), 512);
   tc_fence_before();
   __syncthreads();
@@ -251,6 +266,27 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_tmem_kernel(const Args a) 
       const int c = (int)a.div_strips.div((uint32_t)job), strip = job - c * a.n_strips;
       const Strip st = a.strips[strip];
       const int c0 = ci0 + st.cblk * 32;
+      if (FOLD) {
+        const int q = k_begin + c * KP + st.dc + lane;
+        uint32_t rows = 0;                         // filter rows of this pixel that lie inside the image
+        const float* p = a.x.ptr;
+        if (q >= 0 && q < a.q_total) {
+          const int n = (int)a.img_div.div((uint32_t)q), rem = q - n * img_pitch;
+          const int y = (int)a.row_div.div((uint32_t)rem), x = rem - y * row_pitch, iy = y * a.fold_sh - a.fold_ph, ix = x * a.spw + st.pb;
+          if (x < a.W && ix < a.in_w) {
+            for (int k = 0; k < a.fold_kh; ++k) rows |= (uint32_t)(iy + k * a.fold_dh >= 0 && iy + k * a.fold_dh < a.fold_h) << k;
+            p += n * a.x.s0 + (long long)iy * a.x.s2 + (long long)ix * a.x.s3;
+          }
+        }
+        const int sw = ((lane >> 2) & 1) << 2;     // store_block's register order
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          const int ch = c0 + (i ^ sw);
+          const FoldEntry e = fold_tab[min(ch, g.cig - 1)];
+          val[i] = ch < g.cig && ((rows >> e.ky) & 1u) ? __ldg(p + e.offset) : 0.f;
+        }
+        return false;
+      }
       return tcdw::stage_block(a.x, (long long)group * g.cig + c0, max(0, min(32, g.cig - c0)), a.H, a.W, row_pitch, img_pitch, a.img_div,
                                a.row_div, k_begin + c * KP + (ky0 >= 0 ? dr0 : st.dr) * row_pitch + st.dc, 0, a.q_total, 32, lane, vec, val,
                                a.sph, a.spw, ky0 >= 0 ? pa0 : st.pa, st.pb, a.in_h, a.in_w);
@@ -520,10 +556,18 @@ static void finish_groups(Args& a) {
   }
 }
 
-static Plan make_plan(const ConvGeom& g, size_t budget) {
+static Plan make_plan(const ConvGeom& real, size_t budget) {
   Plan best;
+  // fewer than sixteen input channels: fold the filter rows into the channels (see above)
+  ConvGeom g = real;
+  const bool fold = real.cig < 16;
+  if (fold) {
+    if (real.groups != 1 || real.kh > 31 || real.cig * real.kh > 256 || real.cig * real.kh * real.kw < 9) return best;
+    g.cin = g.cig = real.cig * real.kh;
+    g.kh = 1; g.ph = 0; g.dh = 1; g.sh = 1; g.h = g.oh;
+  }
   // 1x1 filters are bound by the staging of both operands, for which dweight_tc_strip.cu has more warps
-  if (g.kh * g.kw == 1 || g.kw > 8 || g.cog < 16 || g.cig < 16 || g.sh > 127 || g.sw > 127) return best;
+  if ((!fold && (g.kh * g.kw == 1 || g.cig < 16)) || g.kw > 8 || g.cog < 16 || g.sh > 127 || g.sw > 127) return best;
   const int gh = std::max(g.oh, (g.h + g.sh - 1) / g.sh), gw = std::max(g.ow, (g.w + g.sw - 1) / g.sw);
   int pr = 0, pc = 0;
   for (int ky = 0; ky < g.kh; ++ky) pr = std::max(pr, std::abs(floor_div(ky * g.dh - g.ph, g.sh)));
@@ -569,7 +613,7 @@ static Plan make_plan(const ConvGeom& g, size_t budget) {
       auto slower = [&](int sets) { return std::max(1.0 / sets, (double)a.n_strips / (MMA_WARP - 4 * sets)); };
       for (int sets = 2; sets <= std::min(3, a.a_stages); ++sets)
         if (slower(sets) < slower(a.dy_sets)) a.dy_sets = sets;
-      const int fixed_smem = 4 * a.dy_sets * SCRATCH + (int)sizeof(Ctrl) + 1024 + 64;
+      const int fixed_smem = 4 * a.dy_sets * SCRATCH + (int)sizeof(Ctrl) + (fold ? g.cig * (int)sizeof(FoldEntry) : 0) + 1024 + 64;
       a.ring = std::min({MAX_RING, a.ahead + 6, (SMEM_LIMIT - fixed_smem - a.n_strips * MIRROR * 256) / (a.n_strips * KP * 256)});
       if (a.ring < a.ahead + 3 || a.a_stages < 2) continue;
       a.ci_tiles = (cib + nci - 1) / nci;
@@ -616,6 +660,8 @@ static Plan make_plan(const ConvGeom& g, size_t budget) {
   const int kblocks = a.span / KP, chunks = (kblocks + limit - 1) / limit;
   a.chunk_kb = (kblocks + chunks - 1) / chunks;
   a.g = g;
+  a.fold_kh = fold ? real.kh : 0;
+  a.fold_sh = real.sh; a.fold_dh = real.dh; a.fold_ph = real.ph; a.fold_h = real.h;
   return best;
 }
 
@@ -625,13 +671,13 @@ bool plan_bytes(const ConvGeom& g, size_t budget, size_t* bytes) {
   return p.ok;
 }
 
-template <int NG, int NB>
+template <int NG, int NB, bool FOLD = false>
 static int launch(const Args& a, const Plan& p, cudaStream_t st) {
   static std::once_flag once;
   static cudaError_t opt_in = cudaSuccess;
-  std::call_once(once, [] { opt_in = cudaFuncSetAttribute(dweight_tmem_kernel<NG, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448); });
+  std::call_once(once, [] { opt_in = cudaFuncSetAttribute(dweight_tmem_kernel<NG, NB, FOLD>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448); });
   B200_CUDA(opt_in);
-  dweight_tmem_kernel<NG, NB><<<dim3((unsigned)p.tiles, (unsigned)a.splits), THREADS, (size_t)p.smem, st>>>(a);
+  dweight_tmem_kernel<NG, NB, FOLD><<<dim3((unsigned)p.tiles, (unsigned)a.splits), THREADS, (size_t)p.smem, st>>>(a);
   count_launch();
   return launch_check("dweight_tmem_kernel");
 }
@@ -639,6 +685,12 @@ static int launch(const Args& a, const Plan& p, cudaStream_t st) {
 int run(const ConvGeom& g, View4 x, View4 dy, float* dw, void* ws, size_t ws_bytes, cudaStream_t st) {
   Plan p = make_plan(g, ws ? ws_bytes : 0);
   if (!p.ok) return B200_EUNSUPPORTED;
+  // element offsets inside a tensor are 32-bit in the kernel
+  auto span = [](const View4& v, long long n, long long c, long long h, long long w) {
+    return (n - 1) * std::llabs(v.s0) + (c - 1) * std::llabs(v.s1) + (h - 1) * std::llabs(v.s2) + (w - 1) * std::llabs(v.s3);
+  };
+  if (span(x, g.n, g.cin, g.h, g.w) > 2147483647ll - 64 * std::llabs(x.s1) || span(dy, g.n, g.cout, g.oh, g.ow) > 2147483647ll - 64 * std::llabs(dy.s1))
+    return B200_EUNSUPPORTED;
   Args& a = p.a;
   a.x = x; a.dy = dy;
   a.out = a.splits > 1 ? (float*)ws : dw;
@@ -651,10 +703,10 @@ int run(const ConvGeom& g, View4 x, View4 dy, float* dw, void* ws, size_t ws_byt
       if (a.groups[i].n_bits != 3u << 19) return false;
     return true;
   }();
-  const int rc = threes && a.n_groups == 3 ? launch<3, 3>(a, p, st) : threes && a.n_groups == 4 ? launch<4, 3>(a, p, st)
+  const int rc = a.fold_kh ? (a.n_groups == 2 ? launch<2, 0, true>(a, p, st) : a.n_groups == 1 ? launch<1, 0, true>(a, p, st) : launch<0, 0, true>(a, p, st)) : threes && a.n_groups == 3 ? launch<3, 3>(a, p, st) : threes && a.n_groups == 4 ? launch<4, 3>(a, p, st)
                : a.n_groups == 1 ? launch<1, 0>(a, p, st) : a.n_groups == 6 ? launch<6, 0>(a, p, st) : launch<0, 0>(a, p, st);
   if (rc) return rc;
-  if (a.splits > 1) return tcdw::finalize_partials((const float*)ws, dw, g, a.splits, st);
+  if (a.splits > 1) return tcdw::finalize_partials((const float*)ws, dw, a.g, a.splits, st);
   return B200_OK;
 }
 

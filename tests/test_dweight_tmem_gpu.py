@@ -24,6 +24,10 @@ CASES = [  # (xshape, cout, kernel, conv arguments)
     ((2, 32, 15, 14), 96, (3, 3), dict(stride=(3, 2), padding=(0, 1))),
     ((1, 96, 14, 14), 160, (3, 3), dict(padding=(4, 4), dilation=(4, 4))),      # eight rows between the outer taps
     ((2, 64, 14, 14), 64, (3, 3), dict(padding=(1, 1), groups=2)),
+    ((2, 3, 32, 33), 64, (7, 7), dict(stride=(2, 2), padding=(3, 3))),          # filter rows folded into the channels: 21 of 32
+    ((1, 8, 19, 20), 130, (5, 5), dict(padding=(2, 2))),                        # 40: two strips
+    ((3, 1, 17, 16), 16, (3, 3), dict(padding=(1, 1))),
+    ((2, 15, 12, 13), 40, (3, 3), dict(stride=(1, 3), padding=(0, 1), dilation=(2, 1))),
 ]
 
 
