@@ -2,9 +2,9 @@
 // operands.  Replaces attention_forward / attention_backward of the reference
 // (csrc/ops/attention.cpp:16-34) and its sdpa_training shader, dropout included (the same counter-based stream).
 //
-// The products run on the GEMM kernels of this library (b200_bmm: tcgen05 from 128x64x32, CUDA
-// cores below); the score matrix is materialised in the caller's workspace, so this is the
-// composed form of attention, not a single fused pass:
+// Calls without mask, dropout and mask gradient and with heads of 16 to 64 dimensions go to attention_fused.cu.  The rest takes
+// the composed form: the products run on the GEMM kernels of this library (b200_bmm: tcgen05 from 128x64x32, CUDA
+// cores below) and the score matrix is materialised in the caller's workspace:
 //   forward   S = Q K^T;  P = softmax(S * scale + mask) row by row, in place, with the
 //             log-sum-exp kept per row;  O = P V
 //   backward  P again from S and the saved log-sum-exp;  dP = dO V^T;
@@ -14,8 +14,11 @@
 // additive FP32 or one byte per score where zero hides the key (a bool tensor); a row with every key hidden has
 // log-sum-exp -inf and probability 0.  The backward pass can also return the gradient of the additive mask,
 // dM = P (dP - rowsum(dO O)), the unscaled score gradient (sdpa_training.comp:38,40 `aux[index]=ds`).
+#include <algorithm>
 #include <cmath>
+#include <cstdlib>
 
+#include "attention_fused.cuh"
 #include "common.cuh"
 
 namespace b200 {
@@ -297,6 +300,14 @@ int check_mask(const void* mask, int mask_type) {
   return B200_OK;
 }
 
+// The fused kernels take calls without mask, dropout and mask gradient (B200_ATTENTION_COMPOSED=1 pins the composed form: testing aid).
+bool use_fused(int64_t batch, int64_t tq, int64_t tk, int64_t d, int64_t dv, const void* mask, float dropout, const void* dmask, const void* ws,
+               size_t ws_bytes, bool backward) {
+  const char* e = getenv("B200_ATTENTION_COMPOSED");
+  return !(e && e[0] == '1') && !mask && dropout == 0.f && !dmask && fa::supported(batch, tq, tk, d, dv) &&
+         ws && (reinterpret_cast<uintptr_t>(ws) & 15) == 0 && ws_bytes >= fa::workspace(batch, tq, tk, d, backward) && device_status_word();
+}
+
 // -inf -> 0 in place (rows with every key hidden)
 __global__ void __launch_bounds__(kThreads) lse_finite_kernel(float* __restrict__ lse, long long count) {
   const long long i = blockIdx.x * (long long)kThreads + threadIdx.x;
@@ -313,7 +324,8 @@ extern "C" {
 size_t b200_attention_workspace(int64_t batch, int64_t tq, int64_t tk, int64_t d, int64_t dv, int backward) {
   AttentionShape sh;
   if (make_shape(batch, tq, tk, d, dv, &sh)) return 0;
-  return sh.score_bytes * (backward ? 2 : 1);
+  const size_t composed = sh.score_bytes * (backward ? 2 : 1);
+  return fa::supported(batch, tq, tk, d, dv) ? std::max(composed, fa::workspace(batch, tq, tk, d, backward != 0)) : composed;
 }
 
 int b200_attention_forward(int64_t batch, int64_t tq, int64_t tk, int64_t d, int64_t dv, const float* q, const float* k,
@@ -334,6 +346,10 @@ int b200_attention_forward(int64_t batch, int64_t tq, int64_t tk, int64_t d, int
     fill_kernel<<<(unsigned)((rows + kThreads - 1) / kThreads), kThreads, 0, st>>>(lse, -INFINITY, rows);
     count_launch();
     return launch_check("fill_kernel");
+  }
+  if (fa::aligned({q, k, v, out}) && use_fused(batch, tq, tk, d, dv, mask, dropout, nullptr, workspace, workspace_bytes, false)) {
+    note_kernel("attention_forward: fused");
+    return fa::forward(batch, tq, tk, d, q, k, v, causal, scale, out, lse, workspace, st);
   }
   if (!workspace || workspace_bytes < sh.score_bytes) return fail(B200_EWORKSPACE, "attention: workspace smaller than b200_attention_workspace()");
   float* scores = (float*)workspace;
@@ -382,6 +398,10 @@ int b200_attention_backward(int64_t batch, int64_t tq, int64_t tk, int64_t d, in
     return B200_OK;
   }
   if (!grad || !q || !k || !v || !out || !lse) return fail(B200_EINVAL, "attention backward: null tensor");
+  if (fa::aligned({grad, q, k, v, out, dq, dk, dvalue}) && use_fused(batch, tq, tk, d, dv, mask, dropout, dmask, workspace, workspace_bytes, true)) {
+    note_kernel("attention_backward: fused");
+    return fa::backward(batch, tq, tk, d, grad, q, k, v, out, lse, causal, scale, dq, dk, dvalue, workspace, st);
+  }
   if (!workspace || workspace_bytes < 2 * sh.score_bytes)
     return fail(B200_EWORKSPACE, "attention: workspace smaller than b200_attention_workspace()");
   float* p = (float*)workspace;
