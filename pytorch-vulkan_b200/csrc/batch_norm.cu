@@ -23,6 +23,7 @@
 #include <cstdlib>
 
 #include "common.cuh"
+#include "norm_resident.cuh"
 
 namespace b200 {
 namespace {
@@ -629,157 +630,119 @@ __global__ void __launch_bounds__(kThreads) bn_bwd_apply_scalar_kernel(const flo
   }
 }
 
-// ---- small tensors: one CTA per channel, one launch ------------------------------------------------
-// When a channel's values are a few hundred KB at most and there are enough channels to fill the
-// GPU, the three launches above cost more than the traffic.  Here one CTA owns a channel from the
-// first read to the last write, as the reference's workgroup does (batch_norm_forward.comp:18-55,
-// batch_norm_backward.comp:18-66), with a warp per image plane; the second pass finds the channel in
-// L1 / L2.  Planar layout only.
+// ---- channels held in registers, one launch ---------------------------------------------------------
+// Planar tensors whose channels fit the registers of a cluster (norm_resident.cuh): each tensor is read
+// once, and the latency of one load, one exchange and one store replaces that of three launches.
+// 64 images of 256 channels of 14x14: forward 17.7 us with one CTA of 1024 threads a channel and a second
+// read from L2, now 9.8 (the
+// traffic takes 4 at HBM rate; the rest is launch, load latency and the two exchanges); backward 18.7, now 12.5.  512 channels of 7x7: 37 us for both
+// directions in three launches each, now 19.
+constexpr int kUnits = 8, kUnits1 = 16;       // most units a thread holds: forward (16 bytes each), single values
+constexpr int kUnitsBwd = 4;                  // backward: of each of the two tensors
 
-// f(value) / f(x value, g value) over a plane of `len` floats, the warp's lanes striding it with
-// 16-byte loads where the plane is aligned.
-constexpr int kChannelThreads = 1024;  // 32 warps: a channel is spread over as many image planes at once as an SM holds
-
-template <bool TWO, class F>
-__device__ __forceinline__ void plane_stream(const float* __restrict__ p, const float* __restrict__ q, int len, int lane, F&& f) {
-  int done = 0;
-  if (((reinterpret_cast<uintptr_t>(p) | (TWO ? reinterpret_cast<uintptr_t>(q) : 0)) & 15) == 0) {
-    const float4* p4 = reinterpret_cast<const float4*>(p);
-    const float4* q4 = reinterpret_cast<const float4*>(q);
-    const int quads = len >> 2;
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    int i = lane;
-    for (; i + 32 < quads; i += 64) {
-      const float4 a0 = __ldg(p4 + i), a1 = __ldg(p4 + i + 32), b0 = TWO ? __ldg(q4 + i) : zero, b1 = TWO ? __ldg(q4 + i + 32) : zero;
-      f(a0.x, b0.x), f(a0.y, b0.y), f(a0.z, b0.z), f(a0.w, b0.w);
-      f(a1.x, b1.x), f(a1.y, b1.y), f(a1.z, b1.z), f(a1.w, b1.w);
-    }
-    for (; i < quads; i += 32) {
-      const float4 a = __ldg(p4 + i), b = TWO ? __ldg(q4 + i) : zero;
-      f(a.x, b.x), f(a.y, b.y), f(a.z, b.z), f(a.w, b.w);
-    }
-    done = quads * 4;
-  }
-  for (int e = done + lane; e < len; e += 32) f(__ldg(p + e), TWO ? __ldg(q + e) : 0.f);
-}
-// out[e] = f(a, b, r) over a plane; r is the residual value (0 when res is null).
-template <bool TWO, class F>
-__device__ __forceinline__ void plane_map(const float* __restrict__ p, const float* __restrict__ q, const float* __restrict__ res,
-                                          float* __restrict__ out, int len, int lane, F&& f) {
-  int done = 0;
-  const uintptr_t bits = reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(res) |
-                         (TWO ? reinterpret_cast<uintptr_t>(q) : 0);
-  if ((bits & 15) == 0) {
-    const float4* p4 = reinterpret_cast<const float4*>(p);
-    const float4* q4 = reinterpret_cast<const float4*>(q);
-    const float4* r4 = reinterpret_cast<const float4*>(res);
-    float4* o4 = reinterpret_cast<float4*>(out);
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int i = lane; i < (len >> 2); i += 32) {
-      const float4 a = __ldg(p4 + i), b = TWO ? __ldg(q4 + i) : zero, r = res ? __ldg(r4 + i) : zero;
-      o4[i] = make_float4(f(a.x, b.x, r.x), f(a.y, b.y, r.y), f(a.z, b.z, r.z), f(a.w, b.w, r.w));
-    }
-    done = (len >> 2) * 4;
-  }
-  for (int e = done + lane; e < len; e += 32) out[e] = f(__ldg(p + e), TWO ? __ldg(q + e) : 0.f, res ? __ldg(res + e) : 0.f);
-}
-
-__global__ void __launch_bounds__(kChannelThreads) bn_forward_channel_kernel(const float* __restrict__ x, BnShape sh, BnForwardVectors v,
-                                                                       BnPost post, float* __restrict__ y) {
-  const int ch = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const float origin = __ldg(x + (size_t)ch * sh.inner);
+template <int VEC, int N>
+__global__ void __launch_bounds__(nres::THREADS, 4) bn_forward_channel_kernel(const float* __restrict__ x, nres::Rows rows, int inner, float m_count,
+                                                                           BnForwardVectors v, BnPost post, float* __restrict__ y) {
+  auto cluster = nres::cg::this_cluster();
+  const int ch = blockIdx.x, rank = (int)cluster.block_rank();
+  const uint32_t end = min(rows.units, (uint32_t)(rank + 1) * rows.per), u0 = (uint32_t)rank * rows.per + threadIdx.x;
+  const float* base = x + (size_t)ch * inner;
+  const float origin = __ldg(base);
   const float gamma = v.weight ? v.weight[ch * v.w_stride] : 1.f;
   const float beta = v.bias ? v.bias[ch * v.b_stride] : 0.f;
-  Moments acc = {0.f, 0.f, 0.f};
-  for (int img = warp; img < sh.outer; img += kChannelThreads / 32) {
-    const float* base = x + ((size_t)img * sh.c + ch) * sh.inner;
-    const float k = __ldg(base + min(lane, sh.inner - 1));
-    Shifted t;
-    plane_stream<false>(base, nullptr, sh.inner, lane, [&](float xv, float) { t.add(xv, k); });
-    acc = merge(acc, t.moments(k, origin));
-  }
-  __shared__ Moments warp_part[32];
-  acc = warp_merge(acc);
-  if (threadIdx.x < 32) warp_part[threadIdx.x] = Moments{0.f, 0.f, 0.f};
-  __syncthreads();
-  if (lane == 0) warp_part[warp] = acc;
-  __syncthreads();
-  const Moments m = warp_merge(warp_part[lane]);  // every warp folds the partial results itself
-  const float variance = m.m2 / sh.m;
+  // read here: behind the exchange their latency would be the kernel's last
+  const float old_mean = v.running_mean ? v.running_mean[ch * v.rm_stride] : 0.f;
+  const float old_var = v.running_var ? v.running_var[ch * v.rv_stride] : 0.f;
+  nres::Unit<VEC> in[N];
+  uint32_t plane;
+#pragma unroll
+  for (int k = 0; k < N; ++k) in[k].load(base + nres::unit_offset<VEC>(rows, min(u0 + k * nres::THREADS, rows.units - 1), plane), u0 + k * nres::THREADS < end);
+  __shared__ nres::Table<1> t0, t1;
+  const float2 m = nres::row_moments<VEC, N>(in, u0, end, origin, m_count, t0, t1, cluster);
+  const float variance = m.y / m_count;
   const float inv = (variance == 0.f && v.eps == 0.f) ? 0.f : 1.f / sqrtf(variance + v.eps);
-  if (threadIdx.x == 0) {
-    const float mean = origin + m.mean;
+  if (rank == 0 && threadIdx.x == 0) {
+    const float mean = origin + m.x;
     v.save_mean[ch] = mean;
     v.save_inv[ch] = inv;
-    if (v.running_mean) {
-      float* p = v.running_mean + ch * v.rm_stride;
-      *p = (1.f - v.momentum) * *p + v.momentum * mean;
-    }
-    if (v.running_var) {
-      float* p = v.running_var + ch * v.rv_stride;
-      *p = (1.f - v.momentum) * *p + v.momentum * (m.m2 / (sh.m - 1.f));
-    }
+    if (v.running_mean) v.running_mean[ch * v.rm_stride] = (1.f - v.momentum) * old_mean + v.momentum * mean;
+    if (v.running_var) v.running_var[ch * v.rv_stride] = (1.f - v.momentum) * old_var + v.momentum * (m.y / (m_count - 1.f));
   }
-  const float4 k4 = make_float4(origin, m.mean, inv * gamma, beta);
-  for (int img = warp; img < sh.outer; img += kChannelThreads / 32) {
-    const size_t at = ((size_t)img * sh.c + ch) * sh.inner;
-    plane_map<false>(x + at, nullptr, post.res ? post.res + at : nullptr, y + at, sh.inner, lane, [&](float xv, float, float r) {
-      const float o = normalise(xv, k4) + r;
-      return post.relu ? fmaxf(o, 0.f) : o;
-    });
+  const float4 k4 = make_float4(origin, m.x, inv * gamma, beta);
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const uint32_t u = u0 + k * nres::THREADS;
+    if (u >= end) break;
+    const size_t at = (size_t)ch * inner + nres::unit_offset<VEC>(rows, u, plane);
+    nres::Unit<VEC> r;
+    r.load(post.res + (post.res ? at : 0), post.res != nullptr);
+#pragma unroll
+    for (int j = 0; j < VEC; ++j) {
+      r.v[j] += normalise(in[k].v[j], k4);
+      if (post.relu) r.v[j] = fmaxf(r.v[j], 0.f);
+    }
+    r.store(y + at);
   }
 }
 
-__global__ void __launch_bounds__(kChannelThreads) bn_backward_channel_kernel(const float* __restrict__ x, const float* __restrict__ g,
-                                                                        BnShape sh, BnBackwardVectors v, float* __restrict__ dx) {
-  const int ch = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+template <int VEC, int N>
+__global__ void __launch_bounds__(nres::THREADS, 4) bn_backward_channel_kernel(const float* __restrict__ x, const float* __restrict__ g, nres::Rows rows,
+                                                                            int inner, float m_count, BnBackwardVectors v, float* __restrict__ dx) {
+  auto cluster = nres::cg::this_cluster();
+  const int ch = blockIdx.x, rank = (int)cluster.block_rank();
+  const uint32_t end = min(rows.units, (uint32_t)(rank + 1) * rows.per), u0 = (uint32_t)rank * rows.per + threadIdx.x;
+  nres::Unit<VEC> xs[N], gs[N];
+  uint32_t plane;
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const size_t at = (size_t)ch * inner + nres::unit_offset<VEC>(rows, min(u0 + k * nres::THREADS, rows.units - 1), plane);
+    xs[k].load(x + at, u0 + k * nres::THREADS < end);
+    gs[k].load(g + at, u0 + k * nres::THREADS < end);
+  }
   const float mean = v.mean[ch * v.mean_stride];
   float inv = v.inv[ch * v.inv_stride];
   if (!v.training) inv = 1.f / sqrtf(inv + v.eps);
   const float gamma = v.weight ? v.weight[ch * v.w_stride] : 1.f;
   Sums t = {0.f, 0.f, 0.f};
-  for (int img = warp; img < sh.outer; img += kChannelThreads / 32) {
-    const size_t at = ((size_t)img * sh.c + ch) * sh.inner;
-    plane_stream<true>(x + at, g + at, sh.inner, lane, [&](float xv, float gv) { t.add(xv, gv, mean); });
-  }
-  __shared__ Sums warp_part[32];
-  t = warp_sums(t);
-  if (threadIdx.x < 32) warp_part[threadIdx.x] = Sums{0.f, 0.f, 0.f};
-  __syncthreads();
-  if (lane == 0) warp_part[warp] = t;
-  __syncthreads();
-  const Sums s = warp_sums(warp_part[lane]);
-  float fa = s.a, fb = s.b, residual = 0.f;
+#pragma unroll
+  for (int k = 0; k < N; ++k)
+    if (u0 + k * nres::THREADS < end) {
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) t.add(xs[k].v[j], gs[k].v[j], mean);
+    }
+  __shared__ nres::Table<3> table;
+  float s[3] = {t.a, t.b, t.r};
+  nres::cluster_sum(s, table, cluster);
+  float fa = s[0], fb = s[1], residual = 0.f;
   if (v.training) {
-    residual = s.r / sh.m;
+    // the saved mean is rounded to FP32; its low part comes back from sum(x - mean)
+    residual = s[2] / m_count;
     if (residual != 0.f) fb -= residual * fa;
   }
-  if (threadIdx.x == 0) {
+  if (rank == 0 && threadIdx.x == 0) {
     if (v.dw) v.dw[ch] = fb * inv;
     if (v.db) v.db[ch] = fa;
   }
   if (!dx) return;
-  const float4 k4 = make_float4(mean, residual, fa / sh.m, (fb / sh.m) * inv * inv);
+  const float4 k4 = make_float4(mean, residual, fa / m_count, (fb / m_count) * inv * inv);
   const float scale = inv * gamma;
   const bool training = v.training != 0;
-  for (int img = warp; img < sh.outer; img += kChannelThreads / 32) {
-    const size_t at = ((size_t)img * sh.c + ch) * sh.inner;
-    plane_map<true>(x + at, g + at, nullptr, dx + at, sh.inner, lane, [&](float xv, float gv, float) {
-      return training ? input_grad<true>(xv, gv, k4, scale) : input_grad<false>(xv, gv, k4, scale);
-    });
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const uint32_t u = u0 + k * nres::THREADS;
+    if (u >= end) break;
+#pragma unroll
+    for (int j = 0; j < VEC; ++j)
+      gs[k].v[j] = training ? input_grad<true>(xs[k].v[j], gs[k].v[j], k4, scale) : input_grad<false>(xs[k].v[j], gs[k].v[j], k4, scale);
+    gs[k].store(dx + (size_t)ch * inner + nres::unit_offset<VEC>(rows, u, plane));
   }
 }
 
-// One launch pays when a channel is tens to hundreds of KB and the channels fill the GPU.  Measured
-// kernel times (64 images): 256 channels of 14x14 20 us against 26 us for the three launches, 128
-// channels of 28x28 18 against 27; 512 channels of 7x7 (12 KB each) 31 against 21, so short channels
-// keep the three-launch path.
-bool channel_kernel_fits(const BnShape& sh, int layout) {
+// Ranks per channel for the kernels above, or 0: the channel does not fit.
+int channel_ranks(const BnShape& sh, int layout, int vec, int most) {
   static const bool enabled = !(getenv("B200_BN_ONE_LAUNCH") && getenv("B200_BN_ONE_LAUNCH")[0] == '0');  // testing aid
-  if (!enabled) return false;
-  const double channel_bytes = (double)sh.m * sizeof(float);
-  return layout == B200_BN_PLANAR && sh.c >= 64 && channel_bytes >= 32.0 * 1024 && channel_bytes <= 256.0 * 1024 &&
-         channel_bytes * sh.c <= 64.0 * 1024 * 1024;
+  if (!enabled || layout != B200_BN_PLANAR || sh.inner / vec >= (1 << 30) / sh.outer) return 0;
+  return nres::ranks_for((long long)sh.outer * (sh.inner / vec), sh.c, most);
 }
 
 // ---- host side ---------------------------------------------------------------------------------
@@ -901,11 +864,14 @@ int b200_batch_norm_forward_fused(int64_t n, int64_t c, int64_t s, int layout, c
   BnForwardVectors v{weight, bias, running_mean, running_var, weight_stride, bias_stride, running_mean_stride,
                      running_var_stride, save_mean, save_inv, eps, momentum};
   const uint32_t total = (uint32_t)((int64_t)sh.outer * sh.cols);
-  if (training && channel_kernel_fits(sh, layout)) {
-    note_kernel(residual || relu ? "bn_forward_channel_fused" : "bn_forward_channel");
-    bn_forward_channel_kernel<<<(unsigned)sh.c, kChannelThreads, 0, st>>>(x, sh, v, BnPost{residual, relu ? 1 : 0}, y);
-    count_launch();
-    return launch_check("bn_forward_channel_kernel");
+  if (training) {
+    const int vec = sh.inner % 4 == 0 && aligned16(x) && aligned16(y) && aligned16(residual) ? 4 : 1;
+    if (const int ranks = channel_ranks(sh, layout, vec, vec == 4 ? kUnits : kUnits1)) {
+      note_kernel(residual || relu ? "bn_forward_channel_fused" : "bn_forward_channel");
+      const nres::Rows rows = nres::make_rows(sh.outer, sh.inner, vec, (long long)sh.c * sh.inner, ranks);
+      return nres::launch(vec == 4 ? bn_forward_channel_kernel<4, kUnits> : bn_forward_channel_kernel<1, kUnits1>, (unsigned)sh.c, ranks, st, x, rows,
+                          sh.inner, sh.m, v, BnPost{residual, relu ? 1 : 0}, y);
+    }
   }
   if (training) {
     if (p.rows) {
@@ -991,11 +957,14 @@ int b200_batch_norm_backward(int64_t n, int64_t c, int64_t s, int layout, const 
     return launch_check("bn_bwd_pair_kernel");
   }
   const int has_sums = training || dw || db;
-  if (has_sums && channel_kernel_fits(sh, layout)) {
-    note_kernel("bn_backward_channel");
-    bn_backward_channel_kernel<<<(unsigned)sh.c, kChannelThreads, 0, st>>>(x, grad, sh, v, dx);
-    count_launch();
-    return launch_check("bn_backward_channel_kernel");
+  if (has_sums) {
+    const int vec = sh.inner % 4 == 0 && aligned16(x) && aligned16(grad) && aligned16(dx) ? 4 : 1;
+    if (const int ranks = channel_ranks(sh, layout, vec, vec == 4 ? kUnitsBwd : kUnits1)) {
+      note_kernel("bn_backward_channel");
+      const nres::Rows rows = nres::make_rows(sh.outer, sh.inner, vec, (long long)sh.c * sh.inner, ranks);
+      return nres::launch(vec == 4 ? bn_backward_channel_kernel<4, kUnitsBwd> : bn_backward_channel_kernel<1, kUnits1>, (unsigned)sh.c, ranks, st, x,
+                          grad, rows, sh.inner, sh.m, v, dx);
+    }
   }
   if (has_sums) {
     if (p.rows) {

@@ -1,0 +1,144 @@
+// Normalisation rows held in registers: what batch_norm.cu (a row = the planes of one channel) and group_norm.cu (a row = the
+// planes of one sample and group) share.
+//
+// A row that is read for its sums and again for its result costs a second trip to L2 or HBM and, with one CTA a row, leaves the
+// machine to a few hundred long chains.  Here the CTAs of a thread-block cluster share a row: every thread loads its units (16 bytes,
+// or one value where planes are not whole 16-byte pieces) at once, keeps them in registers, the CTAs exchange one partial
+// sum each through distributed shared memory, and the result is computed from the registers.  One trip to memory, one barrier.
+#pragma once
+#include <cooperative_groups.h>
+
+#include "common.cuh"
+
+namespace b200 {
+namespace nres {
+namespace cg = cooperative_groups;
+
+constexpr int THREADS = 256, WARPS = THREADS / 32, MAX_RANKS = 16;
+
+struct Rows {
+  uint32_t units, per;        // units of a row; of one rank
+  uint32_t plane_units;
+  FastDiv plane_div;          // by plane_units
+  long long plane_stride;     // floats
+};
+
+template <int VEC>
+struct Unit {
+  float v[VEC];
+  __device__ __forceinline__ void load(const float* p, bool inside) {
+    if (VEC == 4) {
+      const float4 f = inside ? __ldg(reinterpret_cast<const float4*>(p)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[0] = f.x; v[1 % VEC] = f.y; v[2 % VEC] = f.z; v[3 % VEC] = f.w;
+    } else {
+      v[0] = inside ? __ldg(p) : 0.f;
+    }
+  }
+  __device__ __forceinline__ void store(float* p) const {
+    if (VEC == 4) *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1 % VEC], v[2 % VEC], v[3 % VEC]);
+    else *p = v[0];
+  }
+};
+
+template <int VEC>
+__device__ __forceinline__ long long unit_offset(const Rows& r, uint32_t u, uint32_t& plane) {
+  plane = r.plane_div.div(u);
+  return plane * r.plane_stride + (long long)((u - plane * r.plane_units) * VEC);
+}
+
+__device__ __forceinline__ float warp_total(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// Sums of C values over the cluster, in every thread and in the same order everywhere: each warp leaves its sums with every rank, so
+// that there is one barrier and no second level inside the CTA.  `table` is used once per kernel.
+template <int C>
+using Table = float[MAX_RANKS * WARPS][C];
+template <int C>
+__device__ __forceinline__ void cluster_sum(float (&v)[C], Table<C>& table, cg::cluster_group& cluster) {
+  const int ranks = (int)cluster.num_blocks(), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int c = 0; c < C; ++c) v[c] = warp_total(v[c]);
+  if (lane < ranks) {
+    float* to = cluster.map_shared_rank(&table[cluster.block_rank() * WARPS + warp][0], lane);
+#pragma unroll
+    for (int c = 0; c < C; ++c) to[c] = v[c];
+  }
+  cluster.sync();
+#pragma unroll
+  for (int c = 0; c < C; ++c) v[c] = 0.f;
+  for (int i = lane; i < ranks * WARPS; i += 32) {
+#pragma unroll
+    for (int c = 0; c < C; ++c) v[c] += table[i][c];
+  }
+#pragma unroll
+  for (int c = 0; c < C; ++c) v[c] = warp_total(v[c]);
+}
+
+// Mean relative to `origin` and sum of squared deviations of the row whose units from u0 this thread holds: the mean first, then
+// the deviations themselves (the values are in registers), so that neither a common offset nor an outlier costs precision.
+template <int VEC, int N>
+__device__ __forceinline__ float2 row_moments(const Unit<VEC> (&in)[N], uint32_t u0, uint32_t end, float origin, float count, Table<1>& t0, Table<1>& t1,
+                                              cg::cluster_group& cluster) {
+  float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int k = 0; k < N; ++k)
+#pragma unroll
+    for (int j = 0; j < VEC; ++j) s[(k * VEC + j) & 3] += u0 + k * THREADS < end ? in[k].v[j] - origin : 0.f;
+  float sum[1] = {(s[0] + s[1]) + (s[2] + s[3])}, m2[1];
+  cluster_sum(sum, t0, cluster);
+  const float mean = sum[0] / count;
+  s[0] = s[1] = s[2] = s[3] = 0.f;
+#pragma unroll
+  for (int k = 0; k < N; ++k)
+#pragma unroll
+    for (int j = 0; j < VEC; ++j) {
+      const float d = u0 + k * THREADS < end ? (in[k].v[j] - origin) - mean : 0.f;
+      s[(k * VEC + j) & 3] = fmaf(d, d, s[(k * VEC + j) & 3]);
+    }
+  m2[0] = (s[0] + s[1]) + (s[2] + s[3]);
+  cluster_sum(m2, t1, cluster);
+  return make_float2(mean, m2[0]);
+}
+
+// Ranks of a cluster for rows of `units` when a thread holds up to `most` units, or 0 when even sixteen ranks do not hold one:
+// as few as hold the row (a wider exchange costs more than a fuller thread: 256 channels of 12544 values forward 9.5 us with 2 ranks of
+// eight units a thread, 12.5 with 4 of four), then twice as many while all CTAs still run at once, four to an SM, and a thread has
+// more than two units (20 rows and fewer would leave most SMs idle).
+inline int ranks_for(long long units, long long rows, int most) {
+  long long ranks = (units + (long long)THREADS * most - 1) / ((long long)THREADS * most);
+  if (ranks > MAX_RANKS) return 0;
+  if (ranks > 8) ranks = MAX_RANKS;
+  while (ranks <= MAX_RANKS / 2 && rows * ranks * 2 <= 4ll * sm_count() && units > ranks * THREADS * 2) ranks *= 2;
+  return (int)(ranks > 8 ? MAX_RANKS : ranks);
+}
+
+inline Rows make_rows(int planes, int plane, int vec, long long plane_stride, int ranks) {
+  Rows r{};
+  r.plane_units = (uint32_t)(plane / vec);
+  r.units = (uint32_t)planes * r.plane_units;
+  r.per = (r.units + (uint32_t)ranks - 1) / (uint32_t)ranks;
+  r.plane_div = FastDiv(r.plane_units);
+  r.plane_stride = plane_stride;
+  return r;
+}
+
+// grid (rows, ranks), clusters of `ranks` along y
+template <typename... P, typename... A>
+int launch(void (*kernel)(P...), unsigned rows, int ranks, cudaStream_t st, A... args) {
+  if (ranks > 8) B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(rows, (unsigned)ranks); cfg.blockDim = dim3(THREADS); cfg.stream = st;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = 1; attr.val.clusterDim.y = (unsigned)ranks; attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr; cfg.numAttrs = 1;
+  B200_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+  count_launch();
+  return launch_check("normalisation kernel");
+}
+
+}  // namespace nres
+}  // namespace b200
