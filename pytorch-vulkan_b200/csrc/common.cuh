@@ -125,6 +125,7 @@ struct StripPostOps {
 // Per-group element offsets that turn the grouped 1x1 convolution into a batched GEMM (tc_bmm).
 struct StripBatch {
   long long act_group_extra = 0, w_group_extra = 0, out_pitch = 0, out_group = 0;
+  long long k_total = 0;  // reduction channels of all groups together when the last group has fewer than the others (0: none missing)
 };
 int strip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* bias, long long bias_stride, float* out,
                void* ws, size_t ws_bytes, cudaStream_t st, bool rowmajor = false, float alpha = 1.f, float beta = 1.f,

@@ -77,6 +77,7 @@ struct StripArgs {
   // batched GEMM (groups used as the batch): extra element offsets per group on top of the grouped
   // convolution's own (group * kc channels in, group * nc columns out); 0 / out_channels / nc otherwise
   long long act_group_extra, out_pitch, out_group;
+  int k_total;            // reduction channels of all groups (the last group may have fewer than kc)
   int cb_per_phase;       // kc / 32
   int cblocks;            // strips per tile: forward n_phase * cb_per_phase, dInput cb_per_phase
   int images_per_tile;    // forward: weight stages per tile = cb_per_phase * taps_total
@@ -152,6 +153,33 @@ __device__ __forceinline__ TileCoord tile_coord(const StripArgs& a, int tile) {
     c.m_tile = tn - c.group * a.tiles_m;
   }
   return c;
+}
+
+// 32 consecutive floats of each lane's row (row = null: nothing to store): lanes l, l+4, ..., l+28 exchange 16-byte pieces so that a
+// store instruction covers whole 128-byte lines of four rows instead of 16 bytes of 32 rows, which kept the load/store unit busy for
+// 8000 of the 32000 cycles of a 128x256 tile's products and slowed the producers' loads beside it.
+__device__ __forceinline__ void store_rows32(float (&v)[32], float* row, int lane) {
+  const int i = lane >> 2;
+#pragma unroll
+  for (int s = 1; s < 8; s <<= 1) {
+    const bool upper = (i & s) != 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if ((j & s) == 0) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          float &lo = v[4 * j + e], &hi = v[4 * (j | s) + e];
+          const float other = __shfl_xor_sync(0xffffffffu, upper ? lo : hi, s << 2);
+          if (upper) lo = other; else hi = other;
+        }
+      }
+  }
+  const unsigned long long mine = reinterpret_cast<unsigned long long>(row);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {  // piece i of row 4j + lane % 4
+    float* p = reinterpret_cast<float*>(__shfl_sync(0xffffffffu, mine, 4 * j + (lane & 3)));
+    if (p) reinterpret_cast<float4*>(p)[i] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+  }
 }
 
 template <int BN, int AW>
@@ -333,7 +361,7 @@ __global__ void __launch_bounds__(strip_threads(AW), 1) conv_strip_kernel(const 
     const int chunks = (a.strip_rows + 31) / 32;
     const bool vec_layout = a.act.s1 == 1 && a.kc % 4 == 0 && ((reinterpret_cast<uintptr_t>(a.act.ptr) & 15) == 0) &&
                         (a.act.s0 % 4 == 0) && (a.act.s2 % 4 == 0) && (a.act.s3 % 4 == 0) && (a.act_group_extra % 4 == 0);
-    const bool chunked_layout = vec_layout && a.act.s3 < 256;  // eight lanes per pixel (see below)
+    const bool chunked_layout = vec_layout;
     const int s1 = (int)a.act.s1;
     const int my_units = a.units > (int)blockIdx.x ? (a.units - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
     const int my_tiles = my_units * a.unit;
@@ -361,7 +389,7 @@ __global__ void __launch_bounds__(strip_threads(AW), 1) conv_strip_kernel(const 
       const int phase = a.phase_on_n ? 0 : (int)a.div_cbpp.div((uint32_t)cb), cbl = cb - phase * a.cb_per_phase;
       // the last channel block of a group may be ragged (channel counts that are no multiple of 32):
       // it takes the masked one-value-per-load path, channels beyond the group read as zero
-      const int nvalid = min(KBLK, a.kc - cbl * KBLK);
+      const int nvalid = min(KBLK, min(a.kc, a.k_total - group * a.kc) - cbl * KBLK);
       const bool chunked = chunked_layout && nvalid == KBLK, vec_ok = vec_layout && nvalid == KBLK;
       if (ok) {
         const int n = (int)a.img_div.div((uint32_t)q);
@@ -547,12 +575,11 @@ __global__ void __launch_bounds__(strip_threads(AW), 1) conv_strip_kernel(const 
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.f);
         }
-        if (ok) {
+        if (a.out_rowmajor && a.out_vec4 && nvalid == 32) {
+          store_rows32(v, ok ? a.out + obase + c0 : nullptr, lane);
+        } else if (ok) {
           float* p = a.out + obase + c0 * col_stride;
-          if (a.out_rowmajor && a.out_vec4 && nvalid == 32) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) reinterpret_cast<float4*>(p)[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-          } else if (nvalid == 32) {
+          if (nvalid == 32) {
 #pragma unroll
             for (int j = 0; j < 32; ++j, p += col_stride) *p = v[j];
           } else {
@@ -593,7 +620,7 @@ __global__ void __launch_bounds__(strip_threads(AW), 1) conv_strip_kernel(const 
 // so a weight stage of the main kernel is one bulk copy from a running pointer.
 __global__ void __launch_bounds__(256) stage_weights_kernel(ConvGeom g, View4 w, int is_dx, int bn, int tiles_pp,
                                                             TapTable tt, float* __restrict__ out, long long total,
-                                                            long long w_group_extra) {
+                                                            long long w_group_extra, int k_total, int rows_first) {
   // let the convolution kernel behind this one start its prologue and its activation strips now
   asm volatile("griddepcontrol.launch_dependents;");
   const long long i = blockIdx.x * 256ll + threadIdx.x;
@@ -601,8 +628,11 @@ __global__ void __launch_bounds__(256) stage_weights_kernel(ConvGeom g, View4 w,
   const int kc = is_dx ? g.cog : g.cig, nc = is_dx ? g.cig : g.cog;
   const int cpp = (kc + KBLK - 1) / KBLK;
   // one thread per four adjacent reduction channels: a 16-byte piece of the swizzled row
-  const int k = (int)(i % (KBLK / 4)) * 4;
-  const int row = (int)((i / (KBLK / 4)) % bn);
+  // neighbouring threads take neighbouring columns of a row, or neighbouring rows where those are the adjacent values
+  // (a read along the adjacent values; written rows are 16-byte pieces of their 128 bytes either way)
+  const int in_image = (int)(i % ((KBLK / 4) * bn));
+  const int k = (rows_first ? in_image / bn : in_image % (KBLK / 4)) * 4;
+  const int row = rows_first ? in_image % bn : in_image / (KBLK / 4);
   const long long image = i / ((long long)(KBLK / 4) * bn);
   int grp, n_tile, cbl, tap;
   if (is_dx) {  // [group][phase][tile of the phase][channel block][tap of the phase]
@@ -636,7 +666,7 @@ __global__ void __launch_bounds__(256) stage_weights_kernel(ConvGeom g, View4 w,
                        tt.ky[tap] * w.s2 + tt.kx[tap] * w.s3 + grp * w_group_extra;
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-      if (c + j < kc) v[j] = __ldg(src + j * step);
+      if (c + j < kc && (long long)grp * kc + c + j < k_total) v[j] = __ldg(src + j * step);
   }
   float hi[4], lo[4];
 #pragma unroll
@@ -713,6 +743,13 @@ StripPlan plan_strip_geometry(const ConvGeom& g, bool is_dx) {
   return p;
 }
 
+// Modelled time of `tiles` tiles of `bn` columns, in arbitrary units: a narrow tile feeds the tensor core less per shared-memory byte,
+// and with one tap per strip stages as many activations for fewer products (4096 rows: 1.25, 0.95 and 0.63 us per 32-column block).
+static double width_cost(long long tiles, int bn, bool single_tap) {
+  const double eff = bn == 256 ? 1.0 : bn == 128 ? (single_tap ? 0.66 : 0.85) : (single_tap ? 0.5 : 0.55);
+  return (double)div_up64(tiles, sm_count()) * bn / eff;
+}
+
 static StripPlan plan_strip(const ConvGeom& g, bool is_dx) {
   StripPlan p = plan_strip_geometry(g, is_dx);
   if (!p.ok) return p;
@@ -736,8 +773,7 @@ static StripPlan plan_strip(const ConvGeom& g, bool is_dx) {
       const int left = SMEM_LIMIT - a_stages * a_stage;
       if (left < 2 * w_stage) continue;
       const long long tiles = tiles_m * ((nc + bn - 1) / bn) * g.groups * (is_dx ? p.sph * p.spw : 1);
-      const double eff = bn == 256 ? 1.0 : (bn == 128 ? 0.85 : 0.55);
-      const double cost = (double)div_up64(tiles, sm_count()) * bn / eff;
+      const double cost = width_cost(tiles, bn, single_tap);
       if (!p.ok || cost < best_cost) {
         best_cost = cost;
         p.ok = true;
@@ -814,6 +850,7 @@ int strip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* b
   const int tiles_pp = (nc + plan.bn - 1) / plan.bn;  // column tiles (per output phase in dInput)
   const int tiles_n = is_dx ? tiles_pp * plan.tt.n_phase : tiles_pp;
   const int cpp = (kc + KBLK - 1) / KBLK;  // channel blocks per group, the last one possibly ragged
+  const int k_total = batch && batch->k_total ? (int)batch->k_total : g.groups * kc;
   const long long wcount = (long long)g.groups * tiles_pp * plan.bn * cpp * KBLK * g.kh * g.kw;  // per plane
   const float* wp = staged_images;
   bool staged_here = false;
@@ -822,7 +859,7 @@ int strip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* b
       return fail(B200_EWORKSPACE, "tcgen05 convolution needs a 16-byte aligned workspace of %zu bytes (got %zu)",
                   2 * sizeof(float) * (size_t)wcount, ws_bytes);
     stage_weights_kernel<<<(unsigned)div_up64(wcount / 4, 256), 256, 0, st>>>(g, w, is_dx ? 1 : 0, plan.bn, tiles_pp, plan.tt, (float*)ws, wcount / 4,
-                                                                          batch ? batch->w_group_extra : 0);
+                                                                          batch ? batch->w_group_extra : 0, k_total, std::llabs(is_dx ? w.s1 : w.s0) < std::llabs(is_dx ? w.s0 : w.s1) ? 1 : 0);
     count_launch();
     if (int rc = launch_check("stage_weights_kernel")) return rc;
     wp = (const float*)ws;
@@ -843,6 +880,7 @@ int strip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* b
   a.kc = kc;
   a.nc = nc;
   a.out_channels = is_dx ? g.cin : g.cout;
+  a.k_total = k_total;
   a.act_group_extra = batch ? batch->act_group_extra : 0;
   a.out_pitch = batch ? batch->out_pitch : a.out_channels;
   a.out_group = batch ? batch->out_group : nc;
@@ -862,7 +900,8 @@ int strip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* b
     for (int ph = 0; ph < plan.tt.n_phase; ++ph) most = std::max(most, (int)plan.tt.start[ph + 1] - (int)plan.tt.start[ph]);
     // ... and only while the reduction side is the larger one (256 -> 64 channels forward: 90 -> 69 us); with more output
     // than input (its dInput) the epilogue's stores set the pace and the extra warps only take registers from it (61 -> 80 us)
-    a.wide_producers = most <= 1 && kc > nc ? 1 : 0;
+    // (row-major stores are whole lines and cost less: 1024 -> 1024 columns of a GEMM 198 -> 157 us, but 80 -> 1024 is faster with eight)
+    a.wide_producers = most <= 1 && (kc > nc || (rowmajor && a.cblocks >= 16)) ? 1 : 0;
     if (const char* e = getenv("B200_STRIP_PRODUCERS")) a.wide_producers = atoi(e) == 16 ? 1 : 0;
   }
   const int chunks = (a.strip_rows + 31) / 32;
@@ -915,24 +954,112 @@ int strip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* b
 }
 
 
+// C = the sum of the split-K partial products (in order) + beta * bias[column]; V adjacent values per thread
+template <int V>
+__global__ void __launch_bounds__(256) gemm_finalize_kernel(const float* partial, int splits, long long count, int N, FastDiv by_n, const float* __restrict__ bias,
+                                                            float beta, float* __restrict__ C) {
+  const long long i = (blockIdx.x * 256ll + threadIdx.x) * V;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (i >= count) return;
+  float v[V] = {};
+#pragma unroll 4
+  for (int s = 0; s < splits; ++s) {
+    const float* p = partial + s * count + i;
+    if (V == 4) {
+      const float4 f = *reinterpret_cast<const float4*>(p);
+      v[0] += f.x; v[1 % V] += f.y; v[2 % V] += f.z; v[3 % V] += f.w;
+    } else {
+      v[0] += *p;
+    }
+  }
+  if (bias) {
+    const long long row = count < (1ll << 31) ? by_n.div((uint32_t)i) : i / N;
+    const int col = (int)(i - row * N);
+#pragma unroll
+    for (int j = 0; j < V; ++j) v[j] = fmaf(beta, __ldg(bias + col + j), v[j]);
+  }
+  if (V == 4) *reinterpret_cast<float4*>(C + i) = make_float4(v[0], v[1 % V], v[2 % V], v[3 % V]);
+  else C[i] = v[0];
+}
+
+static ConvGeom gemm_geometry(long long M, long long N, long long K, int groups) {
+  ConvGeom g{};
+  g.n = 1; g.cin = (int)(groups * K); g.cout = (int)(groups * N); g.h = 1; g.w = (int)M; g.kh = g.kw = 1; g.oh = 1; g.ow = (int)M;
+  g.sh = g.sw = 1; g.ph = g.pw = 0; g.dh = g.dw = 1; g.groups = groups; g.cig = (int)K; g.cog = (int)N;
+  return g;
+}
+
+// Slices of the reduction for a product whose tiles leave SMs idle.  Modelled time in microseconds: waves of (32-column blocks of the
+// reduction x the measured time of one at that tile width + prologue and last stores), and for two slices and more a second launch
+// that moves the partial products.  4096x2048 x 2048x512: 74 us as 128 tiles of 128 columns, 57 as two slices of 64 tiles of 256;
+// 2048x4096 x 4096x512: 84 -> 53 with four; 320x8000 x 8000x320: 147 -> 45.
+static int gemm_splits(long long M, long long N, long long K, long long* k_slice) {
+  int best = 1;
+  double best_time = 0.0;
+  *k_slice = K;
+  const long long tiles_m = div_up64(M, tcs::BLOCK_M);
+  for (int splits = 1; splits <= 32 && (splits == 1 || (tiles_m * (splits - 1) < 2ll * sm_count() && K >= 64ll * splits)); ++splits) {
+    const long long slice = splits == 1 ? K : (div_up64(K, splits) + 31) / 32 * 32;
+    if (splits > 1 && (div_up64(K, slice) != splits || splits * std::max(N, slice) > 2147483647ll)) continue;
+    double cost = 0.0, time = 0.0;  // of the width that plan_strip takes
+    for (int bn : {256, 128, 64}) {
+      if (bn > 64 && N <= bn / 2) continue;
+      const long long tiles = tiles_m * div_up64(N, bn) * splits;
+      const double c = tcs::width_cost(tiles, bn, true);
+      if (cost != 0.0 && c >= cost) continue;
+      cost = c;
+      time = (double)div_up64(tiles, sm_count()) * ((double)div_up64(slice, 32) * (bn == 256 ? 1.25 : bn == 128 ? 0.95 : 0.63) + 4.0);
+    }
+    if (splits > 1) time += 3.0 + splits * 2e-6 * (double)M * (double)N;
+    if (best_time == 0.0 || time < best_time) { best_time = time; best = splits; *k_slice = slice; }
+  }
+  return best;
+}
+
 // C[M,N] = alpha * A*B + beta * bias[n] as a 1x1 convolution over an M-pixel image with K input and N
-// output channels, written row-major.  Takes K >= 16 and N >= 16 (a ragged last block of K is padded
-// with zeros); anything else is the caller's CUDA-core kernel.  The staged copy of B comes from the caching allocator and is released on `st`.
+// output channels, written row-major; slices of K ride on the kernel's group dimension, each with its own partial product.  Takes
+// K >= 16 and N >= 16 (a ragged last block of K is padded with zeros); anything else is the caller's CUDA-core kernel.  The staged copy
+// of B and the partial products come from the caching allocator and are released on `st`.
 int tc_gemm(long long M, long long N, long long K, const float* A, long long sa0, long long sa1, const float* B,
             long long sb0, long long sb1, const float* bias, float alpha, float beta, float* C, cudaStream_t st) {
   if (K < 16 || N < 16 || M > 2147483647ll || N > 2147483647ll || K > 2147483647ll)
     return fail(B200_EUNSUPPORTED, "tcgen05 GEMM is incompatible with this shape (needs K >= 16 and N >= 16)");
-  ConvGeom g{};
-  g.n = 1; g.cin = (int)K; g.cout = (int)N; g.h = 1; g.w = (int)M; g.kh = g.kw = 1; g.oh = 1; g.ow = (int)M;
-  g.sh = g.sw = 1; g.ph = g.pw = 0; g.dh = g.dw = 1; g.groups = 1; g.cig = (int)K; g.cog = (int)N;
+  long long slice;
+  const int splits = gemm_splits(M, N, K, &slice);
+  const ConvGeom g = gemm_geometry(M, N, slice, splits);
   if (!tcs::plan_strip(g, false).ok) return fail(B200_EUNSUPPORTED, "tcgen05 GEMM is incompatible with this shape");
   const View4 act{A, 0, sa1, 0, sa0};   // [n=1][c=k][h=1][w=m]
   const View4 wv{B, sb1, sb0, 0, 0};    // [co=n][ci=k][1][1]
+  StripBatch sb;
+  sb.w_group_extra = slice * sb0 - N * sb1;  // slice s starts s*slice rows down B
+  sb.out_pitch = N;
+  sb.out_group = M * N;
+  sb.k_total = K;
   void* ws = nullptr;
-  const size_t ws_bytes = strip_workspace(g, B200_PHASE_FORWARD);
-  if (int rc = b200_malloc(&ws, ws_bytes, st)) return rc;
+  const size_t images = (strip_workspace(g, B200_PHASE_FORWARD) + 255) & ~(size_t)255, partial = splits > 1 ? (size_t)splits * M * N * sizeof(float) : 0;
+  if (int rc = b200_malloc(&ws, images + partial, st)) return rc;
   if (!bias || beta == 0.f) { bias = nullptr; beta = 0.f; }
-  const int rc = strip_conv(g, false, act, wv, bias, 1, C, ws, ws_bytes, st, true, alpha, beta);
+  int rc;
+  if (splits == 1) {
+    rc = strip_conv(g, false, act, wv, bias, 1, C, ws, images, st, true, alpha, beta);
+  } else {
+    float* parts = reinterpret_cast<float*>(static_cast<char*>(ws) + images);
+    rc = strip_conv(g, false, act, wv, nullptr, 1, parts, ws, images, st, true, alpha, 0.f, nullptr, nullptr, &sb);
+    if (!rc) {
+      const long long count = M * N;
+      const bool vec = N % 4 == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3((unsigned)div_up64(vec ? count / 4 : count, 256)); cfg.blockDim = dim3(256); cfg.stream = st;
+      cudaLaunchAttribute attr{};
+      attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr.val.programmaticStreamSerializationAllowed = 1;
+      cfg.attrs = &attr; cfg.numAttrs = 1;
+      const cudaError_t e = cudaLaunchKernelEx(&cfg, vec ? gemm_finalize_kernel<4> : gemm_finalize_kernel<1>, (const float*)parts, splits, count, (int)N,
+                                               FastDiv((uint32_t)N), bias, beta, C);
+      count_launch();
+      rc = e == cudaSuccess ? launch_check("gemm_finalize_kernel") : fail(B200_ECUDA, "gemm_finalize_kernel: %s", cudaGetErrorString(e));
+    }
+  }
   b200_free(ws, st);
   return rc;
 }
@@ -944,9 +1071,7 @@ int tc_bmm(long long batch, long long M, long long N, long long K, const float* 
            const float* B, long long sb_b, long long sb0, long long sb1, float* C, cudaStream_t st) {
   if (K < 16 || N < 16 || M > 2147483647ll || batch * N > 2147483647ll || batch * K > 2147483647ll || batch > 65535)
     return fail(B200_EUNSUPPORTED, "tcgen05 batched GEMM is incompatible with this shape (needs K >= 16 and N >= 16)");
-  ConvGeom g{};
-  g.n = 1; g.cin = (int)(batch * K); g.cout = (int)(batch * N); g.h = 1; g.w = (int)M; g.kh = g.kw = 1; g.oh = 1; g.ow = (int)M;
-  g.sh = g.sw = 1; g.ph = g.pw = 0; g.dh = g.dw = 1; g.groups = (int)batch; g.cig = (int)K; g.cog = (int)N;
+  const ConvGeom g = gemm_geometry(M, N, K, (int)batch);
   if (!tcs::plan_strip(g, false).ok) return fail(B200_EUNSUPPORTED, "tcgen05 batched GEMM is incompatible with this shape");
   const View4 act{A, 0, sa1, 0, sa0};   // [n=1][c=(b,k)][h=1][w=m]
   const View4 wv{B, sb1, sb0, 0, 0};    // [co=(b,n)][ci=k][1][1]
