@@ -127,6 +127,8 @@ struct StripBatch {
   long long act_group_extra = 0, w_group_extra = 0, out_pitch = 0, out_group = 0;
   long long k_total = 0;  // reduction channels of all groups together when the last group has fewer than the others (0: none missing)
 };
+// C[M,N] = alpha * sum of `splits` partial products + beta * bias[n] (null: none) (conv_tc_strip.cu)
+int gemm_finalize(const float* parts, int splits, long long M, long long N, float alpha, const float* bias, float beta, float* C, cudaStream_t st);
 int strip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* bias, long long bias_stride, float* out,
                void* ws, size_t ws_bytes, cudaStream_t st, bool rowmajor = false, float alpha = 1.f, float beta = 1.f,
                const float* staged_images = nullptr,  // images already written for strip_column_tile()

@@ -11,6 +11,8 @@
 //            conv2d_backward_input_tiled_body.glsl:49-93,
 //            conv2d_backward_weight_tiled_body.glsl:42-70 + conv2d_backward_weight_finalize.comp:9-18
 //   GEMM:    csrc/shaders/matmul_strided.comp:1-65, matmul_strided_bias.comp:33-68
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace b200 {
@@ -24,7 +26,7 @@ struct IgemmArgs {
   long long bias_stride;
   float* out;
   long long M, N, K;  // per-group GEMM extents
-  int span;           // dW: positions per split
+  long long span;     // dW and gemm: positions per split
   float alpha, beta;  // gemm epilogue
 };
 
@@ -134,6 +136,10 @@ __device__ __forceinline__ void store_out(const IgemmArgs& p, int group, int spl
   const ConvGeom& g = p.g;
   if (m >= p.M || n >= p.N) return;
   if (PH == PH_GEMM) {
+    if (p.span < p.K) {     // a slice of the reduction: a partial product
+      p.out[((long long)split * p.M + m) * p.N + n] = v;
+      return;
+    }
     float r = p.alpha * v;  // alpha scales the product whether or not a bias follows
     if (p.bias && p.beta != 0.f) r += p.beta * p.bias[n * p.bias_stride];
     p.out[m * p.N + n] = r;
@@ -165,7 +171,7 @@ __global__ void __launch_bounds__(256) simt_igemm_kernel(const IgemmArgs p) {
   const long long n0 = (long long)blockIdx.x * BN;
   const int split = blockIdx.z;
   long long k_begin = 0, k_end = p.K;
-  if (PH == PH_DW) {
+  if (PH == PH_DW || PH == PH_GEMM) {
     k_begin = (long long)split * p.span;
     k_end = min(p.K, k_begin + p.span);
   }
@@ -177,17 +183,27 @@ __global__ void __launch_bounds__(256) simt_igemm_kernel(const IgemmArgs p) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
 
+  // the next step's values are fetched while this one is multiplied (one step took 880 ns, nearly all of it load latency)
+  float ra[4], rb[4];
+  auto fetch = [&](long long k0) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int i = tid + 256 * j;
+      const long long m = m0 + (i >> 4), k = k0 + (i & 15);  // A: 16 consecutive threads walk K
+      ra[j] = (m < p.M && k < k_end) ? fetch_a<PH>(p, group, m, k) : 0.f;
+      const long long kb = k0 + (i >> 6);  // B: 64 consecutive threads walk N (n index fixed per thread)
+      rb[j] = (nctx.valid && kb < k_end) ? fetch_b<PH>(p, nctx, kb) : 0.f;
+    }
+  };
+  fetch(k_begin);
   for (long long k0 = k_begin; k0 < k_end; k0 += BK) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int i = tid + 256 * j;
-      const int am = i >> 4, ak = i & 15;  // A: 16 consecutive threads walk K
-      const long long m = m0 + am, k = k0 + ak;
-      As[ak][am] = (m < p.M && k < k_end) ? fetch_a<PH>(p, group, m, k) : 0.f;
-      const int bk = i >> 6;  // B: 64 consecutive threads walk N (n index fixed per thread)
-      const long long kb = k0 + bk;
-      Bs[bk][tid & 63] = (nctx.valid && kb < k_end) ? fetch_b<PH>(p, nctx, kb) : 0.f;
+      As[i & 15][i >> 4] = ra[j];
+      Bs[i >> 6][tid & 63] = rb[j];
     }
+    if (k0 + BK < k_end) fetch(k0 + BK);
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < BK; ++k) {
@@ -279,7 +295,7 @@ int simt_igemm_dweight(const ConvGeom& g, View4 x, View4 dy, float* dw, float* p
   IgemmArgs p{};
   p.g = g; p.a = dy; p.b = x;
   p.M = g.cog; p.N = (long long)g.cig * g.kh * g.kw; p.K = (long long)g.n * g.oh * g.ow;
-  p.span = splits > 1 ? span : (int)p.K;
+  p.span = splits > 1 ? span : p.K;
   p.out = splits > 1 ? partial : dw;
   if (int rc = launch_igemm<PH_DW>(p, g.groups, splits, st, "simt_igemm_dweight")) return rc;
   if (splits > 1) return finalize_splits(partial, dw, (long long)g.cout * p.N, splits, st);
@@ -293,7 +309,24 @@ int simt_gemm(long long M, long long N, long long K, const float* A, long long s
   p.b = {B, sb0, sb1, 0, 0};
   p.bias = bias; p.bias_stride = 1; p.alpha = alpha; p.beta = beta; p.out = C;
   p.M = M; p.N = N; p.K = K;
-  return launch_igemm<PH_GEMM>(p, 1, 1, st, "simt_gemm");
+  // Slices of the reduction where the 64x64 tiles leave the machine idle: up to four CTAs an SM, each with 64 values of the reduction
+  // or more (below that the second launch costs more than it saves).  100x1000 x 1000x2048: 173 us in one slice, now 47;
+  // 16x4096 x 4096x4096: 215, now 76.
+  const long long tiles = div_up64(M, BM) * div_up64(N, BN);
+  long long splits = std::max(1ll, std::min({4ll * sm_count() / tiles, K / 64, 64ll}));
+  p.span = div_up64(div_up64(std::max(K, 1ll), splits), BK) * BK;
+  splits = std::max<long long>(1, div_up64(K, p.span));
+  if (splits == 1) {
+    p.span = std::max(K, 1ll);
+    return launch_igemm<PH_GEMM>(p, 1, 1, st, "simt_gemm");
+  }
+  void* parts = nullptr;
+  if (int rc = b200_malloc(&parts, (size_t)splits * M * N * sizeof(float), st)) return rc;
+  p.out = (float*)parts;
+  int rc = launch_igemm<PH_GEMM>(p, 1, (int)splits, st, "simt_gemm");
+  if (!rc) rc = gemm_finalize((const float*)parts, (int)splits, M, N, alpha, beta != 0.f ? bias : nullptr, beta, C, st);
+  b200_free(parts, st);
+  return rc;
 }
 
 // ---------------------------------------------------------------------------------------

@@ -954,10 +954,10 @@ int strip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* b
 }
 
 
-// C = the sum of the split-K partial products (in order) + beta * bias[column]; V adjacent values per thread
+// C = alpha * the sum of the split-K partial products (in order) + beta * bias[column]; V adjacent values per thread
 template <int V>
-__global__ void __launch_bounds__(256) gemm_finalize_kernel(const float* partial, int splits, long long count, int N, FastDiv by_n, const float* __restrict__ bias,
-                                                            float beta, float* __restrict__ C) {
+__global__ void __launch_bounds__(256) gemm_finalize_kernel(const float* partial, int splits, long long count, int N, FastDiv by_n, float alpha,
+                                                            const float* __restrict__ bias, float beta, float* __restrict__ C) {
   const long long i = (blockIdx.x * 256ll + threadIdx.x) * V;
   asm volatile("griddepcontrol.wait;" ::: "memory");
   if (i >= count) return;
@@ -972,6 +972,8 @@ __global__ void __launch_bounds__(256) gemm_finalize_kernel(const float* partial
       v[0] += *p;
     }
   }
+#pragma unroll
+  for (int j = 0; j < V; ++j) v[j] *= alpha;
   if (bias) {
     const long long row = count < (1ll << 31) ? by_n.div((uint32_t)i) : i / N;
     const int col = (int)(i - row * N);
@@ -980,6 +982,20 @@ __global__ void __launch_bounds__(256) gemm_finalize_kernel(const float* partial
   }
   if (V == 4) *reinterpret_cast<float4*>(C + i) = make_float4(v[0], v[1 % V], v[2 % V], v[3 % V]);
   else C[i] = v[0];
+}
+
+int gemm_finalize(const float* parts, int splits, long long M, long long N, float alpha, const float* bias, float beta, float* C, cudaStream_t st) {
+  const long long count = M * N;
+  const bool vec = N % 4 == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)div_up64(vec ? count / 4 : count, 256)); cfg.blockDim = dim3(256); cfg.stream = st;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr; cfg.numAttrs = 1;
+  B200_CUDA(cudaLaunchKernelEx(&cfg, vec ? gemm_finalize_kernel<4> : gemm_finalize_kernel<1>, parts, splits, count, (int)N, FastDiv((uint32_t)N), alpha, bias, beta, C));
+  count_launch();
+  return launch_check("gemm_finalize_kernel");
 }
 
 static ConvGeom gemm_geometry(long long M, long long N, long long K, int groups) {
@@ -1045,20 +1061,7 @@ int tc_gemm(long long M, long long N, long long K, const float* A, long long sa0
   } else {
     float* parts = reinterpret_cast<float*>(static_cast<char*>(ws) + images);
     rc = strip_conv(g, false, act, wv, nullptr, 1, parts, ws, images, st, true, alpha, 0.f, nullptr, nullptr, &sb);
-    if (!rc) {
-      const long long count = M * N;
-      const bool vec = N % 4 == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
-      cudaLaunchConfig_t cfg{};
-      cfg.gridDim = dim3((unsigned)div_up64(vec ? count / 4 : count, 256)); cfg.blockDim = dim3(256); cfg.stream = st;
-      cudaLaunchAttribute attr{};
-      attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-      attr.val.programmaticStreamSerializationAllowed = 1;
-      cfg.attrs = &attr; cfg.numAttrs = 1;
-      const cudaError_t e = cudaLaunchKernelEx(&cfg, vec ? gemm_finalize_kernel<4> : gemm_finalize_kernel<1>, (const float*)parts, splits, count, (int)N,
-                                               FastDiv((uint32_t)N), bias, beta, C);
-      count_launch();
-      rc = e == cudaSuccess ? launch_check("gemm_finalize_kernel") : fail(B200_ECUDA, "gemm_finalize_kernel: %s", cudaGetErrorString(e));
-    }
+    if (!rc) rc = gemm_finalize(parts, splits, M, N, 1.f, bias, beta, C, st);
   }
   b200_free(ws, st);
   return rc;
