@@ -141,9 +141,17 @@ bool strip_view_addressable(const ConvGeom& g, bool is_dx, const View4& act, con
 int tc_route(const ConvGeom& g, bool is_dx, const View4& act);  // 0 strip, 1 gather, 2 CUDA-core implicit GEMM (conv_tc.cu)
 // transposed strip kernel (conv_tc_tstrip.cu): filter on M, up to 256 pixels on N; contiguous NCHW results
 bool tstrip_supported(const ConvGeom& g, int phase);
+// modelled time in microseconds of the arrangement's plan for a geometry it supports, and its tile count
+double strip_time(const ConvGeom& g, bool is_dx, long long* tiles);
+double tstrip_time(const ConvGeom& g, bool is_dx, long long* tiles);
+// reduction channels in slices (conv_slices.cu); `ws` holds conv_slices_workspace() bytes
+int conv_slices(const ConvGeom& g, bool is_dx, bool allow_transposed);
+size_t conv_slices_workspace(const ConvGeom& g, bool is_dx, int slices, bool allow_transposed);
+int conv_sliced(const ConvGeom& g, bool is_dx, int slices, bool allow_transposed, View4 act, View4 w, const float* bias, long long bias_stride,
+                const StripPostOps* post, float* out, void* ws, cudaStream_t st);
 size_t tstrip_workspace(const ConvGeom& g, int phase);
 int tstrip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* bias, long long bias_stride, float* out,
-                void* ws, size_t ws_bytes, cudaStream_t st);
+                void* ws, size_t ws_bytes, cudaStream_t st, long long w_group_extra = 0);
 // row kernel (conv_tc_rows.cu): forward passes of layers with fewer than 16 input channels, no workspace
 bool rows_supported(const ConvGeom& g);
 int rows_conv(const ConvGeom& g, View4 x, View4 w, const float* bias, long long bias_stride, float* y, cudaStream_t st);

@@ -605,7 +605,6 @@ static void tc_dweight_plan(const ConvGeom& g, size_t budget, int* splits_out, i
 }
 
 size_t tc_workspace(const ConvGeom& g, int phase, size_t budget, int* splits_out, int* span_out) {
-  (void)budget;
   if (splits_out) *splits_out = 1;
   if (span_out) *span_out = 0;
   if (phase == B200_PHASE_FORWARD && rows_supported(g)) return 0;   // the filter is split inside the kernel
@@ -613,6 +612,15 @@ size_t tc_workspace(const ConvGeom& g, int phase, size_t budget, int* splits_out
     const size_t planes = 2 * sizeof(float) * (size_t)g.cout * g.cig * g.kh * g.kw;  // hi + lo
     size_t need = strip_allowed() && strip_supported(g, phase) ? std::max(planes, strip_workspace(g, phase)) : planes;
     if (strip_allowed() && tstrip_supported(g, phase)) need = std::max(need, tstrip_workspace(g, phase));
+    if (const int slices = strip_allowed() ? conv_slices(g, phase == B200_PHASE_DINPUT, true) : 1; slices > 1) {
+      const size_t more = conv_slices_workspace(g, phase == B200_PHASE_DINPUT, slices, true);  // wanted, not needed
+      if (more <= budget) need = std::max(need, more);
+    }
+    if (phase == B200_PHASE_FORWARD && strip_allowed())   // the fused forward pass has only the strip kernel's epilogue
+      if (const int slices = conv_slices(g, false, false); slices > 1) {
+        const size_t more = conv_slices_workspace(g, false, slices, false);
+        if (more <= budget) need = std::max(need, more);
+      }
     return need;
   }
   if (phase == B200_PHASE_DWEIGHT && strip_allowed() && dweight_strip_supported(g)) {
@@ -728,6 +736,12 @@ int tc_forward(const ConvGeom& g, View4 x, View4 w, const float* bias, long long
     if (rc != B200_EUNSUPPORTED) return rc;   // falls through to the CUDA-core kernel
   }
   int route = tc_route(g, false, x);
+  if (route == 3 || route == 0)
+    if (const int slices = conv_slices(g, false, true);
+        slices > 1 && ws && (reinterpret_cast<uintptr_t>(ws) & 15) == 0 && conv_slices_workspace(g, false, slices, true) <= ws_bytes) {
+      note_kernel(route == 3 ? "tc_tstrip_forward" : "tc_strip_forward");
+      return conv_sliced(g, false, slices, true, x, w, bias, bias_stride, nullptr, y, ws, st);
+    }
   if (route == 3) {
     note_kernel("tc_tstrip_forward");
     const int rc = tstrip_conv(g, false, x, w, bias, bias_stride, y, ws, ws_bytes, st);
@@ -751,6 +765,12 @@ int tc_dinput(const ConvGeom& g, View4 dy, View4 w, const float* bias, long long
               cudaStream_t st, bool* bias_applied) {
   if (bias_applied) *bias_applied = bias != nullptr;
   int route = tc_route(g, true, dy);
+  if (route == 3 || route == 0)
+    if (const int slices = conv_slices(g, true, true);
+        slices > 1 && ws && (reinterpret_cast<uintptr_t>(ws) & 15) == 0 && conv_slices_workspace(g, true, slices, true) <= ws_bytes) {
+      note_kernel(route == 3 ? "tc_tstrip_dinput" : "tc_strip_dinput");
+      return conv_sliced(g, true, slices, true, dy, w, bias, bias_stride, nullptr, dx, ws, st);
+    }
   if (route == 3) {
     note_kernel("tc_tstrip_dinput");
     const int rc = tstrip_conv(g, true, dy, w, bias, bias_stride, dx, ws, ws_bytes, st);

@@ -798,6 +798,17 @@ int strip_column_tile(const ConvGeom& g, bool is_dx) {
   const tcs::StripPlan p = tcs::plan_strip(g, is_dx);
   return p.ok ? p.bn : 0;
 }
+// Waves of tiles times filter stages of a tile times the measured time of a stage at that width (layers of a few waves), and the
+// prologue and epilogue of a wave.
+double strip_time(const ConvGeom& g, bool is_dx, long long* tiles) {
+  const tcs::StripPlan p = tcs::plan_strip(g, is_dx);
+  if (!p.ok) return 1e30;
+  const int kc = is_dx ? g.cog : g.cig, nc = is_dx ? g.cig : g.cog, phases = is_dx ? std::max(1, p.tt.n_phase) : 1;
+  const long long count = div_up64((long long)g.n * (p.gh + p.pr) * (p.gw + p.pc), tcs::BLOCK_M) * ((nc + p.bn - 1) / p.bn) * g.groups * phases;
+  if (tiles) *tiles = count;
+  const double stages = (double)((kc + 31) / 32) * p.tt.taps_total / phases;
+  return (double)div_up64(count, sm_count()) * (stages * (p.bn == 256 ? 0.70 : p.bn == 128 ? 0.48 : 0.38) + 2.0) + 5.0;
+}
 // Bytes of the weight stage images: hi and lo planes with the column count padded to the tile width.
 // The width depends on the image count, so take the largest over the widths the plan may pick.
 size_t strip_workspace(const ConvGeom& g, int phase) {

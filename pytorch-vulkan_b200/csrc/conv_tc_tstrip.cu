@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(tstrip_threads(AW), 1) conv_tstrip_kernel(cons
 // main loop consumes them: forward [group][channel tile][phase][channel block][tap of the phase], dInput
 // [group][phase][channel tile of the phase][channel block][tap of the phase].  One thread per four channels.
 __global__ void __launch_bounds__(256) stage_filter16_kernel(ConvGeom g, View4 w, int is_dx, int tiles_pp, TapTable tt,
-                                                             unsigned char* __restrict__ out, long long total) {
+                                                             unsigned char* __restrict__ out, long long total, long long w_group_extra) {
   asm volatile("griddepcontrol.launch_dependents;");
   const long long i = blockIdx.x * 256ll + threadIdx.x;
   if (i >= total) return;
@@ -493,7 +493,7 @@ __global__ void __launch_bounds__(256) stage_filter16_kernel(ConvGeom g, View4 w
   if (r < nc) {
     const long long step = is_dx ? w.s0 : w.s1;
     const float* src = w.ptr + ((long long)grp * g.cog + (is_dx ? c : r)) * w.s0 + (long long)(is_dx ? r : c) * w.s1 +
-                       tt.ky[tap] * w.s2 + tt.kx[tap] * w.s3;
+                       tt.ky[tap] * w.s2 + tt.kx[tap] * w.s3 + grp * w_group_extra;
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       if (c + j < kc) v[j] = __ldg(src + j * step);
@@ -514,6 +514,7 @@ struct TPlan {
   int pn = 0, strip_rows = 0, a_stages = 0, w_stages = 0, smem = 0;
   int tiles_pp = 0, tiles_m = 0, tiles_p = 0, cpp = 0;
   long long images = 0;   // filter stage images in total
+  double clocks = 0.0;    // modelled duration
 };
 
 // Clocks of one tcgen05.mma of 128 x pn x 8 (TF32) or x 16 (BF16): the tensor pipe needs pn / 2, the
@@ -551,7 +552,7 @@ static TPlan plan_tstrip(const ConvGeom& g, bool is_dx) {
     const long long tiles = div_up64(q_total, pn) * p.tiles_m * g.groups;
     const double cost = (double)div_up64(tiles, sm_count()) * (stages_per_tile * (4.0 * mma_clocks(pn) + 120.0) + 3000.0);
     if (!p.ok || cost < best * 0.995) {   // ties go to the wider tile (fewer filter bytes per output)
-      best = cost;
+      best = p.clocks = cost;
       p.ok = true;
       p.pn = pn; p.strip_rows = rows; p.a_stages = a_stages; p.w_stages = w_stages;
       p.tiles_p = (int)div_up64(q_total, pn);
@@ -581,13 +582,18 @@ bool tstrip_supported(const ConvGeom& g, int phase) {
   }
   return tst::plan_tstrip(g, is_dx).ok;
 }
+double tstrip_time(const ConvGeom& g, bool is_dx, long long* tiles) {
+  const tst::TPlan p = tst::plan_tstrip(g, is_dx);
+  if (tiles) *tiles = (long long)p.tiles_p * p.tiles_m * g.groups;
+  return p.ok ? p.clocks / 1850.0 + 6.0 : 1e30;
+}
 size_t tstrip_workspace(const ConvGeom& g, int phase) {
   const tst::TPlan p = tst::plan_tstrip(g, phase == B200_PHASE_DINPUT);
   return p.ok ? (size_t)p.images * tst::W_STAGE_BYTES : 0;
 }
 
 int tstrip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* bias, long long bias_stride, float* out,
-                void* ws, size_t ws_bytes, cudaStream_t st) {
+                void* ws, size_t ws_bytes, cudaStream_t st, long long w_group_extra) {
   using namespace tst;
   const TPlan plan = plan_tstrip(g, is_dx);
   if (!plan.ok) return fail(B200_EUNSUPPORTED, "transposed strip kernel does not take this geometry");
@@ -597,7 +603,7 @@ int tstrip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* 
   const int kc = is_dx ? g.cog : g.cig, nc = is_dx ? g.cig : g.cog;
   const long long pieces = plan.images * TM * 4;
   stage_filter16_kernel<<<(unsigned)div_up64(pieces, 256), 256, 0, st>>>(g, w, is_dx ? 1 : 0, plan.tiles_pp, plan.geo.tt,
-                                                                         (unsigned char*)ws, pieces);
+                                                                         (unsigned char*)ws, pieces, w_group_extra);
   count_launch();
   if (int rc = launch_check("stage_filter16_kernel")) return rc;
 
