@@ -1,7 +1,7 @@
 // Forward and dInput of dense layers whose tiles leave SMs idle: the reduction channels in slices.
 //
 // A small batch of a deep layer has few pixels and a long reduction: 512 -> 512 channels of one 7x7 image are 8 tiles of 144 filter
-// stages each, 62 us on 8 of 148 SMs; 64 such images fill a wave only with narrow tiles, at 60 % of the tensor core's pace.  Slices of the
+// stages each, 62 us on 8 of 148 SMs (now 21); 64 such images fill a wave only with narrow tiles, at 60 % of the tensor core's pace.  Slices of the
 // reduction channels ride on the group dimension of the strip kernels (slice s of the input is a group of its own), each writes a partial
 // result, and the second kernel here adds them in order with bias, residual and ReLU.
 #include <algorithm>
@@ -13,21 +13,21 @@ namespace {
 
 constexpr int MAX_SLICES = 16;
 
-// out[n][c][p] = sum over s of part[n][s][c][p] + bias[c] + residual, clamped when relu; V adjacent pixels per thread
+// out[n][c][p] = sum over s of part[n][s][c][p] + bias[c] + residual, clamped when relu; V adjacent values of an image per thread
+// (a residual is added only where they are pixels of one row-major plane)
 template <int V>
 __global__ void __launch_bounds__(256) add_slices_kernel(const float* part, int slices, uint32_t count, uint32_t image, FastDiv image_div, FastDiv plane_div,
-                                                         int channels, FastDiv channel_div, FastDiv row_div, int ow, const float* __restrict__ bias,
-                                                         long long bias_stride, View4 res, int relu, float* __restrict__ out) {
-  const uint32_t i = blockIdx.x * 256u + threadIdx.x;      // in units of V
+                                                         FastDiv row_div, const float* __restrict__ bias, long long bias_stride, View4 res, int relu,
+                                                         float* __restrict__ out) {
+  const uint32_t i = (blockIdx.x * 256u + threadIdx.x) * V;
   asm volatile("griddepcontrol.wait;" ::: "memory");
   if (i >= count) return;
-  const uint32_t n = image_div.div(i), plane = plane_div.div(i);
-  const int c = (int)(plane - channel_div.div(plane) * (uint32_t)channels);
-  const float* p = part + ((long long)n * slices * image + (i - n * image)) * V;
+  const uint32_t n = image_div.div(i), in_image = i - n * image;
+  const float* p = part + (long long)n * slices * image + in_image;
   float v[V] = {};
 #pragma unroll 4
   for (int s = 0; s < slices; ++s) {
-    const float* q = p + (long long)s * image * V;
+    const float* q = p + (long long)s * image;
     if (V == 4) {
       const float4 f = *reinterpret_cast<const float4*>(q);
       v[0] += f.x; v[1 % V] += f.y; v[2 % V] += f.z; v[3 % V] += f.w;
@@ -35,20 +35,20 @@ __global__ void __launch_bounds__(256) add_slices_kernel(const float* part, int 
       v[0] += *q;
     }
   }
-  const float b = bias ? __ldg(bias + c * bias_stride) : 0.f;
-  float r[V] = {};
+  if (bias) {
+#pragma unroll
+    for (int j = 0; j < V; ++j) v[j] += __ldg(bias + plane_div.div(in_image + j) * bias_stride);
+  }
   if (res.ptr) {
-    const uint32_t at = (i - plane * plane_div.d) * V, y = row_div.div(at), x = at - y * (uint32_t)ow;
+    const uint32_t c = plane_div.div(in_image), at = in_image - c * plane_div.d, y = row_div.div(at), x = at - y * row_div.d;
     const float* q = res.ptr + n * res.s0 + c * res.s1 + y * res.s2 + x * res.s3;
 #pragma unroll
-    for (int j = 0; j < V; ++j) r[j] = __ldg(q + j);       // V == 4: contiguous planes
+    for (int j = 0; j < V; ++j) v[j] += __ldg(q + j);
   }
 #pragma unroll
-  for (int j = 0; j < V; ++j) {
-    v[j] += b + r[j];
+  for (int j = 0; j < V; ++j)
     if (relu) v[j] = fmaxf(v[j], 0.f);
-  }
-  if (V == 4) reinterpret_cast<float4*>(out)[i] = make_float4(v[0], v[1 % V], v[2 % V], v[3 % V]);
+  if (V == 4) *reinterpret_cast<float4*>(out + i) = make_float4(v[0], v[1 % V], v[2 % V], v[3 % V]);
   else out[i] = v[0];
 }
 
@@ -113,17 +113,16 @@ int conv_sliced(const ConvGeom& g, bool is_dx, int slices, bool allow_transposed
   if (rc) return rc;
   const int channels = is_dx ? g.cin : g.cout, oh = is_dx ? g.h : g.oh, ow = is_dx ? g.w : g.ow;
   const View4 res = post ? post->residual : View4{};
-  const bool vec = oh * ow % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && (!res.ptr || (res.s3 == 1 && res.s2 == ow));
-  const uint32_t v = vec ? 4 : 1, plane = (uint32_t)(oh * ow) / v, count = (uint32_t)(out_count(g, is_dx) / v);
+  const uint32_t plane = (uint32_t)(oh * ow), image = plane * (uint32_t)channels, count = (uint32_t)out_count(g, is_dx);
+  const bool vec = image % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && (!res.ptr || (plane % 4 == 0 && res.s3 == 1 && res.s2 == ow));
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((count + 255) / 256); cfg.blockDim = dim3(256); cfg.stream = st;
+  cfg.gridDim = dim3((count / (vec ? 4 : 1) + 255) / 256); cfg.blockDim = dim3(256); cfg.stream = st;
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr; cfg.numAttrs = 1;
-  B200_CUDA(cudaLaunchKernelEx(&cfg, vec ? add_slices_kernel<4> : add_slices_kernel<1>, (const float*)part, slices, count, plane * (uint32_t)channels,
-                               FastDiv(plane * (uint32_t)channels), FastDiv(plane), channels, FastDiv((uint32_t)channels), FastDiv((uint32_t)ow), ow, bias,
-                               bias_stride, res, post ? post->relu : 0, out));
+  B200_CUDA(cudaLaunchKernelEx(&cfg, vec ? add_slices_kernel<4> : add_slices_kernel<1>, (const float*)part, slices, count, image, FastDiv(image),
+                               FastDiv(plane), FastDiv((uint32_t)ow), bias, bias_stride, res, post ? post->relu : 0, out));
   count_launch();
   return launch_check("add_slices_kernel");
 }

@@ -454,58 +454,45 @@ __global__ void __launch_bounds__(tstrip_threads(AW), 1) conv_tstrip_kernel(cons
 // images the MMA reads: image = [hi: 128 rows x 64 B, SWIZZLE_64B][cross: same], row = output channel of the
 // tile (forward: co, dInput: ci; zero beyond nc), 16 reduction channels per row.  Images are ordered as the
 // main loop consumes them: forward [group][channel tile][phase][channel block][tap of the phase], dInput
-// [group][phase][channel tile of the phase][channel block][tap of the phase].  One thread per four channels.
+// [group][phase][channel tile of the phase][channel block][tap of the phase].  A thread takes four channels of one row and
+// `per_thread` taps (stage_weights_kernel in conv_tc_strip.cu says why).
 __global__ void __launch_bounds__(256) stage_filter16_kernel(ConvGeom g, View4 w, int is_dx, int tiles_pp, TapTable tt,
-                                                             unsigned char* __restrict__ out, long long total, long long w_group_extra) {
+                                                             unsigned char* __restrict__ out, long long total, long long w_group_extra,
+                                                             int rows_first, int per_thread) {
   asm volatile("griddepcontrol.launch_dependents;");
-  const long long i = blockIdx.x * 256ll + threadIdx.x;
+  const long long i = blockIdx.x * 256ll + threadIdx.x;   // [group][channel tile][channel block][row, piece], as stage_weights_kernel
   if (i >= total) return;
   const int kc = is_dx ? g.cog : g.cig, nc = is_dx ? g.cig : g.cog;
   const int cpp = (kc + KB - 1) / KB;
-  const int piece = (int)(i % 4), k = piece * 4;
-  const int row = (int)((i / 4) % TM);
-  const long long image = i / (4ll * TM);
-  int grp, m_tile, cbl, tap;
-  if (is_dx) {
-    const int per_group = tiles_pp * cpp * tt.taps_total;
-    grp = (int)(image / per_group);
-    const int local = (int)(image - (long long)grp * per_group);
-    int phase = 0;
-    while (phase + 1 < tt.n_phase && local >= tiles_pp * cpp * tt.start[phase + 1]) ++phase;
-    const int rel = local - tiles_pp * cpp * tt.start[phase], ntap = tt.start[phase + 1] - tt.start[phase];
-    m_tile = rel / (cpp * ntap);
-    const int rel2 = rel - m_tile * cpp * ntap;
-    cbl = rel2 / ntap;
-    tap = tt.start[phase] + rel2 % ntap;
-  } else {
-    const int per_tile = cpp * tt.taps_total;
-    const int local = (int)(image % per_tile);
-    m_tile = (int)((image / per_tile) % tiles_pp);
-    grp = (int)(image / ((long long)per_tile * tiles_pp));
-    int phase = 0;
-    while (phase + 1 < tt.n_phase && local >= cpp * tt.start[phase + 1]) ++phase;
-    const int rel = local - cpp * tt.start[phase], ntap = tt.start[phase + 1] - tt.start[phase];
-    cbl = rel / ntap;
-    tap = tt.start[phase] + rel % ntap;
-  }
+  const int block = (int)(i / (4 * TM)), in_block = (int)(i - (long long)block * (4 * TM));
+  const int piece = rows_first ? in_block / TM : in_block % 4, k = piece * 4;
+  const int row = rows_first ? in_block % TM : in_block / 4;
+  const int tile_of_all = block / cpp, cbl = block - tile_of_all * cpp, grp = tile_of_all / tiles_pp, m_tile = tile_of_all - grp * tiles_pp;
   const int r = m_tile * TM + row, c = cbl * KB + k;
-  float v[4] = {0.f, 0.f, 0.f, 0.f};
-  if (r < nc) {
-    const long long step = is_dx ? w.s0 : w.s1;
-    const float* src = w.ptr + ((long long)grp * g.cog + (is_dx ? c : r)) * w.s0 + (long long)(is_dx ? r : c) * w.s1 +
-                       tt.ky[tap] * w.s2 + tt.kx[tap] * w.s3 + grp * w_group_extra;
+  const int valid = r < nc ? min(4, kc - c) : 0;
+  const long long step = is_dx ? w.s0 : w.s1;
+  const float* src = w.ptr + ((long long)grp * g.cog + (is_dx ? c : r)) * w.s0 + (long long)(is_dx ? r : c) * w.s1 + grp * w_group_extra;
+  const int t0 = blockIdx.y * per_thread, t1 = min(tt.taps_total, t0 + per_thread);
+  int phase = 0;
+#pragma unroll 3
+  for (int tap = t0; tap < t1; ++tap) {
+    while (tap >= tt.start[phase + 1]) ++phase;
+    const int ntap = tt.start[phase + 1] - tt.start[phase], rel = tap - tt.start[phase];
+    const long long image = is_dx ? (long long)(grp * tt.taps_total + tt.start[phase]) * tiles_pp * cpp + ((long long)m_tile * cpp + cbl) * ntap + rel
+                                  : ((long long)tile_of_all * tt.taps_total + tt.start[phase]) * cpp + cbl * ntap + rel;
+    const float* p = src + tt.ky[tap] * w.s2 + tt.kx[tap] * w.s3;
+    float v[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (c + j < kc) v[j] = __ldg(src + j * step);
+    for (int j = 0; j < 4; ++j) v[j] = j < valid ? __ldg(p + j * step) : 0.f;
+    float hi[4], lo[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) split_tf32(v[j], hi[j], lo[j]);
+    unsigned char* img = out + image * (long long)W_STAGE_BYTES;
+    *reinterpret_cast<float4*>(img + sw64_chunk(row, piece)) = make_float4(hi[0], hi[1], hi[2], hi[3]);
+    unsigned char* cross = img + TM * ROWB;   // [bf16(lo) x16 | bf16(hi) x16], pairing with the activations' [hi | lo]
+    *reinterpret_cast<uint2*>(cross + sw64_chunk(row, piece >> 1) + (piece & 1) * 8) = make_uint2(pack_bf16x2(lo[0], lo[1]), pack_bf16x2(lo[2], lo[3]));
+    *reinterpret_cast<uint2*>(cross + sw64_chunk(row, 2 + (piece >> 1)) + (piece & 1) * 8) = make_uint2(pack_bf16x2(hi[0], hi[1]), pack_bf16x2(hi[2], hi[3]));
   }
-  float hi[4], lo[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) split_tf32(v[j], hi[j], lo[j]);
-  unsigned char* img = out + image * (long long)W_STAGE_BYTES;
-  *reinterpret_cast<float4*>(img + sw64_chunk(row, piece)) = make_float4(hi[0], hi[1], hi[2], hi[3]);
-  unsigned char* cross = img + TM * ROWB;   // [bf16(lo) x16 | bf16(hi) x16], pairing with the activations' [hi | lo]
-  *reinterpret_cast<uint2*>(cross + sw64_chunk(row, piece >> 1) + (piece & 1) * 8) = make_uint2(pack_bf16x2(lo[0], lo[1]), pack_bf16x2(lo[2], lo[3]));
-  *reinterpret_cast<uint2*>(cross + sw64_chunk(row, 2 + (piece >> 1)) + (piece & 1) * 8) = make_uint2(pack_bf16x2(hi[0], hi[1]), pack_bf16x2(hi[2], hi[3]));
 }
 
 struct TPlan {
@@ -601,9 +588,12 @@ int tstrip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* 
   if (!ws || ws_bytes < need || (reinterpret_cast<uintptr_t>(ws) & 15))
     return fail(B200_EWORKSPACE, "tcgen05 convolution needs a 16-byte aligned workspace of %zu bytes (got %zu)", need, ws_bytes);
   const int kc = is_dx ? g.cog : g.cig, nc = is_dx ? g.cig : g.cog;
-  const long long pieces = plan.images * TM * 4;
-  stage_filter16_kernel<<<(unsigned)div_up64(pieces, 256), 256, 0, st>>>(g, w, is_dx ? 1 : 0, plan.tiles_pp, plan.geo.tt,
-                                                                         (unsigned char*)ws, pieces, w_group_extra);
+  const int taps = plan.geo.tt.taps_total;
+  const long long threads = plan.images / taps * TM * 4;
+  const int per_thread = tcs::staged_taps(threads, taps);
+  stage_filter16_kernel<<<dim3((unsigned)div_up64(threads, 256), (unsigned)((taps + per_thread - 1) / per_thread)), 256, 0, st>>>(
+      g, w, is_dx ? 1 : 0, plan.tiles_pp, plan.geo.tt, (unsigned char*)ws, threads, w_group_extra,
+      std::llabs(is_dx ? w.s1 : w.s0) < std::llabs(is_dx ? w.s0 : w.s1) ? 1 : 0, per_thread);
   count_launch();
   if (int rc = launch_check("stage_filter16_kernel")) return rc;
 

@@ -29,6 +29,12 @@ struct StripPlan {
   TapTable tt;
 };
 
+// Taps that a thread of a filter staging kernel takes: as many as leave a CTA of 256 threads for every SM
+inline int staged_taps(long long threads, int taps) {
+  const long long fit = threads * taps / (256ll * sm_count());
+  return (int)(fit < 1 ? 1 : fit < taps ? fit : taps);
+}
+
 // Geometry part of the plan (grid, padding, tap table, shifts); `ok` is false when the strip kernels do not take it.
 StripPlan plan_strip_geometry(const ConvGeom& g, bool is_dx);
 
