@@ -127,6 +127,7 @@ __device__ __forceinline__ float4 drop_weight4(const DropState& d, uint32_t bloc
 __global__ void __launch_bounds__(kThreads) softmax_rows_kernel(float* __restrict__ scores, const void* __restrict__ mask, int mask_type, int tq,
                                                                  int tk, float scale, int causal, float* __restrict__ lse,
                                                                  DropState drop) {
+  wait_previous();
   __shared__ float scratch[kThreads / 32];
   const long long row = blockIdx.x;
   const int i = (int)(row % tq);
@@ -151,6 +152,7 @@ __global__ void __launch_bounds__(kThreads) softmax_rows_kernel(float* __restric
 __global__ void __launch_bounds__(kThreads) softmax_rows_resident_kernel(float* __restrict__ scores, const void* __restrict__ mask,
                                                                           int mask_type, int tq, int tk, float scale, int causal,
                                                                           float* __restrict__ lse, DropState drop) {
+  wait_previous();
   __shared__ float scratch[kThreads / 32];
   const long long row = blockIdx.x;
   const int i = (int)(row % tq), quads = tk >> 2;
@@ -202,6 +204,7 @@ __global__ void __launch_bounds__(kThreads) softmax_rows_resident_kernel(float* 
 // Backward, first elementwise step: s[j] <- P[j] = exp(s[j] * scale + mask - lse[row]).
 __global__ void __launch_bounds__(kThreads) probabilities_kernel(float* __restrict__ scores, const void* __restrict__ mask, int mask_type, int tq,
                                                                   int tk, float scale, int causal, const float* __restrict__ lse) {
+  wait_previous();
   const long long row = blockIdx.x;
   const int i = (int)(row % tq);
   float* s = scores + row * tk;
@@ -232,6 +235,7 @@ __global__ void __launch_bounds__(kThreads) probabilities_kernel(float* __restri
 __global__ void __launch_bounds__(kThreads) score_gradient_kernel(float* __restrict__ dp, float* __restrict__ p,
                                                                    const float* __restrict__ grad, const float* __restrict__ out, int tk,
                                                                    int dv, float scale, float* __restrict__ dmask, DropState drop) {
+  wait_previous();
   __shared__ float scratch[kThreads / 32];
   const long long row = blockIdx.x;
   float delta = 0.f;
@@ -358,8 +362,8 @@ int b200_attention_forward(int64_t batch, int64_t tq, int64_t tk, int64_t d, int
   const uintptr_t mask_align = mask_type == B200_MASK_BYTES ? 3 : 15;
   const bool resident = tk % 4 == 0 && tk <= 16 * kThreads && (reinterpret_cast<uintptr_t>(scores) & 15) == 0 &&
                         (reinterpret_cast<uintptr_t>(mask) & mask_align) == 0;
-  if (resident) softmax_rows_resident_kernel<<<(unsigned)rows, kThreads, 0, st>>>(scores, mask, mask_type, (int)tq, (int)tk, scale, causal, lse, drop);
-  else softmax_rows_kernel<<<(unsigned)rows, kThreads, 0, st>>>(scores, mask, mask_type, (int)tq, (int)tk, scale, causal, lse, drop);
+  if (resident) launch_next(softmax_rows_resident_kernel, (unsigned)rows, kThreads, 0, st, scores, mask, mask_type, (int)tq, (int)tk, scale, causal, lse, drop);
+  else launch_next(softmax_rows_kernel, (unsigned)rows, kThreads, 0, st, scores, mask, mask_type, (int)tq, (int)tk, scale, causal, lse, drop);
   count_launch();
   if (int rc = launch_check("softmax_rows_kernel")) return rc;
   if (dv == 0) return B200_OK;
@@ -407,13 +411,13 @@ int b200_attention_backward(int64_t batch, int64_t tq, int64_t tk, int64_t d, in
   float* p = (float*)workspace;
   float* dp = (float*)((char*)workspace + sh.score_bytes);
   if (int rc = b200_bmm(batch, tq, tk, d, q, tq * d, d, 1, k, tk * d, 1, d, p, B200_ALGO_AUTO, stream)) return rc;
-  probabilities_kernel<<<(unsigned)rows, kThreads, 0, st>>>(p, mask, mask_type, (int)tq, (int)tk, scale, causal, lse);
+  launch_next(probabilities_kernel, (unsigned)rows, kThreads, 0, st, p, mask, mask_type, (int)tq, (int)tk, scale, causal, lse);
   count_launch();
   if (int rc = launch_check("probabilities_kernel")) return rc;
   // dP[b] = dO[b] V[b]^T
   if (int rc = b200_bmm(batch, tq, tk, dv, grad, tq * dv, dv, 1, v, tk * dv, 1, dv, dp, B200_ALGO_AUTO, stream)) return rc;
   // dS in place of dP; with dropout P becomes P w for the product below
-  score_gradient_kernel<<<(unsigned)rows, kThreads, 0, st>>>(dp, p, grad, out, (int)tk, (int)dv, scale, dmask, drop);
+  launch_next(score_gradient_kernel, (unsigned)rows, kThreads, 0, st, dp, p, grad, out, (int)tk, (int)dv, scale, dmask, drop);
   count_launch();
   if (int rc = launch_check("score_gradient_kernel")) return rc;
   // dV[b] = (P w)[b]^T dO[b]

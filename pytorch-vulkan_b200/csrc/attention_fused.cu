@@ -472,6 +472,7 @@ struct StageArgs {
 // One CTA per (block of 64 tokens, batch, task); four values per thread and step.
 template <int DP>
 __global__ void __launch_bounds__(256) stage_kernel(const StageArgs a) {
+  wait_previous();
   asm volatile("griddepcontrol.launch_dependents;");
   const StageTask& t = a.task[blockIdx.z];
   const int blk = blockIdx.x;
@@ -569,7 +570,7 @@ static int forward_dp(int64_t batch, int64_t tq, int64_t tk, int64_t d, const fl
   s.d = (int)d; s.tasks = 2;
   s.task[0] = StageTask{k, ws, nullptr, (int)tk, kb, 1.f};
   s.task[1] = StageTask{v, nullptr, ws + image_bytes(batch, tk, d), (int)tk, kb, 1.f};
-  stage_kernel<DP><<<dim3((unsigned)kb, (unsigned)batch, 2), 256, 0, st>>>(s);
+  launch_next(stage_kernel<DP>, dim3((unsigned)kb, (unsigned)batch, 2), 256, 0, st, s);
   count_launch();
   if (int rc = launch_check("stage_kernel")) return rc;
   Args a{};
@@ -598,7 +599,7 @@ static int backward_dp(int64_t batch, int64_t tq, int64_t tk, int64_t d, const f
   s.task[1] = StageTask{q, q_k, q_mn, (int)tq, qb, scale * LOG2E};
   s.task[2] = StageTask{k, k_k, k_mn, (int)tk, kb, 1.f};
   s.task[3] = StageTask{v, v_k, nullptr, (int)tk, kb, 1.f};
-  stage_kernel<DP><<<dim3((unsigned)std::max(kb, qb), (unsigned)batch, 4), 256, 0, st>>>(s);
+  launch_next(stage_kernel<DP>, dim3((unsigned)std::max(kb, qb), (unsigned)batch, 4), 256, 0, st, s);
   count_launch();
   if (int rc = launch_check("stage_kernel")) return rc;
   Args a{};

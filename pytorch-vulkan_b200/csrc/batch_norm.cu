@@ -85,6 +85,7 @@ struct BnShape {
 
 // rows arrangement: grid (c, slabs); part[slab * c + ch].
 __global__ void __launch_bounds__(kThreads, 8) bn_stats_rows_kernel(const float* __restrict__ x, BnShape sh, Moments* part) {
+  wait_previous();
   const int ch = blockIdx.x, slab = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int units = sh.outer * sh.segs, per = sh.per;
   const int u0 = slab * per, u1 = min(units, u0 + per);
@@ -132,6 +133,7 @@ __global__ void __launch_bounds__(kThreads, 8) bn_stats_rows_kernel(const float*
 // cols % 4 == 0 and a 16-byte aligned tensor); part[slab * cols + col].
 template <int V>
 __global__ void __launch_bounds__(kThreads, 5) bn_stats_cols_kernel(const float* __restrict__ x, BnShape sh, Moments* part) {
+  wait_previous();
   const int cl = (threadIdx.x & 7) * V, prow = threadIdx.x >> 3, slab = blockIdx.y;
   const int col0 = blockIdx.x * 8 * V + cl;
   const int per = sh.per;
@@ -221,6 +223,7 @@ struct BnForwardVectors {
 // normalisation coefficients {origin, mean - origin, inv * gamma, beta}.
 __global__ void __launch_bounds__(kThreads) bn_stats_finalize_kernel(const float* __restrict__ x, BnShape sh, const Moments* part,
                                                                       BnForwardVectors v, float4* coef) {
+  wait_previous();
   const int ch = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (ch >= sh.c) return;
   const int entries = sh.slabs * sh.part_inner;
@@ -250,6 +253,7 @@ __global__ void __launch_bounds__(kThreads) bn_stats_finalize_kernel(const float
 
 // Evaluation: coefficients straight from the running statistics (batch_norm_eval.comp:24-29).
 __global__ void bn_eval_coef_kernel(int c, BnForwardVectors v, float4* coef) {
+  wait_previous();
   const int ch = blockIdx.x * blockDim.x + threadIdx.x;
   if (ch >= c) return;
   const float mean = v.running_mean[ch * v.rm_stride];
@@ -289,6 +293,7 @@ __device__ __forceinline__ float4 post_ops(float4 r, float4 add, int relu) {
 template <bool UNIFORM, bool POST>
 __global__ void __launch_bounds__(kThreads) bn_apply_kernel(const float* __restrict__ x, float* __restrict__ y,
                                                              const float4* __restrict__ coef, uint32_t total, ChannelOf ch, BnPost post) {
+  wait_previous();
   const uint32_t quads = total >> 2, stride = gridDim.x * kThreads;
   const float4* x4 = reinterpret_cast<const float4*>(x);
   const float4* r4 = reinterpret_cast<const float4*>(post.res);
@@ -321,6 +326,7 @@ template <bool POST>
 __global__ void __launch_bounds__(kThreads) bn_apply_cols_kernel(const float* __restrict__ x, float* __restrict__ y,
                                                                   const float4* __restrict__ coef, uint32_t rows, uint32_t c4,
                                                                   uint32_t lanes, BnPost post) {
+  wait_previous();
   const uint32_t t = blockIdx.x * kThreads + threadIdx.x;
   if (t >= lanes) return;
   const uint32_t r0 = t / c4, j = t - r0 * c4;
@@ -349,6 +355,7 @@ __global__ void __launch_bounds__(kThreads) bn_apply_cols_kernel(const float* __
 __global__ void __launch_bounds__(kThreads) bn_apply_scalar_kernel(const float* __restrict__ x, float* __restrict__ y,
                                                                     const float4* __restrict__ coef, uint32_t first, uint32_t total,
                                                                     ChannelOf ch, BnPost post) {
+  wait_previous();
   for (uint64_t i = first + blockIdx.x * (uint64_t)kThreads + threadIdx.x; i < total; i += (uint64_t)gridDim.x * kThreads) {
     float v = normalise(__ldg(x + i), __ldg(coef + ch((uint32_t)i)));
     if (post.res) v += __ldg(post.res + i);
@@ -388,6 +395,7 @@ struct BnBackwardVectors {
 
 __global__ void __launch_bounds__(kThreads, 8) bn_bwd_rows_kernel(const float* __restrict__ x, const float* __restrict__ g, BnShape sh,
                                                                 BnBackwardVectors v, Sums* part) {
+  wait_previous();
   const int ch = blockIdx.x, slab = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int units = sh.outer * sh.segs, per = sh.per;
   const int u0 = slab * per, u1 = min(units, u0 + per);
@@ -430,6 +438,7 @@ __global__ void __launch_bounds__(kThreads, 8) bn_bwd_rows_kernel(const float* _
 template <int V>
 __global__ void __launch_bounds__(kThreads, 5) bn_bwd_cols_kernel(const float* __restrict__ x, const float* __restrict__ g, BnShape sh,
                                                                 BnBackwardVectors v, Sums* part) {
+  wait_previous();
   const int cl = (threadIdx.x & 7) * V, prow = threadIdx.x >> 3, slab = blockIdx.y;
   const int col0 = blockIdx.x * 8 * V + cl;
   const int per = sh.per;
@@ -494,6 +503,7 @@ __global__ void __launch_bounds__(kThreads, 5) bn_bwd_cols_kernel(const float* _
 // has_sums == 0: evaluation mode asked for dx only, nothing was reduced.
 __global__ void __launch_bounds__(kThreads) bn_bwd_finalize_kernel(BnShape sh, const Sums* part, BnBackwardVectors v, int has_sums,
                                                                     float4* coef, float* scale) {
+  wait_previous();
   const int ch = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (ch >= sh.c) return;
   double a = 0.0, b = 0.0, r = 0.0;
@@ -531,6 +541,7 @@ __global__ void __launch_bounds__(kThreads) bn_bwd_finalize_kernel(BnShape sh, c
 // Two values per channel in training mode: the reference switches to the algebraic derivative
 // (batch_norm_backward.comp:24-37), which stays antisymmetric; so does this kernel.
 __global__ void bn_bwd_pair_kernel(const float* __restrict__ x, const float* __restrict__ g, BnShape sh, BnBackwardVectors v, float* dx) {
+  wait_previous();
   const int ch = blockIdx.x * blockDim.x + threadIdx.x;
   if (ch >= sh.c) return;
   const size_t i0 = (size_t)ch * sh.inner;
@@ -559,6 +570,7 @@ template <bool UNIFORM, bool TRAINING>
 __global__ void __launch_bounds__(kThreads) bn_bwd_apply_kernel(const float* __restrict__ x, const float* __restrict__ g,
                                                                  float* __restrict__ dx, const float4* __restrict__ coef,
                                                                  const float* __restrict__ scale, uint32_t total, ChannelOf ch) {
+  wait_previous();
   const uint32_t quads = total >> 2, stride = gridDim.x * kThreads;
   const float4 *x4 = reinterpret_cast<const float4*>(x), *g4 = reinterpret_cast<const float4*>(g);
   float4* d4 = reinterpret_cast<float4*>(dx);
@@ -596,6 +608,7 @@ __global__ void __launch_bounds__(kThreads, 5) bn_bwd_apply_cols_kernel(const fl
                                                                       float* __restrict__ dx, const float4* __restrict__ coef,
                                                                       const float* __restrict__ scale, uint32_t rows, uint32_t c4,
                                                                       uint32_t lanes) {
+  wait_previous();
   const uint32_t t = blockIdx.x * kThreads + threadIdx.x;
   if (t >= lanes) return;
   const uint32_t r0 = t / c4, j = t - r0 * c4;
@@ -624,6 +637,7 @@ __global__ void __launch_bounds__(kThreads) bn_bwd_apply_scalar_kernel(const flo
                                                                         float* __restrict__ dx, const float4* __restrict__ coef,
                                                                         const float* __restrict__ scale, uint32_t first, uint32_t total,
                                                                         ChannelOf ch) {
+  wait_previous();
   for (uint64_t i = first + blockIdx.x * (uint64_t)kThreads + threadIdx.x; i < total; i += (uint64_t)gridDim.x * kThreads) {
     const int c = ch((uint32_t)i);
     dx[i] = input_grad<TRAINING>(TRAINING ? __ldg(x + i) : 0.f, __ldg(g + i), __ldg(coef + c), __ldg(scale + c));
@@ -643,6 +657,7 @@ constexpr int kUnitsBwd = 4;                  // backward: of each of the two te
 template <int VEC, int N>
 __global__ void __launch_bounds__(nres::THREADS, 4) bn_forward_channel_kernel(const float* __restrict__ x, nres::Rows rows, int inner, float m_count,
                                                                            BnForwardVectors v, BnPost post, float* __restrict__ y) {
+  wait_previous();
   auto cluster = nres::cg::this_cluster();
   const int ch = blockIdx.x, rank = (int)cluster.block_rank();
   const uint32_t end = min(rows.units, (uint32_t)(rank + 1) * rows.per), u0 = (uint32_t)rank * rows.per + threadIdx.x;
@@ -688,6 +703,7 @@ __global__ void __launch_bounds__(nres::THREADS, 4) bn_forward_channel_kernel(co
 template <int VEC, int N>
 __global__ void __launch_bounds__(nres::THREADS, 4) bn_backward_channel_kernel(const float* __restrict__ x, const float* __restrict__ g, nres::Rows rows,
                                                                             int inner, float m_count, BnBackwardVectors v, float* __restrict__ dx) {
+  wait_previous();
   auto cluster = nres::cg::this_cluster();
   const int ch = blockIdx.x, rank = (int)cluster.block_rank();
   const uint32_t end = min(rows.units, (uint32_t)(rank + 1) * rows.per), u0 = (uint32_t)rank * rows.per + threadIdx.x;
@@ -876,22 +892,22 @@ int b200_batch_norm_forward_fused(int64_t n, int64_t c, int64_t s, int layout, c
   if (training) {
     if (p.rows) {
       note_kernel("bn_stats_rows+finalize+apply");
-      bn_stats_rows_kernel<<<dim3((unsigned)sh.c, (unsigned)sh.slabs), kThreads, 0, st>>>(x, sh, part);
+      launch_next(bn_stats_rows_kernel, dim3((unsigned)sh.c, (unsigned)sh.slabs), kThreads, 0, st, x, sh, part);
     } else if (sh.cols % 4 == 0 && aligned16(x)) {
       note_kernel("bn_stats_cols+finalize+apply");
-      bn_stats_cols_kernel<4><<<dim3((unsigned)((sh.cols + 31) / 32), (unsigned)sh.slabs), kThreads, 0, st>>>(x, sh, part);
+      launch_next(bn_stats_cols_kernel<4>, dim3((unsigned)((sh.cols + 31) / 32), (unsigned)sh.slabs), kThreads, 0, st, x, sh, part);
     } else {
       note_kernel("bn_stats_cols+finalize+apply");
-      bn_stats_cols_kernel<1><<<dim3((unsigned)((sh.cols + 7) / 8), (unsigned)sh.slabs), kThreads, 0, st>>>(x, sh, part);
+      launch_next(bn_stats_cols_kernel<1>, dim3((unsigned)((sh.cols + 7) / 8), (unsigned)sh.slabs), kThreads, 0, st, x, sh, part);
     }
     count_launch();
     if (int rc = launch_check("bn_stats_kernel")) return rc;
-    bn_stats_finalize_kernel<<<(sh.c + 7) / 8, kThreads, 0, st>>>(x, sh, part, v, coef);
+    launch_next(bn_stats_finalize_kernel, (sh.c + 7) / 8, kThreads, 0, st, x, sh, part, v, coef);
     count_launch();
     if (int rc = launch_check("bn_stats_finalize_kernel")) return rc;
   } else {
     note_kernel("bn_eval_coef+apply");
-    bn_eval_coef_kernel<<<(sh.c + 127) / 128, 128, 0, st>>>(sh.c, v, coef);
+    launch_next(bn_eval_coef_kernel, (sh.c + 127) / 128, 128, 0, st, sh.c, v, coef);
     count_launch();
     if (int rc = launch_check("bn_eval_coef_kernel")) return rc;
   }
@@ -906,25 +922,25 @@ int b200_batch_norm_forward_fused(int64_t n, int64_t c, int64_t s, int layout, c
       const uint32_t c4 = (uint32_t)sh.c / 4, threads = (uint32_t)grid * kThreads;
       const uint32_t lanes = c4 ? threads / c4 * c4 : 0;
       if (sh.inner == 1 && sh.c % 4 == 0 && threads >= c4) {
-        if (fused) bn_apply_cols_kernel<true><<<grid, kThreads, 0, st>>>(x, y, coef, (uint32_t)sh.outer, c4, lanes, post);
-        else bn_apply_cols_kernel<false><<<grid, kThreads, 0, st>>>(x, y, coef, (uint32_t)sh.outer, c4, lanes, post);
+        if (fused) launch_next(bn_apply_cols_kernel<true>, grid, kThreads, 0, st, x, y, coef, (uint32_t)sh.outer, c4, lanes, post);
+        else launch_next(bn_apply_cols_kernel<false>, grid, kThreads, 0, st, x, y, coef, (uint32_t)sh.outer, c4, lanes, post);
       } else if (uniform) {
-        if (fused) bn_apply_kernel<true, true><<<grid, kThreads, 0, st>>>(x, y, coef, total, channel_of(sh, true), post);
-        else bn_apply_kernel<true, false><<<grid, kThreads, 0, st>>>(x, y, coef, total, channel_of(sh, true), post);
+        if (fused) launch_next(bn_apply_kernel<true, true>, grid, kThreads, 0, st, x, y, coef, total, channel_of(sh, true), post);
+        else launch_next(bn_apply_kernel<true, false>, grid, kThreads, 0, st, x, y, coef, total, channel_of(sh, true), post);
       } else {
-        if (fused) bn_apply_kernel<false, true><<<grid, kThreads, 0, st>>>(x, y, coef, total, channel_of(sh, false), post);
-        else bn_apply_kernel<false, false><<<grid, kThreads, 0, st>>>(x, y, coef, total, channel_of(sh, false), post);
+        if (fused) launch_next(bn_apply_kernel<false, true>, grid, kThreads, 0, st, x, y, coef, total, channel_of(sh, false), post);
+        else launch_next(bn_apply_kernel<false, false>, grid, kThreads, 0, st, x, y, coef, total, channel_of(sh, false), post);
       }
       count_launch();
       if (int rc = launch_check("bn_apply_kernel")) return rc;
     }
     if (total & 3) {
-      bn_apply_scalar_kernel<<<1, kThreads, 0, st>>>(x, y, coef, total & ~3u, total, channel_of(sh, false), post);
+      launch_next(bn_apply_scalar_kernel, 1, kThreads, 0, st, x, y, coef, total & ~3u, total, channel_of(sh, false), post);
       count_launch();
       if (int rc = launch_check("bn_apply_scalar_kernel")) return rc;
     }
   } else {
-    bn_apply_scalar_kernel<<<apply_grid(total), kThreads, 0, st>>>(x, y, coef, 0, total, channel_of(sh, false), post);
+    launch_next(bn_apply_scalar_kernel, apply_grid(total), kThreads, 0, st, x, y, coef, 0, total, channel_of(sh, false), post);
     count_launch();
     if (int rc = launch_check("bn_apply_scalar_kernel")) return rc;
   }
@@ -952,7 +968,7 @@ int b200_batch_norm_backward(int64_t n, int64_t c, int64_t s, int layout, const 
   const uint32_t total = (uint32_t)((int64_t)sh.outer * sh.cols);
   if (training && n * s == 2) {
     note_kernel("bn_bwd_pair");
-    bn_bwd_pair_kernel<<<(sh.c + 127) / 128, 128, 0, st>>>(x, grad, sh, v, dx);
+    launch_next(bn_bwd_pair_kernel, (sh.c + 127) / 128, 128, 0, st, x, grad, sh, v, dx);
     count_launch();
     return launch_check("bn_bwd_pair_kernel");
   }
@@ -968,17 +984,17 @@ int b200_batch_norm_backward(int64_t n, int64_t c, int64_t s, int layout, const 
   }
   if (has_sums) {
     if (p.rows) {
-      bn_bwd_rows_kernel<<<dim3((unsigned)sh.c, (unsigned)sh.slabs), kThreads, 0, st>>>(x, grad, sh, v, part);
+      launch_next(bn_bwd_rows_kernel, dim3((unsigned)sh.c, (unsigned)sh.slabs), kThreads, 0, st, x, grad, sh, v, part);
     } else if (sh.cols % 4 == 0 && aligned16(x) && aligned16(grad)) {
-      bn_bwd_cols_kernel<4><<<dim3((unsigned)((sh.cols + 31) / 32), (unsigned)sh.slabs), kThreads, 0, st>>>(x, grad, sh, v, part);
+      launch_next(bn_bwd_cols_kernel<4>, dim3((unsigned)((sh.cols + 31) / 32), (unsigned)sh.slabs), kThreads, 0, st, x, grad, sh, v, part);
     } else {
-      bn_bwd_cols_kernel<1><<<dim3((unsigned)((sh.cols + 7) / 8), (unsigned)sh.slabs), kThreads, 0, st>>>(x, grad, sh, v, part);
+      launch_next(bn_bwd_cols_kernel<1>, dim3((unsigned)((sh.cols + 7) / 8), (unsigned)sh.slabs), kThreads, 0, st, x, grad, sh, v, part);
     }
     count_launch();
     if (int rc = launch_check("bn_bwd_reduce_kernel")) return rc;
   }
   note_kernel(has_sums ? (p.rows ? "bn_bwd_rows+finalize+apply" : "bn_bwd_cols+finalize+apply") : "bn_bwd_finalize+apply");
-  bn_bwd_finalize_kernel<<<(sh.c + 7) / 8, kThreads, 0, st>>>(sh, part, v, has_sums, coef, scale);
+  launch_next(bn_bwd_finalize_kernel, (sh.c + 7) / 8, kThreads, 0, st, sh, part, v, has_sums, coef, scale);
   count_launch();
   if (int rc = launch_check("bn_bwd_finalize_kernel")) return rc;
   if (!dx) return B200_OK;
@@ -991,14 +1007,14 @@ int b200_batch_norm_backward(int64_t n, int64_t c, int64_t s, int layout, const 
     const uint32_t c4 = (uint32_t)sh.c / 4, threads = (uint32_t)grid * kThreads;
     if (sh.inner == 1 && sh.c % 4 == 0 && threads >= c4) {
       const uint32_t lanes = threads / c4 * c4;
-      if (training) bn_bwd_apply_cols_kernel<true><<<grid, kThreads, 0, st>>>(x, grad, dx, coef, scale, (uint32_t)sh.outer, c4, lanes);
-      else bn_bwd_apply_cols_kernel<false><<<grid, kThreads, 0, st>>>(x, grad, dx, coef, scale, (uint32_t)sh.outer, c4, lanes);
+      if (training) launch_next(bn_bwd_apply_cols_kernel<true>, grid, kThreads, 0, st, x, grad, dx, coef, scale, (uint32_t)sh.outer, c4, lanes);
+      else launch_next(bn_bwd_apply_cols_kernel<false>, grid, kThreads, 0, st, x, grad, dx, coef, scale, (uint32_t)sh.outer, c4, lanes);
     } else if (training) {
-      if (uniform) bn_bwd_apply_kernel<true, true><<<grid, kThreads, 0, st>>>(x, grad, dx, coef, scale, total, ch);
-      else bn_bwd_apply_kernel<false, true><<<grid, kThreads, 0, st>>>(x, grad, dx, coef, scale, total, ch);
+      if (uniform) launch_next(bn_bwd_apply_kernel<true, true>, grid, kThreads, 0, st, x, grad, dx, coef, scale, total, ch);
+      else launch_next(bn_bwd_apply_kernel<false, true>, grid, kThreads, 0, st, x, grad, dx, coef, scale, total, ch);
     } else {
-      if (uniform) bn_bwd_apply_kernel<true, false><<<grid, kThreads, 0, st>>>(x, grad, dx, coef, scale, total, ch);
-      else bn_bwd_apply_kernel<false, false><<<grid, kThreads, 0, st>>>(x, grad, dx, coef, scale, total, ch);
+      if (uniform) launch_next(bn_bwd_apply_kernel<true, false>, grid, kThreads, 0, st, x, grad, dx, coef, scale, total, ch);
+      else launch_next(bn_bwd_apply_kernel<false, false>, grid, kThreads, 0, st, x, grad, dx, coef, scale, total, ch);
     }
     count_launch();
     if (int rc = launch_check("bn_bwd_apply_kernel")) return rc;
@@ -1006,8 +1022,8 @@ int b200_batch_norm_backward(int64_t n, int64_t c, int64_t s, int layout, const 
   if (first_scalar < total) {
     const int grid = vec ? 1 : apply_grid(total);
     const ChannelOf ch = channel_of(sh, false);
-    if (training) bn_bwd_apply_scalar_kernel<true><<<grid, kThreads, 0, st>>>(x, grad, dx, coef, scale, first_scalar, total, ch);
-    else bn_bwd_apply_scalar_kernel<false><<<grid, kThreads, 0, st>>>(x, grad, dx, coef, scale, first_scalar, total, ch);
+    if (training) launch_next(bn_bwd_apply_scalar_kernel<true>, grid, kThreads, 0, st, x, grad, dx, coef, scale, first_scalar, total, ch);
+    else launch_next(bn_bwd_apply_scalar_kernel<false>, grid, kThreads, 0, st, x, grad, dx, coef, scale, first_scalar, total, ch);
     count_launch();
     if (int rc = launch_check("bn_bwd_apply_scalar_kernel")) return rc;
   }

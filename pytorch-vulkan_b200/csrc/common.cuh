@@ -32,6 +32,23 @@ inline void count_launch(int n = 1) { g_launches.fetch_add((uint64_t)n, std::mem
 // Checks the launch of the kernel named `what`; to be used right after <<<>>>.
 int launch_check(const char* what);
 
+// A launch that may start while the kernel ahead of it on the stream finishes: every such kernel calls wait_previous() before its first
+// access to memory that another kernel writes or reads, which waits for all of that kernel's work.  Between two short kernels the
+// ordinary boundary costs 1.5 to 2 us (batch norm of 64x256x14x14, forward and backward: 22.6 -> 18.8 us).  Errors stay for launch_check().
+template <typename... P, typename... A>
+void launch_next(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr; cfg.numAttrs = 1;
+  (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<A&&>(args)...);
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+#endif
+
 // ---- device-side geometry ------------------------------------------------------------------
 struct View4 {
   const float* ptr;

@@ -42,6 +42,7 @@ struct GArgs {
 // 32 x 32 for maps up to 32 columns, so that no thread idles on padding).
 template <int CPG, int SX>
 __global__ void __launch_bounds__(THREADS) gconv_fwd_kernel(const GArgs a) {
+  wait_previous();
   constexpr int TWK = 4 * SX, THK = THREADS / SX;         // tile extent
   constexpr int IWK = TWK + 4, IHK = THK + 2;              // with halo; rows padded to a multiple of 4 floats
   __shared__ __align__(16) float s_in[CPG][IHK][IWK];
@@ -178,6 +179,7 @@ __device__ __forceinline__ void cp_async4(float* dst, const float* src, bool ok)
 
 template <int CPG>
 __global__ void __launch_bounds__(DW_THREADS, 3) gconv_dw_kernel(const GdwArgs a) {
+  wait_previous();
   constexpr int NQ = CPG * CPG / 8;             // 4 x 2 channel blocks of a group
   constexpr int STRIPS = DW_THREADS / NQ;       // strips per tile
   constexpr int SX = 4, TR = STRIPS / SX, TW = 8 * SX;   // strips per row, rows, columns
@@ -365,11 +367,11 @@ int group_small_conv(const ConvGeom& g, bool is_dx, View4 in, View4 w, const flo
   if (blocks > 2147483647ll) return fail(B200_ERANGE, "grouped convolution: grid exceeds launch limits");
   const unsigned nb = (unsigned)blocks;
   if (g.cig == 4) {
-    if (narrow) gcs::gconv_fwd_kernel<4, 8><<<nb, gcs::THREADS, 0, st>>>(a);
-    else gcs::gconv_fwd_kernel<4, 16><<<nb, gcs::THREADS, 0, st>>>(a);
+    if (narrow) launch_next(gcs::gconv_fwd_kernel<4, 8>, nb, gcs::THREADS, 0, st, a);
+    else launch_next(gcs::gconv_fwd_kernel<4, 16>, nb, gcs::THREADS, 0, st, a);
   } else {
-    if (narrow) gcs::gconv_fwd_kernel<8, 8><<<nb, gcs::THREADS, 0, st>>>(a);
-    else gcs::gconv_fwd_kernel<8, 16><<<nb, gcs::THREADS, 0, st>>>(a);
+    if (narrow) launch_next(gcs::gconv_fwd_kernel<8, 8>, nb, gcs::THREADS, 0, st, a);
+    else launch_next(gcs::gconv_fwd_kernel<8, 16>, nb, gcs::THREADS, 0, st, a);
   }
   count_launch();
   return launch_check("gconv_fwd_kernel");
@@ -385,8 +387,8 @@ int group_small_dweight(const ConvGeom& g, View4 x, View4 dy, float* dw, float* 
     return fail(B200_EWORKSPACE, "grouped dWeight needs a workspace of %zu bytes (got %zu)", need, ws_bytes);
   a.partial = a.blocks_per_group > 1 ? ws : dw;   // one block per group writes dW directly ([cout][cig][9])
   const long long blocks = (long long)g.groups * a.blocks_per_group;
-  if (g.cig == 4) gcs::gconv_dw_kernel<4><<<(unsigned)blocks, gcs::DW_THREADS, 0, st>>>(a);
-  else gcs::gconv_dw_kernel<8><<<(unsigned)blocks, gcs::DW_THREADS, 0, st>>>(a);
+  if (g.cig == 4) launch_next(gcs::gconv_dw_kernel<4>, (unsigned)blocks, gcs::DW_THREADS, 0, st, a);
+  else launch_next(gcs::gconv_dw_kernel<8>, (unsigned)blocks, gcs::DW_THREADS, 0, st, a);
   count_launch();
   if (int rc = launch_check("gconv_dw_kernel")) return rc;
   if (a.blocks_per_group > 1) return finalize_splits(ws, dw, count, a.blocks_per_group, st);

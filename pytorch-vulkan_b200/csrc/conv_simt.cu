@@ -162,6 +162,7 @@ constexpr int BM = 64, BN = 64, BK = 16;
 
 template <int PH>
 __global__ void __launch_bounds__(256) simt_igemm_kernel(const IgemmArgs p) {
+  wait_previous();
   __shared__ __align__(16) float As[BK][BM + 4];
   __shared__ __align__(16) float Bs[BK][BN + 4];
   const int tid = threadIdx.x;
@@ -228,7 +229,7 @@ static int launch_igemm(const IgemmArgs& p, int groups, int splits, cudaStream_t
   const long long gx = div_up64(p.N, BN), gy = div_up64(p.M, BM) * groups;
   if (gx > 2147483647ll || gy > 65535 || splits > 65535)
     return fail(B200_ERANGE, "%s: grid (%lld,%lld,%d) exceeds launch limits", name, gx, gy, splits);
-  simt_igemm_kernel<PH><<<dim3((unsigned)gx, (unsigned)gy, (unsigned)splits), 256, 0, st>>>(p);
+  launch_next(simt_igemm_kernel<PH>, dim3((unsigned)gx, (unsigned)gy, (unsigned)splits), 256, 0, st, p);
   count_launch();
   return launch_check(name);
 }
@@ -254,6 +255,7 @@ int simt_igemm_dinput(const ConvGeom& g, View4 dy, View4 w, float* dx, cudaStrea
 template <int SLICES>
 __global__ void __launch_bounds__(256) finalize_kernel(const float* __restrict__ partial, float* __restrict__ out,
                                                        long long count, int splits) {
+  wait_previous();
   constexpr int VALUES = 256 / SLICES;
   const int v = threadIdx.x % VALUES, slice = threadIdx.x / VALUES;
   const long long i = (long long)blockIdx.x * VALUES + v;
@@ -284,8 +286,8 @@ __global__ void __launch_bounds__(256) finalize_kernel(const float* __restrict__
 
 int finalize_splits(const float* partial, float* out, long long count, int splits, cudaStream_t st) {
   // eight slices while one thread per value would leave most of the machine idle (two CTAs of 256 per SM)
-  if (splits >= 16 && count < 512ll * sm_count()) finalize_kernel<8><<<(unsigned)div_up64(count, 32), 256, 0, st>>>(partial, out, count, splits);
-  else finalize_kernel<1><<<(unsigned)div_up64(count, 256), 256, 0, st>>>(partial, out, count, splits);
+  if (splits >= 16 && count < 512ll * sm_count()) launch_next(finalize_kernel<8>, (unsigned)div_up64(count, 32), 256, 0, st, partial, out, count, splits);
+  else launch_next(finalize_kernel<1>, (unsigned)div_up64(count, 256), 256, 0, st, partial, out, count, splits);
   count_launch();
   return launch_check("finalize_kernel");
 }

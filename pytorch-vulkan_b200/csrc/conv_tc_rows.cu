@@ -66,6 +66,7 @@ struct RunEntry {
 
 template <int LP, bool UNIT>
 __global__ void __launch_bounds__(THREADS, 1) conv_rows_kernel(const RowsArgs a) {
+  wait_previous();
   extern __shared__ unsigned char smem_raw[];
   const ConvGeom& g = a.g;
   const uint32_t raw = smem_u32(smem_raw), w_base = (raw + 1023u) & ~1023u;
@@ -328,7 +329,7 @@ static int launch_rows(const RowsArgs& a, int smem, cudaStream_t st) {
   static cudaError_t opt_in = cudaSuccess;
   std::call_once(once, [] { opt_in = cudaFuncSetAttribute(conv_rows_kernel<LP, UNIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448); });
   B200_CUDA(opt_in);
-  conv_rows_kernel<LP, UNIT><<<(unsigned)(std::min(a.tiles_m, std::max(1, sm_count() / a.nt_split)) * a.nt_split), THREADS, (size_t)smem, st>>>(a);
+  launch_next(conv_rows_kernel<LP, UNIT>, (unsigned)(std::min(a.tiles_m, std::max(1, sm_count() / a.nt_split)) * a.nt_split), THREADS, (size_t)smem, st, a);
   count_launch();
   return launch_check("conv_rows_kernel");
 }

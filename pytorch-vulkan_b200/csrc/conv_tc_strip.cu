@@ -626,6 +626,7 @@ __global__ void __launch_bounds__(256) stage_weights_kernel(ConvGeom g, View4 w,
                                                             TapTable tt, float* __restrict__ out, long long total,
                                                             long long w_group_extra, int k_total, int rows_first, int per_thread) {
   // let the convolution kernel behind this one start its prologue and its activation strips now
+  wait_previous();
   asm volatile("griddepcontrol.launch_dependents;");
   const long long i = blockIdx.x * 256ll + threadIdx.x;  // [group][tile][channel block][row, piece]
   if (i >= total) return;
@@ -859,7 +860,7 @@ int strip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* b
     const int taps = plan.tt.taps_total;
     const long long threads = wcount / taps / 4;
     const int per_thread = staged_taps(threads, taps);
-    stage_weights_kernel<<<dim3((unsigned)div_up64(threads, 256), (unsigned)((taps + per_thread - 1) / per_thread)), 256, 0, st>>>(
+    launch_next(stage_weights_kernel, dim3((unsigned)div_up64(threads, 256), (unsigned)((taps + per_thread - 1) / per_thread)), 256, 0, st, 
         g, w, is_dx ? 1 : 0, plan.bn, tiles_pp, plan.tt, (float*)ws, threads, batch ? batch->w_group_extra : 0, k_total,
         std::llabs(is_dx ? w.s1 : w.s0) < std::llabs(is_dx ? w.s0 : w.s1) ? 1 : 0, per_thread);
     count_launch();

@@ -459,6 +459,7 @@ __global__ void __launch_bounds__(tstrip_threads(AW), 1) conv_tstrip_kernel(cons
 __global__ void __launch_bounds__(256) stage_filter16_kernel(ConvGeom g, View4 w, int is_dx, int tiles_pp, TapTable tt,
                                                              unsigned char* __restrict__ out, long long total, long long w_group_extra,
                                                              int rows_first, int per_thread) {
+  wait_previous();
   asm volatile("griddepcontrol.launch_dependents;");
   const long long i = blockIdx.x * 256ll + threadIdx.x;   // [group][channel tile][channel block][row, piece], as stage_weights_kernel
   if (i >= total) return;
@@ -591,7 +592,7 @@ int tstrip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* 
   const int taps = plan.geo.tt.taps_total;
   const long long threads = plan.images / taps * TM * 4;
   const int per_thread = tcs::staged_taps(threads, taps);
-  stage_filter16_kernel<<<dim3((unsigned)div_up64(threads, 256), (unsigned)((taps + per_thread - 1) / per_thread)), 256, 0, st>>>(
+  launch_next(stage_filter16_kernel, dim3((unsigned)div_up64(threads, 256), (unsigned)((taps + per_thread - 1) / per_thread)), 256, 0, st, 
       g, w, is_dx ? 1 : 0, plan.tiles_pp, plan.geo.tt, (unsigned char*)ws, threads, w_group_extra,
       std::llabs(is_dx ? w.s1 : w.s0) < std::llabs(is_dx ? w.s0 : w.s1) ? 1 : 0, per_thread);
   count_launch();

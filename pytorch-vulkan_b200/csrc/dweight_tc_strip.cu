@@ -171,6 +171,7 @@ __device__ __noinline__ bool fold_accumulator(FoldArgs f, int c, bool more) {
 
 template <int BN, bool DW_CROSS>
 __global__ void __launch_bounds__(THREADS, 1) dweight_strip_kernel(const DwStripArgs a) {
+  wait_previous();
   extern __shared__ unsigned char smem_raw[];
   const unsigned long long prof_start = a.prof ? global_ns() : 0;
   // the pass that sums the split partials may take its place on the SMs now (it waits for this grid to finish)
@@ -663,7 +664,7 @@ static int launch_dw_strip(const tcdw::DwStripArgs& a, dim3 grid, int smem, cuda
   static cudaError_t opt_in = cudaSuccess;
   std::call_once(once, [] { opt_in = cudaFuncSetAttribute(tcdw::dweight_strip_kernel<BN, CROSS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448); });
   B200_CUDA(opt_in);
-  tcdw::dweight_strip_kernel<BN, CROSS><<<grid, tcdw::THREADS, smem, st>>>(a);
+  launch_next(tcdw::dweight_strip_kernel<BN, CROSS>, grid, tcdw::THREADS, smem, st, a);
   count_launch();
   return launch_check("dweight_strip_kernel");
 }

@@ -122,6 +122,7 @@ __device__ __forceinline__ uint64_t desc64(uint32_t lo, uint32_t hi) {
 // known, the issuing warp needs 175 clocks less per K block of a 3x3 filter.
 template <int NG, int NB, bool FOLD>
 __global__ void __launch_bounds__(THREADS, 1) dweight_tmem_kernel(const Args a) {
+  wait_previous();
   constexpr int GROUPS = NG ? NG : MAX_GROUPS;
   extern __shared__ unsigned char smem_raw[];
   if (a.partial_layout) asm volatile("griddepcontrol.launch_dependents;");
@@ -677,7 +678,7 @@ static int launch(const Args& a, const Plan& p, cudaStream_t st) {
   static cudaError_t opt_in = cudaSuccess;
   std::call_once(once, [] { opt_in = cudaFuncSetAttribute(dweight_tmem_kernel<NG, NB, FOLD>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448); });
   B200_CUDA(opt_in);
-  dweight_tmem_kernel<NG, NB, FOLD><<<dim3((unsigned)p.tiles, (unsigned)a.splits), THREADS, (size_t)p.smem, st>>>(a);
+  launch_next(dweight_tmem_kernel<NG, NB, FOLD>, dim3((unsigned)p.tiles, (unsigned)a.splits), THREADS, (size_t)p.smem, st, a);
   count_launch();
   return launch_check("dweight_tmem_kernel");
 }

@@ -148,6 +148,7 @@ __global__ void __launch_bounds__(kThreads, 3) gn_forward_kernel(const float* __
                                                                  const float* __restrict__ beta, GnShape sh, float eps,
                                                                  float* __restrict__ y, float* __restrict__ means,
                                                                  float* __restrict__ rstds) {
+  wait_previous();
   const int row = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int group = row % sh.groups;
   const size_t base = ((size_t)(row / sh.groups) * sh.c + (size_t)group * sh.cpg) * sh.hw;
@@ -207,6 +208,7 @@ __global__ void __launch_bounds__(kBulkThreads, 1) gn_forward_bulk_kernel(const 
                                                                       float* __restrict__ y, float* __restrict__ means,
                                                                       float* __restrict__ rstds, int blocks, FastDiv plane_quads,
                                                                       int* status) {
+  wait_previous();
   extern __shared__ __align__(128) unsigned char gn_smem[];
   __shared__ __align__(8) unsigned long long full[2];
   __shared__ int abort_flag;
@@ -297,6 +299,7 @@ __global__ void __launch_bounds__(kThreads, 3) gn_backward_kernel(const float* _
                                                                   const float* __restrict__ means, const float* __restrict__ rstds,
                                                                   const float* __restrict__ gamma, GnShape sh, float* __restrict__ dx,
                                                                   float* __restrict__ plane_sums) {
+  wait_previous();
   extern __shared__ float unit_sums[];  // [units][2]
   __shared__ float totals[2];
   const int row = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -367,6 +370,7 @@ __global__ void __launch_bounds__(nres::THREADS, 4) gn_forward_cluster_kernel(co
                                                                            const float* __restrict__ beta, GnShape sh, nres::Rows rows, float eps,
                                                                            float* __restrict__ y, float* __restrict__ means,
                                                                            float* __restrict__ rstds) {
+  wait_previous();
   auto cluster = nres::cg::this_cluster();
   const int row = blockIdx.x, rank = (int)cluster.block_rank();
   const int ch0 = row % sh.groups * sh.cpg;
@@ -402,6 +406,7 @@ __global__ void __launch_bounds__(nres::THREADS, 4) gn_backward_cluster_kernel(c
                                                                             const float* __restrict__ means, const float* __restrict__ rstds,
                                                                             const float* __restrict__ gamma, GnShape sh, nres::Rows rows,
                                                                             float* __restrict__ dx, float* __restrict__ plane_sums) {
+  wait_previous();
   auto cluster = nres::cg::this_cluster();
   __shared__ float2 unit_part[N * nres::THREADS];
   __shared__ float2 plane_part[kResidentChannels];                     // of this rank
@@ -555,7 +560,7 @@ int b200_group_norm_forward(int64_t n, int64_t c, int64_t hw, int64_t groups, co
     });
     B200_CUDA(opt_in);
     note_kernel("gn_forward_bulk");
-    gn_forward_bulk_kernel<<<bulk_grid, kBulkThreads, 2 * block_bytes, st>>>(x, weight, bias, sh, eps, y, mean, rstd, blocks,
+    launch_next(gn_forward_bulk_kernel, bulk_grid, kBulkThreads, 2 * block_bytes, st, x, weight, bias, sh, eps, y, mean, rstd, blocks,
                                                                             FastDiv((uint32_t)(sh.hw / 4)), device_status_word());
     count_launch();
     return launch_check("gn_forward_bulk_kernel");
@@ -565,7 +570,7 @@ int b200_group_norm_forward(int64_t n, int64_t c, int64_t hw, int64_t groups, co
   if (const int ranks = nres::ranks_for((long long)sh.cpg * sh.hw / vec, blocks, vec == 4 ? kUnits : kUnits1))
     return nres::launch(vec == 4 ? gn_forward_cluster_kernel<4, kUnits> : gn_forward_cluster_kernel<1, kUnits1>, (unsigned)blocks, ranks, st, x, weight, bias,
                         sh, nres::make_rows(sh.cpg, sh.hw, vec, sh.hw, ranks), eps, y, mean, rstd);
-  gn_forward_kernel<<<(unsigned)(n * groups), kThreads, 0, st>>>(x, weight, bias, sh, eps, y, mean, rstd);
+  launch_next(gn_forward_kernel, (unsigned)(n * groups), kThreads, 0, st, x, weight, bias, sh, eps, y, mean, rstd);
   count_launch();
   return launch_check("gn_forward_kernel");
 }
@@ -593,7 +598,7 @@ int b200_group_norm_backward(int64_t n, int64_t c, int64_t hw, int64_t groups, c
                               x, mean, rstd, weight, sh, rows, dx, plane_sums))
       return rc;
   } else {
-    gn_backward_kernel<<<(unsigned)blocks, kThreads, (size_t)sh.units * 2 * sizeof(float), st>>>(grad, x, mean, rstd, weight, sh, dx, plane_sums);
+    launch_next(gn_backward_kernel, (unsigned)blocks, kThreads, (size_t)sh.units * 2 * sizeof(float), st, grad, x, mean, rstd, weight, sh, dx, plane_sums);
     count_launch();
     if (int rc = launch_check("gn_backward_kernel")) return rc;
   }

@@ -41,6 +41,7 @@ __device__ __forceinline__ float add4(const float4& v) { return (v.x + v.y) + (v
 template <bool VEC, bool DENSE>
 __global__ void __launch_bounds__(THREADS) reduce_planes_kernel(const float* __restrict__ src, long long chan_stride, Rows rows, uint32_t count,
                                                                 float* __restrict__ out, int accumulate) {
+  wait_previous();
   cg::cluster_group cluster = cg::this_cluster();
   const uint32_t ranks = cluster.num_blocks(), rank = cluster.block_rank();
   const float* base = src + (long long)blockIdx.x * chan_stride;
@@ -84,6 +85,7 @@ __global__ void __launch_bounds__(THREADS) reduce_planes_kernel(const float* __r
 template <int LPR, bool VEC, bool DENSE>
 __global__ void __launch_bounds__(COL_THREADS) reduce_columns_kernel(const float* __restrict__ src, Rows rows, uint32_t count, int cols,
                                                                  float* __restrict__ out, int accumulate) {
+  wait_previous();
   cg::cluster_group cluster = cg::this_cluster();
   const uint32_t cluster_ranks = cluster.num_blocks(), cluster_rank = cluster.block_rank();
   const uint32_t ranks = cluster_ranks * gridDim.z, rank = blockIdx.z * cluster_ranks + cluster_rank;   // shares of the rows
@@ -145,10 +147,12 @@ static int launch_cluster(void (*kernel)(P...), unsigned blocks, int ranks, int 
   if (ranks > 8) B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(blocks, (unsigned)ranks, (unsigned)slabs); cfg.blockDim = dim3(KERNEL_THREADS); cfg.stream = st;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = 1; attr.val.clusterDim.y = (unsigned)ranks; attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr; cfg.numAttrs = 1;
+  cudaLaunchAttribute attr[2] = {};
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = (unsigned)ranks; attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as launch_next()
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = 2;
   B200_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
   count_launch();
   return launch_check("reduce kernel");
