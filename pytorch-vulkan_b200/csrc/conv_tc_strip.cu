@@ -51,8 +51,8 @@ namespace tcs {
 using namespace tc;
 
 constexpr int BLOCK_M = 128, KBLK = 32;
-// Warp roles: 4 epilogue warps, AW strip producers, the weight-copy warp, the MMA warp.  AW is 8, or 16 for layers
-// whose producers set the pace (one tap per staged strip: 1x1 filters): twice the loads in flight per SM.
+// Warp roles: 4 epilogue warps, AW strip producers, the weight-copy warp, the MMA warp.  AW is 8, or 12 for layers
+// whose producers set the pace (one tap per staged strip: 1x1 filters), which fetch a job ahead; sixteen had no registers for that.
 constexpr int EPI_WARPS = 4, W_WARPS = 1;
 constexpr int strip_threads(int aw) { return (EPI_WARPS + aw + W_WARPS + 1) * 32; }
 constexpr int MAX_STAGES = 4;
@@ -92,7 +92,7 @@ struct StripArgs {
   int a_stages, w_stages;
   int out_rowmajor;       // 0: NCHW planes.  1: [pixel][channel] rows (channels-last / GEMM C)
   int out_vec4;           // row-major rows may be written with 16-byte stores
-  int wide_producers;     // 1: the kernel instance with sixteen producer warps
+  int wide_producers;     // 1: the kernel instance with twelve producer warps
   float alpha, beta;      // out = alpha * acc + beta * bias
   View4 res;              // optional residual added after the bias (logical shape of the output), ptr null = none
   int relu;               // clamp at zero last
@@ -361,7 +361,6 @@ __global__ void __launch_bounds__(strip_threads(AW), 1) conv_strip_kernel(const 
     const int chunks = (a.strip_rows + 31) / 32;
     const bool vec_layout = a.act.s1 == 1 && a.kc % 4 == 0 && ((reinterpret_cast<uintptr_t>(a.act.ptr) & 15) == 0) &&
                         (a.act.s0 % 4 == 0) && (a.act.s2 % 4 == 0) && (a.act.s3 % 4 == 0) && (a.act_group_extra % 4 == 0);
-    const bool chunked_layout = vec_layout;
     const int s1 = (int)a.act.s1;
     const int my_units = a.units > (int)blockIdx.x ? (a.units - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
     const int my_tiles = my_units * a.unit;
@@ -369,7 +368,10 @@ __global__ void __launch_bounds__(strip_threads(AW), 1) conv_strip_kernel(const 
     // A warp's consecutive jobs must not be more than a_stages stages apart: a waiter that skips a
     // whole phase of a stage's mbarrier would see the parity of an older phase and run ahead.
     const int a_warps = min(A_WARPS, chunks * a.a_stages);
-    for (int job = aw; job < total_jobs && aw < a_warps; job += a_warps) {
+    // A job's loads are issued before the previous job is converted and stored: a warp that waited for its own loads first
+    // left the tensor core idle for a third of the time where one strip feeds one tap (16384x1024 x 1024x1024: 155 -> 144 us).
+    struct Job { int chunk; uint32_t as, round; bool chunked; };
+    auto fetch = [&](int job, float (&v)[KBLK]) -> Job {
       const uint32_t a_count = a.div_chunks.div((uint32_t)job);
       const int chunk = job - (int)a_count * chunks;
       const uint32_t tile_iter = a.div_cblocks.div(a_count);
@@ -380,8 +382,6 @@ __global__ void __launch_bounds__(strip_threads(AW), 1) conv_strip_kernel(const 
       const int group = tc_.group, m_tile = tc_.m_tile;
       const uint32_t a_round = a.div_a_stages.div(a_count);
       const uint32_t as = a_count - a_round * a.a_stages;
-      const bool pa = PROF_ON(threadIdx.x == EPI_WARPS * 32);
-      PROF_T0(pa);
       const int r = chunk * 32 + lane;
       const int q = m_tile * BLOCK_M - a.halo + r;
       bool ok = r < a.strip_rows && q >= 0 && q < a.q_total;
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(strip_threads(AW), 1) conv_strip_kernel(const 
       // the last channel block of a group may be ragged (channel counts that are no multiple of 32):
       // it takes the masked one-value-per-load path, channels beyond the group read as zero
       const int nvalid = min(KBLK, min(a.kc, a.k_total - group * a.kc) - cbl * KBLK);
-      const bool chunked = chunked_layout && nvalid == KBLK, vec_ok = vec_layout && nvalid == KBLK;
+      const bool chunked = vec_layout && nvalid == KBLK;
       if (ok) {
         const int n = (int)a.img_div.div((uint32_t)q);
         const int rem = q - n * img_pitch;
@@ -400,7 +400,6 @@ __global__ void __launch_bounds__(strip_threads(AW), 1) conv_strip_kernel(const 
         src += n * a.act.s0 + ((long long)group * a.kc + cbl * KBLK) * a.act.s1 + (long long)iy * a.act.s2 + (long long)ix * a.act.s3 +
                (long long)group * a.act_group_extra;
       }
-      float v[KBLK];
       if (chunked) {
         // Channels-last: the 32 channels of a pixel are 128 contiguous bytes.  Eight lanes fetch one
         // pixel (16 bytes each), so a load instruction covers four whole rows; lane r computed row r's
@@ -412,31 +411,23 @@ __global__ void __launch_bounds__(strip_threads(AW), 1) conv_strip_kernel(const 
           const float4 f = ps ? __ldg(ps + (lane & 7)) : make_float4(0.f, 0.f, 0.f, 0.f);
           v[4 * i] = f.x; v[4 * i + 1] = f.y; v[4 * i + 2] = f.z; v[4 * i + 3] = f.w;
         }
-      } else if (vec_ok) {
-        // wide pixels (1 KB apart and more): measured faster with one pixel per lane
-#pragma unroll
-        for (int j = 0; j < KBLK / 4; ++j) {
-          const float4 f = ok ? __ldg(reinterpret_cast<const float4*>(src) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-          v[4 * j] = f.x; v[4 * j + 1] = f.y; v[4 * j + 2] = f.z; v[4 * j + 3] = f.w;
-        }
       } else {
 #pragma unroll
         for (int j = 0; j < KBLK; ++j) v[j] = (ok && j < nvalid) ? __ldg(src + j * s1) : 0.f;  // 32-bit offsets: two instructions per value
       }
-      {
-        const long long tw = pa ? clock64() : 0;
-        if (!mbar_wait(smem_u32(&ctrl->a_empty[as]), (a_round & 1) ^ 1, abort_flag, a.status, STATUS_TIMEOUT_EMPTY)) break;
-        if (pa) atomicAdd(a.prof + 6, (unsigned long long)(clock64() - tw));
-      }
-      const uint32_t p_hi = tiles_base + as * a_stage_bytes, p_lo = p_hi + a_plane;
-      if (chunked) {
+      return Job{chunk, as, a_round, chunked};
+    };
+    auto place = [&](const Job& j, const float (&v)[KBLK]) {
+      const uint32_t p_hi = tiles_base + j.as * a_stage_bytes, p_lo = p_hi + a_plane;
+      const int r = j.chunk * 32 + lane;
+      if (j.chunked) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          const int ri = chunk * 32 + 4 * i + (lane >> 3);  // strip_rows is a multiple of 8
+          const int ri = j.chunk * 32 + 4 * i + (lane >> 3);  // strip_rows is a multiple of 8
           if (ri < a.strip_rows) {
             float h[4], l[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) split_tf32_fast(v[4 * i + j], h[j], l[j]);
+            for (int e = 0; e < 4; ++e) split_tf32_fast(v[4 * i + e], h[e], l[e]);
             const int c4 = (lane & 7) * 4;  // first of this lane's four channels
             sts_f32x4(p_hi + sw128_offset(ri, c4), h[0], h[1], h[2], h[3]);
             if (CROSS_BF16) {
@@ -453,7 +444,7 @@ __global__ void __launch_bounds__(strip_threads(AW), 1) conv_strip_kernel(const 
           for (int c = 0; c < 4; ++c) {  // eight channels: two 16-byte chunks of the hi plane, one each of bf16(hi), bf16(lo)
             float h[8], l[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) split_tf32_fast(v[c * 8 + j], h[j], l[j]);
+            for (int e = 0; e < 8; ++e) split_tf32_fast(v[c * 8 + e], h[e], l[e]);
             sts_f32x4(p_hi + sw128_offset(r, c * 8), h[0], h[1], h[2], h[3]);
             sts_f32x4(p_hi + sw128_offset(r, c * 8 + 4), h[4], h[5], h[6], h[7]);
             sts_b32x4(p_lo + sw128_offset_bf16(r, c * 8), pack_bf16x2(h[0], h[1]), pack_bf16x2(h[2], h[3]),
@@ -466,16 +457,39 @@ __global__ void __launch_bounds__(strip_threads(AW), 1) conv_strip_kernel(const 
           for (int c = 0; c < 8; ++c) {
             float h[4], l[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) split_tf32_fast(v[c * 4 + j], h[j], l[j]);
+            for (int e = 0; e < 4; ++e) split_tf32_fast(v[c * 4 + e], h[e], l[e]);
             const uint32_t o = sw128_offset(r, c * 4);
             sts_f32x4(p_hi + o, h[0], h[1], h[2], h[3]);
             sts_f32x4(p_lo + o, l[0], l[1], l[2], l[3]);
           }
         }
       }
-      fence_proxy_async();
-      mbar_arrive(smem_u32(&ctrl->a_full[as]));
-      PROF_ADD(pa, 7);
+    };
+    if (aw < a_warps && aw < total_jobs) {
+      constexpr bool AHEAD = AW > 8;  // eight warps serve layers of many taps, where the first strip is wanted at once
+      float v[KBLK], ahead[AHEAD ? KBLK : 1];
+      Job j = fetch(aw, v), next = j;
+#pragma unroll 1
+      for (int job = aw;;) {
+        const bool more = job + a_warps < total_jobs;
+        if constexpr (AHEAD) if (more) next = fetch(job + a_warps, ahead);
+        const bool pa = PROF_ON(threadIdx.x == EPI_WARPS * 32);
+        PROF_T0(pa);
+        if (!mbar_wait(smem_u32(&ctrl->a_empty[j.as]), (j.round & 1) ^ 1, abort_flag, a.status, STATUS_TIMEOUT_EMPTY)) break;
+        PROF_ADD(pa, 6);
+        place(j, v);
+        fence_proxy_async();
+        mbar_arrive(smem_u32(&ctrl->a_full[j.as]));
+        if (!more) break;
+        job += a_warps;
+        if constexpr (AHEAD) {
+          j = next;
+#pragma unroll
+          for (int e = 0; e < KBLK; ++e) v[e] = ahead[e];
+        } else {
+          j = fetch(job, v);
+        }
+      }
     }
   } else {
     // ------------------------------ epilogue ------------------------------
@@ -826,7 +840,7 @@ static int launch_strip_aw(const tcs::StripArgs& a, int grid, int smem, cudaStre
 }
 template <int BN>
 static int launch_strip(const tcs::StripArgs& a, int grid, int smem, cudaStream_t st) {
-  return a.wide_producers ? launch_strip_aw<BN, 16>(a, grid, smem, st) : launch_strip_aw<BN, 8>(a, grid, smem, st);
+  return a.wide_producers ? launch_strip_aw<BN, 12>(a, grid, smem, st) : launch_strip_aw<BN, 8>(a, grid, smem, st);
 }
 
 // The kernel forms element offsets inside the activation tensor in 32 bits: true when the view's
@@ -897,15 +911,15 @@ int strip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* b
   a.tiles_m = (int)div_up64(a.q_total, BLOCK_M);
   a.halo = plan.halo; a.strip_rows = plan.strip_rows; a.a_stages = plan.a_stages; a.w_stages = plan.w_stages;
   {
-    // one tap per staged strip (1x1 filters): the MMAs wait for the producers, so sixteen of them run (testing aid:
-    // B200_STRIP_PRODUCERS=8|16 pins either)
+    // one tap per staged strip (1x1 filters): the MMAs wait for the producers, so twelve of them run (testing aid:
+    // B200_STRIP_PRODUCERS=8|12 pins either)
     int most = 0;
     for (int ph = 0; ph < plan.tt.n_phase; ++ph) most = std::max(most, (int)plan.tt.start[ph + 1] - (int)plan.tt.start[ph]);
     // ... and only while the reduction side is the larger one (256 -> 64 channels forward: 90 -> 69 us); with more output
     // than input (its dInput) the epilogue's stores set the pace and the extra warps only take registers from it (61 -> 80 us)
     // (row-major stores are whole lines and cost less: 1024 -> 1024 columns of a GEMM 198 -> 157 us, but 80 -> 1024 is faster with eight)
     a.wide_producers = most <= 1 && (kc > nc || (rowmajor && a.cblocks >= 16)) ? 1 : 0;
-    if (const char* e = getenv("B200_STRIP_PRODUCERS")) a.wide_producers = atoi(e) == 16 ? 1 : 0;
+    if (const char* e = getenv("B200_STRIP_PRODUCERS")) a.wide_producers = atoi(e) > 8 ? 1 : 0;
   }
   const int chunks = (a.strip_rows + 31) / 32;
   const long long tiles_total = (long long)a.tiles_m * a.tiles_n * g.groups;
