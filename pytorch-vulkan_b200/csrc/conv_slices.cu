@@ -7,6 +7,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "plan_cache.cuh"
 
 namespace b200 {
 namespace {
@@ -71,10 +72,8 @@ long long out_count(const ConvGeom& g, bool is_dx) { return is_dx ? (long long)g
 // Slices by the kernels' own time models; 1 when one slice is as good.  A second launch costs about 3 us and the partial results a
 // write and a read, so layers below 12 us, or with two waves of tiles and more, are not looked at further (64 -> 64 channels of one 28x28
 // image, 13 us, gain nothing: half the stages against the second launch).
-int conv_slices(const ConvGeom& g, bool is_dx, bool allow_transposed) {
+static int plan_slices(const ConvGeom& g, bool is_dx, bool transposed) {
   const int kc = is_dx ? g.cout : g.cin, phase = is_dx ? B200_PHASE_DINPUT : B200_PHASE_FORWARD;
-  if (g.groups != 1 || kc % 32 || kc < 64) return 1;
-  const bool transposed = allow_transposed && tstrip_supported(g, phase);
   if (!transposed && !strip_supported(g, phase)) return 1;
   const long long values = out_count(g, is_dx);
   if (values * MAX_SLICES >= 1ll << 31) return 1;
@@ -90,6 +89,13 @@ int conv_slices(const ConvGeom& g, bool is_dx, bool allow_transposed) {
     if (t < 0.95 * best_time) { best = s; best_time = t; }
   }
   return best;
+}
+int conv_slices(const ConvGeom& g, bool is_dx, bool allow_transposed) {
+  const int kc = is_dx ? g.cout : g.cin;
+  if (g.groups != 1 || kc % 32 || kc < 64) return 1;
+  const bool transposed = allow_transposed && tstrip_supported(g, is_dx ? B200_PHASE_DINPUT : B200_PHASE_FORWARD);
+  thread_local PlanCache<int> cache;
+  return cache.get(g, 2 * transposed + is_dx, [&] { return plan_slices(g, is_dx, transposed); });
 }
 
 // Bytes of workspace for that many slices: the filter images and the partial results.

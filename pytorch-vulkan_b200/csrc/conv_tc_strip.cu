@@ -37,6 +37,7 @@
 #include <cuda_bf16.h>
 
 #include "common.cuh"
+#include "plan_cache.cuh"
 #include "strip_plan.cuh"
 #include "tc_common.cuh"
 
@@ -752,7 +753,7 @@ static double width_cost(long long tiles, int bn, bool single_tap) {
   return (double)div_up64(tiles, sm_count()) * bn / eff;
 }
 
-static StripPlan plan_strip(const ConvGeom& g, bool is_dx) {
+static StripPlan make_plan(const ConvGeom& g, bool is_dx) {
   StripPlan p = plan_strip_geometry(g, is_dx);
   if (!p.ok) return p;
   p.ok = false;
@@ -789,6 +790,10 @@ static StripPlan plan_strip(const ConvGeom& g, bool is_dx) {
   }
   return p;
 }
+static const StripPlan& plan_strip(const ConvGeom& g, bool is_dx) {
+  thread_local PlanCache<StripPlan> cache;
+  return cache.get(g, is_dx, [&] { return make_plan(g, is_dx); });
+}
 
 }  // namespace tcs
 
@@ -797,13 +802,13 @@ bool strip_supported(const ConvGeom& g, int phase) {
   return tcs::plan_strip(g, phase == B200_PHASE_DINPUT).ok;
 }
 int strip_column_tile(const ConvGeom& g, bool is_dx) {
-  const tcs::StripPlan p = tcs::plan_strip(g, is_dx);
+  const tcs::StripPlan& p = tcs::plan_strip(g, is_dx);
   return p.ok ? p.bn : 0;
 }
 // Waves of tiles times filter stages of a tile times the measured time of a stage at that width (layers of a few waves), and the
 // prologue and epilogue of a wave.
 double strip_time(const ConvGeom& g, bool is_dx, long long* tiles) {
-  const tcs::StripPlan p = tcs::plan_strip(g, is_dx);
+  const tcs::StripPlan& p = tcs::plan_strip(g, is_dx);
   if (!p.ok) return 1e30;
   const int kc = is_dx ? g.cog : g.cig, nc = is_dx ? g.cig : g.cog, phases = is_dx ? std::max(1, p.tt.n_phase) : 1;
   const long long count = div_up64((long long)g.n * (p.gh + p.pr) * (p.gw + p.pc), tcs::BLOCK_M) * ((nc + p.bn - 1) / p.bn) * g.groups * phases;
@@ -857,7 +862,7 @@ int strip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* b
                void* ws, size_t ws_bytes, cudaStream_t st, bool rowmajor, float alpha, float beta, const float* staged_images,
                const StripPostOps* post, const StripBatch* batch) {
   using namespace tcs;
-  const StripPlan plan = plan_strip(g, is_dx);
+  const StripPlan& plan = plan_strip(g, is_dx);
   if (!plan.ok) return fail(B200_EUNSUPPORTED, "strip kernel does not take this geometry");
   const int kc = is_dx ? g.cog : g.cig, nc = is_dx ? g.cig : g.cog;
   const int tiles_pp = (nc + plan.bn - 1) / plan.bn;  // column tiles (per output phase in dInput)

@@ -34,6 +34,7 @@
 // reference for contiguous NCHW results with at least 65 output channels per group (below that half of every
 // MMA would multiply padding, and conv_tc_strip.cu is the better arrangement).
 #include "common.cuh"
+#include "plan_cache.cuh"
 #include "strip_plan.cuh"
 #include "tc_common.cuh"
 
@@ -511,7 +512,7 @@ static double mma_clocks(int pn) { return std::max(pn / 2.0, (4096.0 + 32.0 * pn
 
 // The pixel tile is the free parameter: wide tiles use the tensor pipe best, but the tile count should fill whole
 // waves of SMs.  Modelled time = waves x (MMAs of a tile x clocks(pn) + a fixed cost per tile).
-static TPlan plan_tstrip(const ConvGeom& g, bool is_dx) {
+static TPlan make_plan(const ConvGeom& g, bool is_dx) {
   TPlan p;
   p.geo = tcs::plan_strip_geometry(g, is_dx);
   if (!p.geo.ok) return p;
@@ -550,6 +551,11 @@ static TPlan plan_tstrip(const ConvGeom& g, bool is_dx) {
   if (p.ok && (long long)p.tiles_p * p.tiles_m * g.groups * p.cpp * ((p.strip_rows + 31) / 32) > 2147483647ll - (1 << 20)) p.ok = false;
   return p;
 }
+static const TPlan& plan_tstrip(const ConvGeom& g, bool is_dx) {
+  thread_local PlanCache<TPlan> cache;
+  const char* pinned = getenv("B200_TSTRIP_PN");
+  return cache.get(g, 2 * (pinned ? (size_t)atoi(pinned) : 0) + is_dx, [&] { return make_plan(g, is_dx); });
+}
 
 }  // namespace tst
 
@@ -571,19 +577,19 @@ bool tstrip_supported(const ConvGeom& g, int phase) {
   return tst::plan_tstrip(g, is_dx).ok;
 }
 double tstrip_time(const ConvGeom& g, bool is_dx, long long* tiles) {
-  const tst::TPlan p = tst::plan_tstrip(g, is_dx);
+  const tst::TPlan& p = tst::plan_tstrip(g, is_dx);
   if (tiles) *tiles = (long long)p.tiles_p * p.tiles_m * g.groups;
   return p.ok ? p.clocks / 1850.0 + 6.0 : 1e30;
 }
 size_t tstrip_workspace(const ConvGeom& g, int phase) {
-  const tst::TPlan p = tst::plan_tstrip(g, phase == B200_PHASE_DINPUT);
+  const tst::TPlan& p = tst::plan_tstrip(g, phase == B200_PHASE_DINPUT);
   return p.ok ? (size_t)p.images * tst::W_STAGE_BYTES : 0;
 }
 
 int tstrip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* bias, long long bias_stride, float* out,
                 void* ws, size_t ws_bytes, cudaStream_t st, long long w_group_extra) {
   using namespace tst;
-  const TPlan plan = plan_tstrip(g, is_dx);
+  const TPlan& plan = plan_tstrip(g, is_dx);
   if (!plan.ok) return fail(B200_EUNSUPPORTED, "transposed strip kernel does not take this geometry");
   const size_t need = (size_t)plan.images * W_STAGE_BYTES;
   if (!ws || ws_bytes < need || (reinterpret_cast<uintptr_t>(ws) & 15))

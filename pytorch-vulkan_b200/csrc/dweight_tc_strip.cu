@@ -26,6 +26,7 @@
 // Replaces csrc/shaders/conv2d_backward_weight_tiled_body.glsl:42-70 and
 // conv2d_backward_weight_finalize.comp:9-18 of the reference for these geometries.
 #include "common.cuh"
+#include "plan_cache.cuh"
 #include "dweight_plan.cuh"
 #include "dweight_stage.cuh"
 #include "tc_common.cuh"
@@ -563,7 +564,7 @@ static inline int floor_div(int a, int b) { return a >= 0 ? a / b : -((-a + b - 
 //   blocks: everything else -- strides, any padding, 1x1: four exact 32-pixel blocks per K
 //           block, either the taps kx = 0..3 of one channel block (each with its own column phase and
 //           offset) or, for a 1x1 filter, four channel blocks.
-static DwStripPlan plan_dw_strip(const ConvGeom& g, size_t budget) {
+static DwStripPlan make_plan(const ConvGeom& g, size_t budget) {
   DwStripPlan p;
   if (g.kw > 8 || g.cog < 16 || g.cig < 16) return p;
   p.kx_groups = (g.kw + 3) / 4;
@@ -640,6 +641,10 @@ static DwStripPlan plan_dw_strip(const ConvGeom& g, size_t budget) {
   p.ok = true;
   return p;
 }
+static const DwStripPlan& plan_dw_strip(const ConvGeom& g, size_t budget) {
+  thread_local PlanCache<DwStripPlan> cache, forced;
+  return (getenv("B200_DW_FORCE_CROSS") ? forced : cache).get(g, budget, [&] { return make_plan(g, budget); });
+}
 
 }  // namespace tcdw
 
@@ -675,7 +680,7 @@ int dweight_strip(const ConvGeom& g, View4 x, View4 dy, float* dw, void* ws, siz
     const int rc = tcdt::run(g, x, dy, dw, ws, ws_bytes, st);
     if (rc != B200_EUNSUPPORTED) return rc;
   }
-  const DwStripPlan plan = plan_dw_strip(g, ws ? ws_bytes : 0);
+  const DwStripPlan& plan = plan_dw_strip(g, ws ? ws_bytes : 0);
   if (!plan.ok) return fail(B200_EUNSUPPORTED, "dWeight strip kernel does not take this geometry");
   // the kernel forms element offsets inside a tensor in 32 bits
   auto span = [](const View4& v, long long n, long long c, long long h, long long w) {

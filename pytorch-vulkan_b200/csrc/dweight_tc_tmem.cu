@@ -34,6 +34,7 @@
 //
 // Replaces csrc/shaders/conv2d_backward_weight_tiled_body.glsl:42-70 of the reference for these geometries.
 #include "common.cuh"
+#include "plan_cache.cuh"
 #include "dweight_stage.cuh"
 #include "dweight_plan.cuh"
 #include "tc_common.cuh"
@@ -665,9 +666,14 @@ static Plan make_plan(const ConvGeom& real, size_t budget) {
   a.fold_sh = real.sh; a.fold_dh = real.dh; a.fold_ph = real.ph; a.fold_h = real.h;
   return best;
 }
+static const Plan& cached_plan(const ConvGeom& g, size_t budget) {
+  thread_local PlanCache<Plan> cache, pinned;
+  if (getenv("B200_DW_CHUNK_KB")) return pinned.get(g, budget + (size_t)atoi(getenv("B200_DW_CHUNK_KB")) * 7919, [&] { return make_plan(g, budget); });
+  return cache.get(g, budget, [&] { return make_plan(g, budget); });
+}
 
 bool plan_bytes(const ConvGeom& g, size_t budget, size_t* bytes) {
-  const Plan p = make_plan(g, budget);
+  const Plan& p = cached_plan(g, budget);
   if (p.ok) *bytes = p.bytes;
   return p.ok;
 }
@@ -684,7 +690,7 @@ static int launch(const Args& a, const Plan& p, cudaStream_t st) {
 }
 
 int run(const ConvGeom& g, View4 x, View4 dy, float* dw, void* ws, size_t ws_bytes, cudaStream_t st) {
-  Plan p = make_plan(g, ws ? ws_bytes : 0);
+  Plan p = cached_plan(g, ws ? ws_bytes : 0);
   if (!p.ok) return B200_EUNSUPPORTED;
   // element offsets inside a tensor are 32-bit in the kernel
   auto span = [](const View4& v, long long n, long long c, long long h, long long w) {
