@@ -194,7 +194,7 @@ int b200_conv_transpose2d_forward(const b200_conv_params* p, b200_view4 x, b200_
 int b200_conv2d_dweight(const b200_conv_params* p, b200_view4 x, b200_view4 dy, float* dw,
                         void* workspace, size_t workspace_bytes, int algo, void* stream);
 /* db[co] = sum dy.  Replaces dispatch(Bias), :692-695, conv2d_backward_bias{,_reduce}.
- * workspace may be NULL (then a single pass per channel is used). */
+ * workspace may be NULL: without it a large, narrow channels-last gradient is summed by fewer CTAs. */
 int b200_conv2d_dbias(const b200_conv_params* p, b200_view4 dy, float* db, void* workspace,
                       size_t workspace_bytes, void* stream);
 
@@ -354,12 +354,13 @@ enum { B200_MASK_NONE = 0, B200_MASK_ADDITIVE = 1, B200_MASK_BYTES = 2 };
  * Philox4x32-10 stream of the reference (csrc/shaders/philox.glsl; state layout of VulkanGenerator::reserve,
  * csrc/vulkan_generator.cpp:17-20), element (row, key) drawing word (row * tk + key) % 4 of block
  * offset + (row * tk + key) / 4.  The backward call must get the same dropout and rng as its forward call.
- * Workspace: the score matrix (forward) or two of them (backward != 0). */
+ * Workspace: the score matrix (forward) or two of them (backward != 0), or the operand images of the fused kernels if larger. */
 size_t b200_attention_workspace(int64_t batch, int64_t tq, int64_t tk, int64_t d, int64_t dv, int backward);
 
 /* out = softmax(q k^T * scale + mask) v and the per-row log-sum-exp.  Replaces attention_forward
- * (csrc/ops/attention.cpp:16-23, shader sdpa_training.comp mode 0).  Composed from b200_bmm and one
- * row-softmax kernel; the scores are materialised in the workspace. */
+ * (csrc/ops/attention.cpp:16-23, shader sdpa_training.comp mode 0).  Calls without mask and
+ * dropout and with d == dv from 16 to 64 run fused; the rest is composed from b200_bmm and one row-softmax kernel, with the
+ * scores materialised in the workspace. */
 int b200_attention_forward(int64_t batch, int64_t tq, int64_t tk, int64_t d, int64_t dv, const float* q, const float* k,
                            const float* v, const void* mask, int mask_type, int causal, float scale, float dropout,
                            const uint32_t* rng, float* out, float* lse, void* workspace, size_t workspace_bytes, void* stream);

@@ -2,8 +2,8 @@
 // group_norm_forward / group_norm_backward_input / group_norm_backward_affine shaders of the
 // reference (csrc/shaders/group_norm_*.comp) and their host side (csrc/ops/group_norm.cpp:76-155).
 //
-// Blocks that fit the registers of a cluster of CTAs are read once (gn_*_cluster_kernel, below).  Larger ones: a (sample, group) block is c/groups adjacent planes, contiguous in memory.  As in the reference
-// one CTA owns one block, but it is a CTA of 16 warps that each stream whole plane segments with
+// Blocks that fit the registers of a cluster of CTAs are read once (gn_*_cluster_kernel, below).  Larger ones: a (sample,
+// group) block is c/groups adjacent planes, contiguous in memory.  As in the reference one CTA owns one block, but it is a CTA of 16 warps that each stream whole plane segments with
 // 16-byte loads, and each kernel makes two passes over its block: the first reads it from HBM, the
 // second finds it in L2 (at most three CTAs of a few hundred KB per SM are in flight, far below the
 // 126 MB of L2).  HBM traffic is therefore one read and one write per tensor element:
