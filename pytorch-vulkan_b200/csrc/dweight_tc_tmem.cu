@@ -568,14 +568,18 @@ static Plan make_plan(const ConvGeom& real, size_t budget) {
     g.cin = g.cig = real.cig * real.kh;
     g.kh = 1; g.ph = 0; g.dh = 1; g.sh = 1; g.h = g.oh;
   }
-  // 1x1 filters are bound by the staging of both operands, for which dweight_tc_strip.cu has more warps
-  if ((!fold && (g.kh * g.kw == 1 || g.cig < 16)) || g.kw > 8 || g.cog < 16 || g.sh > 127 || g.sw > 127) return best;
+  if ((!fold && g.cig < 16) || g.kw > 8 || g.cog < 16 || g.sh > 127 || g.sw > 127) return best;
   const int gh = std::max(g.oh, (g.h + g.sh - 1) / g.sh), gw = std::max(g.ow, (g.w + g.sw - 1) / g.sw);
   int pr = 0, pc = 0;
   for (int ky = 0; ky < g.kh; ++ky) pr = std::max(pr, std::abs(floor_div(ky * g.dh - g.ph, g.sh)));
   for (int kx = 0; kx < g.kw; ++kx) pc = std::max(pc, std::abs(floor_div(kx * g.dw - g.pw, g.sw)));
   const long long q_total = (long long)g.n * (gh + pr) * (gw + pc);
   if (q_total > 2147483647ll - (1 << 20)) return best;
+  // 1x1 filters are bound by the staging of both operands, for which dweight_tc_strip.cu has more warps but needs long splits to fill its
+  // pipeline.  Measured, that kernel against this one: 256 -> 512 channels of 32 x 14x14 38.7 and 28.4 us, 96 -> 131 of 42 x 7x7 31.9 and
+  // 11.9, 32 -> 128 of 64 x 56x56 57 and 45; 512 -> 96 of 64 x 14x14 28.0 and 29.4, 512 -> 128 of 32 x 28x28 34 and 44, 64 -> 64 of
+  // 64 x 56x56 42 and 53: the line is at five million input values, or one block of input channels.
+  if (!fold && g.kh * g.kw == 1 && g.cig > 32 && q_total * g.cig > (5ll << 20)) return best;
   const int row_pitch = gw + pc;
   // shift mode: vertical taps m apart lie a whole number of grid rows apart
   int m = 1;

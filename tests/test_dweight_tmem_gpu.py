@@ -27,6 +27,11 @@ CASES = [  # (xshape, cout, kernel, conv arguments)
     ((2, 3, 32, 33), 64, (7, 7), dict(stride=(2, 2), padding=(3, 3))),          # filter rows folded into the channels: 21 of 32
     ((1, 8, 19, 20), 130, (5, 5), dict(padding=(2, 2))),                        # 40: two strips
     ((3, 1, 17, 16), 16, (3, 3), dict(padding=(1, 1))),
+    ((1, 16, 5, 6), 16, (1, 1), dict()),                                        # 1x1: one K block ...
+    ((2, 96, 7, 7), 131, (1, 1), dict()),
+    ((3, 300, 9, 8), 40, (1, 1), dict(stride=(2, 2))),
+    ((2, 288, 91, 100), 24, (1, 1), dict()),                                    # ... and on either side of the line between the kernels
+    ((2, 289, 91, 100), 24, (1, 1), dict()),
     ((2, 15, 12, 13), 40, (3, 3), dict(stride=(1, 3), padding=(0, 1), dilation=(2, 1))),
 ]
 
