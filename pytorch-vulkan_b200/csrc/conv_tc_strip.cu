@@ -37,6 +37,7 @@
 #include <cuda_bf16.h>
 
 #include "common.cuh"
+#include "gemm_tmem.cuh"
 #include "plan_cache.cuh"
 #include "strip_plan.cuh"
 #include "tc_common.cuh"
@@ -946,6 +947,20 @@ int strip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* b
   a.alpha = alpha; a.beta = beta;
   a.out_vec4 = rowmajor && a.out_pitch % 4 == 0 && a.out_group % 4 == 0 && plan.bn % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0 &&
                a.nc % 4 == 0;
+  // a plain product with wide column tiles: one tap per strip leaves shared memory as the bound, which the kernel with A in tensor memory
+  // relieves (16384x1024 x 1024x1024: 144 -> 131 us); below 65 columns its tiles would be half empty (B200_GEMM_STRIP pins the strip kernel: testing aid)
+  if (rowmajor && !is_dx && !post && g.n == 1 && g.h == 1 && g.kh * g.kw == 1 && plan.bn >= 128 && !getenv("B200_GEMM_STRIP")) {
+    gt::GemmArgs m{};
+    m.A = act.ptr; m.a_m = act.s3; m.a_k = act.s1; m.a_group = kc * act.s1 + a.act_group_extra;
+    m.images = wp; m.bias = bias; m.bias_stride = bias_stride;
+    m.C = out; m.c_pitch = a.out_pitch; m.c_group = a.out_group;
+    m.M = g.w; m.N = nc; m.kc = kc; m.k_total = k_total; m.kblocks = cpp;
+    m.tiles_m = a.tiles_m; m.tiles_n = a.tiles_n; m.tiles = a.tiles_total; m.m_fastest = a.unit == 1;
+    if (kc % 4 == 0 && m.a_group % 4 == 0 && (reinterpret_cast<uintptr_t>(act.ptr) & 15) == 0)
+      m.mode = act.s1 == 1 && act.s3 % 4 == 0 ? 1 : act.s3 == 1 && act.s1 % 4 == 0 ? 2 : 0;
+    m.vec_out = a.out_vec4; m.wait_for_images = a.wait_for_images; m.alpha = alpha; m.beta = beta;
+    return gt::run(m, plan.bn, st);
+  }
   a.status = device_status_word();
   if (!a.status) return fail(B200_ECUDA, "device status word is not allocated");
   static unsigned long long* prof_buf = nullptr;

@@ -1,0 +1,27 @@
+// The GEMM kernel with its left operand in tensor memory (gemm_tc_tmem.cu), launched by conv_tc_strip.cu behind its staging kernel.
+#pragma once
+#include "common.cuh"
+
+namespace b200 {
+namespace gt {
+struct GemmArgs {
+  const float* A;            // A[g][m][k] at g * a_group + m * a_m + k * a_k
+  long long a_m, a_k, a_group;
+  const float* images;       // stage images of B for column tiles of bn: [group][column tile][K block]
+  const float* bias;         // per group and column, or null
+  long long bias_stride;
+  float* C;                  // C[g][m][n] at g * c_group + m * c_pitch + n
+  long long c_pitch, c_group;
+  int M, N, kc, k_total;     // kc: reduction values of a group; k_total: of all groups (the last may have fewer)
+  int kblocks, tiles_m, tiles_n, tiles;
+  int m_fastest;             // tile order
+  int mode;                  // A in lines of 16-byte pieces along k (1) or along m (2), or value by value (0)
+  int vec_out;               // rows of C may be written 16 bytes at a time
+  int wait_for_images;
+  float alpha, beta;
+  int* status;
+  FastDiv div_m, div_n, div_kblocks;
+};
+int run(GemmArgs a, int bn, cudaStream_t st);
+}  // namespace gt
+}  // namespace b200
