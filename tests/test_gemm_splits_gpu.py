@@ -12,7 +12,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("m,n,k", [(128, 64, 64), (128, 64, 128), (320, 320, 8000), (2048, 512, 4096), (130, 70, 1025), (512, 768, 3072), (128, 1000, 999),
-                                   (1, 1, 128), (16, 64, 128), (63, 65, 127), (100, 1000, 2048), (300, 33, 1031), (17, 4096, 143)])
+                                   (1, 1, 128), (16, 64, 128), (63, 65, 127), (100, 1000, 2048), (300, 33, 1031), (17, 4096, 143),
+                                   (2500, 2304, 64), (20500, 128, 96)])
 @pytest.mark.parametrize("ta,tb", [(False, False), (True, False), (False, True)])
 def test_sliced_reduction(m, n, k, ta, tb):
     rng = np.random.default_rng(m + n + k)
