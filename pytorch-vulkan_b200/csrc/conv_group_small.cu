@@ -37,14 +37,34 @@ struct GArgs {
   int transposed;      // dInput: use w[ci][co][2-ky][2-kx]
 };
 
+__device__ __forceinline__ void cp_async(uint32_t dst, const float* src, int bytes, bool inside) {  // zeros where the source lies outside
+  if (bytes == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(inside ? 16 : 0) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(inside ? 4 : 0) : "memory");
+}
+// two FP32 multiply-adds in one instruction, each rounded as fmaf
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ unsigned long long both(float v) {
+  unsigned long long d;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(v));
+  return d;
+}
+
 // y[n, g*CPG + co, y, x] = bias + sum_{ci, ky, kx} in[n, g*CPG + ci, y + ky - 1, x + kx - 1] * W[co][ci][ky][kx]
 // SX strips of 4 pixels per tile row: the tile is (256 / SX) rows x (4 * SX) columns (16 x 64 for wide images,
 // 32 x 32 for maps up to 32 columns, so that no thread idles on padding).
+// One CTA per tile and a few tiles per SM, all in step: a tile's loads are latency, so every one of them is issued before any is waited
+// for (asynchronous copies; through registers four at a time where rows are not 16-byte aligned), and the multiply-adds run two to an
+// instruction, paired over output channels.  256 channels of 16 images of 32x32: 35 us from a
+// sliced view and 25 from a dense one, now 28 and 19.
 template <int CPG, int SX>
-__global__ void __launch_bounds__(THREADS) gconv_fwd_kernel(const GArgs a) {
+__global__ void __launch_bounds__(THREADS, 4) gconv_fwd_kernel(const GArgs a) {
   wait_previous();
   constexpr int TWK = 4 * SX, THK = THREADS / SX;         // tile extent
-  constexpr int IWK = TWK + 4, IHK = THK + 2;              // with halo; rows padded to a multiple of 4 floats
+  constexpr int IWK = TWK + 8, IHK = THK + 2;              // with halo; image column x0 + c at c + 4, so that 16-byte pieces stay aligned
   __shared__ __align__(16) float s_in[CPG][IHK][IWK];
   __shared__ __align__(16) float s_w[CPG][3][3][CPG];   // [ci][ky][kx][co]: the co of one tap are one vector
   const int tid = threadIdx.x;
@@ -65,76 +85,60 @@ __global__ void __launch_bounds__(THREADS) gconv_fwd_kernel(const GArgs a) {
                                  : a.w.ptr[(chan0 + co) * a.w.s0 + ci * a.w.s1 + ky * a.w.s2 + kx * a.w.s3];
     s_w[ci][ky][kx][co] = v;
   }
-  // input tile with halo (tile column c is image column x0 - 1 + c); out-of-image pixels are zero
+  // input tile with halo; out-of-image pixels are zero
   const float* src = a.in.ptr + n * a.in.s0 + chan0 * a.in.s1;
+  const uint32_t tile = (uint32_t)__cvta_generic_to_shared(&s_in[0][0][0]);
+  auto copy = [&](int ci, int r, int c, int bytes) {      // c: image column relative to x0
+    const int y = y0 - 1 + r, x = x0 + c;
+    const bool inside = y >= 0 && y < a.h && x >= 0 && x < a.w_;
+    cp_async(tile + 4u * (uint32_t)((ci * IHK + r) * IWK + c + 4), inside ? src + (ci * a.in.s1 + y * a.in.s2 + x * a.in.s3) : a.in.ptr, bytes, inside);
+  };
   const bool rows_vec = a.in.s3 == 1 && a.in.s2 % 4 == 0 && a.in.s1 % 4 == 0 && a.in.s0 % 4 == 0 &&
                         ((reinterpret_cast<uintptr_t>(a.in.ptr) & 15) == 0) && x0 + TWK <= a.w_;
-  if (rows_vec) {
-    // planes with contiguous rows: the interior of a tile row as 16-byte loads (all of a thread's loads are issued
-    // before the first is used), the two halo columns as scalars
-    constexpr int VEC = CPG * IHK * SX;                     // float4 pieces of the interior
-#pragma unroll
-    for (int i0 = 0; i0 < VEC; i0 += THREADS) {
-      const int i = i0 + tid;
-      if (VEC % THREADS == 0 || i < VEC) {
-        const int c4 = i % SX, r = (i / SX) % IHK, ci = i / (SX * IHK);
-        const int y = y0 - 1 + r;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (y >= 0 && y < a.h) v = __ldg(reinterpret_cast<const float4*>(src + ci * a.in.s1 + (long long)y * a.in.s2 + x0) + c4);
-        float* d = &s_in[ci][r][1 + 4 * c4];
-        d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
-      }
-    }
-    for (int i = tid; i < CPG * IHK * 2; i += THREADS) {
-      const int side = i & 1, r = (i >> 1) % IHK, ci = i / (2 * IHK);
-      const int y = y0 - 1 + r, x = side ? x0 + TWK : x0 - 1;
-      s_in[ci][r][side ? TWK + 1 : 0] = (y >= 0 && y < a.h && x >= 0 && x < a.w_) ? __ldg(src + ci * a.in.s1 + (long long)y * a.in.s2 + x) : 0.f;
-    }
+  if (rows_vec) {              // planes with contiguous rows: 16 bytes at a time, the two halo columns alone
+    for (int i = tid; i < CPG * IHK * SX; i += THREADS) copy(i / (SX * IHK), (i / SX) % IHK, 4 * (i % SX), 16);
+    for (int i = tid; i < CPG * IHK * 2; i += THREADS) copy(i / (2 * IHK), (i >> 1) % IHK, i & 1 ? TWK : -1, 4);
   } else if (a.in.s1 == 1) {   // channels-last: the channels of a pixel are adjacent
-#pragma unroll 4
-    for (int i = tid; i < CPG * IHK * (TWK + 2); i += THREADS) {
-      const int ci = i % CPG, c = (i / CPG) % (TWK + 2), r = i / (CPG * (TWK + 2));
-      const int y = y0 - 1 + r, x = x0 - 1 + c;
-      s_in[ci][r][c] = (y >= 0 && y < a.h && x >= 0 && x < a.w_) ? __ldg(src + ci + (long long)y * a.in.s2 + (long long)x * a.in.s3) : 0.f;
-    }
+    for (int i = tid; i < CPG * IHK * (TWK + 2); i += THREADS) copy(i % CPG, i / (CPG * (TWK + 2)), (i / CPG) % (TWK + 2) - 1, 4);
   } else {
-#pragma unroll 4
-    for (int i = tid; i < CPG * IHK * (TWK + 2); i += THREADS) {
-      const int c = i % (TWK + 2), r = (i / (TWK + 2)) % IHK, ci = i / ((TWK + 2) * IHK);
-      const int y = y0 - 1 + r, x = x0 - 1 + c;
-      s_in[ci][r][c] = (y >= 0 && y < a.h && x >= 0 && x < a.w_) ? __ldg(src + ci * a.in.s1 + (long long)y * a.in.s2 + (long long)x * a.in.s3) : 0.f;
-    }
+    for (int i = tid; i < CPG * IHK * (TWK + 2); i += THREADS) copy(i / ((TWK + 2) * IHK), (i / (TWK + 2)) % IHK, i % (TWK + 2) - 1, 4);
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
 
   const int tx = tid % SX, ty = tid / SX;   // strip of 4 pixels: row ty, columns 4*tx .. 4*tx+3
-  float acc[CPG][4];
+  unsigned long long pair[CPG / 2][4];      // output channels 2q and 2q + 1 of four pixels
 #pragma unroll
-  for (int co = 0; co < CPG; ++co)
+  for (int q = 0; q < CPG / 2; ++q)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[co][j] = 0.f;
+    for (int j = 0; j < 4; ++j) pair[q][j] = 0ull;
 #pragma unroll
   for (int ci = 0; ci < CPG; ++ci) {
 #pragma unroll
     for (int ky = 0; ky < 3; ++ky) {
-      const float4 p0 = *reinterpret_cast<const float4*>(&s_in[ci][ty + ky][4 * tx]);
-      const float2 p1 = *reinterpret_cast<const float2*>(&s_in[ci][ty + ky][4 * tx + 4]);
-      const float v[6] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y};
+      const float* row = &s_in[ci][ty + ky][4 * tx + 3];
+      const float4 p = *reinterpret_cast<const float4*>(row + 1);
+      const unsigned long long v[6] = {both(row[0]), both(p.x), both(p.y), both(p.z), both(p.w), both(row[5])};
 #pragma unroll
       for (int kx = 0; kx < 3; ++kx) {
-        float wv[CPG];
+        unsigned long long wv[CPG / 2];
 #pragma unroll
         for (int q = 0; q < CPG / 4; ++q) {
-          const float4 t = *reinterpret_cast<const float4*>(&s_w[ci][ky][kx][4 * q]);
-          wv[4 * q] = t.x; wv[4 * q + 1] = t.y; wv[4 * q + 2] = t.z; wv[4 * q + 3] = t.w;
+          const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(&s_w[ci][ky][kx][4 * q]);
+          wv[2 * q] = t.x; wv[2 * q + 1] = t.y;
         }
 #pragma unroll
-        for (int co = 0; co < CPG; ++co)
+        for (int q = 0; q < CPG / 2; ++q)
 #pragma unroll
-          for (int j = 0; j < 4; ++j) acc[co][j] = fmaf(v[j + kx], wv[co], acc[co][j]);
+          for (int j = 0; j < 4; ++j) pair[q][j] = fma2(v[j + kx], wv[q], pair[q][j]);
       }
     }
   }
+  float acc[CPG][4];
+#pragma unroll
+  for (int q = 0; q < CPG / 2; ++q)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) asm("mov.b64 {%0, %1}, %2;" : "=f"(acc[2 * q][j]), "=f"(acc[2 * q + 1][j]) : "l"(pair[q][j]));
   const int y = y0 + ty, x = x0 + 4 * tx;
   if (y >= a.h || x >= a.w_) return;
   const long long plane = (long long)a.h * a.w_;
