@@ -956,10 +956,12 @@ int strip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* b
     m.C = out; m.c_pitch = a.out_pitch; m.c_group = a.out_group;
     m.M = g.w; m.N = nc; m.kc = kc; m.k_total = k_total; m.kblocks = cpp;
     m.tiles_m = a.tiles_m; m.tiles_n = a.tiles_n; m.tiles = a.tiles_total; m.m_fastest = a.unit == 1;
-    if (kc % 4 == 0 && m.a_group % 4 == 0 && (reinterpret_cast<uintptr_t>(act.ptr) & 15) == 0)
-      m.mode = act.s1 == 1 && act.s3 % 4 == 0 ? 1 : act.s3 == 1 && act.s1 % 4 == 0 ? 2 : 0;
+    m.mode = act.s1 == 1 ? 1 : act.s3 == 1 ? 2 : 0;
+    m.pieces16 = (m.mode == 1 ? act.s3 : act.s1) % 4 == 0 && (m.mode == 2 || kc % 4 == 0) && m.a_group % 4 == 0 && (reinterpret_cast<uintptr_t>(act.ptr) & 15) == 0;
     m.vec_out = a.out_vec4; m.wait_for_images = a.wait_for_images; m.alpha = alpha; m.beta = beta;
-    return gt::run(m, plan.bn, st);
+    // rows of A along m that are not 16-byte aligned are better read straight into the strip producers' registers (51 against 66 us for
+    // 1111x16000 x 16000x77), as is A without a contiguous dimension
+    if (m.mode != 0 && (m.mode == 1 || m.pieces16)) return gt::run(m, plan.bn, st);
   }
   a.status = device_status_word();
   if (!a.status) return fail(B200_ECUDA, "device status word is not allocated");

@@ -71,8 +71,10 @@ __device__ __forceinline__ void transpose_pieces(float (&v)[32], int lane) {
   }
 }
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int bytes) {   // the rest of the 16 bytes becomes zero
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+template <int BYTES>
+__device__ __forceinline__ void cp_async(uint32_t dst, const void* src, int bytes) {   // the rest of BYTES becomes zero
+  if (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -188,15 +190,24 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const GemmArgs a)
       const int c = set + n * SETS;
       if (a.mode != 0 && c < total) {
         const Block k = locate(c);
-        const int lines = a.mode == 1 ? k.rows : k.valid, inside = (a.mode == 1 ? k.valid : k.rows) - (lane & 7) * 4;
-        const int bytes = max(0, min(16, inside * 4));
+        const int lines = a.mode == 1 ? k.rows : k.valid, length = a.mode == 1 ? k.valid : k.rows;
         const long long pitch = a.mode == 1 ? a.a_m : a.a_k;
-        const float* p = k.src + (long long)(lane >> 3) * pitch + (lane & 7) * 4;
         const uint32_t slot = slots + (uint32_t)(n % DEPTH) * SLOT;
+        if (a.pieces16) {
+          const int bytes = max(0, min(16, (length - (lane & 7) * 4) * 4));
+          const float* p = k.src + (long long)(lane >> 3) * pitch + (lane & 7) * 4;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int r = 4 * j + (lane >> 3), size = r < lines ? bytes : 0;
-          cp_async16(slot + (uint32_t)(r * 128 + (((lane & 7) ^ (r & 7)) << 4)), size ? p + 4ll * j * pitch : a.A, size);
+          for (int j = 0; j < 8; ++j) {
+            const int r = 4 * j + (lane >> 3), size = r < lines ? bytes : 0;
+            cp_async<16>(slot + (uint32_t)(r * 128 + (((lane & 7) ^ (r & 7)) << 4)), size ? p + 4ll * j * pitch : a.A, size);
+          }
+        } else {                     // lines that start anywhere: a value at a time, a warp to a line
+          const float* p = k.src + lane;
+#pragma unroll 8
+          for (int r = 0; r < 32; ++r) {
+            const int size = r < lines && lane < length ? 4 : 0;
+            cp_async<4>(slot + (uint32_t)(r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4), size ? p + r * pitch : a.A, size);
+          }
         }
       }
       cp_async_commit();
@@ -293,13 +304,19 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const GemmArgs a)
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] *= a.alpha;
         }
-        if (a.vec_out && left == 32) {
+        if (left == 32) {
           transpose_pieces(v, lane);  // whole lines: piece i of row 4j + lane % 4
           float* p = a.C + t.group * a.c_group + (long long)(t.m * M_TILE + quarter * 32 + (lane & 3)) * a.c_pitch + n0 + c0 + (lane >> 2) * 4;
+          if (a.vec_out) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j)
-            if (t.m * M_TILE + quarter * 32 + 4 * j + (lane & 3) < a.M)
-              *reinterpret_cast<float4*>(p + 4ll * j * a.c_pitch) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+            for (int j = 0; j < 8; ++j)
+              if (t.m * M_TILE + quarter * 32 + 4 * j + (lane & 3) < a.M)
+                *reinterpret_cast<float4*>(p + 4ll * j * a.c_pitch) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+          } else {                    // rows of C that are not 16-byte aligned (a row to a lane: 151 us for 16000x77 x 77x1111, now 71)
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (t.m * M_TILE + quarter * 32 + (j & ~3) + (lane & 3) < a.M) p[(long long)(j & ~3) * a.c_pitch + (j & 3)] = v[j];
+          }
         } else if (row < a.M) {
 #pragma unroll
           for (int j = 0; j < 32; ++j)
