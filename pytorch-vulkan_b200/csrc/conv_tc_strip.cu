@@ -649,8 +649,10 @@ __global__ void __launch_bounds__(256) stage_weights_kernel(ConvGeom g, View4 w,
   const int kc = is_dx ? g.cog : g.cig, nc = is_dx ? g.cig : g.cog;
   const int cpp = (kc + KBLK - 1) / KBLK;
   const int block = (int)(i / ((KBLK / 4) * bn)), in_block = (int)(i - (long long)block * ((KBLK / 4) * bn));
-  const int k = (rows_first ? in_block / bn : in_block % (KBLK / 4)) * 4;
-  const int row = rows_first ? in_block % bn : in_block / (KBLK / 4);
+  // rows first: eight adjacent rows (32 bytes read) by four pieces (64 bytes written) to a warp; with a warp along the rows alone the
+  // writes were 16 bytes of 32 lines (weight gradient of a 4096x512 -> 2048 linear layer 46.5 us, now 43.4)
+  const int k = (rows_first ? in_block >> 3 & 7 : in_block % (KBLK / 4)) * 4;
+  const int row = rows_first ? (in_block & 7) | in_block >> 6 << 3 : in_block / (KBLK / 4);
   const int tile_of_all = block / cpp, cbl = block - tile_of_all * cpp, grp = tile_of_all / tiles_pp, n_tile = tile_of_all - grp * tiles_pp;
   const int r = n_tile * bn + row, c = cbl * KBLK + k;
   // rows beyond the column count and channels beyond a ragged last block are zero

@@ -467,8 +467,8 @@ __global__ void __launch_bounds__(256) stage_filter16_kernel(ConvGeom g, View4 w
   const int kc = is_dx ? g.cog : g.cig, nc = is_dx ? g.cig : g.cog;
   const int cpp = (kc + KB - 1) / KB;
   const int block = (int)(i / (4 * TM)), in_block = (int)(i - (long long)block * (4 * TM));
-  const int piece = rows_first ? in_block / TM : in_block % 4, k = piece * 4;
-  const int row = rows_first ? in_block % TM : in_block / 4;
+  const int piece = rows_first ? in_block >> 3 & 3 : in_block % 4, k = piece * 4;
+  const int row = rows_first ? (in_block & 7) | in_block >> 5 << 3 : in_block / 4;
   const int tile_of_all = block / cpp, cbl = block - tile_of_all * cpp, grp = tile_of_all / tiles_pp, m_tile = tile_of_all - grp * tiles_pp;
   const int r = m_tile * TM + row, c = cbl * KB + k;
   const int valid = r < nc ? min(4, kc - c) : 0;
