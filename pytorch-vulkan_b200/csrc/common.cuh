@@ -55,6 +55,12 @@ struct View4 {
   long long s0, s1, s2, s3;
 };
 inline View4 to_view(const b200_view4& v) { return {v.ptr, v.stride[0], v.stride[1], v.stride[2], v.stride[3]}; }
+// Channels-last loads of four channels at once, from channel blocks that start at multiples of four within a group of `per_group` channels:
+// true when every such piece starts on 16 bytes, in every pixel and every group (with 34 channels a group the second one starts 136 bytes in).
+__host__ __device__ inline bool channel_quads_aligned(const View4& v, int per_group, int groups) {
+  return v.s1 == 1 && (reinterpret_cast<uintptr_t>(v.ptr) & 15) == 0 && v.s0 % 4 == 0 && v.s2 % 4 == 0 && v.s3 % 4 == 0 &&
+         (groups == 1 || per_group % 4 == 0);
+}
 inline View4 contiguous_view(const float* p, long long d1, long long d2, long long d3) {
   return {p, d1 * d2 * d3, d2 * d3, d3, 1};
 }

@@ -321,10 +321,7 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_strip_kernel(const DwStrip
     }
   } else {
     // ---- producers: job j of K block kb goes to warp (kb*tasks + j) % 16 ----
-    const bool x_vec = a.x.s1 == 1 && ((reinterpret_cast<uintptr_t>(a.x.ptr) & 15) == 0) && a.x.s0 % 4 == 0 &&
-                       a.x.s2 % 4 == 0 && a.x.s3 % 4 == 0;
-    const bool y_vec = a.dy.s1 == 1 && ((reinterpret_cast<uintptr_t>(a.dy.ptr) & 15) == 0) && a.dy.s0 % 4 == 0 &&
-                       a.dy.s2 % 4 == 0 && a.dy.s3 % 4 == 0;
+    const bool x_vec = channel_quads_aligned(a.x, g.cig, g.groups), y_vec = channel_quads_aligned(a.dy, g.cog, g.groups);
     const int total_jobs = kblocks * tasks;  // kblocks <= 2^26, tasks <= 16
     // ---- folding the accumulator into `out` (warps 0 .. 4*nacc-1): lane = row of the accumulator = (block, channel) ----
     // Chunk c of the reduction is complete when the MMA thread's commit flips `accum` for the c-th time.  The first

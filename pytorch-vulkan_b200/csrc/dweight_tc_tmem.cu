@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_tmem_kernel(const Args a) 
     if (leader) umma_commit(smem_u32(&ctrl->accum));
   } else if (warp >= dy_warps) {
     // ---- input chunks: job j = (chunk, strip) goes to warp j mod (warps in use) ----
-    const bool vec = a.x.s1 == 1 && ((reinterpret_cast<uintptr_t>(a.x.ptr) & 15) == 0) && a.x.s0 % 4 == 0 && a.x.s2 % 4 == 0 && a.x.s3 % 4 == 0;
+    const bool vec = channel_quads_aligned(a.x, g.cig, g.groups);
     const int jobs = (kblocks + a.ahead) * a.n_strips;
     // consecutive jobs of a warp stay within `ring` chunks of each other (a waiter must not skip a phase of a slot's barrier)
     const int active = min(MMA_WARP - dy_warps, a.n_strips * a.ring);

@@ -1,0 +1,54 @@
+"""Host checks of rules that decide which path a call takes: the functions of common.cuh that the kernels and their launchers share,
+compiled with g++ and compared with the property they stand for."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CUDA_INC = "/usr/local/cuda/include"
+pytestmark = pytest.mark.skipif(shutil.which("g++") is None or not os.path.isdir(CUDA_INC), reason="needs g++ and the CUDA headers")
+
+
+def _run(tmp_path, source):
+    src = tmp_path / "check.cpp"
+    src.write_text(source)
+    gxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
+    subprocess.check_call([gxx, "-O1", "-std=c++17", "-x", "c++", str(src), "-o", str(tmp_path / "check"), "-I", os.path.join(ROOT, "pytorch-vulkan_b200", "csrc"),
+                           "-I", os.path.join(ROOT, "include"), "-I", CUDA_INC])
+    out = subprocess.run([str(tmp_path / "check")], capture_output=True, text=True)
+    assert out.returncode == 0, out.stdout + out.stderr
+    return out.stdout
+
+
+def test_channel_quads_are_aligned_in_every_group(tmp_path):
+    """Every address that a 16-byte load of a channels-last view would use, over groups whose channel count is no multiple of four and pixels
+    that are padded, offset or sliced: the rule may only say yes where all of them are whole 16-byte pieces, and says it for whole layers."""
+    out = _run(tmp_path, r"""
+#include <cstdio>
+#include "common.cuh"
+int main() {
+  int yes = 0, wrong = 0, missed = 0;
+  for (int groups = 1; groups <= 3; ++groups)
+    for (int per = 30; per <= 68; ++per)
+      for (int pad = 0; pad <= 4; ++pad)
+        for (int offset = 0; offset <= 4; ++offset) {
+          const long long pixel = (long long)groups * per + pad, row = 5 * pixel, image = 3 * row;
+          const b200::View4 v{reinterpret_cast<const float*>(4096) + offset, image, 1, row, pixel};
+          bool aligned = true;
+          for (int n = 0; n < 2; ++n)
+            for (int x = 0; x < 3; ++x)
+              for (int g = 0; g < groups; ++g)
+                for (int c = 0; c < 8; c += 4)
+                  aligned &= reinterpret_cast<uintptr_t>(v.ptr + n * v.s0 + n * v.s2 + x * v.s3 + (long long)g * per + c) % 16 == 0;
+          const bool said = b200::channel_quads_aligned(v, per, groups);
+          yes += said;
+          wrong += said && !aligned;
+          missed += !said && aligned;
+        }
+  printf("%d %d %d\n", yes, wrong, missed);
+  return wrong != 0 || missed != 0 || yes == 0;
+}
+""")
+    assert int(out.split()[1]) == 0
