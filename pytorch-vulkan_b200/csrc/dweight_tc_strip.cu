@@ -518,7 +518,7 @@ int finalize_partials(const float* partial, float* dw, const ConvGeom& g, int sp
   const long long count = (long long)g.cout * g.cig * g.kh * g.kw;
   cudaLaunchConfig_t cfg{};
   const int taps = g.kh * g.kw;
-  const bool vec = g.cig % 4 == 0;
+  const bool vec = g.cig % 4 == 0 && (reinterpret_cast<uintptr_t>(partial) & 15) == 0;   // the caller's workspace may start anywhere
   // channels per block: all of them if they fit the default shared memory, fewer while the blocks do not fill the SMs
   // twice (down to 16: shorter runs waste the sectors at their ends); a single channel needs no shared memory
   int ch_log2 = 0;

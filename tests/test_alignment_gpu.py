@@ -1,4 +1,6 @@
 """Calls whose operands or scratch start off 16 bytes where a kernel has a 16-byte path: the path may not be taken, results stay right."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -24,3 +26,27 @@ def test_grouped_channels_last_dweight(cig, cog, groups, kernel, variant, monkey
     dw = b200conv.conv2d_backward(NHWC(go), NHWC(x), w, padding=pad, groups=groups, mask=(False, True, False), algo="tc")[1]
     assert b200conv.last_kernel() == "tc_strip_dweight" and b200conv.device_status() == 0
     assert oracle.rel_l2(dw, want) <= 1e-5
+
+
+def _dweight(g, x, go, kw, offset, budget):
+    """dWeight through the C ABI with scratch that starts `offset` bytes into its allocation."""
+    L, P = b200conv.lib(), ctypes.c_void_p
+    p = b200conv.geometry(g.x_shape, g.w_shape[0], g.w_shape[2:], **kw)
+    n = b200conv.workspace_bytes(p, b200conv.PHASE_DWEIGHT, budget=budget)
+    assert n > 0                                                       # split: the partial sums go through the scratch
+    vx, vg, ws, dw = b200conv.DeviceView(x), b200conv.DeviceView(go), b200conv.DeviceBuffer(n + 16), b200conv.DeviceBuffer(4 * int(np.prod(g.w_shape)))
+    b200conv.check(L.b200_conv2d_dweight(ctypes.byref(p), vx.view4(), vg.view4(), P(dw.ptr), P(ws.ptr + offset), n, b200conv.ALGO_AUTO, None))
+    return dw.to_numpy(g.w_shape)
+
+
+# one reader of the partial sums for each route: the tensor-memory kernel (3x3), the shared-memory one (1x1, many pixels), grouped
+@pytest.mark.parametrize("offset", [4, 8, 12])
+@pytest.mark.parametrize("xshape,cout,kernel,kw", [((4, 64, 28, 28), 64, (3, 3), dict(padding=(1, 1))), ((8, 256, 52, 52), 64, (1, 1), dict()),
+                                                   ((4, 64, 32, 32), 64, (3, 3), dict(padding=(1, 1), groups=8))], ids=["3x3", "1x1", "grouped"])
+def test_dweight_scratch_off_16_bytes(xshape, cout, kernel, kw, offset):
+    rng = np.random.default_rng(offset)
+    g = oracle.geometry(xshape, cout, kernel, **kw)
+    x, go = rng.standard_normal(g.x_shape, dtype=np.float32), rng.standard_normal(g.y_shape, dtype=np.float32)
+    want = oracle.torch_conv_all(x, np.zeros(g.w_shape, np.float32), None, go, (1, 1), kw.get("padding", (0, 0)), (1, 1), kw.get("groups", 1))[2]
+    got = _dweight(g, x, go, kw, offset, 64 << 20)
+    assert b200conv.device_status() == 0 and oracle.rel_l2(got, want) <= 1e-5
