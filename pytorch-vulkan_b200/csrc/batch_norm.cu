@@ -657,6 +657,7 @@ constexpr int kUnitsBwd = 4;                  // backward: of each of the two te
 template <int VEC, int N>
 __global__ void __launch_bounds__(nres::THREADS, 4) bn_forward_channel_kernel(const float* __restrict__ x, nres::Rows rows, int inner, float m_count,
                                                                            BnForwardVectors v, BnPost post, float* __restrict__ y) {
+  cluster_announce();
   wait_previous();
   auto cluster = nres::cg::this_cluster();
   const int ch = blockIdx.x, rank = (int)cluster.block_rank();
@@ -703,6 +704,7 @@ __global__ void __launch_bounds__(nres::THREADS, 4) bn_forward_channel_kernel(co
 template <int VEC, int N>
 __global__ void __launch_bounds__(nres::THREADS, 4) bn_backward_channel_kernel(const float* __restrict__ x, const float* __restrict__ g, nres::Rows rows,
                                                                             int inner, float m_count, BnBackwardVectors v, float* __restrict__ dx) {
+  cluster_announce();
   wait_previous();
   auto cluster = nres::cg::this_cluster();
   const int ch = blockIdx.x, rank = (int)cluster.block_rank();
@@ -728,6 +730,7 @@ __global__ void __launch_bounds__(nres::THREADS, 4) bn_backward_channel_kernel(c
     }
   __shared__ nres::Table<3> table;
   float s[3] = {t.a, t.b, t.r};
+  cluster_wait_started();
   nres::cluster_sum(s, table, cluster);
   float fa = s[0], fb = s[1], residual = 0.f;
   if (v.training) {

@@ -47,6 +47,11 @@ void launch_next(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem,
 }
 #ifdef __CUDACC__
 __device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Another CTA's shared memory may be touched only once that CTA has started, which being in one cluster does not promise: every thread
+// announces itself at the kernel's entry and waits for the others just before the first remote store, so that the exchange passes under
+// the loads between the two.  Both are executed by all threads of the cluster, in this order, before any other cluster barrier.
+__device__ __forceinline__ void cluster_announce() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait_started() { asm volatile("barrier.cluster.wait;" ::: "memory"); }
 #endif
 
 // ---- device-side geometry ------------------------------------------------------------------

@@ -370,6 +370,7 @@ __global__ void __launch_bounds__(nres::THREADS, 4) gn_forward_cluster_kernel(co
                                                                            const float* __restrict__ beta, GnShape sh, nres::Rows rows, float eps,
                                                                            float* __restrict__ y, float* __restrict__ means,
                                                                            float* __restrict__ rstds) {
+  cluster_announce();
   wait_previous();
   auto cluster = nres::cg::this_cluster();
   const int row = blockIdx.x, rank = (int)cluster.block_rank();
@@ -406,6 +407,7 @@ __global__ void __launch_bounds__(nres::THREADS, 4) gn_backward_cluster_kernel(c
                                                                             const float* __restrict__ means, const float* __restrict__ rstds,
                                                                             const float* __restrict__ gamma, GnShape sh, nres::Rows rows,
                                                                             float* __restrict__ dx, float* __restrict__ plane_sums) {
+  cluster_announce();
   wait_previous();
   auto cluster = nres::cg::this_cluster();
   __shared__ float2 unit_part[N * nres::THREADS];
@@ -436,6 +438,7 @@ __global__ void __launch_bounds__(nres::THREADS, 4) gn_backward_cluster_kernel(c
     unit_part[k * nres::THREADS + threadIdx.x] = make_float2(s1, s2);
   }
   __syncthreads();
+  cluster_wait_started();
   const int p0 = (int)rows.plane_div.div(begin), p1 = begin < end ? (int)rows.plane_div.div(end - 1) + 1 : p0;
   for (int p = p0 + warp; p < p1; p += nres::WARPS) {
     const uint32_t a = max(begin, (uint32_t)p * rows.plane_units) - begin, b = min(end, (uint32_t)(p + 1) * rows.plane_units) - begin;

@@ -53,7 +53,8 @@ __device__ __forceinline__ float warp_total(float v) {
 }
 
 // Sums of C values over the cluster, in every thread and in the same order everywhere: each warp leaves its sums with every rank, so
-// that there is one barrier and no second level inside the CTA.  `table` is used once per kernel.
+// that there is one barrier and no second level inside the CTA.  `table` is used once per kernel.  A kernel's first sum follows its
+// cluster_announce() and a cluster_wait_started().
 template <int C>
 using Table = float[MAX_RANKS * WARPS][C];
 template <int C>
@@ -88,6 +89,7 @@ __device__ __forceinline__ float2 row_moments(const Unit<VEC> (&in)[N], uint32_t
 #pragma unroll
     for (int j = 0; j < VEC; ++j) s[(k * VEC + j) & 3] += u0 + k * THREADS < end ? in[k].v[j] - origin : 0.f;
   float sum[1] = {(s[0] + s[1]) + (s[2] + s[3])}, m2[1];
+  cluster_wait_started();
   cluster_sum(sum, t0, cluster);
   const float mean = sum[0] / count;
   s[0] = s[1] = s[2] = s[3] = 0.f;

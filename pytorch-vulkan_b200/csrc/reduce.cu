@@ -41,6 +41,7 @@ __device__ __forceinline__ float add4(const float4& v) { return (v.x + v.y) + (v
 template <bool VEC, bool DENSE>
 __global__ void __launch_bounds__(THREADS) reduce_planes_kernel(const float* __restrict__ src, long long chan_stride, Rows rows, uint32_t count,
                                                                 float* __restrict__ out, int accumulate) {
+  cluster_announce();
   wait_previous();
   cg::cluster_group cluster = cg::this_cluster();
   const uint32_t ranks = cluster.num_blocks(), rank = cluster.block_rank();
@@ -65,6 +66,7 @@ __global__ void __launch_bounds__(THREADS) reduce_planes_kernel(const float* __r
   __shared__ float slab_part[MAX_CLUSTER];
   if ((threadIdx.x & 31) == 0) warp_part[threadIdx.x >> 5] = sum;
   __syncthreads();
+  cluster_wait_started();
   if (threadIdx.x == 0) {
     float v = 0.f;
 #pragma unroll
@@ -85,6 +87,7 @@ __global__ void __launch_bounds__(THREADS) reduce_planes_kernel(const float* __r
 template <int LPR, bool VEC, bool DENSE>
 __global__ void __launch_bounds__(COL_THREADS) reduce_columns_kernel(const float* __restrict__ src, Rows rows, uint32_t count, int cols,
                                                                  float* __restrict__ out, int accumulate) {
+  cluster_announce();
   wait_previous();
   cg::cluster_group cluster = cg::this_cluster();
   const uint32_t cluster_ranks = cluster.num_blocks(), cluster_rank = cluster.block_rank();
@@ -127,6 +130,7 @@ __global__ void __launch_bounds__(COL_THREADS) reduce_columns_kernel(const float
   __shared__ float slab_part[MAX_CLUSTER][4 * LPR];
   if (lane < LPR) warp_part[warp][lane] = sum;
   __syncthreads();
+  cluster_wait_started();
   if (threadIdx.x < 4 * LPR) {
     float v = 0.f;
 #pragma unroll

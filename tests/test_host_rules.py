@@ -52,3 +52,36 @@ int main() {
 }
 """)
     assert int(out.split()[1]) == 0
+
+
+CLUSTER_SOURCES = ("reduce.cu", "batch_norm.cu", "group_norm.cu", "norm_resident.cuh")
+
+
+def _functions(name):
+    """(name, body) of the kernels and device functions of a source file that hold or reach a store into another CTA's shared memory."""
+    import re
+    with open(os.path.join(ROOT, "pytorch-vulkan_b200", "csrc", name)) as f:
+        text = re.sub(r"//[^\n]*", "", f.read())
+    for m in re.finditer(r"\n__(?:global|device)__[^;{]*?\b(\w+)\([^;{]*\)\s*\{", text):
+        end = text.find("\n}", m.end())
+        yield m.group(1), m.group(0).startswith("\n__global__"), text[m.end():end]
+
+
+def test_clusters_wait_until_every_cta_has_started():
+    """CUDA allows access to another CTA's shared memory only once that CTA runs.  In every kernel that reaches such a store, all threads
+    announce themselves before anything else, and wait for the other CTAs before the first store."""
+    waits_itself = {"row_moments"}          # holds the wait ahead of its first sum
+    checked = 0
+    for name in CLUSTER_SOURCES:
+        for function, kernel, body in _functions(name):
+            stores = [body.find(w) for w in ("map_shared_rank", "cluster_sum(", "row_moments<") if w in body]
+            if not stores or function == "cluster_sum":
+                continue
+            waited, first = body.find("cluster_wait_started()"), min(stores)
+            inside = any(f + "<" in body and body.find(f + "<") == first for f in waits_itself)
+            assert inside or 0 <= waited < first, f"{name}: {function} stores into another CTA before it knows that it runs"
+            if kernel:
+                announced = body.find("cluster_announce()")
+                assert 0 <= announced < body.find("wait_previous()"), f"{name}: {function} does not announce itself first"
+                checked += 1
+    assert checked == 6
