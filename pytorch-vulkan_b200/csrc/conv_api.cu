@@ -239,7 +239,7 @@ int b200_conv2d_forward_fused(const b200_conv_params* p, b200_view4 x, b200_view
   if (chosen == B200_ALGO_TC && strip_supported(g, B200_PHASE_FORWARD)) {
     note_kernel("tc_strip_forward_fused");
     if (const int slices = y_channels_last || !strip_view_addressable(g, false, to_view(x), nullptr) ? 1 : conv_slices(g, false, false);
-        slices > 1 && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0 && conv_slices_workspace(g, false, slices, false) <= workspace_bytes)
+        slices > 1 && workspace && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0 && conv_slices_workspace(g, false, slices, false) <= workspace_bytes)
       return conv_sliced(g, false, slices, false, to_view(x), to_view(w), bias, bias_stride, &post, y, workspace, st);
     const int rc = strip_conv(g, false, to_view(x), to_view(w), bias, bias_stride, y, workspace, workspace_bytes, st,
                               y_channels_last != 0, 1.f, 1.f, nullptr, &post);

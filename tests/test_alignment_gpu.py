@@ -50,3 +50,17 @@ def test_dweight_scratch_off_16_bytes(xshape, cout, kernel, kw, offset):
     want = oracle.torch_conv_all(x, np.zeros(g.w_shape, np.float32), None, go, (1, 1), kw.get("padding", (0, 0)), (1, 1), kw.get("groups", 1))[2]
     got = _dweight(g, x, go, kw, offset, 64 << 20)
     assert b200conv.device_status() == 0 and oracle.rel_l2(got, want) <= 1e-5
+
+
+@pytest.mark.parametrize("channels,hw", [(512, 7), (64, 28)])          # with the reduction in slices, and whole
+@pytest.mark.parametrize("offset", [None, 4])                          # no scratch at all, scratch that is not 16-byte aligned
+def test_fused_forward_refuses_unusable_scratch(channels, hw, offset):
+    L, P = b200conv.lib(), ctypes.c_void_p
+    p = b200conv.geometry((1, channels, hw, hw), channels, (3, 3), padding=(1, 1))
+    n = 256 << 20                                                      # as much as the caller says, nothing of it may be touched
+    x, w = b200conv.DeviceView(np.zeros((1, channels, hw, hw), np.float32)), b200conv.DeviceView(np.zeros((channels, channels, 3, 3), np.float32))
+    y, ws = b200conv.DeviceBuffer(4 * channels * hw * hw), b200conv.DeviceBuffer(16)
+    none = b200conv.View4(None, (ctypes.c_int64 * 4)(0, 0, 0, 0))
+    scratch = None if offset is None else P(ws.ptr + offset)
+    with pytest.raises(b200conv.B200Error, match="workspace"):
+        b200conv.check(L.b200_conv2d_forward_fused(ctypes.byref(p), x.view4(), w.view4(), None, 0, none, 1, P(y.ptr), 0, scratch, n, b200conv.ALGO_TC, None))
