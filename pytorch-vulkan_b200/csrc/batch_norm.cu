@@ -645,12 +645,8 @@ __global__ void __launch_bounds__(kThreads) bn_bwd_apply_scalar_kernel(const flo
 }
 
 // ---- channels held in registers, one launch ---------------------------------------------------------
-// Planar tensors whose channels fit the registers of a cluster (norm_resident.cuh): each tensor is read
-// once, and the latency of one load, one exchange and one store replaces that of three launches.
-// 64 images of 256 channels of 14x14: forward 17.7 us with one CTA of 1024 threads a channel and a second
-// read from L2, now 9.8 (the
-// traffic takes 4 at HBM rate; the rest is launch, load latency and the two exchanges); backward 18.7, now 12.5.  512 channels of 7x7: 37 us for both
-// directions in three launches each, now 19.
+// Planar tensors whose channels fit the registers of a cluster (norm_resident.cuh) and gain by it (norm_plan.cuh): each tensor is
+// read once, and the latency of one load, one exchange and one store replaces that of three launches.
 constexpr int kUnits = 8, kUnits1 = 16;       // most units a thread holds: forward (16 bytes each), single values
 constexpr int kUnitsBwd = 4;                  // backward: of each of the two tensors
 
@@ -757,11 +753,11 @@ __global__ void __launch_bounds__(nres::THREADS, 4) bn_backward_channel_kernel(c
   }
 }
 
-// Ranks per channel for the kernels above, or 0: the channel does not fit.
-int channel_ranks(const BnShape& sh, int layout, int vec, int most) {
-  static const bool enabled = !(getenv("B200_BN_ONE_LAUNCH") && getenv("B200_BN_ONE_LAUNCH")[0] == '0');  // testing aid
-  if (!enabled || layout != B200_BN_PLANAR || sh.inner / vec >= (1 << 30) / sh.outer) return 0;
-  return nres::ranks_for((long long)sh.outer * (sh.inner / vec), sh.c, most);
+// Ranks per channel for the kernels above, or 0: the streaming kernels take the call.
+int channel_ranks(const BnShape& sh, int layout, int vec, int most, bool backward) {
+  if (layout != B200_BN_PLANAR || sh.inner / vec >= (1 << 30) / sh.outer) return 0;
+  const nres::RankPlan p = nres::plan_ranks((long long)sh.outer * (sh.inner / vec), sh.c, most, sm_count());
+  return nres::batch_norm_resident(p, vec, sh.inner, backward) ? p.ranks : 0;
 }
 
 // ---- host side ---------------------------------------------------------------------------------
@@ -885,7 +881,7 @@ int b200_batch_norm_forward_fused(int64_t n, int64_t c, int64_t s, int layout, c
   const uint32_t total = (uint32_t)((int64_t)sh.outer * sh.cols);
   if (training) {
     const int vec = sh.inner % 4 == 0 && aligned16(x) && aligned16(y) && aligned16(residual) ? 4 : 1;
-    if (const int ranks = channel_ranks(sh, layout, vec, vec == 4 ? kUnits : kUnits1)) {
+    if (const int ranks = channel_ranks(sh, layout, vec, vec == 4 ? kUnits : kUnits1, false)) {
       note_kernel(residual || relu ? "bn_forward_channel_fused" : "bn_forward_channel");
       const nres::Rows rows = nres::make_rows(sh.outer, sh.inner, vec, (long long)sh.c * sh.inner, ranks);
       return nres::launch(vec == 4 ? bn_forward_channel_kernel<4, kUnits> : bn_forward_channel_kernel<1, kUnits1>, (unsigned)sh.c, ranks, st, x, rows,
@@ -978,7 +974,7 @@ int b200_batch_norm_backward(int64_t n, int64_t c, int64_t s, int layout, const 
   const int has_sums = training || dw || db;
   if (has_sums) {
     const int vec = sh.inner % 4 == 0 && aligned16(x) && aligned16(grad) && aligned16(dx) ? 4 : 1;
-    if (const int ranks = channel_ranks(sh, layout, vec, vec == 4 ? kUnitsBwd : kUnits1)) {
+    if (const int ranks = channel_ranks(sh, layout, vec, vec == 4 ? kUnitsBwd : kUnits1, true)) {
       note_kernel("bn_backward_channel");
       const nres::Rows rows = nres::make_rows(sh.outer, sh.inner, vec, (long long)sh.c * sh.inner, ranks);
       return nres::launch(vec == 4 ? bn_backward_channel_kernel<4, kUnitsBwd> : bn_backward_channel_kernel<1, kUnits1>, (unsigned)sh.c, ranks, st, x,

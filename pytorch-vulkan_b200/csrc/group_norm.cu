@@ -488,6 +488,12 @@ __global__ void __launch_bounds__(nres::THREADS, 4) gn_backward_cluster_kernel(c
   }
 }
 
+// Ranks per block for the kernels above, or 0: the streaming kernels take the call.
+int block_ranks(const GnShape& sh, int blocks, int vec, int most, bool backward) {
+  const nres::RankPlan p = nres::plan_ranks((long long)sh.cpg * sh.hw / vec, blocks, most, sm_count());
+  return nres::group_norm_resident(p, vec, sh.hw, backward, blocks <= 3 * sm_count()) ? p.ranks : 0;
+}
+
 // dgamma[ch] = sum over samples of s2, dbeta[ch] = sum of s1 (the result of
 // group_norm_backward_affine.comp:16-31).  One warp per channel: lane l adds samples l, l + 32, ...
 // in order and the lanes are folded by shuffles, so the result does not depend on the launch.
@@ -570,7 +576,7 @@ int b200_group_norm_forward(int64_t n, int64_t c, int64_t hw, int64_t groups, co
   }
   note_kernel("gn_forward");
   const int vec = sh.hw % 4 == 0 && aligned ? 4 : 1;
-  if (const int ranks = nres::ranks_for((long long)sh.cpg * sh.hw / vec, blocks, vec == 4 ? kUnits : kUnits1))
+  if (const int ranks = block_ranks(sh, blocks, vec, vec == 4 ? kUnits : kUnits1, false))
     return nres::launch(vec == 4 ? gn_forward_cluster_kernel<4, kUnits> : gn_forward_cluster_kernel<1, kUnits1>, (unsigned)blocks, ranks, st, x, weight, bias,
                         sh, nres::make_rows(sh.cpg, sh.hw, vec, sh.hw, ranks), eps, y, mean, rstd);
   launch_next(gn_forward_kernel, (unsigned)(n * groups), kThreads, 0, st, x, weight, bias, sh, eps, y, mean, rstd);
@@ -594,7 +600,7 @@ int b200_group_norm_backward(int64_t n, int64_t c, int64_t hw, int64_t groups, c
   note_kernel(affine ? "gn_backward+affine" : "gn_backward");
   const bool aligned = ((reinterpret_cast<uintptr_t>(grad) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dx)) & 15) == 0;
   const int vec = sh.hw % 4 == 0 && aligned ? 4 : 1, blocks = (int)(n * groups);
-  const int ranks = sh.cpg <= kResidentChannels ? nres::ranks_for((long long)sh.cpg * sh.hw / vec, blocks, vec == 4 ? kUnitsBwd : kUnits1) : 0;
+  const int ranks = sh.cpg <= kResidentChannels ? block_ranks(sh, blocks, vec, vec == 4 ? kUnitsBwd : kUnits1, true) : 0;
   if (ranks) {
     const nres::Rows rows = nres::make_rows(sh.cpg, sh.hw, vec, sh.hw, ranks);
     if (int rc = nres::launch(vec == 4 ? gn_backward_cluster_kernel<4, kUnitsBwd> : gn_backward_cluster_kernel<1, kUnits1>, (unsigned)blocks, ranks, st, grad,

@@ -9,12 +9,13 @@
 #include <cooperative_groups.h>
 
 #include "common.cuh"
+#include "norm_plan.cuh"
 
 namespace b200 {
 namespace nres {
 namespace cg = cooperative_groups;
 
-constexpr int THREADS = 256, WARPS = THREADS / 32, MAX_RANKS = 16;
+constexpr int THREADS = PLAN_THREADS, WARPS = THREADS / 32, MAX_RANKS = PLAN_MAX_RANKS;
 
 struct Rows {
   uint32_t units, per;        // units of a row; of one rank
@@ -103,18 +104,6 @@ __device__ __forceinline__ float2 row_moments(const Unit<VEC> (&in)[N], uint32_t
   m2[0] = (s[0] + s[1]) + (s[2] + s[3]);
   cluster_sum(m2, t1, cluster);
   return make_float2(mean, m2[0]);
-}
-
-// Ranks of a cluster for rows of `units` when a thread holds up to `most` units, or 0 when even sixteen ranks do not hold one:
-// as few as hold the row (a wider exchange costs more than a fuller thread: 256 channels of 12544 values forward 9.5 us with 2 ranks of
-// eight units a thread, 12.5 with 4 of four), then twice as many while all CTAs still run at once, four to an SM, and a thread has
-// more than two units (20 rows and fewer would leave most SMs idle).
-inline int ranks_for(long long units, long long rows, int most) {
-  long long ranks = (units + (long long)THREADS * most - 1) / ((long long)THREADS * most);
-  if (ranks > MAX_RANKS) return 0;
-  if (ranks > 8) ranks = MAX_RANKS;
-  while (ranks <= MAX_RANKS / 2 && rows * ranks * 2 <= 4ll * sm_count() && units > ranks * THREADS * 2) ranks *= 2;
-  return (int)(ranks > 8 ? MAX_RANKS : ranks);
 }
 
 inline Rows make_rows(int planes, int plane, int vec, long long plane_stride, int ranks) {

@@ -85,3 +85,39 @@ def test_clusters_wait_until_every_cta_has_started():
                 assert 0 <= announced < body.find("wait_previous()"), f"{name}: {function} does not announce itself first"
                 checked += 1
     assert checked == 6
+
+
+def test_norm_rank_plans_hold_their_rows(tmp_path):
+    """Every plan for a row that stays resident gives its threads all units (no more than `most` each, no rank empty for want of units), widens
+    only as far as all CTAs run at once, and the rows that the resident kernels took at a loss stream: forward passes of single values over
+    several waves of wide clusters."""
+    _run(tmp_path, r"""
+#include <cstdio>
+#include <initializer_list>
+#include "norm_plan.cuh"
+using namespace b200::nres;
+int main() {
+  int wrong = 0, resident = 0, streams = 0;
+  const int sms = 148;
+  for (int most : {4, 8, 16})
+    for (long long units = 1; units < 80000; units = units * 9 / 8 + 1)
+      for (long long rows = 1; rows < 5000; rows = rows * 3 / 2 + 1) {
+        const RankPlan p = plan_ranks(units, rows, most, sms);
+        const long long holds = 256ll * most;
+        if (units > 16 * holds) { wrong += p.ranks != 0; continue; }
+        wrong += p.ranks < 1 || p.ranks > 16 || (units + p.ranks - 1) / p.ranks > holds || p.need != (units + holds - 1) / holds;
+        if (p.ranks != p.need) wrong += p.ranks > 8 || rows * p.ranks > 4 * sms || units <= p.ranks / 2 * 512;
+        for (int vec : {1, 4})
+          for (int backward = 0; backward < 2; ++backward)
+            for (long long plane : {49, 225, 900, 3136}) {
+              const bool b = batch_norm_resident(p, vec, plane, backward), g = group_norm_resident(p, vec, plane, backward, rows <= 3 * sms);
+              (b ? resident : streams) += 1;
+              if (p.waves <= 1.0 || vec == 4 || backward) wrong += !b || !g;
+              else if (p.need > 8 && p.waves > 4.0) wrong += b || g;
+              else if (p.need > 4 && p.waves > 2.0 && plane > 256) wrong += b || (p.need <= 8 && g);
+            }
+      }
+  printf("%d %d %d\n", wrong, resident, streams);
+  return wrong != 0 || resident == 0 || streams == 0;
+}
+""")
