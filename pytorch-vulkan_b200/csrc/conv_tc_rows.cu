@@ -1,10 +1,17 @@
 // Persistent tcgen05 kernel for convolution forward passes with a SHORT reduction (input channels x taps up to a few
-// hundred): a network's first layer (1, 3 or 4 input channels, 3x3 or 7x7 filters).  FP32 by the split-precision scheme of
-// tc_common.cuh.
+// hundred): a network's first layer (1, 3 or 4 input channels, 3x3 or 7x7 filters).  FP32 by three TF32 products (tc_common.cuh).
+//
+// These layers ran in plain FP32 before, so their sums are kept close to it.  The tensor core truncates every addition to the accumulator:
+// with the BF16 cross terms of the other kernels in one chain of 48 steps, a 7x7 layer of 3 channels was off by 1.1e-6 against 2.2e-7
+// in FP32.  Here the cross terms are TF32 too (their operands cost the same bytes, and the producers save the packing), and beyond
+// two K blocks they go to an accumulator of their own, where they lose nothing that counts; the chain of the main products then has
+// 48 steps at most (SEG_KB), and the epilogue adds the pieces in FP32: 5.6e-7 for that layer, 8.7e-7 for the longest reductions (3.5e-6 in
+// one chain; FP32 4.4e-7).  The time is that of one BF16 chain within 2 %, but for 7x7 filters with more than 64 output channels, whose single
+// pair of accumulators makes the next tile's products wait (5 images of 179x179, 3 -> 112 channels: 44.5 us, now 56.4).
 //
 // What bounds these layers and what follows from it.  A 3 -> 64 channel 7x7 layer has 147 products per output: the whole
 // filter fits shared memory, so every CTA splits it once and keeps it (no staging kernel, no workspace), and the tensor
-// work is small enough that feeding the tensor core is the problem: 1307 us on the CUDA-core kernel, 137 us here (batch 64,
+// work is small enough that feeding the tensor core is the problem: 1307 us on the CUDA-core kernel, 141 us here (batch 64,
 // 224x224, stride 2), of which the loads are a fifth and the tensor-memory stores with their splits a third.  The im2col rows are therefore never written to shared
 // memory: a producer thread owns one output pixel (one accumulator row), gathers 32 of its reduction values straight
 // into registers (coalesced across the warp's consecutive pixels, L1 serving the overlap of the windows), splits them and
@@ -13,9 +20,9 @@
 // that reading both operands from shared memory takes.
 //
 // CTA roles: warps 0-3 epilogue, GROUPS groups of four producer warps (a group stages one K block of 128 pixels x 32
-// reduction values at a time; three groups fit the register file beside the rest), one MMA warp.  Tensor memory: two accumulators
-// and (512 - 2 * columns) / 64 operand stages of 64 columns (32 TF32 values; 16 columns of bf16 pairs of the high parts, 16 of
-// the low parts).
+// reduction values at a time; three groups fit the register file beside the rest: eight epilogue warps would leave 80 registers a thread and
+// spills), one MMA warp.  Tensor memory: two accumulators, or pairs of them (main, cross; one pair where they have more than 64 columns), the
+// rest operand stages of 64 columns (32 high parts, 32 low parts).
 //
 // Replaces csrc/shaders/conv2d_tiled_body.glsl:53-86 of the reference for these geometries.
 #include "common.cuh"
@@ -23,6 +30,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 namespace b200 {
 namespace tcr {
@@ -32,6 +40,7 @@ constexpr int BLOCK_M = 128, KBLK = 32, EPI_WARPS = 4;
 constexpr int GROUPS = 3;
 constexpr int MMA_WARP = EPI_WARPS + 4 * GROUPS, THREADS = (MMA_WARP + 1) * 32;
 constexpr int MAX_STAGES = 6, MAX_RUNS = 1024;
+constexpr int SEG_KB = 12;      // K blocks (of four main steps) per accumulation chain
 constexpr int SMEM_LIMIT = 232448 - 2048;
 constexpr uint32_t STAGE_COLS = 64;
 
@@ -44,9 +53,11 @@ struct RowsArgs {
   // The window of a pixel is `runs` runs of `run_len` values `run_step` elements apart (unit step where memory allows: the taps
   // of a filter row in NCHW, the taps x channels of a row in channels-last), each padded to LP reduction indices.
   int runs, run_len, nkb;
+  int segs, seg_kb;      // accumulation chains of a tile, K blocks of one
   long long run_step;
   int channels_last;     // a run holds (kx, ci) rather than kx
   int bn, acc_cols, ntn; // columns per tile (multiple of 16), accumulator pitch in tensor memory, column tiles of a CTA
+  int bufs;              // accumulators, or pairs of them
   int nt_split;          // CTAs that share a pixel tile, each with its own `ntn` column tiles (a filter too large for one CTA)
   int stages, tiles_m;
   uint32_t m_total;      // output pixels
@@ -64,13 +75,14 @@ struct RunEntry {
   int ky;                // filter row (its bit of the row mask)
 };
 
-template <int LP, bool UNIT>
+// PAIR: the cross terms have an accumulator of their own
+template <int LP, bool UNIT, bool PAIR>
 __global__ void __launch_bounds__(THREADS, 1) conv_rows_kernel(const RowsArgs a) {
   wait_previous();
   extern __shared__ unsigned char smem_raw[];
   const ConvGeom& g = a.g;
   const uint32_t raw = smem_u32(smem_raw), w_base = (raw + 1023u) & ~1023u;
-  const uint32_t w_plane = (uint32_t)a.bn * 128u, w_block = 2u * w_plane;   // one K block of one column tile: hi plane, cross plane
+  const uint32_t w_plane = (uint32_t)a.bn * 128u, w_block = 2u * w_plane;   // one K block of one column tile: high parts, low parts
   unsigned char* w_smem = smem_raw + (w_base - raw);
   RunEntry* tab = reinterpret_cast<RunEntry*>(w_smem + (size_t)a.ntn * a.nkb * w_block);
   Ctrl* ctrl = reinterpret_cast<Ctrl*>(tab + a.nkb * (KBLK / LP));
@@ -102,7 +114,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv_rows_kernel(const RowsArgs a)
     }
     tab[r] = e;
   }
-  // the filter, split once per CTA: per (column tile, K block) a TF32 plane and a plane of [bf16(lo) x32 | bf16(hi) x32] rows
+  // the filter, split once per CTA: per (column tile, K block) a plane of the high parts and one of the low parts
   for (int i = threadIdx.x; i < a.ntn * a.nkb * a.bn * 8; i += THREADS) {
     const int piece = i & 7, rest = i >> 3, row_all = rest % (a.ntn * a.bn), kb = rest / (a.ntn * a.bn);
     const int nt = row_all / a.bn, row = row_all - nt * a.bn;
@@ -120,45 +132,49 @@ __global__ void __launch_bounds__(THREADS, 1) conv_rows_kernel(const RowsArgs a)
     }
     const uint32_t plane = w_base + (uint32_t)(nt * a.nkb + kb) * w_block;
     sts_f32x4(plane + sw128_offset(row, piece * 4), hi[0], hi[1], hi[2], hi[3]);
-    sts_b32x2(plane + w_plane + sw128_offset_bf16(row, piece * 4), pack_bf16x2(lo[0], lo[1]), pack_bf16x2(lo[2], lo[3]));
-    sts_b32x2(plane + w_plane + sw128_offset_bf16(row, 32 + piece * 4), pack_bf16x2(hi[0], hi[1]), pack_bf16x2(hi[2], hi[3]));
+    sts_f32x4(plane + w_plane + sw128_offset(row, piece * 4), lo[0], lo[1], lo[2], lo[3]);
   }
   fence_proxy_async();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&ctrl->tmem_base);
-  const uint32_t a_cols = tmem_base + 2u * (uint32_t)a.acc_cols;   // first operand stage
+  const uint32_t acc_pitch = (uint32_t)a.acc_cols * (PAIR ? 2u : 1u), a_cols = tmem_base + (uint32_t)a.bufs * acc_pitch;   // a_cols: first operand stage
   const int my_tiles = a.tiles_m > (int)cta ? (a.tiles_m - (int)cta + (int)ctas - 1) / (int)ctas : 0;
   const int jobs_per_tile = a.ntn * a.nkb;
 
   if (warp == MMA_WARP) {
     const bool leader = elect_one();
-    const uint32_t idesc = make_idesc_tf32(BLOCK_M, a.bn), idesc_cross = make_idesc_bf16(BLOCK_M, a.bn);
+    const uint32_t idesc = make_idesc_tf32(BLOCK_M, a.bn);
     const uint64_t w_desc = make_kmajor_sw128_desc(w_base);
-    uint32_t s = 0, par = 0, t_count = 0;
+    uint32_t s = 0, par = 0, ab = 0, acc_par = 1;
     bool alive = true;
     for (int t = 0; t < my_tiles && alive; ++t) {
-      for (int nt = 0; nt < a.ntn && alive; ++nt, ++t_count) {
-        const uint32_t ab = t_count & 1u;
-        if (!warp_wait(smem_u32(&ctrl->acc_empty[ab]), ((t_count >> 1) & 1u) ^ 1u, abort_flag, a.status, STATUS_TIMEOUT_ACCUM)) { alive = false; break; }
-        tc_fence_after();
-        const uint32_t acc = tmem_base + ab * (uint32_t)a.acc_cols;
-        for (int kb = 0; kb < a.nkb; ++kb) {
-          if (!warp_wait(smem_u32(&ctrl->full[s]), par, abort_flag, a.status, STATUS_TIMEOUT_FULL)) { alive = false; break; }
+      for (int nt = 0; nt < a.ntn && alive; ++nt) {
+        for (int seg = 0; seg < a.segs && alive; ++seg) {
+          if (!warp_wait(smem_u32(&ctrl->acc_empty[ab]), acc_par, abort_flag, a.status, STATUS_TIMEOUT_ACCUM)) { alive = false; break; }
           tc_fence_after();
-          const uint32_t ta = a_cols + s * STAGE_COLS;
-          const uint64_t bh = w_desc + (uint64_t)((uint32_t)(nt * a.nkb + kb) * (w_block >> 4)), bc = bh + (w_plane >> 4);
-          if (leader) {
+          const uint32_t acc = tmem_base + ab * acc_pitch, cross = PAIR ? acc + (uint32_t)a.acc_cols : acc;
+          const int kb0 = seg * a.seg_kb, kb1 = min(a.nkb, kb0 + a.seg_kb);
+          for (int kb = kb0; kb < kb1; ++kb) {
+            if (!warp_wait(smem_u32(&ctrl->full[s]), par, abort_flag, a.status, STATUS_TIMEOUT_FULL)) { alive = false; break; }
+            tc_fence_after();
+            const uint32_t ta = a_cols + s * STAGE_COLS, later = (uint32_t)(kb != kb0);
+            const uint64_t bh = w_desc + (uint64_t)((uint32_t)(nt * a.nkb + kb) * (w_block >> 4)), bl = bh + (w_plane >> 4);
+            if (leader) {
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk) umma_tf32_ts(acc, ta + 8 * kk, bh + 2 * kk, idesc, (uint32_t)((kb | kk) != 0));
+              for (int kk = 0; kk < 4; ++kk) umma_tf32_ts(cross, ta + 8 * kk, bl + 2 * kk, idesc, kk ? 1u : later);
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk) umma_bf16_ts(acc, ta + 32 + 8 * kk, bc + 2 * kk, idesc_cross, 1);
-            umma_commit(smem_u32(&ctrl->empty[s]));
+              for (int kk = 0; kk < 4; ++kk) umma_tf32_ts(cross, ta + 32 + 8 * kk, bh + 2 * kk, idesc, 1);
+#pragma unroll
+              for (int kk = 0; kk < 4; ++kk) umma_tf32_ts(acc, ta + 8 * kk, bh + 2 * kk, idesc, kk || !PAIR ? 1u : later);
+              umma_commit(smem_u32(&ctrl->empty[s]));
+            }
+            if (++s == (uint32_t)a.stages) { s = 0; par ^= 1; }
           }
-          if (++s == (uint32_t)a.stages) { s = 0; par ^= 1; }
+          if (alive && leader) umma_commit(smem_u32(&ctrl->acc_full[ab]));
+          if (++ab == (uint32_t)a.bufs) { ab = 0; acc_par ^= 1u; }
         }
-        if (alive && leader) umma_commit(smem_u32(&ctrl->acc_full[ab]));
       }
     }
   } else if (warp >= EPI_WARPS) {
@@ -203,17 +219,12 @@ __global__ void __launch_bounds__(THREADS, 1) conv_rows_kernel(const RowsArgs a)
       tc_fence_after();
       const uint32_t ta = a_cols + s * STAGE_COLS + lane_base;
       uint32_t r[32], c[32];
-      float lo[KBLK];
 #pragma unroll
       for (int i = 0; i < KBLK; ++i) {
-        float h;
-        split_tf32_fast(v[i], h, lo[i]);
+        float h, l;
+        split_tf32_fast(v[i], h, l);
         r[i] = __float_as_uint(h);
-      }
-#pragma unroll
-      for (int i = 0; i < KBLK / 2; ++i) {
-        c[i] = pack_bf16x2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
-        c[16 + i] = pack_bf16x2(lo[2 * i], lo[2 * i + 1]);
+        c[i] = __float_as_uint(l);
       }
       tmem_st32(ta, r);
       tmem_st32(ta + 32, c);
@@ -233,7 +244,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv_rows_kernel(const RowsArgs a)
   } else {
     // ------------------------------ epilogue: lane = pixel, a warp stores 32 consecutive pixels of one channel ------------------------------
     const long long plane = (long long)g.oh * g.ow;
-    uint32_t t_count = 0;
+    uint32_t ab = 0, acc_par = 0;
     bool alive = true;
     for (int t = 0; t < my_tiles && alive; ++t) {
       const uint32_t m = (cta + (uint32_t)t * ctas) * BLOCK_M + (uint32_t)(warp * 32 + lane);
@@ -243,34 +254,41 @@ __global__ void __launch_bounds__(THREADS, 1) conv_rows_kernel(const RowsArgs a)
         const uint32_t n = a.img_div.div(m), rem = m - n * (uint32_t)plane;
         obase = (long long)n * g.cout * plane + rem;
       }
-      for (int nt = 0; nt < a.ntn; ++nt, ++t_count) {
-        const uint32_t ab = t_count & 1u;
+      for (int piece = 0; piece < a.ntn * a.segs; ++piece) {    // (column tile, chain)
+        const int nt = a.segs == 1 ? piece : piece / a.segs, seg = piece - nt * a.segs;
         const int cols = min(a.bn, g.cout - ch0 - nt * a.bn);   // may be <= 0 in the last CTA of a split
-        if (!warp_wait(smem_u32(&ctrl->acc_full[ab]), (t_count >> 1) & 1u, abort_flag, a.status, STATUS_TIMEOUT_ACCUM)) { alive = false; break; }
+        const uint32_t done = smem_u32(&ctrl->acc_empty[ab]);
+        if (!warp_wait(smem_u32(&ctrl->acc_full[ab]), acc_par, abort_flag, a.status, STATUS_TIMEOUT_ACCUM)) { alive = false; break; }
         tc_fence_after();
         if (cols <= 0) {
           tc_fence_before();
-          mbar_arrive(smem_u32(&ctrl->acc_empty[ab]));
+          mbar_arrive(done);
         }
-        const uint32_t acc = tmem_base + ab * (uint32_t)a.acc_cols + ((uint32_t)(warp * 32) << 16);
+        const uint32_t acc = tmem_base + ab * acc_pitch + ((uint32_t)(warp * 32) << 16);
+        if (++ab == (uint32_t)a.bufs) { ab = 0; acc_par ^= 1u; }
 #pragma unroll 1
         for (int c0 = 0; c0 < cols; c0 += 32) {
           float v[32];
-          tmem_ld32(acc + (uint32_t)c0, v);
+          if (PAIR) tmem_ld32_sum(acc + (uint32_t)c0, acc + (uint32_t)(a.acc_cols + c0), v);
+          else tmem_ld32(acc + (uint32_t)c0, v);
           if (c0 + 32 >= cols) {
             tc_fence_before();
-            mbar_arrive(smem_u32(&ctrl->acc_empty[ab]));
+            mbar_arrive(done);
           }
           const int nvalid = min(32, cols - c0);
           const int ch = ch0 + nt * a.bn + c0;
-          if (a.bias) {
+          if (a.bias && seg == 0) {
             float bv = lane < nvalid ? __ldg(a.bias + (long long)(ch + lane) * a.bias_stride) : 0.f;
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] += __shfl_sync(0xffffffffu, bv, i);
           }
           if (ok) {
             float* p = a.out + obase + (long long)ch * plane;
-            if (nvalid == 32) {
+            if (PAIR && seg > 0) {      // onto what this thread stored for the chain before: one writer per address, in program order
+#pragma unroll
+              for (int i = 0; i < 32; ++i, p += plane)
+                if (i < nvalid) atomicAdd(p, v[i]);
+            } else if (nvalid == 32) {
 #pragma unroll
               for (int i = 0; i < 32; ++i, p += plane) *p = v[i];
             } else {
@@ -293,7 +311,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv_rows_kernel(const RowsArgs a)
 
 struct RowsPlan {
   bool ok = false;
-  int runs = 0, run_len = 0, lp = 0, nkb = 0, ntn = 0, nt_split = 1, bn = 0, acc_cols = 0, stages = 0, smem = 0;
+  int runs = 0, run_len = 0, lp = 0, nkb = 0, ntn = 0, nt_split = 1, bn = 0, acc_cols = 0, pair = 0, bufs = 0, stages = 0, smem = 0;
 };
 // `channels_last`: the values of a filter row (taps x channels) are adjacent, so they form one run.
 static RowsPlan plan_rows(const ConvGeom& g, bool channels_last) {
@@ -316,20 +334,22 @@ static RowsPlan plan_rows(const ConvGeom& g, bool channels_last) {
   p.nt_split = ((g.cout + p.bn - 1) / p.bn + p.ntn - 1) / p.ntn;
   if (p.nt_split > 8) return p;
   p.acc_cols = (p.bn + 31) / 32 * 32;
-  p.stages = std::min<int>(MAX_STAGES, (512 - 2 * p.acc_cols) / (int)STAGE_COLS);
+  p.pair = p.nkb > 2;
+  p.bufs = p.pair && p.acc_cols > 64 ? 1 : 2;
+  p.stages = std::min<int>(MAX_STAGES, (512 - (p.bufs * p.acc_cols << p.pair)) / (int)STAGE_COLS);
   const long long smem = bytes(p.ntn, p.bn);
   p.smem = (int)smem;
   p.ok = (long long)g.n * g.oh * g.ow < 2147483647ll - (1 << 20);
   return p;
 }
 
-template <int LP, bool UNIT>
+template <int LP, bool UNIT, bool PAIR>
 static int launch_rows(const RowsArgs& a, int smem, cudaStream_t st) {
   static std::once_flag once;
   static cudaError_t opt_in = cudaSuccess;
-  std::call_once(once, [] { opt_in = cudaFuncSetAttribute(conv_rows_kernel<LP, UNIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448); });
+  std::call_once(once, [] { opt_in = cudaFuncSetAttribute(conv_rows_kernel<LP, UNIT, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448); });
   B200_CUDA(opt_in);
-  launch_next(conv_rows_kernel<LP, UNIT>, (unsigned)(std::min(a.tiles_m, std::max(1, sm_count() / a.nt_split)) * a.nt_split), THREADS, (size_t)smem, st, a);
+  launch_next(conv_rows_kernel<LP, UNIT, PAIR>, (unsigned)(std::min(a.tiles_m, std::max(1, sm_count() / a.nt_split)) * a.nt_split), THREADS, (size_t)smem, st, a);
   count_launch();
   return launch_check("conv_rows_kernel");
 }
@@ -353,7 +373,8 @@ int rows_conv(const ConvGeom& g, View4 x, View4 w, const float* bias, long long 
   a.g = g; a.x = x; a.w = w; a.bias = bias; a.bias_stride = bias_stride; a.out = y;
   a.runs = plan.runs; a.run_len = plan.run_len; a.channels_last = channels_last ? 1 : 0;
   a.run_step = channels_last ? 1 : g.dw * x.s3;
-  a.nkb = plan.nkb; a.bn = plan.bn; a.acc_cols = plan.acc_cols; a.ntn = plan.ntn; a.nt_split = plan.nt_split; a.stages = plan.stages;
+  a.segs = (plan.nkb + SEG_KB - 1) / SEG_KB; a.seg_kb = (plan.nkb + a.segs - 1) / a.segs;
+  a.nkb = plan.nkb; a.bn = plan.bn; a.acc_cols = plan.acc_cols; a.ntn = plan.ntn; a.nt_split = plan.nt_split; a.bufs = plan.bufs; a.stages = plan.stages;
   a.m_total = (uint32_t)((long long)g.n * g.oh * g.ow);
   a.tiles_m = (int)div_up64(a.m_total, BLOCK_M);
   if ((long long)a.tiles_m * plan.ntn * plan.nkb > 2147483647ll) return fail(B200_EUNSUPPORTED, "row kernel: job count exceeds 32 bits");
@@ -363,11 +384,16 @@ int rows_conv(const ConvGeom& g, View4 x, View4 w, const float* bias, long long 
   a.status = device_status_word();
   if (!a.status) return fail(B200_ECUDA, "device status word is not allocated");
   const bool unit = a.run_step == 1;
+  auto launch = [&](auto lp) {
+    constexpr int LP = decltype(lp)::value;
+    return plan.pair ? (unit ? launch_rows<LP, true, true>(a, plan.smem, st) : launch_rows<LP, false, true>(a, plan.smem, st))
+                     : (unit ? launch_rows<LP, true, false>(a, plan.smem, st) : launch_rows<LP, false, false>(a, plan.smem, st));
+  };
   switch (plan.lp) {
-    case 4: return unit ? launch_rows<4, true>(a, plan.smem, st) : launch_rows<4, false>(a, plan.smem, st);
-    case 8: return unit ? launch_rows<8, true>(a, plan.smem, st) : launch_rows<8, false>(a, plan.smem, st);
-    case 16: return unit ? launch_rows<16, true>(a, plan.smem, st) : launch_rows<16, false>(a, plan.smem, st);
-    default: return unit ? launch_rows<32, true>(a, plan.smem, st) : launch_rows<32, false>(a, plan.smem, st);
+    case 4: return launch(std::integral_constant<int, 4>{});
+    case 8: return launch(std::integral_constant<int, 8>{});
+    case 16: return launch(std::integral_constant<int, 16>{});
+    default: return launch(std::integral_constant<int, 32>{});
   }
 }
 

@@ -41,3 +41,27 @@ def test_narrow_forward(xshape, cout, kernel, kw, layout):
     assert b200conv.last_kernel() == "tc_rows_forward" and b200conv.device_status() == 0
     assert oracle.rel_l2(y, want) <= 1e-5
     assert oracle.rel_l2(b200conv.conv2d_forward(x, w, None, algo="tc", **kw), want - b[None, :, None, None]) <= 1e-5
+
+
+# The layers of this kernel were computed in FP32 on the CUDA cores before it.  Its main products add up in chains of at most 48 truncating
+# steps, each of which loses half a unit in the last place on average, 2^-24, of a sum that has reached half of its size on average:
+# 48 * 2^-25 * 0.72 (the mean of a unit in the last place over the value) = 1.0e-6 at most; the split itself stays below 2e-7.
+@pytest.mark.parametrize("xshape,cout,kernel,kw", [
+    ((2, 3, 64, 64), 64, (7, 7), dict(stride=(2, 2), padding=(3, 3))),       # six K blocks, one chain
+    ((1, 14, 21, 21), 82, (5, 5), dict(padding=(2, 2))),                     # eighteen: two chains
+    ((2, 15, 19, 18), 130, (7, 7), dict(padding=(3, 3))),                    # twenty-seven: three chains, two column tiles
+    ((1, 11, 24, 24), 16, (7, 1), dict(padding=(3, 0))),
+    ((40, 1, 30, 30), 48, (3, 3), dict(padding=(1, 1))),                     # several tiles per CTA
+], ids=lambda v: "x".join(map(str, v)) if isinstance(v, tuple) else str(v) if isinstance(v, int) else "")
+@pytest.mark.parametrize("layout", ["nchw", "nhwc"])
+def test_narrow_forward_keeps_fp32(xshape, cout, kernel, kw, layout):
+    rng = np.random.default_rng(sum(xshape) + cout)
+    g = oracle.geometry(xshape, cout, kernel, **kw)
+    x, b = rng.standard_normal(g.x_shape, dtype=np.float32), rng.standard_normal(cout, dtype=np.float32)
+    w = (rng.standard_normal(g.w_shape, dtype=np.float32) / np.sqrt(np.prod(g.w_shape[1:]))).astype(np.float32)
+    want = oracle.torch_conv_all(x, w, b, np.zeros(g.y_shape, np.float32), kw.get("stride", (1, 1)), kw.get("padding", (0, 0)), (1, 1), 1)[0]
+    if layout == "nhwc":
+        x = np.ascontiguousarray(x.transpose(0, 2, 3, 1)).transpose(0, 3, 1, 2)
+    y = b200conv.conv2d_forward(x, w, b, algo="tc", **kw)
+    assert b200conv.last_kernel() == "tc_rows_forward" and b200conv.device_status() == 0
+    assert oracle.rel_l2(y, want) <= 1.2e-6
