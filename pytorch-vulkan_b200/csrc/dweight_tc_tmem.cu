@@ -58,6 +58,9 @@ constexpr int ACC_COLS = 384;                // accumulator columns at most (two
 constexpr int SCRATCH = 32 * 36 * 4;         // transpose tile of a dY warp
 constexpr int SMEM_LIMIT = 232448 - 2048;
 constexpr int CHUNK_KB = 96;                 // K blocks per accumulation chain (see dweight_tc_strip.cu)
+// ... of layers with fewer than 32 (input channel, tap) pairs per group, which ran in FP32 on the CUDA cores before: 49 images of 95x95, 3 -> 80
+// channels, 3x3, off by 1.4e-5 in chains of 96, 1.0e-6 in chains of 4 (FP32 7.6e-7; in chains of 2 8e-7); 87 us, now 116 (FP32 613).
+constexpr int CHUNK_KB_FP32 = 4;
 
 struct Strip {       // one staged input strip
   signed char cblk;  // channel block within the CTA's tile
@@ -602,6 +605,8 @@ static Plan make_plan(const ConvGeom& real, size_t budget) {
   const int cib = (g.cig + 31) / 32;
   const size_t dw_bytes = sizeof(float) * (size_t)g.cout * g.cig * g.kh * g.kw;
   const long long kb_total = div_up64(q_total - q_first, KP);
+  int limit = real.cig * real.kh * real.kw < 32 ? CHUNK_KB_FP32 : CHUNK_KB;
+  if (const char* e = getenv("B200_DW_CHUNK_KB")) limit = std::max(1, atoi(e));   // testing aid: chain length in K blocks
   double best_cost = 0;
   for (int nci : {1, 2, 3, 4, 6, 8}) {
     if (nci > cib && nci > 1) break;
@@ -638,7 +643,7 @@ static Plan make_plan(const ConvGeom& real, size_t budget) {
         sp = std::min<long long>({sp, std::max<long long>(1, kb_total / 6), 65535, std::max<long long>(1, (long long)(budget / dw_bytes))});
         if (sp < 1) continue;
         const double per = (double)div_up64(kb_total, sp), waves = (double)div_up64(p.tiles * sp, sm_count());
-        const double cost = waves * (per * kb_clk + per / CHUNK_KB * 2500.0 + 6000.0 + 150.0 * a.n_slots) +
+        const double cost = waves * (per * kb_clk + per / limit * 2500.0 + 6000.0 + 150.0 * a.n_slots) +
                             (sp > 1 ? 3000.0 + (double)(sp + 1) * dw_bytes / 2200.0 : 0.0);
         if (!best.ok || cost < best_cost) {
           best_cost = cost;
@@ -661,8 +666,6 @@ static Plan make_plan(const ConvGeom& real, size_t budget) {
   a.img_div = FastDiv((uint32_t)((gh + pr) * row_pitch)); a.row_div = FastDiv((uint32_t)row_pitch);
   a.div_strips = FastDiv((uint32_t)a.n_strips); a.div_ring = FastDiv((uint32_t)a.ring);
   a.sph = g.sh; a.spw = g.sw; a.in_h = g.h; a.in_w = g.w; a.out_h = g.oh; a.out_w = g.ow;
-  int limit = CHUNK_KB;
-  if (const char* e = getenv("B200_DW_CHUNK_KB")) limit = std::max(1, atoi(e));   // testing aid: chain length in K blocks
   const int kblocks = a.span / KP, chunks = (kblocks + limit - 1) / limit;
   a.chunk_kb = (kblocks + chunks - 1) / chunks;
   a.g = g;
