@@ -645,18 +645,37 @@ static const DwStripPlan& plan_dw_strip(const ConvGeom& g, size_t budget) {
 
 }  // namespace tcdw
 
-static bool tmem_allowed() {
-  const char* e = getenv("B200_DW_VARIANT");   // "strip" pins the kernel with both operands in shared memory (testing aid)
-  return !(e && !strcmp(e, "strip"));
+// B200_DW_VARIANT pins a kernel (testing aid): "strip" the one with both operands in shared memory, "tmem" the other where it takes the geometry.
+enum class Variant { BY_RULE, STRIP, TMEM };
+static Variant variant() {
+  const char* e = getenv("B200_DW_VARIANT");
+  return !e ? Variant::BY_RULE : !strcmp(e, "strip") ? Variant::STRIP : !strcmp(e, "tmem") ? Variant::TMEM : Variant::BY_RULE;
 }
 bool dweight_strip_supported(const ConvGeom& g) {
-  size_t bytes;
-  return tcdw::plan_dw_strip(g, 0).ok || (tmem_allowed() && tcdt::plan_bytes(g, 0, &bytes));
+  tcdt::PlanInfo info;
+  return tcdw::plan_dw_strip(g, 0).ok || (variant() != Variant::STRIP && tcdt::plan_info(g, 0, &info));
+}
+// The tensor-memory kernel gives a CTA of up to 64 output channels all vertical taps of an input block, where this one has a CTA for each
+// tap.  That pays while the splits fill the machine; where they cannot (little or no scratch, few pixels) its CTAs are a third as many and
+// do a third more per K block.  Per K block and for the rest of a CTA, measured: 0.74 us (six slots; 0.31 per strip of a strided input) and
+// 0.70 (1x1 filters) + 6 against 0.51 (0.60 in four blocks) + 4.  16 -> 62 channels of 7x 21x21, stride 2, no scratch: 45.6 and 25.3 us;
+// 38 -> 32 of 5x 46x46, no scratch: 265 and 181; 16 -> 64 of 61x61 x 14 with all the scratch it wants: 27.4 and 28.9.
+static bool strip_is_faster(const ConvGeom& g, const tcdt::PlanInfo& t, const tcdw::DwStripPlan& s) {
+  if (!s.ok || g.cig * g.kh * g.kw < 32) return false;   // few products: short chains, which only the tensor-memory kernel has
+  if (g.cog > 64 || s.nacc != 1 || !(t.shift || g.kh * g.kw == 1)) return false;
+  const double tmem = 6.0 + t.kblocks * (t.shift ? std::max(0.74 * t.slots / 6, 0.31 * t.strips) : 0.70);
+  const double strip = 4.0 + (double)(s.span / tcdw::KP) * (s.xblocks == 1 ? 0.51 : 0.60);
+  return strip < 0.85 * tmem;
+}
+// Whether the tensor-memory kernel takes the call.
+static bool tmem_takes(const ConvGeom& g, size_t budget, const tcdw::DwStripPlan& s, tcdt::PlanInfo* t) {
+  const Variant pinned = variant();
+  return pinned != Variant::STRIP && tcdt::plan_info(g, budget, t) && (pinned == Variant::TMEM || !strip_is_faster(g, *t, s));
 }
 size_t dweight_strip_workspace(const ConvGeom& g, size_t budget) {
-  size_t bytes = 0;
-  if (tmem_allowed() && tcdt::plan_bytes(g, budget, &bytes)) return bytes;
-  return tcdw::plan_dw_strip(g, budget).bytes;
+  tcdt::PlanInfo t;
+  const tcdw::DwStripPlan& s = tcdw::plan_dw_strip(g, budget);
+  return tmem_takes(g, budget, s, &t) ? t.bytes : s.bytes;
 }
 
 template <int BN, bool CROSS>
@@ -673,11 +692,12 @@ static int launch_dw_strip(const tcdw::DwStripArgs& a, dim3 grid, int smem, cuda
 
 int dweight_strip(const ConvGeom& g, View4 x, View4 dy, float* dw, void* ws, size_t ws_bytes, cudaStream_t st) {
   using namespace tcdw;
-  if (tmem_allowed()) {
+  const DwStripPlan& plan = plan_dw_strip(g, ws ? ws_bytes : 0);
+  tcdt::PlanInfo t;
+  if (tmem_takes(g, ws ? ws_bytes : 0, plan, &t)) {
     const int rc = tcdt::run(g, x, dy, dw, ws, ws_bytes, st);
     if (rc != B200_EUNSUPPORTED) return rc;
   }
-  const DwStripPlan& plan = plan_dw_strip(g, ws ? ws_bytes : 0);
   if (!plan.ok) return fail(B200_EUNSUPPORTED, "dWeight strip kernel does not take this geometry");
   // the kernel forms element offsets inside a tensor in 32 bits
   auto span = [](const View4& v, long long n, long long c, long long h, long long w) {

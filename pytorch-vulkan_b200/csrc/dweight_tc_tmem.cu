@@ -679,9 +679,9 @@ static const Plan& cached_plan(const ConvGeom& g, size_t budget) {
   return cache.get(g, budget, [&] { return make_plan(g, budget); });
 }
 
-bool plan_bytes(const ConvGeom& g, size_t budget, size_t* bytes) {
+bool plan_info(const ConvGeom& g, size_t budget, PlanInfo* info) {
   const Plan& p = cached_plan(g, budget);
-  if (p.ok) *bytes = p.bytes;
+  if (p.ok) *info = PlanInfo{p.bytes, p.a.span / KP, p.a.n_strips, p.a.n_slots, p.a.shift_rows != 0};
   return p.ok;
 }
 
