@@ -318,12 +318,15 @@ int simt_gemm(long long M, long long N, long long K, const float* A, long long s
   long long splits = std::max(1ll, std::min({4ll * sm_count() / tiles, K / 64, 64ll}));
   p.span = div_up64(div_up64(std::max(K, 1ll), splits), BK) * BK;
   splits = std::max<long long>(1, div_up64(K, p.span));
-  if (splits == 1) {
+  // One slice needs no scratch: under stream capture, where the pool would hand the block on while the graph still uses it and where a cold
+  // pool may not allocate, and where the device has no memory left.
+  void* parts = nullptr;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (splits > 1 && cudaStreamIsCapturing(st, &capture) != cudaSuccess) (void)cudaGetLastError();
+  if (splits == 1 || capture != cudaStreamCaptureStatusNone || b200_malloc(&parts, (size_t)splits * M * N * sizeof(float), st)) {
     p.span = std::max(K, 1ll);
     return launch_igemm<PH_GEMM>(p, 1, 1, st, "simt_gemm");
   }
-  void* parts = nullptr;
-  if (int rc = b200_malloc(&parts, (size_t)splits * M * N * sizeof(float), st)) return rc;
   p.out = (float*)parts;
   int rc = launch_igemm<PH_GEMM>(p, 1, (int)splits, st, "simt_gemm");
   if (!rc) rc = gemm_finalize((const float*)parts, (int)splits, M, N, alpha, beta != 0.f ? bias : nullptr, beta, C, st);

@@ -1082,19 +1082,28 @@ int tc_gemm(long long M, long long N, long long K, const float* A, long long sa0
   if (K < 16 || N < 16 || M > 2147483647ll || N > 2147483647ll || K > 2147483647ll)
     return fail(B200_EUNSUPPORTED, "tcgen05 GEMM is incompatible with this shape (needs K >= 16 and N >= 16)");
   long long slice;
-  const int splits = gemm_splits(M, N, K, &slice);
-  const ConvGeom g = gemm_geometry(M, N, slice, splits);
+  int splits = gemm_splits(M, N, K, &slice);
+  ConvGeom g = gemm_geometry(M, N, slice, splits);
   if (!tcs::plan_strip(g, false).ok) return fail(B200_EUNSUPPORTED, "tcgen05 GEMM is incompatible with this shape");
   const View4 act{A, 0, sa1, 0, sa0};   // [n=1][c=k][h=1][w=m]
   const View4 wv{B, sb1, sb0, 0, 0};    // [co=n][ci=k][1][1]
+  void* ws = nullptr;
+  size_t images = (strip_workspace(g, B200_PHASE_FORWARD) + 255) & ~(size_t)255;
+  int status = b200_malloc(&ws, images + (splits > 1 ? (size_t)splits * M * N * sizeof(float) : 0), st);
+  if (status && splits > 1) {           // no room for the partial products: one slice
+    splits = 1;
+    slice = K;
+    g = gemm_geometry(M, N, K, 1);
+    if (!tcs::plan_strip(g, false).ok) return status;
+    images = (strip_workspace(g, B200_PHASE_FORWARD) + 255) & ~(size_t)255;
+    status = b200_malloc(&ws, images, st);
+  }
+  if (status) return status;
   StripBatch sb;
   sb.w_group_extra = slice * sb0 - N * sb1;  // slice s starts s*slice rows down B
   sb.out_pitch = N;
   sb.out_group = M * N;
   sb.k_total = K;
-  void* ws = nullptr;
-  const size_t images = (strip_workspace(g, B200_PHASE_FORWARD) + 255) & ~(size_t)255, partial = splits > 1 ? (size_t)splits * M * N * sizeof(float) : 0;
-  if (int rc = b200_malloc(&ws, images + partial, st)) return rc;
   if (!bias || beta == 0.f) { bias = nullptr; beta = 0.f; }
   int rc;
   if (splits == 1) {

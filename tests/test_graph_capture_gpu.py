@@ -75,3 +75,34 @@ def test_captured_layer_replays_on_new_inputs(xshape, cout, kernel, stride, padd
     got = (y.cpu().numpy(), dx.cpu().numpy(), dw.cpu().numpy())
     errs = [oracle.rel_l2(a, e) for a, e in zip(got, want[:3])]
     assert max(errs) <= 1e-4, errs
+
+
+@pytest.mark.parametrize("m,n,k", [(100, 1000, 2048), (16, 512, 4096), (5, 7, 3000)])
+def test_captured_products_of_few_rows_take_no_scratch(m, n, k):
+    """Products with fewer than 128 rows slice their reduction with scratch from the pool; a captured call may not, since the pool would hand the
+    block to the next caller while the graph still writes it."""
+    lib, P, f = b200conv.lib(), ctypes.c_void_p, ctypes.c_float
+    gen = torch.Generator(device="cuda").manual_seed(m + n + k)
+    a, b, c = torch.randn(m, k, device="cuda", generator=gen), torch.randn(k, n, device="cuda", generator=gen), torch.empty(m, n, device="cuda")
+
+    def issue(stream):
+        b200conv.check(lib.b200_gemm(m, n, k, P(a.data_ptr()), k, 1, P(b.data_ptr()), n, 1, None, f(1.0), f(0.0), P(c.data_ptr()), 0, stream))
+
+    def stats():
+        out = (ctypes.c_uint64 * 4)()
+        b200conv.check(lib.b200_mem_stats(out))
+        return list(out)
+    issue(None)
+    torch.cuda.synchronize()
+    b200conv.check(lib.b200_empty_cache())             # a cold pool, which a capture could not fill either
+    before = stats()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        issue(P(torch.cuda.current_stream().cuda_stream))
+    assert stats() == before
+    a.copy_(torch.randn(m, k, device="cuda", generator=gen))
+    c.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    want = a.double() @ b.double()
+    assert float((c.double() - want).norm() / want.norm()) <= 1e-5 and b200conv.device_status() == 0
