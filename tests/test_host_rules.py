@@ -121,3 +121,53 @@ int main() {
   return wrong != 0 || resident == 0 || streams == 0;
 }
 """)
+
+
+def test_plan_table_holds_a_network(tmp_path):
+    """The layers of ResNet-50, forward and dInput: every plan is made once, whatever the batch, and kept through the following steps; more
+    layers than the table has places still get plans of their own."""
+    _run(tmp_path, r"""
+#include <cstdio>
+#include <vector>
+#include "plan_cache.cuh"
+namespace b200 { int sm_count() { return 148; } }
+using namespace b200;
+static ConvGeom layer(int n, int cin, int cout, int hw, int k, int s) {
+  const int p = (k - 1) / 2, o = (hw + 2 * p - k) / s + 1;
+  return ConvGeom{n, cin, cout, hw, hw, k, k, o, o, s, s, p, p, 1, 1, 1, cin, cout};
+}
+int main() {
+  int wrong = 0;
+  for (int n : {1, 2, 8, 32, 64, 100, 256}) {
+    std::vector<ConvGeom> net{layer(n, 3, 64, 224, 7, 2)};
+    const int blocks[] = {3, 4, 6, 3};
+    int cin = 64, hw = 56;
+    for (int stage = 0; stage < 4; ++stage)
+      for (int b = 0; b < blocks[stage]; ++b) {
+        const int width = 64 << stage, s = stage > 0 && b == 0 ? 2 : 1;
+        net.push_back(layer(n, cin, width, hw, 1, 1));
+        net.push_back(layer(n, width, width, hw, 3, s));
+        if (b == 0) net.push_back(layer(n, cin, 4 * width, hw, 1, s));
+        hw /= s;
+        net.push_back(layer(n, width, 4 * width, hw, 1, 1));
+        cin = 4 * width;
+      }
+    PlanCache<int> cache;
+    int made = 0, first = 0;
+    for (int step = 0; step < 4; ++step) {
+      for (size_t i = 0; i < net.size(); ++i)
+        for (int is_dx = 0; is_dx < 2; ++is_dx) {
+          const int want = net[i].cin * 100000 + net[i].cout * 20 + net[i].h + 7 * net[i].kh + 3 * net[i].sh + is_dx;
+          wrong += cache.get(net[i], is_dx, [&] { ++made; return want; }) != want;
+        }
+      if (step == 0) first = made;
+    }
+    printf("batch %d: %d layers, %d plans made\n", n, (int)net.size(), made);
+    wrong += made != first;
+  }
+  PlanCache<int> cache;
+  for (int step = 0; step < 2; ++step)
+    for (int i = 1; i < 5000; ++i) wrong += cache.get(layer(1, i, 16, 8, 3, 1), 0, [&] { return i; }) != i;
+  return wrong != 0;
+}
+""")
