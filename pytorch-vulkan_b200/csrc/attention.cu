@@ -16,7 +16,6 @@
 // dM = P (dP - rowsum(dO O)), the unscaled score gradient (sdpa_training.comp:38,40 `aux[index]=ds`).
 #include <algorithm>
 #include <cmath>
-#include <cstdlib>
 
 #include "attention_fused.cuh"
 #include "common.cuh"
@@ -304,11 +303,10 @@ int check_mask(const void* mask, int mask_type) {
   return B200_OK;
 }
 
-// The fused kernels take calls without mask, dropout and mask gradient (B200_ATTENTION_COMPOSED=1 pins the composed form: testing aid).
+// The fused kernels take calls without mask, dropout and mask gradient.
 bool use_fused(int64_t batch, int64_t tq, int64_t tk, int64_t d, int64_t dv, const void* mask, float dropout, const void* dmask, const void* ws,
                size_t ws_bytes, bool backward) {
-  const char* e = getenv("B200_ATTENTION_COMPOSED");
-  return !(e && e[0] == '1') && !mask && dropout == 0.f && !dmask && fa::supported(batch, tq, tk, d, dv) &&
+  return !mask && dropout == 0.f && !dmask && fa::supported(batch, tq, tk, d, dv) &&
          ws && (reinterpret_cast<uintptr_t>(ws) & 15) == 0 && ws_bytes >= fa::workspace(batch, tq, tk, d, backward) && device_status_word();
 }
 

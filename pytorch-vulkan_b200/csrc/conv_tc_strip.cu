@@ -919,15 +919,13 @@ int strip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* b
   a.tiles_m = (int)div_up64(a.q_total, BLOCK_M);
   a.halo = plan.halo; a.strip_rows = plan.strip_rows; a.a_stages = plan.a_stages; a.w_stages = plan.w_stages;
   {
-    // one tap per staged strip (1x1 filters): the MMAs wait for the producers, so twelve of them run (testing aid:
-    // B200_STRIP_PRODUCERS=8|12 pins either)
+    // one tap per staged strip (1x1 filters): the MMAs wait for the producers, so twelve of them run
     int most = 0;
     for (int ph = 0; ph < plan.tt.n_phase; ++ph) most = std::max(most, (int)plan.tt.start[ph + 1] - (int)plan.tt.start[ph]);
     // ... and only while the reduction side is the larger one (256 -> 64 channels forward: 90 -> 69 us); with more output
     // than input (its dInput) the epilogue's stores set the pace and the extra warps only take registers from it (61 -> 80 us)
     // (row-major stores are whole lines and cost less: 1024 -> 1024 columns of a GEMM 198 -> 157 us, but 80 -> 1024 is faster with eight)
     a.wide_producers = most <= 1 && (kc > nc || (rowmajor && a.cblocks >= 16)) ? 1 : 0;
-    if (const char* e = getenv("B200_STRIP_PRODUCERS")) a.wide_producers = atoi(e) > 8 ? 1 : 0;
   }
   const int chunks = (a.strip_rows + 31) / 32;
   const long long tiles_total = (long long)a.tiles_m * a.tiles_n * g.groups;
@@ -950,20 +948,21 @@ int strip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* b
   a.out_vec4 = rowmajor && a.out_pitch % 4 == 0 && a.out_group % 4 == 0 && plan.bn % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0 &&
                a.nc % 4 == 0;
   // a plain product with wide column tiles: one tap per strip leaves shared memory as the bound, which the kernel with A in tensor memory
-  // relieves (16384x1024 x 1024x1024: 144 -> 131 us); below 65 columns its tiles would be half empty (B200_GEMM_STRIP pins the strip kernel: testing aid)
-  if (rowmajor && !is_dx && !post && g.n == 1 && g.h == 1 && g.kh * g.kw == 1 && plan.bn >= 128 && !getenv("B200_GEMM_STRIP")) {
+  // relieves (16384x1024 x 1024x1024: 144 -> 131 us); below 65 columns its tiles would be half empty
+  if (rowmajor && !is_dx && !post && g.n == 1 && g.h == 1 && g.kh * g.kw == 1 && plan.bn >= 128) {
     gt::GemmArgs m{};
     m.A = act.ptr; m.a_m = act.s3; m.a_k = act.s1; m.a_group = kc * act.s1 + a.act_group_extra;
     m.images = wp; m.bias = bias; m.bias_stride = bias_stride;
     m.C = out; m.c_pitch = a.out_pitch; m.c_group = a.out_group;
     m.M = g.w; m.N = nc; m.kc = kc; m.k_total = k_total; m.kblocks = cpp;
     m.tiles_m = a.tiles_m; m.tiles_n = a.tiles_n; m.tiles = a.tiles_total; m.m_fastest = a.unit == 1;
-    m.mode = act.s1 == 1 ? 1 : act.s3 == 1 ? 2 : 0;
-    m.pieces16 = (m.mode == 1 ? act.s3 : act.s1) % 4 == 0 && (m.mode == 2 || kc % 4 == 0) && m.a_group % 4 == 0 && (reinterpret_cast<uintptr_t>(act.ptr) & 15) == 0;
+    const bool lines = act.s1 == 1 || act.s3 == 1;
+    m.along_k = act.s1 == 1;
+    m.pieces16 = (m.along_k ? act.s3 : act.s1) % 4 == 0 && (!m.along_k || kc % 4 == 0) && m.a_group % 4 == 0 && (reinterpret_cast<uintptr_t>(act.ptr) & 15) == 0;
     m.vec_out = a.out_vec4; m.wait_for_images = a.wait_for_images; m.alpha = alpha; m.beta = beta;
     // rows of A along m that are not 16-byte aligned are better read straight into the strip producers' registers (51 against 66 us for
     // 1111x16000 x 16000x77), as is A without a contiguous dimension
-    if (m.mode != 0 && (m.mode == 1 || m.pieces16)) return gt::run(m, plan.bn, st);
+    if (lines && (m.along_k || m.pieces16)) return gt::run(m, plan.bn, st);
   }
   a.status = device_status_word();
   if (!a.status) return fail(B200_ECUDA, "device status word is not allocated");

@@ -527,9 +527,7 @@ static TPlan make_plan(const ConvGeom& g, bool is_dx) {
   const double stages_per_tile = is_dx ? (double)p.cpp * tt.taps_total / std::max(1, tt.n_phase) : (double)p.cpp * tt.taps_total;
   const int span = p.geo.shift_hi - p.geo.shift_lo;
   double best = 0.0;
-  int pn_hi = 256, pn_lo = 32;
-  if (const char* e = getenv("B200_TSTRIP_PN")) pn_hi = pn_lo = std::max(16, std::min(256, atoi(e) / 16 * 16));  // testing aid
-  for (int pn = pn_hi; pn >= pn_lo; pn -= 16) {
+  for (int pn = 256; pn >= 32; pn -= 16) {
     const int rows = (pn + span + 7) / 8 * 8;
     const int a_stage = rows * ROWB * 2;
     int a_stages = 0, w_stages = 0;
@@ -553,8 +551,7 @@ static TPlan make_plan(const ConvGeom& g, bool is_dx) {
 }
 static const TPlan& plan_tstrip(const ConvGeom& g, bool is_dx) {
   thread_local PlanCache<TPlan> cache;
-  const char* pinned = getenv("B200_TSTRIP_PN");
-  return cache.get(g, 2 * (pinned ? (size_t)atoi(pinned) : 0) + is_dx, [&] { return make_plan(g, is_dx); });
+  return cache.get(g, is_dx, [&] { return make_plan(g, is_dx); });
 }
 
 }  // namespace tst
@@ -565,8 +562,7 @@ bool tstrip_supported(const ConvGeom& g, int phase) {
   const bool is_dx = phase == B200_PHASE_DINPUT;
   const int nc = is_dx ? g.cig : g.cog;
   const int last = nc % tst::TM;
-  int least = 65;
-  if (const char* e = getenv("B200_TSTRIP_MIN")) least = std::max(16, atoi(e));  // testing aid
+  const int least = 65;
   if (nc < least || (last != 0 && last < least && nc < 4 * tst::TM)) return false;   // at most a quarter of the rows may be padding
   // a 1x1 filter is bound by HBM and by the epilogue, not by the MMAs, and a strided dInput splits into phases of two
   // or three taps each: both keep the arrangement with pixels on M, whose epilogue stores straight from registers
@@ -651,9 +647,8 @@ int tstrip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* 
   B200_CUDA(opt_in);
   // A strided forward pass stages one strip per input phase and gets only one to four taps of MMAs out of it (a
   // stride-1 strip feeds all nine): the producers set the pace, so sixteen run (128 -> 128 channels, 56x56 stride 2:
-  // 87 -> 81 us NCHW, 94 -> 73 us channels-last; stride-1 layers are unchanged either way).  B200_TSTRIP_PRODUCERS=8|16 pins it.
-  bool wide = !is_dx && (g.sh > 1 || g.sw > 1);
-  if (const char* e = getenv("B200_TSTRIP_PRODUCERS")) wide = atoi(e) == 16;
+  // 87 -> 81 us NCHW, 94 -> 73 us channels-last; stride-1 layers are unchanged either way).
+  const bool wide = !is_dx && (g.sh > 1 || g.sw > 1);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)std::min(a.tiles_total, sm_count())); cfg.blockDim = dim3(tstrip_threads(wide ? 16 : 8));
   cfg.dynamicSmemBytes = (size_t)plan.smem; cfg.stream = st;

@@ -536,7 +536,7 @@ int finalize_partials(const float* partial, float* dw, const ConvGeom& g, int sp
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
-  if (!getenv("B200_DW_NO_PDL")) { cfg.attrs = &attr; cfg.numAttrs = 1; }
+  cfg.attrs = &attr; cfg.numAttrs = 1;
   B200_CUDA(cudaLaunchKernelEx(&cfg, v4 ? finalize_partials_kernel<4> : finalize_partials_kernel<1>, partial, dw, count, splits,
                                g.cig, taps, slices, ch_log2, FastDiv((uint32_t)chunks), FastDiv((uint32_t)units)));
   count_launch();
@@ -592,7 +592,7 @@ static DwStripPlan make_plan(const ConvGeom& g, size_t budget) {
   // Several channel blocks per CTA share every staged dY block (one TMEM accumulator each): less dY
   // staging per MMA.  The column tile then stays at 128 (TMEM holds 512 columns).
   if (p.xblocks == 1 && g.cig >= 64) {
-    p.cross = g.cig >= 128 || getenv("B200_DW_FORCE_CROSS") != nullptr;
+    p.cross = g.cig >= 128;
     p.nacc = p.cross && g.cig > 64 ? 4 : 2;
     p.bn = g.cog <= 64 ? 64 : 128;
   } else {
@@ -639,8 +639,8 @@ static DwStripPlan make_plan(const ConvGeom& g, size_t budget) {
   return p;
 }
 static const DwStripPlan& plan_dw_strip(const ConvGeom& g, size_t budget) {
-  thread_local PlanCache<DwStripPlan> cache, forced;
-  return (getenv("B200_DW_FORCE_CROSS") ? forced : cache).get(g, budget, [&] { return make_plan(g, budget); });
+  thread_local PlanCache<DwStripPlan> cache;
+  return cache.get(g, budget, [&] { return make_plan(g, budget); });
 }
 
 }  // namespace tcdw

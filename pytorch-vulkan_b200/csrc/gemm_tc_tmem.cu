@@ -175,7 +175,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const GemmArgs a)
     // ------------------------------ producers ------------------------------
     const int quarter = warp & 3, set = (warp - EPI_WARPS) >> 2;
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16, slots = w_base + W_STAGES * W_BYTES + (uint32_t)(warp - EPI_WARPS) * (DEPTH * SLOT);
-    const int a_k = (int)a.a_k;                   // views span less than 2^31 elements (checked by the host)
     const int total = my_tiles * a.kblocks;       // below 2^31 (checked by the host)
     struct Block { const float* src; int rows, valid; };        // rows of this warp inside the matrix, values of this K block
     auto locate = [&](int c) -> Block {
@@ -188,10 +187,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const GemmArgs a)
     // the 32 x 32 values of a job as 32 lines of 128 bytes, eight lanes to a line; what lies outside is zero
     auto issue = [&](int n) {
       const int c = set + n * SETS;
-      if (a.mode != 0 && c < total) {
+      if (c < total) {
         const Block k = locate(c);
-        const int lines = a.mode == 1 ? k.rows : k.valid, length = a.mode == 1 ? k.valid : k.rows;
-        const long long pitch = a.mode == 1 ? a.a_m : a.a_k;
+        const int lines = a.along_k ? k.rows : k.valid, length = a.along_k ? k.valid : k.rows;
+        const long long pitch = a.along_k ? a.a_m : a.a_k;
         const uint32_t slot = slots + (uint32_t)(n % DEPTH) * SLOT;
         if (a.pieces16) {
           const int bytes = max(0, min(16, (length - (lane & 7) * 4) * 4));
@@ -201,12 +200,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const GemmArgs a)
             const int r = 4 * j + (lane >> 3), size = r < lines ? bytes : 0;
             cp_async<16>(slot + (uint32_t)(r * 128 + (((lane & 7) ^ (r & 7)) << 4)), size ? p + 4ll * j * pitch : a.A, size);
           }
-        } else {                     // lines that start anywhere: a value at a time, a warp to a line
+        } else {                     // lines along k that start anywhere: a value at a time, a warp to a line
           const float* p = k.src + lane;
 #pragma unroll 8
           for (int r = 0; r < 32; ++r) {
-            const int size = r < lines && lane < length ? 4 : 0;
-            cp_async<4>(slot + (uint32_t)(r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4), size ? p + r * pitch : a.A, size);
+            const int size = r < k.rows && lane < k.valid ? 4 : 0;
+            cp_async<4>(slot + (uint32_t)(r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4), size ? p + r * a.a_m : a.A, size);
           }
         }
       }
@@ -217,24 +216,17 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const GemmArgs a)
 #pragma unroll 1
       for (int n = 0, c = set; c < total; ++n, c += SETS) {
         float v[32];
-        if (a.mode != 0) {
-          cp_async_wait<DEPTH - 1>();
-          __syncwarp();
-          const uint32_t slot = slots + (uint32_t)(n % DEPTH) * SLOT;
-          if (a.mode == 1) {         // lines are rows: 16 bytes at a time of this lane's line
+        cp_async_wait<DEPTH - 1>();
+        __syncwarp();
+        const uint32_t slot = slots + (uint32_t)(n % DEPTH) * SLOT;
+        if (a.along_k) {             // lines are rows: 16 bytes at a time of this lane's line
 #pragma unroll
-            for (int j = 0; j < 8; ++j) lds_f32x4(slot + (uint32_t)(lane * 128 + ((j ^ (lane & 7)) << 4)), v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-          } else {                   // lines are values of the reduction: this lane's row out of each
+          for (int j = 0; j < 8; ++j) lds_f32x4(slot + (uint32_t)(lane * 128 + ((j ^ (lane & 7)) << 4)), v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+        } else {                     // lines are values of the reduction: this lane's row out of each
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = lds_f32(slot + (uint32_t)(j * 128 + (((lane >> 2) ^ (j & 7)) << 4) + (lane & 3) * 4));
-          }
-          __syncwarp();
-        } else {
-          const Block k = locate(c);
-          const float* p = k.src + (long long)lane * a.a_m;
-#pragma unroll
-          for (int j = 0; j < KBLK; ++j) v[j] = lane < k.rows && j < k.valid ? __ldg(p + j * a_k) : 0.f;  // 32-bit offsets: two instructions per value
+          for (int j = 0; j < 32; ++j) v[j] = lds_f32(slot + (uint32_t)(j * 128 + (((lane >> 2) ^ (j & 7)) << 4) + (lane & 3) * 4));
         }
+        __syncwarp();
         issue(n + DEPTH);
         const uint32_t as = (uint32_t)c % A_STAGES, round = (uint32_t)c / A_STAGES;
         if (!warp_wait(smem_u32(&ctrl->a_empty[as]), (round & 1u) ^ 1u, abort_flag, a.status, STATUS_TIMEOUT_EMPTY)) break;

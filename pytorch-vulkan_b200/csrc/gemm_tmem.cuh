@@ -15,8 +15,8 @@ struct GemmArgs {
   int M, N, kc, k_total;     // kc: reduction values of a group; k_total: of all groups (the last may have fewer)
   int kblocks, tiles_m, tiles_n, tiles;
   int m_fastest;             // tile order
-  int mode;                  // A in lines along k (1) or along m (2), or with neither contiguous (0)
-  int pieces16;              // the lines start at multiples of 16 bytes
+  int along_k;               // A in lines along k, else along m
+  int pieces16;              // the lines start at multiples of 16 bytes (always so along m)
   int vec_out;               // rows of C may be written 16 bytes at a time
   int wait_for_images;
   float alpha, beta;
