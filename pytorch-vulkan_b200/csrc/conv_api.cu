@@ -95,7 +95,11 @@ static int select(const ConvGeom& g, int phase, int algo, size_t workspace) {
   // The tcgen05 forward / dInput kernels stage the split filter in the caller's workspace; a caller that
   // brings none (or too little) gets the CUDA-core kernels, which need no scratch.  dWeight runs unsplit
   // without a workspace.  (A forced B200_ALGO_TC keeps reporting the workspace error.)
-  if (tc_supported(g, phase) &&
+  // A handful of products per result, few results and wide column tiles: the row kernel's prologue (every CTA splits the filter) costs more than
+  // the layer.  Measured, row kernel against CUDA cores: 3 -> 119 channels of 3x 8x8, 1x1, 7.2 and 4.3 us; 8 -> 117 of 2x 15x15 7.7 and 6.2;
+  // on the other side of each bound 6 -> 103 of 3x 17x17 7.6 and 8.3, 8 -> 60 of 9x 8x8 5.7 and 6.2, 15 -> 119 of 2x 13x13 8.9 and 10.6.
+  const bool few = phase == B200_PHASE_FORWARD && cols <= 10 && g.cog > 64 && rows * g.cog <= 70000 && rows_supported(g);
+  if (tc_supported(g, phase) && !few &&
       (phase == B200_PHASE_DWEIGHT || tc_workspace(g, phase, workspace, nullptr, nullptr) <= workspace))
     return B200_ALGO_TC;
   // grouped 3x3 layers with 4 or 8 channels per group have kernels of their own behind the tiled candidate

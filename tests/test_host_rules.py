@@ -171,3 +171,13 @@ int main() {
   return wrong != 0;
 }
 """)
+
+
+@pytest.mark.parametrize("n,cin,cout,hw,k,tc", [(3, 3, 119, 8, 1, False), (2, 8, 117, 15, 1, False), (3, 6, 103, 17, 1, True), (9, 8, 60, 8, 1, True),
+                                                (2, 15, 119, 13, 1, True), (1, 1, 80, 29, 3, False), (1, 1, 80, 30, 3, True), (8, 3, 64, 16, 3, True)])
+def test_forward_passes_of_a_few_products_stay_on_the_cuda_cores(n, cin, cout, hw, k, tc):
+    import b200conv
+    p = b200conv.geometry((n, cin, hw, hw), cout, (k, k), padding=(k // 2, k // 2))
+    chosen = b200conv.select(p, b200conv.PHASE_FORWARD)
+    assert (chosen == b200conv.ALGO_TC) == tc
+    assert b200conv.select(p, b200conv.PHASE_FORWARD, b200conv.ALGO_TC) == b200conv.ALGO_TC      # still there when asked for
