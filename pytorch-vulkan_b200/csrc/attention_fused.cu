@@ -2,7 +2,7 @@
 // 64 dimensions: the scores never reach memory.  FP32 by the split-precision scheme of tc_common.cuh.
 //
 // What bounds it and what follows from that.  The composed form (attention.cu) writes, rewrites and reads the [tokens,
-// tokens] matrix: 144 us forward and 265 us backward for 16 heads of 1024 tokens x 64, of which 60 us are products.  Here a CTA owns 128
+// tokens] matrix: 139 us forward and 258 us backward for 16 heads of 1024 tokens x 64, of which 60 us are products.  Here a CTA owns 128
 // rows of one result and walks the other side's tokens in blocks of 64 columns:
 //   S = own1 * col1^T                    (both operands in shared memory)
 //   [dP = own2 * col2^T]
@@ -18,7 +18,7 @@
 // blocks, so that the element-wise work of one runs under the products of the other; a stream is eight warps, a thread half a row
 // (32 columns: 64 left 168 registers a thread and 8 warps, which could not hide the latency of their own chain).  In the forward
 // pass each stream keeps its own maximum, sum and accumulator, merged at the end, and rescales its accumulator only when the maximum
-// has grown by more than 8 (a factor 256 of head room in FP32).  The column operands are split once per call into ready-made
+// has grown by more than 8 (a factor 256 of head room in FP32; the method of FlashAttention-4).  The column operands are split once per call into ready-made
 // shared-memory images by stage_kernel, which also prepares log-sum-exp and delta; one thread fetches them with bulk copies.
 //
 // Measured, 16 heads of 1024 tokens x 64: forward 139 us composed -> 39 with four warps a stream -> 31; backward 258 -> 151 (three

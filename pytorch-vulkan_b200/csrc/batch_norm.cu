@@ -8,7 +8,8 @@
 // run on the CUDA cores with 16-byte loads, several loads in flight per lane, and grids of a
 // few CTAs per SM; nothing here is GEMM-shaped.
 //
-// Two arrangements cover every shape:
+// Planar channels that gain by it are held in the registers of a cluster of CTAs and read once (norm_resident.cuh, norm_plan.cuh); two
+// streaming arrangements cover every shape:
 //   rows     inner >= 256: the channel's elements lie in `outer` contiguous planes.  A warp
 //            streams one plane segment at a time (like the reference's one-workgroup-per-channel
 //            loop, but with the channel cut into (channel, slab) CTAs).

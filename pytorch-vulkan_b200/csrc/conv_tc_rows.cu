@@ -361,7 +361,7 @@ bool rows_supported(const ConvGeom& g) { return g.cig < 16 && tcr::plan_rows(g, 
 
 int rows_conv(const ConvGeom& g, View4 x, View4 w, const float* bias, long long bias_stride, float* y, cudaStream_t st) {
   using namespace tcr;
-  // channels-last: one run per filter row while the padded runs are no longer than the NCHW ones
+  // channels-last with dense pixels: a filter row's taps x channels are adjacent and form one run, where such a run has 31 values at most
   bool channels_last = g.cin > 1 && x.s1 == 1 && x.s3 == g.cin && g.dw == 1;
   RowsPlan plan = plan_rows(g, channels_last);
   if (channels_last && !plan.ok) plan = plan_rows(g, channels_last = false);

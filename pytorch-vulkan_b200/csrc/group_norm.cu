@@ -357,10 +357,9 @@ __global__ void __launch_bounds__(kThreads, 3) gn_backward_kernel(const float* _
 
 // ---- blocks held in registers ----------------------------------------------------------------------
 // The same results with a block shared by the CTAs of a cluster (norm_resident.cuh), wherever its values
-// fit their registers: each tensor is read once, and the shares are small enough that the last wave costs little.
-// 16 samples of 512 channels of 32x32 in 32 groups (512 blocks of 64 KB, 1.15 waves of the kernels above):
-// forward 20.9 us, now 18.7; backward with the sums
-// over the batch 33.0, now 26.7.  32 samples of 1280 channels of 8x8: 24.8 and 27.2 us, now 12.2 and 18.7.
+// fit their registers and that pays (norm_plan.cuh): each tensor is read once, and the shares are small enough that the last wave costs little.
+// 16 samples of 512 channels of 32x32 in 32 groups (512 blocks of 64 KB, 1.15 waves of the kernels above), both directions: 44.4 us
+// with the backward kernel above, 40.7 with this one.  32 samples of 1280 channels of 8x8: 24.8 and 27.2 us, now 12.2 and 18.7.
 constexpr int kUnits = 8, kUnits1 = 16;  // most units a thread holds: forward (16 bytes each), single values
 constexpr int kUnitsBwd = 4;             // backward: of each of the two tensors
 constexpr int kResidentChannels = 64;    // most channels per group in the backward kernel
