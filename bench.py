@@ -71,7 +71,7 @@ LAYERS = [
 WORKLOAD = "resnet50-style layer sweep, batch 64, 6 layers x {NCHW, channels-last}, fwd+dInput+dWeight, FP32"
 L2_NOTE = "inputs larger than L2 (1.7 GB working set per step), no flush needed"
 NUMERICS = ("split-precision FP32 on tcgen05, FP32 accumulate: TF32 hi*hi + BF16 cross terms (dWeight: the same, "
-            "or three TF32 passes where the plan says so); FP32 FMA on the CUDA-core paths")
+            "or three TF32 passes, as the first-layer forward); FP32 FMA on the CUDA-core paths")
 
 
 def peaks():
@@ -263,11 +263,12 @@ class Layer:
 
 
 # dram__bytes_read.sum + dram__bytes_write.sum of ONE launch of the family's kernel on ONE layer of the sweep
-# (named in the note), from the ncu capture summarised in the strip-kernel summary under profiles/: bytes of
+# (named in the note), from the ncu captures summarised in profiles/: bytes of
 # that capture, not a live measurement and not a figure for the whole family.
 NCU_TRAFFIC_ONE_LAYER = {
-    "tc_strip_dweight": {"bytes_per_launch": 54.4e6, "layer": "128->128 28x28 3x3 batch 64 NCHW",
-                         "note": "51.5 MB read + 2.9 MB written per launch against 51.9 MB algorithmic (x + dy + dW)"},
+    "tc_strip_dweight": {"bytes_per_launch": 51.5e6, "layer": "128->128 28x28 3x3 batch 64 NCHW",
+                         "note": "51.5 MB read per launch of dweight_tmem_kernel (x + dy); its partial sums were still in L2 "
+                                 "when the capture ended"},
     "tc_tstrip_forward": {"bytes_per_launch": 26.9e6, "layer": "128->128 28x28 3x3 batch 64 NCHW",
                           "note": "26.9 MB read per launch (x + filter); the 25.7 MB output was still in L2 when the capture ended"},
     "tc_tstrip_dinput": {"bytes_per_launch": 26.9e6, "layer": "128->128 28x28 3x3 batch 64 NCHW",
@@ -739,7 +740,7 @@ def main():
                     "traffic_note": traffic.get("note"),
                     "peak_source": f"{pk['source']}: sustained bf16 {pk['bf16_sustained']} TFLOP/s / 2 (TF32 rate); the split-precision "
                                    "scheme issues one TF32 and one BF16 pass of equal duration per algorithmic MAC (ceiling = peak/2), "
-                                   "three TF32 passes where the dWeight plan keeps 3xTF32 (peak/3)",
+                                   "three TF32 passes in dweight_strip_kernel: 1x1 filters, below 128 input channels (peak/3)",
                     "families": fam_stats,
                     "families_timed": ("an event pair around every library call in an eager pass of the same steps right before the "
                                        "timed region (the timed region replays a CUDA graph)") if graph is not None

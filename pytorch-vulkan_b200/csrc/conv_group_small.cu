@@ -163,7 +163,8 @@ __global__ void __launch_bounds__(THREADS, 4) gconv_fwd_kernel(const GArgs a) {
 // Bound by the FP32 multiply-adds (CPG * 9 per dy value) and by the shared-memory reads that feed them.  A thread owns
 // strips of 8 pixels and a 4 x 2 block of (output, input) channels: its 72 sums stay in registers, and the ten x values of
 // a filter row feed 4 * 3 * 8 multiply-adds, so the reads take under half the time of the arithmetic (one output channel
-// and 4 pixels per thread read as much for an eighth of the work: 151 us at 256 channels, 32x32, batch 16; 14 us now).
+// and 4 pixels per thread read as much for an eighth of the work: 151 us at 256 channels, 32x32, batch 16; 32 us now, the
+// input a channel slice of a wider tensor).
 // Tiles of (128 / NQ / SX) rows x 8*SX columns arrive by 4-byte cp.async (any strides; zero fill outside the image), one or
 // two tiles ahead of the one being used.
 struct GdwArgs {

@@ -11,7 +11,7 @@
 //
 // What bounds these layers and what follows from it.  A 3 -> 64 channel 7x7 layer has 147 products per output: the whole
 // filter fits shared memory, so every CTA splits it once and keeps it (no staging kernel, no workspace), and the tensor
-// work is small enough that feeding the tensor core is the problem: 1307 us on the CUDA-core kernel, 141 us here (batch 64,
+// work is small enough that feeding the tensor core is the problem: 1307 us on the CUDA-core kernel, 135 us here (batch 64,
 // 224x224, stride 2), of which the loads are a fifth and the tensor-memory stores with their splits a third.  The im2col rows are therefore never written to shared
 // memory: a producer thread owns one output pixel (one accumulator row), gathers 32 of its reduction values straight
 // into registers (coalesced across the warp's consecutive pixels, L1 serving the overlap of the windows), splits them and
