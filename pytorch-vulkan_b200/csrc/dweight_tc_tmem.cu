@@ -57,6 +57,7 @@ constexpr int MAX_RING = 24, MAX_A = 6, MAX_STRIPS = 8, MAX_GROUPS = 8, MAX_SLOT
 constexpr int ACC_COLS = 384;                // accumulator columns at most (two 64-column dY stages need the rest)
 constexpr int SCRATCH = 32 * 36 * 4;         // transpose tile of a dY warp
 constexpr int SMEM_LIMIT = 232448 - 2048;
+constexpr int NO_PIXEL = -2147483647 - 1;    // an element offset that no admitted view has (strides may be negative, run() bounds their span)
 constexpr int CHUNK_KB = 96;                 // K blocks per accumulation chain (see dweight_tc_strip.cu)
 // ... of layers with fewer than 32 (input channel, tap) pairs per group, which ran in FP32 on the CUDA cores before: 49 images of 95x95, 3 -> 80
 // channels, 3x3, off by 1.4e-5 in chains of 96, 1.0e-6 in chains of 4 (FP32 7.6e-7; in chains of 2 8e-7); 87 us, now 116 (FP32 613).
@@ -340,7 +341,7 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_tmem_kernel(const Args a) 
     const float* src = a.dy.ptr + chan_off;
     // lane = pixel (channels apart in memory) or lane = channel (channels adjacent)
     auto load = [&](int k, float (&v)[32]) {
-      int off = -1;                                // element offset of this lane's pixel, -1 where the contraction has nothing
+      int off = NO_PIXEL;                          // element offset of this lane's pixel, -1 where the contraction has nothing
       {
         const int qx = k_begin + k * KP + lane, q = qx + dq;
         if (qx < k_end && q >= 0 && q < a.q_total) {
@@ -358,15 +359,15 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_tmem_kernel(const Args a) 
 #pragma unroll
         for (int i = 0; i < 32; i += 4) {            // four pixels' offsets per read
           const int4 o = *reinterpret_cast<const int4*>(offs + i);
-          v[i] = o.x >= 0 && lane < chans ? __ldg(mine + o.x) : 0.f;
-          v[i + 1] = o.y >= 0 && lane < chans ? __ldg(mine + o.y) : 0.f;
-          v[i + 2] = o.z >= 0 && lane < chans ? __ldg(mine + o.z) : 0.f;
-          v[i + 3] = o.w >= 0 && lane < chans ? __ldg(mine + o.w) : 0.f;
+          v[i] = o.x != NO_PIXEL && lane < chans ? __ldg(mine + o.x) : 0.f;
+          v[i + 1] = o.y != NO_PIXEL && lane < chans ? __ldg(mine + o.y) : 0.f;
+          v[i + 2] = o.z != NO_PIXEL && lane < chans ? __ldg(mine + o.z) : 0.f;
+          v[i + 3] = o.w != NO_PIXEL && lane < chans ? __ldg(mine + o.w) : 0.f;
         }
       } else {
-        const float* p = src + (off >= 0 ? off : 0);
+        const float* p = src + (off != NO_PIXEL ? off : 0);
 #pragma unroll
-        for (int i = 0; i < 32; ++i, p += s1) v[i] = off >= 0 && i < chans ? __ldg(p) : 0.f;
+        for (int i = 0; i < 32; ++i, p += s1) v[i] = off != NO_PIXEL && i < chans ? __ldg(p) : 0.f;
       }
     };
     auto advance = [&] {

@@ -36,7 +36,7 @@ CASES = [  # (xshape, cout, kernel, conv arguments)
 ]
 
 
-def _run(case, layout, budget=64 << 20, gate=1e-5):
+def _run(case, layout, budget=64 << 20, gate=1e-5, flip=None):
     xshape, cout, kernel, kw = case
     rng = np.random.default_rng(sum(xshape) + cout)
     g = oracle.geometry(xshape, cout, kernel, **kw)
@@ -44,7 +44,8 @@ def _run(case, layout, budget=64 << 20, gate=1e-5):
     w = np.zeros(g.w_shape, np.float32)
     want = oracle.torch_conv_all(x, w, None, go, kw.get("stride", (1, 1)), kw.get("padding", (0, 0)), kw.get("dilation", (1, 1)), kw.get("groups", 1))[2]
     lay = (lambda a: np.ascontiguousarray(a.transpose(0, 2, 3, 1)).transpose(0, 3, 1, 2)) if layout == "nhwc" else (lambda a: a)
-    dw = b200conv.conv2d_backward(lay(go), lay(x), w, mask=(False, True, False), algo="tc", budget=budget, **kw)[1]
+    mirror = lambda a: lay(np.ascontiguousarray(a[flip]))[flip] if flip else lay(a)  # noqa: E731  the same values through negative strides
+    dw = b200conv.conv2d_backward(mirror(go), mirror(x), w, mask=(False, True, False), algo="tc", budget=budget, **kw)[1]
     assert b200conv.last_kernel() == "tc_strip_dweight" and b200conv.device_status() == 0
     assert oracle.rel_l2(dw, want) <= gate
 
@@ -53,6 +54,17 @@ def _run(case, layout, budget=64 << 20, gate=1e-5):
 @pytest.mark.parametrize("case", CASES, ids=lambda c: "x".join(map(str, c[0])) + f"-co{c[1]}-k{c[2][0]}x{c[2][1]}")
 def test_dweight(case, layout):
     _run(case, layout)
+
+
+_BACK, _ALL = slice(None, None, -1), slice(None)
+
+
+@pytest.mark.parametrize("flip", [(_BACK,), (_ALL, _ALL, _BACK), (_ALL, _ALL, _ALL, _BACK), (_ALL, _BACK), (_BACK, _ALL, _BACK, _BACK)],
+                         ids=["images", "rows", "columns", "channels", "images-rows-columns"])
+@pytest.mark.parametrize("layout", ["nchw", "nhwc"])
+@pytest.mark.parametrize("case", [CASES[0], CASES[5], CASES[14], CASES[18]], ids=lambda c: "x".join(map(str, c[0])))
+def test_views_with_negative_strides(case, layout, flip):
+    _run(case, layout, flip=flip)
 
 
 @pytest.mark.parametrize("case", [CASES[0], CASES[5], CASES[7]], ids=lambda c: "x".join(map(str, c[0])))
