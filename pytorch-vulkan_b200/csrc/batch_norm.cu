@@ -670,8 +670,8 @@ __global__ void __launch_bounds__(nres::THREADS, 4) bn_forward_channel_kernel(co
   uint32_t plane;
 #pragma unroll
   for (int k = 0; k < N; ++k) in[k].load(base + nres::unit_offset<VEC>(rows, min(u0 + k * nres::THREADS, rows.units - 1), plane), u0 + k * nres::THREADS < end);
-  __shared__ nres::Table<1> t0, t1;
-  const float2 m = nres::row_moments<VEC, N>(in, u0, end, origin, m_count, t0, t1, cluster);
+  __shared__ nres::Table<3> table;
+  const float2 m = nres::row_moments<VEC, N>(in, u0, end, origin, m_count, table, cluster);
   const float variance = m.y / m_count;
   const float inv = (variance == 0.f && v.eps == 0.f) ? 0.f : 1.f / sqrtf(variance + v.eps);
   if (rank == 0 && threadIdx.x == 0) {

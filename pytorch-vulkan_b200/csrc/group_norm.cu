@@ -380,8 +380,8 @@ __global__ void __launch_bounds__(nres::THREADS, 4) gn_forward_cluster_kernel(co
   nres::Unit<VEC> in[N];
 #pragma unroll
   for (int k = 0; k < N; ++k) in[k].load(x + base + (size_t)min(u0 + k * nres::THREADS, rows.units - 1) * VEC, u0 + k * nres::THREADS < end);
-  __shared__ nres::Table<1> t0, t1;
-  const float2 total = nres::row_moments<VEC, N>(in, u0, end, origin, sh.count, t0, t1, cluster);
+  __shared__ nres::Table<3> table;
+  const float2 total = nres::row_moments<VEC, N>(in, u0, end, origin, sh.count, table, cluster);
   const float mean_rel = total.x, rstd = 1.f / sqrtf(total.y / sh.count + eps);
   if (rank == 0 && threadIdx.x == 0) {
     means[row] = origin + mean_rel;
