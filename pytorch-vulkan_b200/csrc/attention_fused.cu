@@ -148,7 +148,7 @@ __device__ __forceinline__ void attention_tile(const Args& a) {
   const uint32_t colb = cols + STAGES * C_STAGE;
   Ctrl* ctrl = reinterpret_cast<Ctrl*>(smem_raw + (colb - raw) + STAGES * COL_BYTES);
   volatile int* abort_flag = &ctrl->abort_flag;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int row0 = blockIdx.x * M;
   const long long batch = blockIdx.y;
   if (row0 >= a.rows) return;

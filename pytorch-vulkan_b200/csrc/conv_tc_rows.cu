@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv_rows_kernel(const RowsArgs a)
   RunEntry* tab = reinterpret_cast<RunEntry*>(w_smem + (size_t)a.ntn * a.nkb * w_block);
   Ctrl* ctrl = reinterpret_cast<Ctrl*>(tab + a.nkb * (KBLK / LP));
   volatile int* abort_flag = &ctrl->abort_flag;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int ch0 = (int)(blockIdx.x % (unsigned)a.nt_split) * a.ntn * a.bn;   // first output channel of this CTA
   const uint32_t cta = blockIdx.x / (unsigned)a.nt_split, ctas = gridDim.x / (unsigned)a.nt_split;
 

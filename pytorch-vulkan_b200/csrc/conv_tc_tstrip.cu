@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(tstrip_threads(AW), 1) conv_tstrip_kernel(cons
   const uint32_t tbuf_base = w_base + a.w_stages * W_RING_BYTES;
   Ctrl* ctrl = reinterpret_cast<Ctrl*>(smem_raw + (tbuf_base - raw) + TBUF_BYTES);
   volatile int* abort_flag = &ctrl->abort_flag;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   constexpr uint32_t ACC_COLS = 256, TMEM_COLS = 512;
   const long long prof_c0 = (B200_ROLE_PROFILE && a.prof) ? clock64() : 0;
 

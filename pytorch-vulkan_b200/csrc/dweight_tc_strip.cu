@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_strip_kernel(const DwStrip
   const uint32_t stage_bytes = x_bytes + 2u * y_plane;
   Ctrl* ctrl = reinterpret_cast<Ctrl*>(smem_raw + (base - raw) + a.stages * stage_bytes);
   volatile int* abort_flag = &ctrl->abort_flag;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int x_halves = a.xr > 32 ? 2 : 1;                      // a strip = rows 0..31 and 32..47; an exact block = 32 rows
   const int kx0 = (int)(blockIdx.x % (unsigned)a.kx_groups) * 4;  // first horizontal tap of this CTA
   // taps beyond the filter width of a narrow filter are not staged (their accumulator rows are never

@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_tmem_kernel(const Args a) 
   Ctrl* ctrl = reinterpret_cast<Ctrl*>(scratch_all + dy_warps * SCRATCH);
   FoldEntry* fold_tab = reinterpret_cast<FoldEntry*>(ctrl + 1);   // [cig]
   volatile int* abort_flag = &ctrl->abort_flag;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < MAX_RING; ++s) {

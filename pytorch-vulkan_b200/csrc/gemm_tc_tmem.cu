@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const GemmArgs a)
   const uint32_t raw = smem_u32(smem_raw), w_base = (raw + 1023u) & ~1023u;
   Ctrl* ctrl = reinterpret_cast<Ctrl*>(smem_raw + (w_base - raw) + W_STAGES * W_BYTES + 4 * SETS * DEPTH * SLOT);
   volatile int* abort_flag = &ctrl->abort_flag;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < A_STAGES; ++s) {
       mbar_init(smem_u32(&ctrl->a_full[s]), 4);

@@ -20,6 +20,12 @@ constexpr int STATUS_TIMEOUT_TMA = 4;    // bulk copy never landed
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
+// Index of this warp in the CTA, as a value that the compiler knows to be the same in all lanes: what a warp's role and its jobs are computed from
+// then runs on the uniform datapath.  From threadIdx alone it takes every role for divergent code, and each load, tensor-memory access and MMA there
+// moves its descriptors to uniform registers again (R2UR: 12 to 24 for every MMA of dWeight and of the first layer, now 1 or 2).  dWeight
+// of 64 x 128 -> 128 channels, 56x56, stride 2, channels-last 92 -> 66 us, of 512 -> 512, 7x7, 77 -> 71; first-layer forward 138 -> 126,
+// attention of 16x1024x64 28.8 + 97.7 -> 26.5 + 92.7.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
