@@ -131,11 +131,12 @@ __device__ __forceinline__ void store_block_chunks(const float (&val)[32], int r
 }
 // Store for the lane = row pattern; val[j] holds channel j ^ 4 in lanes 4-7 of every eight (see stage_block).
 template <bool DW_CROSS>
-__device__ __forceinline__ void store_block(const float (&val)[32], int rows, int row0, const BlockPlanes& pl, int lane) {
+__device__ __forceinline__ void store_block(const float (&val)[32], int rows, int row0, const BlockPlanes& pl, int lane, int chans = 32) {
   if (lane >= rows) return;
   const uint32_t sw = (uint32_t)((lane >> 2) & 1);
 #pragma unroll
   for (int m = 0; m < 4; ++m) {
+    if (8 * m >= chans) break;   // nothing reads what lies in these columns
     float h0[4], l0[4], h1[4], l1[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {

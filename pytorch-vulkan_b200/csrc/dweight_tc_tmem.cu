@@ -22,7 +22,9 @@
 //
 // FOLD (fewer than sixteen input channels: a network's first layer): the (input channel, ky) pairs of a pixel take the place of the
 // channels of a strip, 21 of 32 for 3 channels and a 7x7 filter, and the taps kx stay row offsets.  dW is then that of a
-// one-row filter over cin * kh channels, whose layout it already has.
+// one-row filter over cin * kh channels, whose layout it already has.  Four offsets of these channels come with one read, pieces of eight
+// channels beyond the last are neither loaded nor stored, and filter rows are tested only where the image cuts some off (one read
+// and test a value took 28 instructions for each; 186 -> 181 us on that layer).
 //
 // The pixel grid, the split of the contraction over CTAs, the chunked accumulation (the tensor core truncates: CHUNK_KB) and
 // the partial layout [split][cout][kh*kw][cin/g] are those of dweight_tc_strip.cu.
@@ -31,6 +33,9 @@
 //
 // CTA roles: two or three sets of four dY warps (set s stages K blocks = s mod sets, a warp the lanes of its quarter; they
 // also fold the accumulator), then input warps up to warp 14, warp 15 MMA issue.  All waits are bounded.
+// Where 64 or fewer output channels leave lanes 64-127 empty and no second tap fills them (folded layers, 1x1 filters), the warps of those
+// quarters stage input, and four sets of two warps stage dY: a dY block is a load from memory, a conversion and a store in one warp, so
+// the number of warps that have one on its way sets the pace.  3 -> 64 channels, 7x7, stride 2, 64x224x224: 186 us, now 144.
 //
 // Replaces csrc/shaders/conv2d_backward_weight_tiled_body.glsl:42-70 of the reference for these geometries.
 #include "common.cuh"
@@ -53,10 +58,12 @@ constexpr int KP = 32;                       // pixels per K block
 constexpr int HALO = 8;                      // rows that horizontal taps may reach beyond a K block's own
 constexpr int MIRROR = KP + HALO;            // rows repeated behind the end of a ring
 constexpr int MMA_WARP = 15, THREADS = 512;
+constexpr int NARROW_X_WARPS = 7;            // warps 2, 3, 6, 7, 10, 11, 14
 constexpr int MAX_RING = 24, MAX_A = 6, MAX_STRIPS = 8, MAX_GROUPS = 8, MAX_SLOTS = 12;
 constexpr int ACC_COLS = 384;                // accumulator columns at most (two 64-column dY stages need the rest)
 constexpr int SCRATCH = 32 * 36 * 4;         // transpose tile of a dY warp
 constexpr int SMEM_LIMIT = 232448 - 2048;
+constexpr int FOLD_MAX = 256;                // (input channel, filter row) pairs at most
 constexpr int NO_PIXEL = -2147483647 - 1;    // an element offset that no admitted view has (strides may be negative, run() bounds their span)
 constexpr int CHUNK_KB = 96;                 // K blocks per accumulation chain (see dweight_tc_strip.cu)
 // ... of layers with fewer than 32 (input channel, tap) pairs per group, which ran in FP32 on the CUDA cores before: 49 images of 95x95, 3 -> 80
@@ -88,6 +95,7 @@ struct Args {
   int q_first, q_total;       // contraction range [q_first, q_total); q_first < 0 in shift mode
   FastDiv img_div, row_div, div_strips, div_ring;
   int dy_sets, ahead;         // sets of dY warps; chunks a K block reads beyond its own
+  int narrow;                 // 64 or fewer output channels and no shift: a set is two warps, the warps of the other quarters stage input
   int span, splits;
   int shift_rows;             // shift mode: lanes 64-127 hold dY this many grid pixels ahead (0: off)
   int nci, ci_tiles, ky_tiles, co_tiles;
@@ -101,15 +109,14 @@ struct Args {
   int* status;
 };
 
-struct FoldEntry {
-  int offset, ky;            // elements from the window's first row; filter row
-};
 
 struct Ctrl {
   unsigned long long x_full[MAX_RING], x_empty[MAX_RING], a_full[MAX_A], a_empty[MAX_A], accum, drained;
   uint32_t tmem_base;
   int abort_flag;
 };
+
+constexpr int FOLD_AT = ((int)sizeof(Ctrl) + 15) / 16 * 16;   // the fold table behind Ctrl, in 16-byte pieces
 
 // whether the phase has completed, without the suspension of try_wait
 __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
@@ -136,9 +143,10 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_tmem_kernel(const Args a) 
   const uint32_t ring_pixels = (uint32_t)(a.ring * KP), ring_rows = ring_pixels + MIRROR;
   const uint32_t strip_bytes = ring_rows * 256u;                 // hi ring (128-byte rows), then bf16(hi) and bf16(lo) rings (64-byte rows)
   unsigned char* scratch_all = smem_raw + (base - raw) + a.n_strips * strip_bytes;
-  const int dy_warps = 4 * a.dy_sets;
+  const int dy_quarters = a.narrow ? 2 : 4, dy_warps = dy_quarters * a.dy_sets;
   Ctrl* ctrl = reinterpret_cast<Ctrl*>(scratch_all + dy_warps * SCRATCH);
-  FoldEntry* fold_tab = reinterpret_cast<FoldEntry*>(ctrl + 1);   // [cig]
+  int* fold_off = reinterpret_cast<int*>(scratch_all + dy_warps * SCRATCH + FOLD_AT);   // [cig up to a multiple of 32] elements from the window's first row
+  int* fold_ky = fold_off + FOLD_MAX;                                                   // filter row
   volatile int* abort_flag = &ctrl->abort_flag;
   const int warp = warp_index(), lane = threadIdx.x & 31;
 
@@ -148,7 +156,7 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_tmem_kernel(const Args a) 
       mbar_init(smem_u32(&ctrl->x_empty[s]), 1);
     }
     for (int s = 0; s < MAX_A; ++s) {
-      mbar_init(smem_u32(&ctrl->a_full[s]), 4);
+      mbar_init(smem_u32(&ctrl->a_full[s]), (uint32_t)dy_quarters);
       mbar_init(smem_u32(&ctrl->a_empty[s]), 1);
     }
     mbar_init(smem_u32(&ctrl->accum), 1);
@@ -157,9 +165,10 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_tmem_kernel(const Args a) 
     fence_barrier_init();
   }
   if (FOLD)
-    for (int c = threadIdx.x; c < g.cig; c += THREADS) {
+    for (int c = threadIdx.x; c < (g.cig + 31) / 32 * 32; c += THREADS) {
       const int ci = c / a.fold_kh, ky = c - ci * a.fold_kh;
-      fold_tab[c] = FoldEntry{(int)(ci * a.x.s1 + (long long)(ky * a.fold_dh) * a.x.s2), ky};
+      fold_off[c] = c < g.cig ? (int)(ci * a.x.s1 + (long long)(ky * a.fold_dh) * a.x.s2) : 0;
+      fold_ky[c] = c < g.cig ? ky : 31;                           // 31: no pixel has that row
     }
   if (warp == MMA_WARP) tmem_alloc(smem_u32(&ctrl->tmem_base), 512);
   tc_fence_before();
@@ -255,13 +264,13 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_tmem_kernel(const Args a) 
       }
     }
     if (leader) umma_commit(smem_u32(&ctrl->accum));
-  } else if (warp >= dy_warps) {
+  } else if (a.narrow ? (warp & 3) >= 2 : warp >= dy_warps) {
     // ---- input chunks: job j = (chunk, strip) goes to warp j mod (warps in use) ----
     const bool vec = channel_quads_aligned(a.x, g.cig, g.groups);
     const int jobs = (kblocks + a.ahead) * a.n_strips;
     // consecutive jobs of a warp stay within `ring` chunks of each other (a waiter must not skip a phase of a slot's barrier)
-    const int active = min(MMA_WARP - dy_warps, a.n_strips * a.ring);
-    const int xw = warp - dy_warps;
+    const int active = min(a.narrow ? NARROW_X_WARPS : MMA_WARP - dy_warps, a.n_strips * a.ring);
+    const int xw = a.narrow ? (warp >> 2) * 2 + (warp & 1) : warp - dy_warps;
     int dr0 = 0, pa0 = 0;
     if (ky0 >= 0) {
       const int oy = ky0 * g.dh - g.ph;
@@ -275,6 +284,7 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_tmem_kernel(const Args a) 
       if (FOLD) {
         const int q = k_begin + c * KP + st.dc + lane;
         uint32_t rows = 0;                         // filter rows of this pixel that lie inside the image
+        const uint32_t whole = (1u << a.fold_kh) - 1u;
         const float* p = a.x.ptr;
         if (q >= 0 && q < a.q_total) {
           const int n = (int)a.img_div.div((uint32_t)q), rem = q - n * img_pitch;
@@ -285,11 +295,21 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_tmem_kernel(const Args a) 
           }
         }
         const int sw = ((lane >> 2) & 1) << 2;     // store_block's register order
+        const bool inside = rows != 0;
+        const bool all_rows = __all_sync(0xffffffffu, rows == whole || !inside);   // no row cut off by the image: one predicate for the pixel
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const int ch = c0 + (i ^ sw);
-          const FoldEntry e = fold_tab[min(ch, g.cig - 1)];
-          val[i] = ch < g.cig && ((rows >> e.ky) & 1u) ? __ldg(p + e.offset) : 0.f;
+        for (int m = 0; m < 32; m += 4) {
+          if (c0 + (m & ~7) >= g.cig) break;       // the columns of these channels are never read
+          const int at = c0 + (m ^ sw);
+          const int4 o = *reinterpret_cast<const int4*>(fold_off + at);
+          if (all_rows) {
+            val[m] = inside ? __ldg(p + o.x) : 0.f; val[m + 1] = inside ? __ldg(p + o.y) : 0.f;
+            val[m + 2] = inside ? __ldg(p + o.z) : 0.f; val[m + 3] = inside ? __ldg(p + o.w) : 0.f;
+          } else {
+            const int4 k = *reinterpret_cast<const int4*>(fold_ky + at);
+            val[m] = (rows >> k.x) & 1u ? __ldg(p + o.x) : 0.f; val[m + 1] = (rows >> k.y) & 1u ? __ldg(p + o.y) : 0.f;
+            val[m + 2] = (rows >> k.z) & 1u ? __ldg(p + o.z) : 0.f; val[m + 3] = (rows >> k.w) & 1u ? __ldg(p + o.w) : 0.f;
+          }
         }
         return false;
       }
@@ -314,16 +334,16 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_tmem_kernel(const Args a) 
       for (int i = 0; i < copies; ++i) {
         const int row0 = slot * KP + i * (int)ring_pixels, rows = i ? min(KP, MIRROR - slot * KP) : KP;
         if (chunked) tcdw::store_block_chunks<true>(val, rows, row0, pl, lane);
-        else tcdw::store_block<true>(val, rows, row0, pl, lane);
+        else tcdw::store_block<true>(val, rows, row0, pl, lane, FOLD ? g.cig - ci0 - a.strips[strip].cblk * 32 : 32);
       }
       fence_proxy_async();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&ctrl->x_full[slot]));
     }
-  } else {
+  } else if (!a.narrow || (warp >> 2) < a.dy_sets) {
     // ---- dY: lane = output channel (tensor-memory lane quarter * 32 + lane), columns = pixels ----
     const int set = warp >> 2, quarter = warp & 3;
-    float* scratch = reinterpret_cast<float*>(scratch_all + warp * SCRATCH);
+    float* scratch = reinterpret_cast<float*>(scratch_all + (set * dy_quarters + quarter) * SCRATCH);
     const bool shift = a.shift_rows != 0;
     const int cq = co0 + (shift ? (quarter & 1) : quarter) * 32;           // first channel of this warp
     const int dq = shift && quarter >= 2 ? a.shift_rows : 0;
@@ -568,7 +588,7 @@ static Plan make_plan(const ConvGeom& real, size_t budget) {
   ConvGeom g = real;
   const bool fold = real.cig < 16;
   if (fold) {
-    if (real.groups != 1 || real.kh > 31 || real.cig * real.kh > 256 || real.cig * real.kh * real.kw < 9) return best;
+    if (real.groups != 1 || real.kh > 31 || real.cig * real.kh > FOLD_MAX || real.cig * real.kh * real.kw < 9) return best;
     g.cin = g.cig = real.cig * real.kh;
     g.kh = 1; g.ph = 0; g.dh = 1; g.sh = 1; g.h = g.oh;
   }
@@ -625,7 +645,10 @@ static Plan make_plan(const ConvGeom& real, size_t budget) {
       auto slower = [&](int sets) { return std::max(1.0 / sets, (double)a.n_strips / (MMA_WARP - 4 * sets)); };
       for (int sets = 2; sets <= std::min(3, a.a_stages); ++sets)
         if (slower(sets) < slower(a.dy_sets)) a.dy_sets = sets;
-      const int fixed_smem = 4 * a.dy_sets * SCRATCH + (int)sizeof(Ctrl) + (fold ? g.cig * (int)sizeof(FoldEntry) : 0) + 1024 + 64;
+      // lanes 64-127 have no channels: their warps stage input instead
+      a.narrow = g.cog <= 64 && !shift;
+      if (a.narrow) a.dy_sets = std::min(4, a.a_stages);
+      const int fixed_smem = (a.narrow ? 2 : 4) * a.dy_sets * SCRATCH + (int)sizeof(Ctrl) + (fold ? 2 * FOLD_MAX * (int)sizeof(int) + 16 : 0) + 1024 + 64;
       a.ring = std::min({MAX_RING, a.ahead + 6, (SMEM_LIMIT - fixed_smem - a.n_strips * MIRROR * 256) / (a.n_strips * KP * 256)});
       if (a.ring < a.ahead + 3 || a.a_stages < 2) continue;
       a.ci_tiles = (cib + nci - 1) / nci;
@@ -638,7 +661,8 @@ static Plan make_plan(const ConvGeom& real, size_t budget) {
       // of the staging warps (about 2400 clocks per job and warp)
       const int dy_jobs = shift ? 2 * std::min(2, (g.cog + 31) / 32) : std::min(4, (g.cog + 31) / 32);
       const double mma = 128.0 * a.n_slots + 100.0 + 60.0 * a.n_groups + 30.0 * (a.n_strips + dy_jobs);
-      const double kb_clk = std::max({mma, 4096.0 * (a.n_strips + dy_jobs) / 22.0, 2400.0 * slower(a.dy_sets)});
+      const double kb_clk = std::max({mma, 4096.0 * (a.n_strips + dy_jobs) / 22.0,
+                                      2400.0 * (a.narrow ? std::max(1.0 / a.dy_sets, (double)a.n_strips / NARROW_X_WARPS) : slower(a.dy_sets))});
       for (int w = 0; w <= 3; ++w) {
         long long sp = w == 0 ? 1 : w * (long long)sm_count() / p.tiles;
         sp = std::min<long long>({sp, std::max<long long>(1, kb_total / 6), 65535, std::max<long long>(1, (long long)(budget / dw_bytes))});
