@@ -180,6 +180,10 @@ int conv_sliced(const ConvGeom& g, bool is_dx, int slices, bool allow_transposed
 size_t tstrip_workspace(const ConvGeom& g, int phase);
 int tstrip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* bias, long long bias_stride, float* out,
                 void* ws, size_t ws_bytes, cudaStream_t st, long long w_group_extra = 0);
+// one-launch kernel for layers of a few tiles (conv_tc_small.cu), no workspace
+bool conv_small_wanted(const ConvGeom& g, bool is_dx, bool allow_transposed);
+int conv_small(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* bias, long long bias_stride, const StripPostOps* post, float* out,
+               cudaStream_t st);
 // row kernel (conv_tc_rows.cu): forward passes of layers with fewer than 16 input channels, no workspace
 bool rows_supported(const ConvGeom& g);
 int rows_conv(const ConvGeom& g, View4 x, View4 w, const float* bias, long long bias_stride, float* y, cudaStream_t st);

@@ -122,6 +122,12 @@ static int reconsider_for_layout(const ConvGeom& g, int phase, int algo, int cho
   return tc_workspace(g, phase, workspace, nullptr, nullptr) <= workspace ? B200_ALGO_TC : chosen;
 }
 
+// The automatic choice of the tcgen05 kernels goes to the one-launch kernel where a layer has few tiles; a forced candidate keeps the strip
+// kernels, and so does a workspace that they would refuse.
+static bool takes_one_launch(const ConvGeom& g, bool is_dx, int algo, int chosen, const void* workspace, bool fused = false) {
+  return algo == B200_ALGO_AUTO && chosen == B200_ALGO_TC && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0 && conv_small_wanted(g, is_dx, !fused);
+}
+
 }  // namespace b200
 
 using namespace b200;
@@ -203,6 +209,10 @@ int b200_conv2d_forward(const b200_conv_params* p, b200_view4 x, b200_view4 w, c
   chosen = reconsider_for_layout(g, B200_PHASE_FORWARD, algo, chosen, x, workspace ? workspace_bytes : 0);
   cudaStream_t st = (cudaStream_t)stream;
   if (!bias) bias_stride = 0;
+  if (takes_one_launch(g, false, algo, chosen, workspace)) {
+    note_kernel("tc_strip_forward");
+    return conv_small(g, false, to_view(x), to_view(w), bias, bias_stride, nullptr, y, st);
+  }
   switch (chosen) {
     case B200_ALGO_WINOGRAD:
       note_kernel("winograd_f4_forward");
@@ -242,6 +252,8 @@ int b200_conv2d_forward_fused(const b200_conv_params* p, b200_view4 x, b200_view
   // the strip kernel applies everything in its epilogue and can write [pixel][channel] rows
   if (chosen == B200_ALGO_TC && strip_supported(g, B200_PHASE_FORWARD)) {
     note_kernel("tc_strip_forward_fused");
+    if (!y_channels_last && takes_one_launch(g, false, algo, chosen, workspace, true))
+      return conv_small(g, false, to_view(x), to_view(w), bias, bias_stride, &post, y, st);
     if (const int slices = y_channels_last || !strip_view_addressable(g, false, to_view(x), nullptr) ? 1 : conv_slices(g, false, false);
         slices > 1 && workspace && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0 && conv_slices_workspace(g, false, slices, false) <= workspace_bytes)
       return conv_sliced(g, false, slices, false, to_view(x), to_view(w), bias, bias_stride, &post, y, workspace, st);
@@ -278,6 +290,12 @@ static int dinput_with_bias(const b200_conv_params* p, b200_view4 dy, b200_view4
       bias_applied = true;
       break;
     case B200_ALGO_TC:
+      if (takes_one_launch(g, true, algo, chosen, workspace)) {
+        note_kernel("tc_strip_dinput");
+        rc = conv_small(g, true, to_view(dy), to_view(w), bias, bias_stride, nullptr, dx, st);
+        bias_applied = true;
+        break;
+      }
       note_kernel("tc_igemm_dinput");
       rc = tc_dinput(g, to_view(dy), to_view(w), bias, bias_stride, dx, workspace, workspace_bytes, st, &bias_applied);
       break;
