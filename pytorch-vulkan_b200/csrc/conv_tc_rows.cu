@@ -20,8 +20,9 @@
 // that reading both operands from shared memory takes.
 //
 // CTA roles: warps 0-3 epilogue, GROUPS groups of four producer warps (a group stages one K block of 128 pixels x 32
-// reduction values at a time; three groups fit the register file beside the rest: eight epilogue warps would leave 80 registers a thread and
-// spills), one MMA warp.  Tensor memory: two accumulators, or pairs of them (main, cross; one pair where they have more than 64 columns), the
+// reduction values at a time), one MMA warp.  A K block is loads, a conversion and a store in one warp, so four groups are faster than three although
+// they leave 80 registers a thread (some spills): 3 -> 64 channels, 7x7, stride 2, 64x224x224 126 -> 118 us; where a CTA has fewer than seven K
+// blocks the larger CTA starts later than it gains (8 images of 120x120, 4 -> 32 channels, 3x3, 6.5 and 7.0 us).  Tensor memory: two accumulators, or pairs of them (main, cross; one pair where they have more than 64 columns), the
 // rest operand stages of 64 columns (32 high parts, 32 low parts).
 //
 // Replaces csrc/shaders/conv2d_tiled_body.glsl:53-86 of the reference for these geometries.
@@ -37,9 +38,10 @@ namespace tcr {
 using namespace tc;
 
 constexpr int BLOCK_M = 128, KBLK = 32, EPI_WARPS = 4;
-constexpr int GROUPS = 3;
-constexpr int MMA_WARP = EPI_WARPS + 4 * GROUPS, THREADS = (MMA_WARP + 1) * 32;
+template <int GROUPS> constexpr int MMA_WARP_OF = EPI_WARPS + 4 * GROUPS;
+template <int GROUPS> constexpr int THREADS_OF = (MMA_WARP_OF<GROUPS> + 1) * 32;
 constexpr int MAX_STAGES = 6, MAX_RUNS = 1024;
+constexpr int FOUR_GROUPS_FROM = 7;   // K blocks of a CTA
 constexpr int SEG_KB = 12;      // K blocks (of four main steps) per accumulation chain
 constexpr int SMEM_LIMIT = 232448 - 2048;
 constexpr uint32_t STAGE_COLS = 64;
@@ -76,8 +78,9 @@ struct RunEntry {
 };
 
 // PAIR: the cross terms have an accumulator of their own
-template <int LP, bool UNIT, bool PAIR>
-__global__ void __launch_bounds__(THREADS, 1) conv_rows_kernel(const RowsArgs a) {
+template <int LP, bool UNIT, bool PAIR, int GROUPS>
+__global__ void __launch_bounds__(THREADS_OF<GROUPS>, 1) conv_rows_kernel(const RowsArgs a) {
+  constexpr int MMA_WARP = MMA_WARP_OF<GROUPS>, THREADS = THREADS_OF<GROUPS>;
   wait_previous();
   extern __shared__ unsigned char smem_raw[];
   const ConvGeom& g = a.g;
@@ -343,15 +346,22 @@ static RowsPlan plan_rows(const ConvGeom& g, bool channels_last) {
   return p;
 }
 
-template <int LP, bool UNIT, bool PAIR>
-static int launch_rows(const RowsArgs& a, int smem, cudaStream_t st) {
+template <int LP, bool UNIT, bool PAIR, int GROUPS>
+static int launch_groups(const RowsArgs& a, unsigned ctas, int smem, cudaStream_t st) {
   static std::once_flag once;
   static cudaError_t opt_in = cudaSuccess;
-  std::call_once(once, [] { opt_in = cudaFuncSetAttribute(conv_rows_kernel<LP, UNIT, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448); });
+  std::call_once(once, [] { opt_in = cudaFuncSetAttribute(conv_rows_kernel<LP, UNIT, PAIR, GROUPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448); });
   B200_CUDA(opt_in);
-  launch_next(conv_rows_kernel<LP, UNIT, PAIR>, (unsigned)(std::min(a.tiles_m, std::max(1, sm_count() / a.nt_split)) * a.nt_split), THREADS, (size_t)smem, st, a);
+  launch_next(conv_rows_kernel<LP, UNIT, PAIR, GROUPS>, ctas, THREADS_OF<GROUPS>, (size_t)smem, st, a);
   count_launch();
   return launch_check("conv_rows_kernel");
+}
+template <int LP, bool UNIT, bool PAIR>
+static int launch_rows(const RowsArgs& a, int smem, cudaStream_t st) {
+  const int share = std::min(a.tiles_m, std::max(1, sm_count() / a.nt_split));   // CTAs that share the pixel tiles
+  const unsigned ctas = (unsigned)(share * a.nt_split);
+  const bool many = div_up64(a.tiles_m, share) * a.ntn * a.nkb >= FOUR_GROUPS_FROM;
+  return many ? launch_groups<LP, UNIT, PAIR, 4>(a, ctas, smem, st) : launch_groups<LP, UNIT, PAIR, 3>(a, ctas, smem, st);
 }
 
 }  // namespace tcr
