@@ -174,9 +174,11 @@ double strip_time(const ConvGeom& g, bool is_dx, long long* tiles);
 double tstrip_time(const ConvGeom& g, bool is_dx, long long* tiles);
 // reduction channels in slices (conv_slices.cu); `ws` holds conv_slices_workspace() bytes
 int conv_slices(const ConvGeom& g, bool is_dx, bool allow_transposed);
+double conv_slices_time(const ConvGeom& g, bool is_dx);   // modelled time of the strip kernel, in slices where that is better
 size_t conv_slices_workspace(const ConvGeom& g, bool is_dx, int slices, bool allow_transposed);
 int conv_sliced(const ConvGeom& g, bool is_dx, int slices, bool allow_transposed, View4 act, View4 w, const float* bias, long long bias_stride,
                 const StripPostOps* post, float* out, void* ws, cudaStream_t st);
+bool tstrip_stacks(const ConvGeom& g, bool is_dx);   // 64 or fewer output channels, two taps to a tile: better than the strip kernel
 size_t tstrip_workspace(const ConvGeom& g, int phase);
 int tstrip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* bias, long long bias_stride, float* out,
                 void* ws, size_t ws_bytes, cudaStream_t st, long long w_group_extra = 0);

@@ -72,13 +72,14 @@ long long out_count(const ConvGeom& g, bool is_dx) { return is_dx ? (long long)g
 // Slices by the kernels' own time models; 1 when one slice is as good.  A second launch costs about 3 us and the partial results a
 // write and a read, so layers below 12 us, or with two waves of tiles and more, are not looked at further (64 -> 64 channels of one 28x28
 // image, 13 us, gain nothing: half the stages against the second launch).
-static int plan_slices(const ConvGeom& g, bool is_dx, bool transposed) {
+static int plan_slices(const ConvGeom& g, bool is_dx, bool transposed, double* time = nullptr) {
   const int kc = is_dx ? g.cout : g.cin, phase = is_dx ? B200_PHASE_DINPUT : B200_PHASE_FORWARD;
   if (!transposed && !strip_supported(g, phase)) return 1;
   const long long values = out_count(g, is_dx);
   if (values * MAX_SLICES >= 1ll << 31) return 1;
   long long tiles;
   const double whole = transposed ? tstrip_time(g, is_dx, &tiles) : strip_time(g, is_dx, &tiles);
+  if (time) *time = whole;
   if (whole < 12.0 || tiles >= 2ll * sm_count()) return 1;
   int best = 1;
   double best_time = whole;
@@ -88,7 +89,14 @@ static int plan_slices(const ConvGeom& g, bool is_dx, bool transposed) {
     const double t = (transposed ? tstrip_time(gs, is_dx, nullptr) : strip_time(gs, is_dx, nullptr)) + 3.0 + (double)values * (8.0 * s + 4.0) * 2e-7;
     if (t < 0.95 * best_time) { best = s; best_time = t; }
   }
+  if (time) *time = best_time;
   return best;
+}
+double conv_slices_time(const ConvGeom& g, bool is_dx) {
+  const int kc = is_dx ? g.cout : g.cin;
+  double time = strip_time(g, is_dx, nullptr);
+  if (g.groups == 1 && kc % 32 == 0 && kc >= 64) plan_slices(g, is_dx, false, &time);
+  return time;
 }
 int conv_slices(const ConvGeom& g, bool is_dx, bool allow_transposed) {
   const int kc = is_dx ? g.cout : g.cin;

@@ -612,6 +612,8 @@ size_t tc_workspace(const ConvGeom& g, int phase, size_t budget, int* splits_out
     const size_t planes = 2 * sizeof(float) * (size_t)g.cout * g.cig * g.kh * g.kw;  // hi + lo
     size_t need = strip_allowed() && strip_supported(g, phase) ? std::max(planes, strip_workspace(g, phase)) : planes;
     if (strip_allowed() && tstrip_supported(g, phase)) need = std::max(need, tstrip_workspace(g, phase));
+    if (strip_allowed() && tstrip_stacks(g, phase == B200_PHASE_DINPUT))
+      if (const size_t more = tstrip_workspace(g, phase); more <= budget) need = std::max(need, more);   // wanted, not needed
     if (const int slices = strip_allowed() ? conv_slices(g, phase == B200_PHASE_DINPUT, true) : 1; slices > 1) {
       const size_t more = conv_slices_workspace(g, phase == B200_PHASE_DINPUT, slices, true);  // wanted, not needed
       if (more <= budget) need = std::max(need, more);
@@ -736,6 +738,10 @@ int tc_forward(const ConvGeom& g, View4 x, View4 w, const float* bias, long long
     if (rc != B200_EUNSUPPORTED) return rc;   // falls through to the CUDA-core kernel
   }
   int route = tc_route(g, false, x);
+  if (route == 0 && ws && (reinterpret_cast<uintptr_t>(ws) & 15) == 0 && tstrip_stacks(g, false) && tstrip_workspace(g, B200_PHASE_FORWARD) <= ws_bytes) {
+    note_kernel("tc_strip_forward");
+    return tstrip_conv(g, false, x, w, bias, bias_stride, y, ws, ws_bytes, st);
+  }
   if (route == 3 || route == 0)
     if (const int slices = conv_slices(g, false, true);
         slices > 1 && ws && (reinterpret_cast<uintptr_t>(ws) & 15) == 0 && conv_slices_workspace(g, false, slices, true) <= ws_bytes) {
@@ -765,6 +771,10 @@ int tc_dinput(const ConvGeom& g, View4 dy, View4 w, const float* bias, long long
               cudaStream_t st, bool* bias_applied) {
   if (bias_applied) *bias_applied = bias != nullptr;
   int route = tc_route(g, true, dy);
+  if (route == 0 && ws && (reinterpret_cast<uintptr_t>(ws) & 15) == 0 && tstrip_stacks(g, true) && tstrip_workspace(g, B200_PHASE_DINPUT) <= ws_bytes) {
+    note_kernel("tc_strip_dinput");
+    return tstrip_conv(g, true, dy, w, bias, bias_stride, dx, ws, ws_bytes, st);
+  }
   if (route == 3 || route == 0)
     if (const int slices = conv_slices(g, true, true);
         slices > 1 && ws && (reinterpret_cast<uintptr_t>(ws) & 15) == 0 && conv_slices_workspace(g, true, slices, true) <= ws_bytes) {

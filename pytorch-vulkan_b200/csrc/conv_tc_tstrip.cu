@@ -31,8 +31,7 @@
 // All hand-offs are mbarriers with bounded waits.
 //
 // Replaces csrc/shaders/conv2d_tiled_body.glsl:53-86 and conv2d_backward_input_tiled_body.glsl:49-93 of the
-// reference for contiguous NCHW results with at least 65 output channels per group (below that half of every
-// MMA would multiply padding, and conv_tc_strip.cu is the better arrangement).
+// reference for contiguous NCHW results with at least 65 output channels per group, and for fewer where two taps can share a tile.
 #include "common.cuh"
 #include "plan_cache.cuh"
 #include "strip_plan.cuh"
@@ -81,6 +80,7 @@ struct TArgs {
   int cb_per_phase, cblocks, images_per_tile;
   int tiles_m, tiles_p, tiles_total;
   int pn;                 // pixels per tile: a multiple of 16, at most 256
+  int delta, step;        // stacked taps: grid pixels between the two taps of a stack (0: off); pixels that a tile completes, pn - delta
   int q_total;
   FastDiv img_div, row_div, div_tiles_p, div_tiles_m, div_tiles_pp, div_chunks, div_cblocks, div_cbpp, div_a_stages;
   int halo, strip_rows;   // rows staged before a tile's first pixel; rows per stage (a multiple of 8)
@@ -102,6 +102,13 @@ struct TArgs {
 #endif
 #define TPROF(slot, stmt) do { if (B200_ROLE_PROFILE && a.prof && blockIdx.x == 0) { const long long t0__ = clock64(); stmt; atomicAdd(a.prof + (slot), (unsigned long long)(clock64() - t0__)); } else { stmt; } } while (0)
 
+// Second tap of a stack (filter column, NO_TAP: none) where 64 or fewer output channels leave half of the filter rows to it
+constexpr unsigned char NO_TAP = 255;
+struct Stacked {
+  int delta = 0;
+  unsigned char kx[MAX_TAPS];
+};
+
 struct Ctrl {
   unsigned long long a_full[MAX_A_STAGES], a_empty[MAX_A_STAGES], w_full[MAX_W_STAGES], w_empty[MAX_W_STAGES], acc_full[2], acc_empty[2];
   uint32_t tmem_base;
@@ -113,6 +120,14 @@ struct Ctrl {
 // byte offset of 16-byte chunk `c` (0..3) of row `row` in a plane of 64-byte rows, SWIZZLE_64B
 __device__ __host__ __forceinline__ uint32_t sw64_chunk(int row, int c) {
   return (uint32_t)(row * ROWB + ((c ^ ((row >> 1) & 3)) << 4));
+}
+// barrier of the epilogue warps; with a predicate, true for all where it is true for each
+__device__ __forceinline__ void epilogue_sync() { asm volatile("barrier.cta.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory"); }
+__device__ __forceinline__ bool epilogue_all(bool mine) {
+  int all;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbarrier.cta.red.and.pred q, 1, %2, p;\n\tselp.b32 %0, 1, 0, q;\n\t}"
+               : "=r"(all) : "r"((int)mine), "n"(EPI_WARPS * 32) : "memory");
+  return all != 0;
 }
 // K-major operand descriptor for a plane of 64-byte rows, SWIZZLE_64B: 8-row groups 512 bytes apart
 __device__ __forceinline__ uint64_t make_kmajor_sw64_desc(uint32_t smem_addr) {
@@ -307,7 +322,7 @@ __global__ void __launch_bounds__(tstrip_threads(AW), 1) conv_tstrip_kernel(cons
       const int phase = a.phase_on_m ? 0 : (int)a.div_cbpp.div((uint32_t)cb), cbl = cb - phase * a.cb_per_phase;
       const int nvalid = min(KB, a.kc - cbl * KB);
       const bool chunked = vec_layout && nvalid == KB;   // channels-last: four lanes fetch the 64 bytes of a pixel
-      const int q0 = tc_.p_tile * a.pn - a.halo + chunk * 32;
+      const int q0 = tc_.p_tile * a.step - a.halo + chunk * 32;
       float v[KB];
       // row -> address of its first channel (0 = the row is padding)
       const float* src = nullptr;
@@ -378,21 +393,27 @@ __global__ void __launch_bounds__(tstrip_threads(AW), 1) conv_tstrip_kernel(cons
     // Warp w owns accumulator lanes 32w .. 32w+31 (output channels).  tcgen05.ld hands thread = channel its 32
     // consecutive pixels; a 32x33 shared-memory tile turns that into thread = pixel, so that each store
     // instruction writes 32 consecutive pixels of one channel plane.
-    float* tb = reinterpret_cast<float*>(smem_raw + (tbuf_base - raw)) + warp * (32 * 33);
+    // Stacked taps: the lanes of warps 2 and 3 hold what the second taps add, `delta` pixels further on; every warp then adds and stores
+    // half of the channels of a pair of tiles.
+    float* tiles = reinterpret_cast<float*>(smem_raw + (tbuf_base - raw));
+    float* tb = tiles + warp * (32 * 33);
+    const int pair = a.delta ? warp & 1 : warp;
     for (int t = 0; t < my_tiles; ++t) {
       const TileCoord tc_ = tile_coord(a, (int)blockIdx.x + t * (int)gridDim.x);
       const int phase_m = a.phase_on_m ? (int)a.div_tiles_pp.div((uint32_t)tc_.m_tile) : 0;
-      const int c0 = (tc_.m_tile - phase_m * a.tiles_pp) * TM + warp * 32;   // first channel (within the group) of this warp
+      const int c0 = (tc_.m_tile - phase_m * a.tiles_pp) * TM + pair * 32;   // first channel (within the group) of this warp
       const int nch = min(32, a.nc - c0);                                       // channels of this warp that exist (may be <= 0)
       const uint32_t ab = (uint32_t)t & 1u;
       const bool has_taps = !a.phase_on_m || ctrl->tap_start[phase_m + 1] > ctrl->tap_start[phase_m];
       float bv = 0.f;  // lane j holds the bias of channel c0 + j
       if (a.bias && lane < nch) bv = __ldg(a.bias + ((long long)tc_.group * a.nc + c0 + lane) * a.bias_stride);
-      if (!mbar_wait(smem_u32(&ctrl->acc_full[ab]), ((uint32_t)t >> 1) & 1u, abort_flag, a.status, STATUS_TIMEOUT_ACCUM)) break;
+      bool complete = mbar_wait(smem_u32(&ctrl->acc_full[ab]), ((uint32_t)t >> 1) & 1u, abort_flag, a.status, STATUS_TIMEOUT_ACCUM);
+      if (a.delta) complete = epilogue_all(complete);   // the warps meet below: all of them go on, or none
+      if (!complete) break;
       tc_fence_after();
-      const uint32_t tmem_acc = tmem_base + ab * ACC_COLS + ((uint32_t)(warp * 32) << 16);
-      const int q_tile = tc_.p_tile * a.pn;
-      const int cols = min(a.pn, a.q_total - q_tile);
+      const uint32_t tmem_acc = tmem_base + ab * ACC_COLS + ((uint32_t)(warp * 32) << 16) + (uint32_t)(warp >= 2 ? a.delta : 0);
+      const int q_tile = tc_.p_tile * a.step;
+      const int cols = min(a.step, a.q_total - q_tile);
       const int nchunks = (cols + 31) / 32;
       const long long plane = (long long)a.out_h * a.out_w;
       const long long te__ = (B200_ROLE_PROFILE && a.prof && blockIdx.x == 0 && threadIdx.x == 0) ? clock64() : 0;
@@ -405,7 +426,7 @@ __global__ void __launch_bounds__(tstrip_threads(AW), 1) conv_tstrip_kernel(cons
           tc_fence_before();
           mbar_arrive(smem_u32(&ctrl->acc_empty[ab]));
         }
-        if (nch <= 0) continue;
+        if (nch <= 0 && !a.delta) continue;
         // this lane's pixel of the chunk
         const int q = q_tile + ch * 32 + lane;
         bool ok = ch * 32 + lane < cols;
@@ -418,6 +439,21 @@ __global__ void __launch_bounds__(tstrip_threads(AW), 1) conv_tstrip_kernel(cons
           if (a.phase_on_m) { y = y * a.osh + ctrl->ph_a[phase_m]; x = x * a.osw + ctrl->ph_b[phase_m]; }
           ok = ok && y < a.out_h && x < a.out_w;
           obase = ((n * a.out_channels + (long long)tc_.group * a.nc + c0) * a.out_h + y) * a.out_w + x;
+        }
+        if (a.delta) {
+          epilogue_sync();   // the previous chunk's reads of the tiles are done
+#pragma unroll
+          for (int j = 0; j < 32; ++j) tb[lane * 33 + j] = v[j];
+          epilogue_sync();
+          const int first = (warp >> 1) * 16;
+          const float *lower = tiles + pair * (32 * 33) + first * 33 + lane, *upper = lower + 2 * 32 * 33;
+          float* p = a.out + obase + first * plane;
+#pragma unroll
+          for (int c = 0; c < 16; ++c, p += plane) {
+            const float val = lower[c * 33] + upper[c * 33] + __shfl_sync(0xffffffffu, bv, first + c);
+            if (ok && first + c < nch) *p = val;
+          }
+          continue;
         }
         __syncwarp();   // the previous chunk's reads of the tile are done
 #pragma unroll
@@ -457,7 +493,8 @@ __global__ void __launch_bounds__(tstrip_threads(AW), 1) conv_tstrip_kernel(cons
 // main loop consumes them: forward [group][channel tile][phase][channel block][tap of the phase], dInput
 // [group][phase][channel tile of the phase][channel block][tap of the phase].  A thread takes four channels of one row and
 // `per_thread` taps (stage_weights_kernel in conv_tc_strip.cu says why).
-__global__ void __launch_bounds__(256) stage_filter16_kernel(ConvGeom g, View4 w, int is_dx, int tiles_pp, TapTable tt,
+// Stacked taps: rows 64 to 127 are those of the second tap of each stack.
+__global__ void __launch_bounds__(256) stage_filter16_kernel(ConvGeom g, View4 w, int is_dx, int tiles_pp, TapTable tt, Stacked stacked,
                                                              unsigned char* __restrict__ out, long long total, long long w_group_extra,
                                                              int rows_first, int per_thread) {
   wait_previous();
@@ -470,7 +507,8 @@ __global__ void __launch_bounds__(256) stage_filter16_kernel(ConvGeom g, View4 w
   const int piece = rows_first ? in_block >> 3 & 3 : in_block % 4, k = piece * 4;
   const int row = rows_first ? (in_block & 7) | in_block >> 5 << 3 : in_block / 4;
   const int tile_of_all = block / cpp, cbl = block - tile_of_all * cpp, grp = tile_of_all / tiles_pp, m_tile = tile_of_all - grp * tiles_pp;
-  const int r = m_tile * TM + row, c = cbl * KB + k;
+  const bool second = stacked.delta && row >= 64;
+  const int r = m_tile * TM + (second ? row - 64 : row), c = cbl * KB + k;
   const int valid = r < nc ? min(4, kc - c) : 0;
   const long long step = is_dx ? w.s0 : w.s1;
   const float* src = w.ptr + ((long long)grp * g.cog + (is_dx ? c : r)) * w.s0 + (long long)(is_dx ? r : c) * w.s1 + grp * w_group_extra;
@@ -482,10 +520,11 @@ __global__ void __launch_bounds__(256) stage_filter16_kernel(ConvGeom g, View4 w
     const int ntap = tt.start[phase + 1] - tt.start[phase], rel = tap - tt.start[phase];
     const long long image = is_dx ? (long long)(grp * tt.taps_total + tt.start[phase]) * tiles_pp * cpp + ((long long)m_tile * cpp + cbl) * ntap + rel
                                   : ((long long)tile_of_all * tt.taps_total + tt.start[phase]) * cpp + cbl * ntap + rel;
-    const float* p = src + tt.ky[tap] * w.s2 + tt.kx[tap] * w.s3;
+    const int kx = second ? stacked.kx[tap] : tt.kx[tap], here = kx == NO_TAP ? 0 : valid;
+    const float* p = src + tt.ky[tap] * w.s2 + kx * w.s3;
     float v[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) v[j] = j < valid ? __ldg(p + j * step) : 0.f;
+    for (int j = 0; j < 4; ++j) v[j] = j < here ? __ldg(p + j * step) : 0.f;
     float hi[4], lo[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) split_tf32(v[j], hi[j], lo[j]);
@@ -503,6 +542,7 @@ struct TPlan {
   int pn = 0, strip_rows = 0, a_stages = 0, w_stages = 0, smem = 0;
   int tiles_pp = 0, tiles_m = 0, tiles_p = 0, cpp = 0;
   long long images = 0;   // filter stage images in total
+  Stacked stacked;
   double clocks = 0.0;    // modelled duration
 };
 
@@ -512,11 +552,38 @@ static double mma_clocks(int pn) { return std::max(pn / 2.0, (4096.0 + 32.0 * pn
 
 // The pixel tile is the free parameter: wide tiles use the tensor pipe best, but the tile count should fill whole
 // waves of SMs.  Modelled time = waves x (MMAs of a tile x clocks(pn) + a fixed cost per tile).
+// Taps in stacks of two: neighbouring filter columns of one row and phase, the one that reads further on second.  False where the filter
+// does not gain by it (fewer than a quarter of the steps saved) or its taps lie too far apart.
+static bool stack_taps(TapTable& tt, bool is_dx, Stacked& s) {
+  TapTable out = tt;
+  out.taps_total = 0;
+  s.delta = 0;
+  for (int ph = 0; ph < tt.n_phase; ++ph) {
+    for (int t = tt.start[ph]; t < tt.start[ph + 1];) {
+      const bool two = t + 1 < tt.start[ph + 1] && tt.ky[t + 1] == tt.ky[t];
+      const int first = two && is_dx ? t + 1 : t, second = two ? (is_dx ? t : t + 1) : -1, i = out.taps_total++;
+      out.ky[i] = tt.ky[first]; out.kx[i] = tt.kx[first]; out.shift[i] = tt.shift[first];
+      s.kx[i] = two ? tt.kx[second] : NO_TAP;
+      if (two) {
+        const int d = tt.shift[second] - tt.shift[first];
+        if (d < 1 || d > 16 || (s.delta && d != s.delta)) return false;
+        s.delta = d;
+      }
+      t += two ? 2 : 1;
+    }
+    out.start[ph + 1] = (unsigned char)out.taps_total;
+  }
+  if (!s.delta || 4 * out.taps_total > 3 * tt.taps_total) return false;
+  tt = out;
+  return true;
+}
+
 static TPlan make_plan(const ConvGeom& g, bool is_dx) {
   TPlan p;
   p.geo = tcs::plan_strip_geometry(g, is_dx);
   if (!p.geo.ok) return p;
   const int kc = is_dx ? g.cog : g.cig, nc = is_dx ? g.cig : g.cog;
+  if (nc <= TM / 2 && ((is_dx && p.geo.tt.n_phase > 1) || !stack_taps(p.geo.tt, is_dx, p.stacked))) return p;
   const TapTable& tt = p.geo.tt;
   p.cpp = (kc + KB - 1) / KB;
   p.tiles_pp = (nc + TM - 1) / TM;
@@ -528,6 +595,8 @@ static TPlan make_plan(const ConvGeom& g, bool is_dx) {
   const int span = p.geo.shift_hi - p.geo.shift_lo;
   double best = 0.0;
   for (int pn = 256; pn >= 32; pn -= 16) {
+    const int step = pn - p.stacked.delta;
+    if (p.stacked.delta && (step + 31) / 32 * 32 + p.stacked.delta > 256) continue;   // what the epilogue reads of an accumulator
     const int rows = (pn + span + 7) / 8 * 8;
     const int a_stage = rows * ROWB * 2;
     int a_stages = 0, w_stages = 0;
@@ -536,13 +605,13 @@ static TPlan make_plan(const ConvGeom& g, bool is_dx) {
       if (left >= 2 * (int)W_RING_BYTES) { a_stages = as; w_stages = std::min(MAX_W_STAGES, left / (int)W_RING_BYTES); break; }
     }
     if (!a_stages) continue;
-    const long long tiles = div_up64(q_total, pn) * p.tiles_m * g.groups;
+    const long long tiles = div_up64(q_total, step) * p.tiles_m * g.groups;
     const double cost = (double)div_up64(tiles, sm_count()) * (stages_per_tile * (4.0 * mma_clocks(pn) + 120.0) + 3000.0);
     if (!p.ok || cost < best * 0.995) {   // ties go to the wider tile (fewer filter bytes per output)
       best = p.clocks = cost;
       p.ok = true;
       p.pn = pn; p.strip_rows = rows; p.a_stages = a_stages; p.w_stages = w_stages;
-      p.tiles_p = (int)div_up64(q_total, pn);
+      p.tiles_p = (int)div_up64(q_total, step);
       p.smem = a_stages * a_stage + w_stages * (int)W_RING_BYTES + TBUF_BYTES + 1024 + (int)sizeof(Ctrl) + 64;
     }
   }
@@ -572,6 +641,16 @@ bool tstrip_supported(const ConvGeom& g, int phase) {
   }
   return tst::plan_tstrip(g, is_dx).ok;
 }
+// 64 or fewer output channels: half of the filter rows would multiply padding, so two taps share a tile (rows 0-63 one, 64-127 its
+// neighbour); a step then costs what it does at 128 channels and there are two thirds as many for a 3-wide filter.
+// 64 -> 64 channels of 8x 56x56: forward 18.6 us in the strip kernel, 15.9 here, dInput 17.9 and 15.5; 40 random 3x3 layers with 64 channels or
+// fewer on a side, forward 0.86 and dInput 0.85 of the time (worst 1.03, a layer that keeps its kernel).  The line is where the models of both meet.
+bool tstrip_stacks(const ConvGeom& g, bool is_dx) {
+  const int nc = is_dx ? g.cig : g.cog;
+  if (nc > tst::TM / 2 || !tst::plan_tstrip(g, is_dx).ok) return false;
+  if (const char* v = getenv("B200_CONV_TC_VARIANT")) return !strcmp(v, "stacked");   // testing aid
+  return tstrip_time(g, is_dx, nullptr) < 0.9 * conv_slices_time(g, is_dx);
+}
 double tstrip_time(const ConvGeom& g, bool is_dx, long long* tiles) {
   const tst::TPlan& p = tst::plan_tstrip(g, is_dx);
   if (tiles) *tiles = (long long)p.tiles_p * p.tiles_m * g.groups;
@@ -595,7 +674,7 @@ int tstrip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* 
   const long long threads = plan.images / taps * TM * 4;
   const int per_thread = tcs::staged_taps(threads, taps);
   launch_next(stage_filter16_kernel, dim3((unsigned)div_up64(threads, 256), (unsigned)((taps + per_thread - 1) / per_thread)), 256, 0, st, 
-      g, w, is_dx ? 1 : 0, plan.tiles_pp, plan.geo.tt, (unsigned char*)ws, threads, w_group_extra,
+      g, w, is_dx ? 1 : 0, plan.tiles_pp, plan.geo.tt, plan.stacked, (unsigned char*)ws, threads, w_group_extra,
       std::llabs(is_dx ? w.s1 : w.s0) < std::llabs(is_dx ? w.s0 : w.s1) ? 1 : 0, per_thread);
   count_launch();
   if (int rc = launch_check("stage_filter16_kernel")) return rc;
@@ -616,7 +695,7 @@ int tstrip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* 
   a.images_per_tile = plan.cpp * plan.geo.tt.taps_total;
   a.tiles_m = plan.tiles_m; a.tiles_p = plan.tiles_p;
   a.tiles_total = plan.tiles_p * plan.tiles_m * g.groups;
-  a.pn = plan.pn;
+  a.pn = plan.pn; a.delta = plan.stacked.delta; a.step = plan.pn - plan.stacked.delta;
   a.q_total = (int)((long long)g.n * (a.H + a.pr) * (a.W + a.pc));
   a.img_div = FastDiv((uint32_t)((a.H + a.pr) * (a.W + a.pc)));
   a.row_div = FastDiv((uint32_t)(a.W + a.pc));
