@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_strip_kernel(const DwStrip
   const uint32_t stage_bytes = x_bytes + 2u * y_plane;
   Ctrl* ctrl = reinterpret_cast<Ctrl*>(smem_raw + (base - raw) + a.stages * stage_bytes);
   volatile int* abort_flag = &ctrl->abort_flag;
-  const int warp = warp_index(), lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int x_halves = a.xr > 32 ? 2 : 1;                      // a strip = rows 0..31 and 32..47; an exact block = 32 rows
   const int kx0 = (int)(blockIdx.x % (unsigned)a.kx_groups) * 4;  // first horizontal tap of this CTA
   // taps beyond the filter width of a narrow filter are not staged (their accumulator rows are never
@@ -658,12 +658,13 @@ bool dweight_strip_supported(const ConvGeom& g) {
 // The tensor-memory kernel gives a CTA of up to 64 output channels all vertical taps of an input block, where this one has a CTA for each
 // tap.  That pays while the splits fill the machine; where they cannot (little or no scratch, few pixels) its CTAs are a third as many and
 // do a third more per K block.  Per K block and for the rest of a CTA, measured: 0.74 us (six slots; 0.31 per strip of a strided input) and
-// 0.70 (1x1 filters) + 6 against 0.51 (0.60 in four blocks) + 4.  16 -> 62 channels of 7x 21x21, stride 2, no scratch: 45.6 and 25.3 us;
+// 6 against 0.51 (0.60 in four blocks) + 4.  (1x1 filters always gain by the tensor-memory kernel's idle warps: 432 -> 64 channels of 5x 7x7
+// 10.8 us here, 7.8 there.)  16 -> 62 channels of 7x 21x21, stride 2, no scratch: 45.6 and 25.3 us;
 // 38 -> 32 of 5x 46x46, no scratch: 265 and 181; 16 -> 64 of 61x61 x 14 with all the scratch it wants: 27.4 and 28.9.
 static bool strip_is_faster(const ConvGeom& g, const tcdt::PlanInfo& t, const tcdw::DwStripPlan& s) {
   if (!s.ok || g.cig * g.kh * g.kw < 32) return false;   // few products: short chains, which only the tensor-memory kernel has
-  if (g.cog > 64 || s.nacc != 1 || !(t.shift || g.kh * g.kw == 1)) return false;
-  const double tmem = 6.0 + t.kblocks * (t.shift ? std::max(0.74 * t.slots / 6, 0.31 * t.strips) : 0.70);
+  if (g.cog > 64 || s.nacc != 1 || !t.shift) return false;
+  const double tmem = 6.0 + t.kblocks * std::max(0.74 * t.slots / 6, 0.31 * t.strips);
   const double strip = 4.0 + (double)(s.span / tcdw::KP) * (s.xblocks == 1 ? 0.51 : 0.60);
   return strip < 0.85 * tmem;
 }

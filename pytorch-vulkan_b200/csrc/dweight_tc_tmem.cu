@@ -603,7 +603,9 @@ static Plan make_plan(const ConvGeom& real, size_t budget) {
   // pipeline.  Measured, that kernel against this one: 256 -> 512 channels of 32 x 14x14 38.7 and 28.4 us, 96 -> 131 of 42 x 7x7 31.9 and
   // 11.9, 32 -> 128 of 64 x 56x56 57 and 45; 512 -> 96 of 64 x 14x14 28.0 and 29.4, 512 -> 128 of 32 x 28x28 34 and 44, 64 -> 64 of
   // 64 x 56x56 42 and 53: the line is at five million input values, or one block of input channels.
-  if (!fold && g.kh * g.kw == 1 && g.cig > 32 && q_total * g.cig > (5ll << 20)) return best;
+  // Fewer than 64 input channels leave that kernel's rows half empty, with one value to a load in the ragged block: where wide outputs repeat it,
+  // this one is faster at any size (48 -> 256 of 33 x 92x92 233 and 125 us, 61 -> 400 of 20 x 88x88 211 and 138; 64 -> 192 of 27 x 77x77 69 and 73).
+  if (!fold && g.kh * g.kw == 1 && g.cig > 32 && !(g.cig < 64 && g.cog > 128) && q_total * g.cig > (5ll << 20)) return best;
   const int row_pitch = gw + pc;
   // shift mode: vertical taps m apart lie a whole number of grid rows apart
   int m = 1;
