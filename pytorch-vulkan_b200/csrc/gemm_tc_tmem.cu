@@ -27,7 +27,7 @@ constexpr int M_TILE = 128, KBLK = 32;
 constexpr int EPI_WARPS = 8, SETS = 2, W_WARP = EPI_WARPS + 4 * SETS, MMA_WARP = W_WARP + 1, THREADS = (MMA_WARP + 1) * 32;
 constexpr int DEPTH = 3;             // jobs of a producer warp on their way
 constexpr uint32_t SLOT = 4096;      // one of them: 32 lines of 128 bytes
-constexpr int A_STAGES = 4, MAX_W_STAGES = 4;
+constexpr int A_STAGES = 4, MAX_W_STAGES = 8;
 template <int BN> constexpr int W_RING = BN == 256 ? 2 : 4;
 
 struct Ctrl {
@@ -88,9 +88,14 @@ __device__ __forceinline__ void lds_f32x4(uint32_t addr, float& a, float& b, flo
   asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(a), "=f"(b), "=f"(c), "=f"(d) : "r"(addr) : "memory");
 }
 
-template <int BN>
+// PLANES: 1x1 convolutions of NCHW planes (a line of A is 32 pixels of a channel, a tile 128 pixels of an image) whose filter fits shared
+// memory: it is fetched once and stays.  Such a layer is bound by HBM, so what counts is the bytes on their way: 96 KB of asynchronous copies a
+// CTA against the 48 KB that the strip kernel's twelve producer warps hold in registers, and no filter traffic beside them.  64 images of 56x56:
+// 256 -> 64 channels 71 us in the strip kernel, 57 here (4.5 TB/s), 64 -> 256 61 and 51.
+template <int BN, bool PLANES>
 __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const GemmArgs a) {
-  constexpr int NACC = 256 / BN, W_STAGES = W_RING<BN>;
+  constexpr int NACC = 256 / BN;
+  const int W_STAGES = PLANES ? a.kblocks : W_RING<BN>;
   constexpr uint32_t W_BYTES = BN * 256u;
   extern __shared__ unsigned char smem_raw[];
   const uint32_t raw = smem_u32(smem_raw), w_base = (raw + 1023u) & ~1023u;
@@ -143,10 +148,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const GemmArgs a)
 #pragma unroll
           for (int k = 0; k < 4; ++k) umma_bf16_ts(d, ta + 32 + 8 * k, bc + 2 * k, id16, 1);
           umma_commit(smem_u32(&ctrl->a_empty[as]));
-          umma_commit(smem_u32(&ctrl->w_empty[ws]));
+          if (!PLANES) umma_commit(smem_u32(&ctrl->w_empty[ws]));
         }
         if (++as == A_STAGES) { as = 0; a_par ^= 1u; }
-        if (++ws == (uint32_t)W_STAGES) { ws = 0; w_par ^= 1u; }
+        if (++ws == (uint32_t)W_STAGES) { ws = 0; w_par ^= PLANES ? 0u : 1u; }
       }
       if (alive && leader) umma_commit(smem_u32(&ctrl->acc_full[ab]));
     }
@@ -155,9 +160,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const GemmArgs a)
       if (a.wait_for_images) asm volatile("griddepcontrol.wait;" ::: "memory");  // only this thread reads what the kernel ahead writes
       uint32_t ws = 0, par = 1, issued = 0;
       bool alive = true;
-      for (int i = 0; i < my_tiles && alive; ++i) {
+      for (int i = 0; i < (PLANES ? min(my_tiles, 1) : my_tiles) && alive; ++i) {
         const Tile t = tile_of(a, (int)blockIdx.x + i * (int)gridDim.x);
-        const unsigned char* img = reinterpret_cast<const unsigned char*>(a.images) + ((long long)t.group * a.tiles_n + t.n) * a.kblocks * (long long)W_BYTES;
+        const unsigned char* img = reinterpret_cast<const unsigned char*>(a.images) + ((long long)(PLANES ? 0 : t.group) * a.tiles_n + t.n) * a.kblocks * (long long)W_BYTES;
         for (int kb = 0; kb < a.kblocks; ++kb, img += W_BYTES) {
           if (!mbar_wait(smem_u32(&ctrl->w_empty[ws]), par, abort_flag, a.status, STATUS_TIMEOUT_EMPTY)) { alive = false; break; }
           mbar_expect_tx(smem_u32(&ctrl->w_full[ws]), W_BYTES);
@@ -174,7 +179,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const GemmArgs a)
   } else if (warp >= EPI_WARPS) {
     // ------------------------------ producers ------------------------------
     const int quarter = warp & 3, set = (warp - EPI_WARPS) >> 2;
-    const uint32_t lane_base = (uint32_t)(quarter * 32) << 16, slots = w_base + W_STAGES * W_BYTES + (uint32_t)(warp - EPI_WARPS) * (DEPTH * SLOT);
+    const uint32_t lane_base = (uint32_t)(quarter * 32) << 16, slots = w_base + (uint32_t)W_STAGES * W_BYTES + (uint32_t)(warp - EPI_WARPS) * (DEPTH * SLOT);
     const int total = my_tiles * a.kblocks;       // below 2^31 (checked by the host)
     struct Block { const float* src; int rows, valid; };        // rows of this warp inside the matrix, values of this K block
     auto locate = [&](int c) -> Block {
@@ -182,7 +187,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const GemmArgs a)
       const Tile t = tile_of(a, (int)blockIdx.x + it * (int)gridDim.x);
       const int row0 = t.m * M_TILE + quarter * 32, k0 = kb * KBLK;
       return Block{a.A + t.group * a.a_group + (long long)k0 * a.a_k + (long long)row0 * a.a_m, a.M - row0,
-                   min(KBLK, min(a.kc, a.k_total - t.group * a.kc) - k0)};
+                   min(KBLK, (PLANES ? a.kc : min(a.kc, a.k_total - t.group * a.kc)) - k0)};
     };
     // the 32 x 32 values of a job as 32 lines of 128 bytes, eight lanes to a line; what lies outside is zero
     auto issue = [&](int n) {
@@ -289,14 +294,21 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const GemmArgs a)
         }
         const int left = min(32, cols - c0);
         if (a.bias) {
-          const float b = lane < left ? a.beta * __ldg(a.bias + ((long long)t.group * a.N + n0 + c0 + lane) * a.bias_stride) : 0.f;
+          const float b = lane < left ? a.beta * __ldg(a.bias + ((PLANES ? 0 : (long long)t.group * a.N) + n0 + c0 + lane) * a.bias_stride) : 0.f;
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = fmaf(a.alpha, v[j], __shfl_sync(0xffffffffu, b, j));
         } else {
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] *= a.alpha;
         }
-        if (left == 32) {
+        if (PLANES) {                 // lane = pixel: 32 pixels of a channel to a store
+          float* p = a.C + t.group * a.c_group + (long long)(n0 + c0) * a.c_pitch + row;
+          if (row < a.M) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j, p += a.c_pitch)
+              if (j < left) *p = v[j];
+          }
+        } else if (left == 32) {
           transpose_pieces(v, lane);  // whole lines: piece i of row 4j + lane % 4
           float* p = a.C + t.group * a.c_group + (long long)(t.m * M_TILE + quarter * 32 + (lane & 3)) * a.c_pitch + n0 + c0 + (lane >> 2) * 4;
           if (a.vec_out) {
@@ -325,16 +337,16 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const GemmArgs a)
   }
 }
 
-template <int BN>
+template <int BN, bool PLANES>
 static int launch(const GemmArgs& a, cudaStream_t st) {
   static std::once_flag once;
   static cudaError_t opt_in = cudaSuccess;
-  std::call_once(once, [] { opt_in = cudaFuncSetAttribute(gemm_tmem_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448); });
+  std::call_once(once, [] { opt_in = cudaFuncSetAttribute(gemm_tmem_kernel<BN, PLANES>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448); });
   B200_CUDA(opt_in);
-  const size_t smem = (size_t)W_RING<BN> * BN * 256 + 4 * SETS * DEPTH * SLOT + 1024 + sizeof(Ctrl) + 64;
+  const size_t smem = (size_t)(PLANES ? a.kblocks : W_RING<BN>) * BN * 256 + 4 * SETS * DEPTH * SLOT + 1024 + sizeof(Ctrl) + 64;
   const dim3 grid((unsigned)std::min(a.tiles, sm_count()));
-  if (a.wait_for_images) launch_next(gemm_tmem_kernel<BN>, grid, THREADS, smem, st, a);
-  else gemm_tmem_kernel<BN><<<grid, THREADS, smem, st>>>(a);
+  if (a.wait_for_images) launch_next(gemm_tmem_kernel<BN, PLANES>, grid, THREADS, smem, st, a);
+  else gemm_tmem_kernel<BN, PLANES><<<grid, THREADS, smem, st>>>(a);
   count_launch();
   return launch_check("gemm_tmem_kernel");
 }
@@ -343,7 +355,8 @@ int run(GemmArgs a, int bn, cudaStream_t st) {
   a.status = device_status_word();
   if (!a.status) return fail(B200_ECUDA, "device status word is not allocated");
   a.div_m = FastDiv((uint32_t)a.tiles_m); a.div_n = FastDiv((uint32_t)a.tiles_n); a.div_kblocks = FastDiv((uint32_t)a.kblocks);
-  return bn == 256 ? launch<256>(a, st) : launch<128>(a, st);
+  if (a.planes) return bn == 256 ? launch<256, true>(a, st) : bn == 128 ? launch<128, true>(a, st) : launch<64, true>(a, st);
+  return bn == 256 ? launch<256, false>(a, st) : launch<128, false>(a, st);
 }
 
 }  // namespace gt

@@ -19,10 +19,12 @@ struct GemmArgs {
   int pieces16;              // the lines start at multiples of 16 bytes (always so along m)
   int vec_out;               // rows of C may be written 16 bytes at a time
   int wait_for_images;
+  int planes;                // 1x1 convolution on pixel planes: a group is an image, all share B and the bias, C[g][n][m] at g * c_group + n * c_pitch + m
   float alpha, beta;
   int* status;
   FastDiv div_m, div_n, div_kblocks;
 };
 int run(GemmArgs a, int bn, cudaStream_t st);
+constexpr int PLANES_B = 128 << 10;   // bytes of B's images that the planes form keeps in shared memory
 }  // namespace gt
 }  // namespace b200
