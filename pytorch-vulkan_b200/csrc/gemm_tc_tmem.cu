@@ -10,7 +10,7 @@
 // CTA roles (576 threads, persistent over tiles of 128 x BN): warps 0-7 epilogue, warps 8-15 producers (two sets of four; a warp
 // serves the 32 rows of its quarter of the tensor memory), warp 16 one thread streaming the images of B
 // that stage_weights_kernel wrote, warp 17 tensor-memory allocation and MMA issue.
-// Tensor memory: columns 0-255 the accumulators (one of 256 columns or two of 128), 256-511 four stages of A: 32 columns of
+// Tensor memory: columns 0-255 the accumulators (one of 256 columns, two of 128 or four of 64), 256-511 four stages of A: 32 columns of
 // TF32 values, 16 of BF16 pairs of the high parts, 16 of the low parts.
 #include <algorithm>
 #include <mutex>
@@ -27,11 +27,11 @@ constexpr int M_TILE = 128, KBLK = 32;
 constexpr int EPI_WARPS = 8, SETS = 2, W_WARP = EPI_WARPS + 4 * SETS, MMA_WARP = W_WARP + 1, THREADS = (MMA_WARP + 1) * 32;
 constexpr int DEPTH = 3;             // jobs of a producer warp on their way
 constexpr uint32_t SLOT = 4096;      // one of them: 32 lines of 128 bytes
-constexpr int A_STAGES = 4, MAX_W_STAGES = 8;
+constexpr int A_STAGES = 4, MAX_W_STAGES = 8, MAX_ACC = 4;
 template <int BN> constexpr int W_RING = BN == 256 ? 2 : 4;
 
 struct Ctrl {
-  unsigned long long a_full[A_STAGES], a_empty[A_STAGES], w_full[MAX_W_STAGES], w_empty[MAX_W_STAGES], acc_full[2], acc_empty[2];
+  unsigned long long a_full[A_STAGES], a_empty[A_STAGES], w_full[MAX_W_STAGES], w_empty[MAX_W_STAGES], acc_full[MAX_ACC], acc_empty[MAX_ACC];
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -95,6 +95,7 @@ __device__ __forceinline__ void lds_f32x4(uint32_t addr, float& a, float& b, flo
 template <int BN, bool PLANES>
 __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const GemmArgs a) {
   constexpr int NACC = 256 / BN;
+  static_assert(NACC <= MAX_ACC, "a barrier pair for every accumulator");
   const int W_STAGES = PLANES ? a.kblocks : W_RING<BN>;
   constexpr uint32_t W_BYTES = BN * 256u;
   extern __shared__ unsigned char smem_raw[];

@@ -12,6 +12,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("n,cin,cout,h,w", [
     (60, 256, 64, 24, 22), (75, 16, 16, 16, 33), (64, 40, 33, 26, 30), (64, 64, 256, 28, 28), (60, 128, 100, 22, 26), (60, 33, 200, 24, 24),
     (1, 64, 64, 195, 196),
+    (64, 32, 48, 84, 84),      # two dozen tiles to a CTA: every accumulator is used again and again
 ])
 @pytest.mark.parametrize("sliced", [False, True])
 def test_forward_and_dinput(n, cin, cout, h, w, sliced):
