@@ -219,7 +219,7 @@ int b200_conv2d_forward(const b200_conv_params* p, b200_view4 x, b200_view4 w, c
       return winograd_conv(g, false, to_view(x), to_view(w), bias, bias_stride, y, workspace, workspace_bytes, st);
     case B200_ALGO_TC:
       note_kernel("tc_igemm_forward");
-      return tc_forward(g, to_view(x), to_view(w), bias, bias_stride, y, workspace, workspace_bytes, st);
+      return tc_forward(g, to_view(x), to_view(w), bias, bias_stride, y, workspace, workspace_bytes, st, algo == B200_ALGO_AUTO);
     case B200_ALGO_TILED:
       if (group_small_supported(g)) {   // few channels per group: the tile follows the group (conv_group_small.cu)
         note_kernel("group_small_forward");
@@ -297,7 +297,7 @@ static int dinput_with_bias(const b200_conv_params* p, b200_view4 dy, b200_view4
         break;
       }
       note_kernel("tc_igemm_dinput");
-      rc = tc_dinput(g, to_view(dy), to_view(w), bias, bias_stride, dx, workspace, workspace_bytes, st, &bias_applied);
+      rc = tc_dinput(g, to_view(dy), to_view(w), bias, bias_stride, dx, workspace, workspace_bytes, st, &bias_applied, algo == B200_ALGO_AUTO);
       break;
     case B200_ALGO_TILED:
       if (group_small_supported(g)) {

@@ -731,14 +731,14 @@ int tc_route(const ConvGeom& g, bool is_dx, const View4& act) {
 }
 
 int tc_forward(const ConvGeom& g, View4 x, View4 w, const float* bias, long long bias_stride, float* y, void* ws,
-               size_t ws_bytes, cudaStream_t st) {
+               size_t ws_bytes, cudaStream_t st, bool automatic) {
   if (rows_supported(g)) {
     note_kernel("tc_rows_forward");
     const int rc = rows_conv(g, x, w, bias, bias_stride, y, st);
     if (rc != B200_EUNSUPPORTED) return rc;   // falls through to the CUDA-core kernel
   }
   int route = tc_route(g, false, x);
-  if (route == 0 && ws && (reinterpret_cast<uintptr_t>(ws) & 15) == 0 && tstrip_stacks(g, false) && tstrip_workspace(g, B200_PHASE_FORWARD) <= ws_bytes) {
+  if (automatic && route != 3 && ws && (reinterpret_cast<uintptr_t>(ws) & 15) == 0 && tstrip_stacks(g, false) && tstrip_workspace(g, B200_PHASE_FORWARD) <= ws_bytes) {
     note_kernel("tc_strip_forward");
     return tstrip_conv(g, false, x, w, bias, bias_stride, y, ws, ws_bytes, st);
   }
@@ -768,10 +768,10 @@ int tc_forward(const ConvGeom& g, View4 x, View4 w, const float* bias, long long
   return simt_igemm_forward(g, x, w, bias, bias_stride, y, st);
 }
 int tc_dinput(const ConvGeom& g, View4 dy, View4 w, const float* bias, long long bias_stride, float* dx, void* ws, size_t ws_bytes,
-              cudaStream_t st, bool* bias_applied) {
+              cudaStream_t st, bool* bias_applied, bool automatic) {
   if (bias_applied) *bias_applied = bias != nullptr;
   int route = tc_route(g, true, dy);
-  if (route == 0 && ws && (reinterpret_cast<uintptr_t>(ws) & 15) == 0 && tstrip_stacks(g, true) && tstrip_workspace(g, B200_PHASE_DINPUT) <= ws_bytes) {
+  if (automatic && route != 3 && ws && (reinterpret_cast<uintptr_t>(ws) & 15) == 0 && tstrip_stacks(g, true) && tstrip_workspace(g, B200_PHASE_DINPUT) <= ws_bytes) {
     note_kernel("tc_strip_dinput");
     return tstrip_conv(g, true, dy, w, bias, bias_stride, dx, ws, ws_bytes, st);
   }

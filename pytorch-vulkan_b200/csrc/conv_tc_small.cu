@@ -339,7 +339,7 @@ static int launch(const SmallArgs& a, const SmallPlan& p, cudaStream_t st) {
 // with slices of the reduction they stay below 16 us.
 bool conv_small_wanted(const ConvGeom& g, bool is_dx, bool allow_transposed) {
   const tsm::SmallPlan& p = tsm::plan_small(g, is_dx);
-  if (!p.ranks) return false;
+  if (!p.ranks || getenv("B200_CONV_TC_VARIANT")) return false;   // testing aid: a pinned kernel
   const bool transposed = allow_transposed && tstrip_supported(g, is_dx ? B200_PHASE_DINPUT : B200_PHASE_FORWARD);
   return p.time < 0.75 * std::min(16.0, transposed ? tstrip_time(g, is_dx, nullptr) : strip_time(g, is_dx, nullptr));
 }

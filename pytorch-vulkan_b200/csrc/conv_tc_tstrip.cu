@@ -644,7 +644,8 @@ bool tstrip_supported(const ConvGeom& g, int phase) {
 // 64 or fewer output channels: half of the filter rows would multiply padding, so two taps share a tile (rows 0-63 one, 64-127 its
 // neighbour); a step then costs what it does at 128 channels and there are two thirds as many for a 3-wide filter.
 // 64 -> 64 channels of 8x 56x56: forward 18.6 us in the strip kernel, 15.9 here, dInput 17.9 and 15.5; 40 random 3x3 layers with 64 channels or
-// fewer on a side, forward 0.86 and dInput 0.85 of the time (worst 1.03, a layer that keeps its kernel).  The line is where the models of both meet.
+// fewer on a side, forward 0.86 and dInput 0.85 of the time (worst 1.03, a layer that keeps its kernel).  The line is where the models of both meet.  Only the automatic choice
+// comes here: a forced candidate stays on the strip kernel, whose sums are those of the fused forward pass bit for bit.
 bool tstrip_stacks(const ConvGeom& g, bool is_dx) {
   const int nc = is_dx ? g.cig : g.cog;
   if (nc > tst::TM / 2 || !tst::plan_tstrip(g, is_dx).ok) return false;

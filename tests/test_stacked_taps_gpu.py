@@ -14,7 +14,7 @@ CASES = [  # (xshape, cout, kernel, conv arguments)
     ((1, 16, 5, 6), 16, (3, 3), dict(padding=(1, 1))),
     ((3, 40, 23, 17), 33, (3, 3), dict(padding=(2, 2), dilation=(2, 2))),
     ((2, 48, 9, 31), 50, (2, 2), dict(padding=(0, 1))),
-    ((1, 32, 19, 300), 32, (5, 5), dict(padding=(2, 2))),
+    ((1, 32, 19, 100), 32, (5, 5), dict(padding=(2, 2))),          # (four rows of 102 pixels beside a tile still fit shared memory)
     ((2, 33, 31, 30), 64, (3, 3), dict(stride=(2, 2), padding=(1, 1))),
     ((1, 32, 40, 41), 64, (1, 7), dict(padding=(0, 3))),
     ((2, 96, 14, 15), 96, (3, 3), dict(padding=(1, 1), groups=3)),
@@ -35,7 +35,7 @@ def test_forward_and_dinput(case, layout, monkeypatch):
     b = rng.standard_normal(cout, dtype=np.float32)
     y64, dx64 = oracle.torch_conv_all(x, w, b, go, kw.get("stride", (1, 1)), kw.get("padding", (0, 0)), kw.get("dilation", (1, 1)), kw.get("groups", 1))[:2]
     lay = (lambda a: np.ascontiguousarray(a.transpose(0, 2, 3, 1)).transpose(0, 3, 1, 2)) if layout == "nhwc" else (lambda a: a)
-    y = b200conv.conv2d_forward(lay(x), w, b, algo="tc", **kw)
-    assert b200conv.device_status() == 0 and oracle.rel_l2(y, y64) <= 1e-5
-    dx = b200conv.conv2d_backward(lay(go), lay(x), w, mask=(True, False, False), algo="tc", **kw)[0]
-    assert b200conv.device_status() == 0 and oracle.rel_l2(dx, dx64) <= 1e-5
+    y = b200conv.conv2d_forward(lay(x), w, b, **kw)
+    assert b200conv.last_kernel() == "tc_strip_forward" and b200conv.device_status() == 0 and oracle.rel_l2(y, y64) <= 1e-5
+    dx = b200conv.conv2d_backward(lay(go), lay(x), w, mask=(True, False, False), **kw)[0]
+    assert b200conv.last_kernel() == "tc_strip_dinput" and b200conv.device_status() == 0 and oracle.rel_l2(dx, dx64) <= 1e-5
