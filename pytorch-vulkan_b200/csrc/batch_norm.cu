@@ -650,6 +650,7 @@ __global__ void __launch_bounds__(kThreads) bn_bwd_apply_scalar_kernel(const flo
 // read once, and the latency of one load, one exchange and one store replaces that of three launches.
 constexpr int kUnits = 8, kUnits1 = 16;       // most units a thread holds: forward (16 bytes each), single values
 constexpr int kUnitsBwd = 4;                  // backward: of each of the two tensors
+constexpr int kUnitsParked = 5, kParkedX = 2; // backward of several waves: the gradient's units and so many of the input's in shared memory
 
 template <int VEC, int N>
 __global__ void __launch_bounds__(nres::THREADS, 4) bn_forward_channel_kernel(const float* __restrict__ x, nres::Rows rows, int inner, float m_count,
@@ -698,32 +699,47 @@ __global__ void __launch_bounds__(nres::THREADS, 4) bn_forward_channel_kernel(co
   }
 }
 
-template <int VEC, int N>
-__global__ void __launch_bounds__(nres::THREADS, 4) bn_backward_channel_kernel(const float* __restrict__ x, const float* __restrict__ g, nres::Rows rows,
-                                                                            int inner, float m_count, BnBackwardVectors v, float* __restrict__ dx) {
+// Bound by latency: a wave of CTAs loads, meets and stores in step, so fewer and fuller waves are faster.  With everything in registers (PARK false)
+// four CTAs fit an SM; with the gradient and two units of the input in shared memory a thread holds five units of each tensor instead of four and
+// six CTAs fit.  256 channels of 64x14x14: one wave of 768 CTAs instead of 1.7 waves of 1024, forward and backward 17.9 -> 17.0 us; 704 of 5100 values
+// 10.9 -> 8.3, 976 of 41472 118.6 -> 90.4.
+template <int VEC, int N, bool PARK>
+__global__ void __launch_bounds__(nres::THREADS, PARK ? 6 : 4) bn_backward_channel_kernel(const float* __restrict__ x, const float* __restrict__ g,
+                                                                                       nres::Rows rows, int inner, float m_count, BnBackwardVectors v,
+                                                                                       float* __restrict__ dx) {
   cluster_announce();
   wait_previous();
   auto cluster = nres::cg::this_cluster();
   const int ch = blockIdx.x, rank = (int)cluster.block_rank();
   const uint32_t end = min(rows.units, (uint32_t)(rank + 1) * rows.per), u0 = (uint32_t)rank * rows.per + threadIdx.x;
-  nres::Unit<VEC> xs[N], gs[N];
+  constexpr int XP = PARK ? kParkedX : 0, GP = PARK ? N : 0;
+  __shared__ __align__(16) nres::Parked<VEC, GP ? GP : 1> gs_parked;
+  __shared__ __align__(16) nres::Parked<VEC, XP ? XP : 1> xs_parked;
+  nres::Unit<VEC> xs[N], gs[GP ? 1 : N];
   uint32_t plane;
 #pragma unroll
   for (int k = 0; k < N; ++k) {
     const size_t at = (size_t)ch * inner + nres::unit_offset<VEC>(rows, min(u0 + k * nres::THREADS, rows.units - 1), plane);
-    xs[k].load(x + at, u0 + k * nres::THREADS < end);
-    gs[k].load(g + at, u0 + k * nres::THREADS < end);
+    const bool inside = u0 + k * nres::THREADS < end;
+    if (k < XP) xs_parked.load(k, x + at, inside);
+    else xs[k].load(x + at, inside);
+    if (GP) gs_parked.load(k, g + at, inside);
+    else gs[k % (GP ? 1 : N)].load(g + at, inside);
   }
+  auto x_unit = [&](int k) { return k < XP ? xs_parked.unit(k < XP ? k : 0) : xs[k]; };
+  auto g_unit = [&](int k) { return GP ? gs_parked.unit(GP ? k : 0) : gs[k % (GP ? 1 : N)]; };
   const float mean = v.mean[ch * v.mean_stride];
   float inv = v.inv[ch * v.inv_stride];
   if (!v.training) inv = 1.f / sqrtf(inv + v.eps);
   const float gamma = v.weight ? v.weight[ch * v.w_stride] : 1.f;
   Sums t = {0.f, 0.f, 0.f};
+  if (GP) gs_parked.arrive();
 #pragma unroll
   for (int k = 0; k < N; ++k)
     if (u0 + k * nres::THREADS < end) {
+      const nres::Unit<VEC> xu = x_unit(k), gu = g_unit(k);
 #pragma unroll
-      for (int j = 0; j < VEC; ++j) t.add(xs[k].v[j], gs[k].v[j], mean);
+      for (int j = 0; j < VEC; ++j) t.add(xu.v[j], gu.v[j], mean);
     }
   __shared__ nres::Table<3> table;
   float s[3] = {t.a, t.b, t.r};
@@ -747,14 +763,24 @@ __global__ void __launch_bounds__(nres::THREADS, 4) bn_backward_channel_kernel(c
   for (int k = 0; k < N; ++k) {
     const uint32_t u = u0 + k * nres::THREADS;
     if (u >= end) break;
+    const nres::Unit<VEC> xu = x_unit(k);
+    nres::Unit<VEC> gu = g_unit(k);
 #pragma unroll
-    for (int j = 0; j < VEC; ++j)
-      gs[k].v[j] = training ? input_grad<true>(xs[k].v[j], gs[k].v[j], k4, scale) : input_grad<false>(xs[k].v[j], gs[k].v[j], k4, scale);
-    gs[k].store(dx + (size_t)ch * inner + nres::unit_offset<VEC>(rows, u, plane));
+    for (int j = 0; j < VEC; ++j) gu.v[j] = training ? input_grad<true>(xu.v[j], gu.v[j], k4, scale) : input_grad<false>(xu.v[j], gu.v[j], k4, scale);
+    gu.store(dx + (size_t)ch * inner + nres::unit_offset<VEC>(rows, u, plane));
   }
 }
 
 // Ranks per channel for the kernels above, or 0: the streaming kernels take the call.
+// Where the parked form (bn_backward_channel_kernel) is the faster one: beyond one wave of the other, if fewer ranks hold a channel or everything runs
+// at once.  Measured, gain over the other form on 60 random layers: 1.00 to 1.38, median 1.08, within the line (but 8 -> 7 ranks .93, and .97 to 1.03
+// where the second wave is up to a fifth full); .89 to 1.06, median .95, where the ranks stay and a wave does not hold all.
+bool parks(const BnShape& sh, int ranks, int parked_ranks) {
+  const double waves = (double)sh.c * parked_ranks / (6.0 * sm_count());
+  if ((long long)sh.c * ranks <= 4ll * sm_count() || parked_ranks == 0) return false;
+  return waves <= 1.0 || (waves >= 1.2 && parked_ranks * 7 <= ranks * 6);
+}
+
 int channel_ranks(const BnShape& sh, int layout, int vec, int most, bool backward) {
   if (layout != B200_BN_PLANAR || sh.inner / vec >= (1 << 30) / sh.outer) return 0;
   const nres::RankPlan p = nres::plan_ranks((long long)sh.outer * (sh.inner / vec), sh.c, most, sm_count());
@@ -975,11 +1001,16 @@ int b200_batch_norm_backward(int64_t n, int64_t c, int64_t s, int layout, const 
   const int has_sums = training || dw || db;
   if (has_sums) {
     const int vec = sh.inner % 4 == 0 && aligned16(x) && aligned16(grad) && aligned16(dx) ? 4 : 1;
-    if (const int ranks = channel_ranks(sh, layout, vec, vec == 4 ? kUnitsBwd : kUnits1, true)) {
+    if (int ranks = channel_ranks(sh, layout, vec, vec == 4 ? kUnitsBwd : kUnits1, true)) {
       note_kernel("bn_backward_channel");
+      const int parked_ranks = channel_ranks(sh, layout, vec, kUnitsParked, true);
+      const bool park = vec == 4 && parks(sh, ranks, parked_ranks);
+      if (park) ranks = parked_ranks;
       const nres::Rows rows = nres::make_rows(sh.outer, sh.inner, vec, (long long)sh.c * sh.inner, ranks);
-      return nres::launch(vec == 4 ? bn_backward_channel_kernel<4, kUnitsBwd> : bn_backward_channel_kernel<1, kUnits1>, (unsigned)sh.c, ranks, st, x,
-                          grad, rows, sh.inner, sh.m, v, dx);
+      return nres::launch(vec == 1 ? bn_backward_channel_kernel<1, kUnits1, false>
+                          : park   ? bn_backward_channel_kernel<4, kUnitsParked, true>
+                                   : bn_backward_channel_kernel<4, kUnitsBwd, false>,
+                          (unsigned)sh.c, ranks, st, x, grad, rows, sh.inner, sh.m, v, dx);
     }
   }
   if (has_sums) {

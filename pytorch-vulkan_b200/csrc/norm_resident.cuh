@@ -41,6 +41,29 @@ struct Unit {
   }
 };
 
+// Units that wait in shared memory instead of registers, each thread's own: what a backward pass holds of its second tensor, so that six CTAs fit an
+// SM where registers for both tensors leave room for four.
+template <int VEC, int N>
+struct Parked {
+  float v[N][THREADS * VEC];
+  __device__ __forceinline__ void load(int k, const float* p, bool inside) {   // asynchronous: arrive() before the first read
+    const uint32_t to = (uint32_t)__cvta_generic_to_shared(&v[k][threadIdx.x * VEC]);
+    if (VEC == 4) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(p), "r"(inside ? 16 : 0) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to), "l"(p), "r"(inside ? 4 : 0) : "memory");
+  }
+  static __device__ __forceinline__ void arrive() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+  __device__ __forceinline__ Unit<VEC> unit(int k) const {
+    Unit<VEC> u;
+    if (VEC == 4) {
+      const float4 f = *reinterpret_cast<const float4*>(&v[k][threadIdx.x * VEC]);
+      u.v[0] = f.x; u.v[1 % VEC] = f.y; u.v[2 % VEC] = f.z; u.v[3 % VEC] = f.w;
+    } else {
+      u.v[0] = v[k][threadIdx.x];
+    }
+    return u;
+  }
+};
+
 template <int VEC>
 __device__ __forceinline__ long long unit_offset(const Rows& r, uint32_t u, uint32_t& plane) {
   plane = r.plane_div.div(u);
