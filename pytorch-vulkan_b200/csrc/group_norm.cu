@@ -362,6 +362,7 @@ __global__ void __launch_bounds__(kThreads, 3) gn_backward_kernel(const float* _
 // with the backward kernel above, 40.7 with this one.  32 samples of 1280 channels of 8x8: 24.8 and 27.2 us, now 12.2 and 18.7.
 constexpr int kUnits = 8, kUnits1 = 16;  // most units a thread holds: forward (16 bytes each), single values
 constexpr int kUnitsBwd = 4;             // backward: of each of the two tensors
+constexpr int kUnitsParked = 6;          // backward of wide rows: the gradient's units in shared memory
 constexpr int kResidentChannels = 64;    // most channels per group in the backward kernel
 
 template <int VEC, int N>
@@ -400,8 +401,9 @@ __global__ void __launch_bounds__(nres::THREADS, 4) gn_forward_cluster_kernel(co
 }
 
 // Each unit's two sums go through shared memory so that a warp can add those of one plane in order; a plane cut by a rank's
-// boundary is put together by rank 0.
-template <int VEC, int N>
+// boundary is put together by rank 0.  PARK: the gradient waits in shared memory and a thread holds six units of each tensor instead of four, so
+// that half as wide a cluster, or one at all where sixteen CTAs did not hold a row, takes it.
+template <int VEC, int N, bool PARK>
 __global__ void __launch_bounds__(nres::THREADS, 4) gn_backward_cluster_kernel(const float* __restrict__ dy, const float* __restrict__ x,
                                                                             const float* __restrict__ means, const float* __restrict__ rstds,
                                                                             const float* __restrict__ gamma, GnShape sh, nres::Rows rows,
@@ -417,22 +419,27 @@ __global__ void __launch_bounds__(nres::THREADS, 4) gn_backward_cluster_kernel(c
   const int ch0 = row % sh.groups * sh.cpg;
   const uint32_t begin = min(rows.units, (uint32_t)rank * rows.per), end = min(rows.units, (uint32_t)(rank + 1) * rows.per), u0 = begin + threadIdx.x;
   const size_t base = (size_t)row * sh.cpg * sh.hw;
-  nres::Unit<VEC> xs[N], gs[N];
+  __shared__ __align__(16) nres::Parked<VEC, PARK ? N : 1> parked;
+  nres::Unit<VEC> xs[N], gs[PARK ? 1 : N];
 #pragma unroll
   for (int k = 0; k < N; ++k) {
     const size_t at = base + (size_t)min(u0 + k * nres::THREADS, rows.units - 1) * VEC;
     xs[k].load(x + at, u0 + k * nres::THREADS < end);
-    gs[k].load(dy + at, u0 + k * nres::THREADS < end);
+    if (PARK) parked.load(k, dy + at, u0 + k * nres::THREADS < end);
+    else gs[k % (PARK ? 1 : N)].load(dy + at, u0 + k * nres::THREADS < end);
   }
+  auto g_unit = [&](int k) { return PARK ? parked.unit(PARK ? k : 0) : gs[k % (PARK ? 1 : N)]; };
   const float mean = __ldg(means + row), rstd = __ldg(rstds + row);
+  if (PARK) parked.arrive();
 #pragma unroll
   for (int k = 0; k < N; ++k) {
     float s1 = 0.f, s2 = 0.f;
+    const nres::Unit<VEC> gu = g_unit(k);
 #pragma unroll
     for (int j = 0; j < VEC; ++j) {
       xs[k].v[j] = (xs[k].v[j] - mean) * rstd;
-      s1 += gs[k].v[j];
-      s2 = fmaf(gs[k].v[j], xs[k].v[j], s2);
+      s1 += gu.v[j];
+      s2 = fmaf(gu.v[j], xs[k].v[j], s2);
     }
     unit_part[k * nres::THREADS + threadIdx.x] = make_float2(s1, s2);
   }
@@ -481,9 +488,10 @@ __global__ void __launch_bounds__(nres::THREADS, 4) gn_backward_cluster_kernel(c
     const uint32_t u = u0 + k * nres::THREADS;
     if (u >= end) break;
     const float w = gamma ? __ldg(gamma + ch0 + (int)rows.plane_div.div(u)) : 1.f;
+    nres::Unit<VEC> gu = g_unit(k);
 #pragma unroll
-    for (int j = 0; j < VEC; ++j) gs[k].v[j] = rstd * (gs[k].v[j] * w - avg - xs[k].v[j] * avg_z);
-    gs[k].store(dx + base + (size_t)u * VEC);
+    for (int j = 0; j < VEC; ++j) gu.v[j] = rstd * (gu.v[j] * w - avg - xs[k].v[j] * avg_z);
+    gu.store(dx + base + (size_t)u * VEC);
   }
 }
 
@@ -491,6 +499,26 @@ __global__ void __launch_bounds__(nres::THREADS, 4) gn_backward_cluster_kernel(c
 int block_ranks(const GnShape& sh, int blocks, int vec, int most, bool backward) {
   const nres::RankPlan p = nres::plan_ranks((long long)sh.cpg * sh.hw / vec, blocks, most, sm_count());
   return nres::group_norm_resident(p, vec, sh.hw, backward, blocks <= 3 * sm_count()) ? p.ranks : 0;
+}
+
+// The backward kernel's form.  Parked where four units of each tensor do not hold the row, need nine ranks or more and most of a wave, or take more
+// than one wave while six are one wave of two thirds as many ranks.  Measured on 150 random layers, the gain over what took them before: rows that
+// only the parked form holds 1.20 to 3.38, median 1.5, over the streaming kernel (32 rows of 74420 values 30.6 -> 9.1 us); rows of nine ranks or more
+// .98 to 1.27, median 1.06 (half a wave and less .90); two thirds as many ranks in one wave 1.15 to 1.29; elsewhere .87 to .98.
+struct BackwardPlan {
+  int ranks = 0;
+  bool park = false;
+};
+BackwardPlan backward_plan(const GnShape& sh, int blocks, int vec) {
+  BackwardPlan p;
+  if (sh.cpg > kResidentChannels) return p;
+  p.ranks = block_ranks(sh, blocks, vec, vec == 4 ? kUnitsBwd : kUnits1, true);
+  const int parked = vec == 4 ? block_ranks(sh, blocks, vec, kUnitsParked, true) : 0;
+  const long long slots = 4ll * sm_count();
+  p.park = parked && (p.ranks == 0 || (p.ranks >= 9 && 10ll * blocks * p.ranks > 7 * slots) ||
+                      ((long long)blocks * p.ranks > slots && (long long)blocks * parked <= slots && parked * 3 <= p.ranks * 2));
+  if (p.park) p.ranks = parked;
+  return p;
 }
 
 // dgamma[ch] = sum over samples of s2, dbeta[ch] = sum of s1 (the result of
@@ -599,11 +627,14 @@ int b200_group_norm_backward(int64_t n, int64_t c, int64_t hw, int64_t groups, c
   note_kernel(affine ? "gn_backward+affine" : "gn_backward");
   const bool aligned = ((reinterpret_cast<uintptr_t>(grad) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dx)) & 15) == 0;
   const int vec = sh.hw % 4 == 0 && aligned ? 4 : 1, blocks = (int)(n * groups);
-  const int ranks = sh.cpg <= kResidentChannels ? block_ranks(sh, blocks, vec, vec == 4 ? kUnitsBwd : kUnits1, true) : 0;
+  const BackwardPlan plan = backward_plan(sh, blocks, vec);
+  const int ranks = plan.ranks;
   if (ranks) {
     const nres::Rows rows = nres::make_rows(sh.cpg, sh.hw, vec, sh.hw, ranks);
-    if (int rc = nres::launch(vec == 4 ? gn_backward_cluster_kernel<4, kUnitsBwd> : gn_backward_cluster_kernel<1, kUnits1>, (unsigned)blocks, ranks, st, grad,
-                              x, mean, rstd, weight, sh, rows, dx, plane_sums))
+    if (int rc = nres::launch(vec == 1    ? gn_backward_cluster_kernel<1, kUnits1, false>
+                              : plan.park ? gn_backward_cluster_kernel<4, kUnitsParked, true>
+                                          : gn_backward_cluster_kernel<4, kUnitsBwd, false>,
+                              (unsigned)blocks, ranks, st, grad, x, mean, rstd, weight, sh, rows, dx, plane_sums))
       return rc;
   } else {
     launch_next(gn_backward_kernel, (unsigned)blocks, kThreads, (size_t)sh.units * 2 * sizeof(float), st, grad, x, mean, rstd, weight, sh, dx, plane_sums);

@@ -1,10 +1,11 @@
-"""Backward passes of batch norm that keep a tensor in shared memory beside the registers (one wave instead of several), at
-the lines of the rule that chooses them and with ragged last units, against the FP64 oracle."""
+"""Backward passes of the normalisations that keep a tensor in shared memory beside the registers (one wave instead of several, rows that four units a
+thread do not hold), at the lines of the rules that choose them and with ragged last units, against the FP64 oracles."""
 import numpy as np
 import pytest
 
 import b200conv
 from oracle import batch_norm_oracle as bn
+from oracle import group_norm_oracle as gn
 from oracle import oracle
 
 pytestmark = pytest.mark.gpu
@@ -25,3 +26,18 @@ def test_batch_norm(shape):
         second = inv if training else (1 / inv.astype(np.float64) ** 2 - 1e-5).astype(np.float32)
         for got, e in zip(b200conv.batch_norm_backward(g, x, w, mean, second, training, 1e-5), bn.backward(g, x, w, mean, second, training, 1e-5, dtype=np.float64)):
             assert oracle.rel_l2(got, e) <= 5 * GATE
+
+
+# (n, c, h, w), groups: nine ranks of four units, the widest row of four and of six units and the first beyond it, one wave with two thirds of the ranks
+GN = [((3, 9, 64, 64), 1), ((1, 64, 32, 32), 1), ((1, 65, 32, 32), 1), ((1, 24, 64, 64), 1), ((1, 48, 128, 64), 2), ((1, 49, 32, 64), 1), ((2, 14, 81, 84), 2),
+      ((20, 96, 22, 66), 32)]
+
+
+@pytest.mark.parametrize("shape,groups", GN, ids=lambda v: "x".join(map(str, v)) if isinstance(v, tuple) else f"g{v}")
+def test_group_norm(shape, groups):
+    rng = np.random.default_rng(sum(shape) + groups)
+    x, g = rng.standard_normal(shape, dtype=np.float32) + np.float32(3), rng.standard_normal(shape, dtype=np.float32)
+    w, b = rng.standard_normal(shape[1]).astype(np.float32), rng.standard_normal(shape[1]).astype(np.float32)
+    y, mean, rstd = b200conv.group_norm_forward(x, groups, w, b, 1e-5)
+    for got, e in zip(b200conv.group_norm_backward(g, x, mean, rstd, groups, w), gn.backward(g, x, mean, rstd, groups, w, dtype=np.float64)):
+        assert oracle.rel_l2(got, e) <= 5 * GATE
