@@ -672,7 +672,7 @@ __global__ void __launch_bounds__(nres::THREADS, 4) bn_forward_channel_kernel(co
 #pragma unroll
   for (int k = 0; k < N; ++k) in[k].load(base + nres::unit_offset<VEC>(rows, min(u0 + k * nres::THREADS, rows.units - 1), plane), u0 + k * nres::THREADS < end);
   __shared__ nres::Table<3> table;
-  const float2 m = nres::row_moments<VEC, N>(in, u0, end, origin, m_count, table, cluster);
+  const float2 m = nres::row_moments<VEC, N>([&](int k) { return in[k]; }, N, u0, end, origin, m_count, table, cluster);
   const float variance = m.y / m_count;
   const float inv = (variance == 0.f && v.eps == 0.f) ? 0.f : 1.f / sqrtf(variance + v.eps);
   if (rank == 0 && threadIdx.x == 0) {
@@ -713,8 +713,8 @@ __global__ void __launch_bounds__(nres::THREADS, PARK ? 6 : 4) bn_backward_chann
   const int ch = blockIdx.x, rank = (int)cluster.block_rank();
   const uint32_t end = min(rows.units, (uint32_t)(rank + 1) * rows.per), u0 = (uint32_t)rank * rows.per + threadIdx.x;
   constexpr int XP = PARK ? kParkedX : 0, GP = PARK ? N : 0;
-  __shared__ __align__(16) nres::Parked<VEC, GP ? GP : 1> gs_parked;
-  __shared__ __align__(16) nres::Parked<VEC, XP ? XP : 1> xs_parked;
+  __shared__ __align__(16) float parked[(GP + XP ? GP + XP : 1) * nres::THREADS * VEC];
+  const nres::Staged<VEC> gs_parked{parked}, xs_parked{parked + GP * nres::THREADS * VEC};
   nres::Unit<VEC> xs[N], gs[GP ? 1 : N];
   uint32_t plane;
 #pragma unroll
@@ -911,7 +911,7 @@ int b200_batch_norm_forward_fused(int64_t n, int64_t c, int64_t s, int layout, c
     if (const int ranks = channel_ranks(sh, layout, vec, vec == 4 ? kUnits : kUnits1, false)) {
       note_kernel(residual || relu ? "bn_forward_channel_fused" : "bn_forward_channel");
       const nres::Rows rows = nres::make_rows(sh.outer, sh.inner, vec, (long long)sh.c * sh.inner, ranks);
-      return nres::launch(vec == 4 ? bn_forward_channel_kernel<4, kUnits> : bn_forward_channel_kernel<1, kUnits1>, (unsigned)sh.c, ranks, st, x, rows,
+      return nres::launch(vec == 4 ? bn_forward_channel_kernel<4, kUnits> : bn_forward_channel_kernel<1, kUnits1>, (unsigned)sh.c, ranks, 0, st, x, rows,
                           sh.inner, sh.m, v, BnPost{residual, relu ? 1 : 0}, y);
     }
   }
@@ -1010,7 +1010,7 @@ int b200_batch_norm_backward(int64_t n, int64_t c, int64_t s, int layout, const 
       return nres::launch(vec == 1 ? bn_backward_channel_kernel<1, kUnits1, false>
                           : park   ? bn_backward_channel_kernel<4, kUnitsParked, true>
                                    : bn_backward_channel_kernel<4, kUnitsBwd, false>,
-                          (unsigned)sh.c, ranks, st, x, grad, rows, sh.inner, sh.m, v, dx);
+                          (unsigned)sh.c, ranks, 0, st, x, grad, rows, sh.inner, sh.m, v, dx);
     }
   }
   if (has_sums) {

@@ -363,6 +363,7 @@ __global__ void __launch_bounds__(kThreads, 3) gn_backward_kernel(const float* _
 constexpr int kUnits = 8, kUnits1 = 16;  // most units a thread holds: forward (16 bytes each), single values
 constexpr int kUnitsBwd = 4;             // backward: of each of the two tensors
 constexpr int kUnitsParked = 6;          // backward of wide rows: the gradient's units in shared memory
+constexpr int kStagedForward = 54 * 1024, kStagedBackward = 46 * 1024;  // rows in shared memory: bytes of a CTA of which four fit an SM
 constexpr int kResidentChannels = 64;    // most channels per group in the backward kernel
 
 template <int VEC, int N>
@@ -382,7 +383,7 @@ __global__ void __launch_bounds__(nres::THREADS, 4) gn_forward_cluster_kernel(co
 #pragma unroll
   for (int k = 0; k < N; ++k) in[k].load(x + base + (size_t)min(u0 + k * nres::THREADS, rows.units - 1) * VEC, u0 + k * nres::THREADS < end);
   __shared__ nres::Table<3> table;
-  const float2 total = nres::row_moments<VEC, N>(in, u0, end, origin, sh.count, table, cluster);
+  const float2 total = nres::row_moments<VEC, N>([&](int k) { return in[k]; }, N, u0, end, origin, sh.count, table, cluster);
   const float mean_rel = total.x, rstd = 1.f / sqrtf(total.y / sh.count + eps);
   if (rank == 0 && threadIdx.x == 0) {
     means[row] = origin + mean_rel;
@@ -419,7 +420,8 @@ __global__ void __launch_bounds__(nres::THREADS, 4) gn_backward_cluster_kernel(c
   const int ch0 = row % sh.groups * sh.cpg;
   const uint32_t begin = min(rows.units, (uint32_t)rank * rows.per), end = min(rows.units, (uint32_t)(rank + 1) * rows.per), u0 = begin + threadIdx.x;
   const size_t base = (size_t)row * sh.cpg * sh.hw;
-  __shared__ __align__(16) nres::Parked<VEC, PARK ? N : 1> parked;
+  __shared__ __align__(16) float gs_parked[(PARK ? N : 1) * nres::THREADS * VEC];
+  const nres::Staged<VEC> parked{gs_parked};
   nres::Unit<VEC> xs[N], gs[PARK ? 1 : N];
 #pragma unroll
   for (int k = 0; k < N; ++k) {
@@ -495,19 +497,167 @@ __global__ void __launch_bounds__(nres::THREADS, 4) gn_backward_cluster_kernel(c
   }
 }
 
+// Rows beyond the registers of sixteen CTAs: the CTAs' shares are fetched into shared memory asynchronously and each tensor is read once.  The kernels
+// with a CTA for a row read it again for each pass and leave the chip to as many CTAs as there are rows; the rule and what it measured stand at
+// forward_staged() and backward_plan().  Bound by latency with few rows, by memory beyond two waves.  `n`: units of a thread.
+template <int VEC>
+__global__ void __launch_bounds__(nres::THREADS, 4) gn_forward_staged_kernel(const float* __restrict__ x, const float* __restrict__ gamma,
+                                                                          const float* __restrict__ beta, GnShape sh, nres::Rows rows, int n, float eps,
+                                                                          float* __restrict__ y, float* __restrict__ means, float* __restrict__ rstds) {
+  cluster_announce();
+  wait_previous();
+  auto cluster = nres::cg::this_cluster();
+  extern __shared__ __align__(16) float staged[];
+  __shared__ nres::Table<3> table;
+  const nres::Staged<VEC> in{staged};
+  const int row = blockIdx.x, rank = (int)cluster.block_rank();
+  const int ch0 = row % sh.groups * sh.cpg;
+  const uint32_t end = min(rows.units, (uint32_t)(rank + 1) * rows.per), u0 = (uint32_t)rank * rows.per + threadIdx.x;
+  const size_t base = (size_t)row * sh.cpg * sh.hw;
+  const float origin = __ldg(x + base);
+#pragma unroll 8
+  for (int k = 0; k < n; ++k) in.load(k, x + base + (size_t)min(u0 + k * nres::THREADS, rows.units - 1) * VEC, u0 + k * nres::THREADS < end);
+  in.arrive();
+  const float2 total = nres::row_moments<VEC, 8>([&](int k) { return in.unit(k); }, n, u0, end, origin, sh.count, table, cluster);
+  const float mean_rel = total.x, rstd = 1.f / sqrtf(total.y / sh.count + eps);
+  if (rank == 0 && threadIdx.x == 0) {
+    means[row] = origin + mean_rel;
+    rstds[row] = rstd;
+  }
+#pragma unroll 4
+  for (int k = 0; k < n; ++k) {
+    const uint32_t u = u0 + k * nres::THREADS;
+    if (u >= end) break;
+    const int ch = ch0 + (int)rows.plane_div.div(u);
+    const float scale = rstd * (gamma ? __ldg(gamma + ch) : 1.f), shift = beta ? __ldg(beta + ch) : 0.f;
+    nres::Unit<VEC> v = in.unit(k);
+#pragma unroll
+    for (int j = 0; j < VEC; ++j) v.v[j] = ((v.v[j] - origin) - mean_rel) * scale + shift;
+    v.store(y + base + (size_t)u * VEC);
+  }
+}
+
+// As gn_backward_cluster_kernel; with both tensors in shared memory a warp adds a plane's units themselves, and where a rank has fewer planes than
+// warps each plane is cut into parts.
+template <int VEC>
+__global__ void __launch_bounds__(nres::THREADS, 4) gn_backward_staged_kernel(const float* __restrict__ dy, const float* __restrict__ x,
+                                                                           const float* __restrict__ means, const float* __restrict__ rstds,
+                                                                           const float* __restrict__ gamma, GnShape sh, nres::Rows rows, int n,
+                                                                           float* __restrict__ dx, float* __restrict__ plane_sums) {
+  cluster_announce();
+  wait_previous();
+  auto cluster = nres::cg::this_cluster();
+  extern __shared__ __align__(16) float staged[];
+  __shared__ float2 part[kResidentChannels];                           // of this rank: planes, or parts of them
+  __shared__ float2 all_part[nres::MAX_RANKS][kResidentChannels];      // rank 0: planes of every rank
+  __shared__ float2 rank_part[nres::MAX_RANKS];
+  const nres::Staged<VEC> xs{staged}, gs{staged + n * nres::THREADS * VEC};
+  const int row = blockIdx.x, ranks = (int)cluster.num_blocks(), rank = (int)cluster.block_rank(), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int ch0 = row % sh.groups * sh.cpg;
+  const uint32_t begin = min(rows.units, (uint32_t)rank * rows.per), end = min(rows.units, (uint32_t)(rank + 1) * rows.per), u0 = begin + threadIdx.x;
+  const size_t base = (size_t)row * sh.cpg * sh.hw;
+#pragma unroll 4
+  for (int k = 0; k < n; ++k) {
+    const size_t at = base + (size_t)min(u0 + k * nres::THREADS, rows.units - 1) * VEC;
+    xs.load(k, x + at, u0 + k * nres::THREADS < end);
+    gs.load(k, dy + at, u0 + k * nres::THREADS < end);
+  }
+  const float mean = __ldg(means + row), rstd = __ldg(rstds + row);
+  xs.arrive();
+  __syncthreads();
+  cluster_wait_started();
+  const int p0 = (int)rows.plane_div.div(begin), planes = begin < end ? (int)rows.plane_div.div(end - 1) + 1 - p0 : 0;
+  const int cut = planes && planes < nres::WARPS ? nres::WARPS / planes : 1;
+  for (int i = warp; i < planes * cut; i += nres::WARPS) {
+    const uint32_t p = (uint32_t)(p0 + i / cut), a = max(begin, p * rows.plane_units) - begin, b = min(end, (p + 1) * rows.plane_units) - begin;
+    const uint32_t share = (b - a + cut - 1) / cut, first = a + (uint32_t)(i % cut) * share, last = min(b, first + share);
+    float s1[4] = {0.f, 0.f, 0.f, 0.f}, s2[4] = {0.f, 0.f, 0.f, 0.f};
+    auto add = [&](uint32_t u, int slot) {
+      const nres::Unit<VEC> xu = xs.at(u), gu = gs.at(u);
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) {
+        s1[(slot + j) & 3] += gu.v[j];
+        s2[(slot + j) & 3] = fmaf(gu.v[j], (xu.v[j] - mean) * rstd, s2[(slot + j) & 3]);
+      }
+    };
+    uint32_t u = first + lane;
+    for (; u + 96 < last; u += 128) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) add(u + 32 * q, q);
+    }
+    for (; u < last; u += 32) add(u, 0);
+    const float t1 = warp_sum((s1[0] + s1[1]) + (s1[2] + s1[3])), t2 = warp_sum((s2[0] + s2[1]) + (s2[2] + s2[3]));
+    if (lane == 0) part[i] = make_float2(t1, t2);
+  }
+  __syncthreads();
+  if (warp == 0) {
+    float a = 0.f, b = 0.f;
+    for (int i = lane; i < planes; i += 32) {
+      float s1 = 0.f, s2 = 0.f;
+      for (int q = 0; q < cut; ++q) s1 += part[i * cut + q].x, s2 += part[i * cut + q].y;
+      if (plane_sums) *cluster.map_shared_rank(&all_part[rank][p0 + i], 0) = make_float2(s1, s2);
+      const float w = gamma ? __ldg(gamma + ch0 + p0 + i) : 1.f;
+      a = fmaf(w, s1, a);
+      b = fmaf(w, s2, b);
+    }
+    a = warp_sum(a);
+    b = warp_sum(b);
+    if (lane < ranks) *cluster.map_shared_rank(&rank_part[rank], lane) = make_float2(a, b);
+  }
+  cluster.sync();
+  asm volatile("griddepcontrol.launch_dependents;");
+  if (plane_sums && rank == 0)
+    for (int p = threadIdx.x; p < sh.cpg; p += nres::THREADS) {
+      const int r0 = (int)((uint32_t)p * rows.plane_units / rows.per), r1 = (int)(((uint32_t)(p + 1) * rows.plane_units - 1) / rows.per);
+      float s1 = 0.f, s2 = 0.f;
+      for (int r = r0; r <= r1; ++r) s1 += all_part[r][p].x, s2 += all_part[r][p].y;
+      reinterpret_cast<float2*>(plane_sums)[(size_t)(row / sh.groups) * sh.c + ch0 + p] = make_float2(s1, s2);
+    }
+  if (!dx) return;
+  float avg = 0.f, avg_z = 0.f;
+  for (int r = 0; r < ranks; ++r) avg += rank_part[r].x, avg_z += rank_part[r].y;
+  avg /= sh.count;
+  avg_z /= sh.count;
+#pragma unroll 4
+  for (int k = 0; k < n; ++k) {
+    const uint32_t u = u0 + k * nres::THREADS;
+    if (u >= end) break;
+    const float w = gamma ? __ldg(gamma + ch0 + (int)rows.plane_div.div(u)) : 1.f;
+    const nres::Unit<VEC> xu = xs.unit(k);
+    nres::Unit<VEC> gu = gs.unit(k);
+#pragma unroll
+    for (int j = 0; j < VEC; ++j) gu.v[j] = rstd * (gu.v[j] * w - avg - (xu.v[j] - mean) * rstd * avg_z);
+    gu.store(dx + base + (size_t)u * VEC);
+  }
+}
+
 // Ranks per block for the kernels above, or 0: the streaming kernels take the call.
 int block_ranks(const GnShape& sh, int blocks, int vec, int most, bool backward) {
   const nres::RankPlan p = nres::plan_ranks((long long)sh.cpg * sh.hw / vec, blocks, most, sm_count());
   return nres::group_norm_resident(p, vec, sh.hw, backward, blocks <= 3 * sm_count()) ? p.ranks : 0;
 }
 
+// Forward rows that no cluster's registers hold: up to 409600 values.  Measured on random layers against the kernel with a CTA for a row: pieces of 16
+// bytes 1.6 to 3.1 times as fast (32 rows of 154652 values 38.1 -> 12.1 us, 96 of 332928 129 -> 76), single values 1.2 to 3.0 (416 rows of
+// 103968 157 -> 131, 64 of 274428 211 -> 71).  Rows of single values that fit but stream (norm_plan.cuh) gain nothing: .80 to 1.07.
+nres::StagedPlan forward_staged(const GnShape& sh, int vec) {
+  const long long units = (long long)sh.cpg * sh.hw / vec;
+  if (nres::plan_ranks(units, 1, vec == 4 ? kUnits : kUnits1, sm_count()).ranks) return {};
+  return nres::plan_staged(units, 4 * vec, kStagedForward);
+}
+
 // The backward kernel's form.  Parked where four units of each tensor do not hold the row, need nine ranks or more and most of a wave, or take more
 // than one wave while six are one wave of two thirds as many ranks.  Measured on 150 random layers, the gain over what took them before: rows that
 // only the parked form holds 1.20 to 3.38, median 1.5, over the streaming kernel (32 rows of 74420 values 30.6 -> 9.1 us); rows of nine ranks or more
 // .98 to 1.27, median 1.06 (half a wave and less .90); two thirds as many ranks in one wave 1.15 to 1.29; elsewhere .87 to .98.
+// Rows beyond both, up to 204800 values, wait in shared memory altogether: 1.1 to 2.6 times as fast as the kernel with a CTA for a row (32 rows of
+// 154652 values 67.4 -> 25.9 us; single values 64 of 136367 123 -> 56, 416 of 103968 212 -> 195).  Where six units hold a row they are the faster form: 32
+// rows of 82944 values 9.3 against 12.5.  With two CTAs to an SM and many rows the other kernel is level: 288 rows of 148104 values 158 -> 165, 96 of
+// 184960 107 -> 62.
 struct BackwardPlan {
   int ranks = 0;
   bool park = false;
+  nres::StagedPlan staged;
 };
 BackwardPlan backward_plan(const GnShape& sh, int blocks, int vec) {
   BackwardPlan p;
@@ -518,6 +668,8 @@ BackwardPlan backward_plan(const GnShape& sh, int blocks, int vec) {
   p.park = parked && (p.ranks == 0 || (p.ranks >= 9 && 10ll * blocks * p.ranks > 7 * slots) ||
                       ((long long)blocks * p.ranks > slots && (long long)blocks * parked <= slots && parked * 3 <= p.ranks * 2));
   if (p.park) p.ranks = parked;
+  if (p.ranks == 0) p.staged = nres::plan_staged((long long)sh.cpg * sh.hw / vec, 8 * vec, kStagedBackward);
+  if (vec == 4 && p.staged.units > 8 && blocks > 256) p.staged = {};
   return p;
 }
 
@@ -604,8 +756,12 @@ int b200_group_norm_forward(int64_t n, int64_t c, int64_t hw, int64_t groups, co
   note_kernel("gn_forward");
   const int vec = sh.hw % 4 == 0 && aligned ? 4 : 1;
   if (const int ranks = block_ranks(sh, blocks, vec, vec == 4 ? kUnits : kUnits1, false))
-    return nres::launch(vec == 4 ? gn_forward_cluster_kernel<4, kUnits> : gn_forward_cluster_kernel<1, kUnits1>, (unsigned)blocks, ranks, st, x, weight, bias,
-                        sh, nres::make_rows(sh.cpg, sh.hw, vec, sh.hw, ranks), eps, y, mean, rstd);
+    return nres::launch(vec == 4 ? gn_forward_cluster_kernel<4, kUnits> : gn_forward_cluster_kernel<1, kUnits1>, (unsigned)blocks, ranks, 0, st, x, weight,
+                        bias, sh, nres::make_rows(sh.cpg, sh.hw, vec, sh.hw, ranks), eps, y, mean, rstd);
+  if (const nres::StagedPlan staged = forward_staged(sh, vec); staged.ranks)
+    return nres::launch(vec == 4 ? gn_forward_staged_kernel<4> : gn_forward_staged_kernel<1>, (unsigned)blocks, staged.ranks,
+                        (size_t)staged.units * nres::THREADS * 4 * vec, st, x, weight, bias, sh, nres::make_rows(sh.cpg, sh.hw, vec, sh.hw, staged.ranks),
+                        staged.units, eps, y, mean, rstd);
   launch_next(gn_forward_kernel, (unsigned)(n * groups), kThreads, 0, st, x, weight, bias, sh, eps, y, mean, rstd);
   count_launch();
   return launch_check("gn_forward_kernel");
@@ -634,7 +790,13 @@ int b200_group_norm_backward(int64_t n, int64_t c, int64_t hw, int64_t groups, c
     if (int rc = nres::launch(vec == 1    ? gn_backward_cluster_kernel<1, kUnits1, false>
                               : plan.park ? gn_backward_cluster_kernel<4, kUnitsParked, true>
                                           : gn_backward_cluster_kernel<4, kUnitsBwd, false>,
-                              (unsigned)blocks, ranks, st, grad, x, mean, rstd, weight, sh, rows, dx, plane_sums))
+                              (unsigned)blocks, ranks, 0, st, grad, x, mean, rstd, weight, sh, rows, dx, plane_sums))
+      return rc;
+  } else if (plan.staged.ranks) {
+    const nres::Rows rows = nres::make_rows(sh.cpg, sh.hw, vec, sh.hw, plan.staged.ranks);
+    if (int rc = nres::launch(vec == 4 ? gn_backward_staged_kernel<4> : gn_backward_staged_kernel<1>, (unsigned)blocks, plan.staged.ranks,
+                              (size_t)plan.staged.units * nres::THREADS * 8 * vec, st, grad, x, mean, rstd, weight, sh, rows, plan.staged.units, dx,
+                              plane_sums))
       return rc;
   } else {
     launch_next(gn_backward_kernel, (unsigned)blocks, kThreads, (size_t)sh.units * 2 * sizeof(float), st, grad, x, mean, rstd, weight, sh, dx, plane_sums);

@@ -51,6 +51,23 @@ inline RankPlan plan_ranks(long long units, long long rows, int most, int sms) {
   return p;
 }
 
+// Rows whose units wait in the shared memory of a cluster's CTAs, `unit_bytes` for each: as few ranks as hold the row with four CTAs to an SM
+// (`quarter` bytes each), or sixteen with up to two to an SM.
+constexpr int PLAN_STAGED_BYTES = 100 * 1024;
+struct StagedPlan {
+  int ranks = 0;        // 0: the row does not fit
+  int units = 0;        // of a thread
+};
+inline StagedPlan plan_staged(long long units, int unit_bytes, int quarter) {
+  StagedPlan p;
+  const long long holds = (long long)PLAN_THREADS * (quarter / (PLAN_THREADS * unit_bytes)), need = (units + holds - 1) / holds;
+  const long long ranks = need < PLAN_MAX_RANKS ? need : PLAN_MAX_RANKS, per = (units + ranks - 1) / ranks, mine = (per + PLAN_THREADS - 1) / PLAN_THREADS;
+  if (mine * PLAN_THREADS * unit_bytes > PLAN_STAGED_BYTES) return p;
+  p.ranks = (int)ranks;
+  p.units = (int)mine;
+  return p;
+}
+
 // The line through the table above, for rows beyond one wave; `plane`: values of a plane, `vec`: values of a unit.
 inline bool batch_norm_resident(const RankPlan& p, int vec, long long plane, bool backward) {
   if (p.ranks == 0) return false;

@@ -41,27 +41,27 @@ struct Unit {
   }
 };
 
-// Units that wait in shared memory instead of registers, each thread's own: what a backward pass holds of its second tensor, so that six CTAs fit an
-// SM where registers for both tensors leave room for four.
-template <int VEC, int N>
-struct Parked {
-  float v[N][THREADS * VEC];
-  __device__ __forceinline__ void load(int k, const float* p, bool inside) {   // asynchronous: arrive() before the first read
-    const uint32_t to = (uint32_t)__cvta_generic_to_shared(&v[k][threadIdx.x * VEC]);
+// Units that wait in shared memory instead of registers, each thread's own: unit k of a thread is unit k * THREADS + its index of the CTA.
+template <int VEC>
+struct Staged {
+  float* v;
+  __device__ __forceinline__ void load(int k, const float* p, bool inside) const {   // asynchronous: arrive() before the first read
+    const uint32_t to = (uint32_t)__cvta_generic_to_shared(v + (k * THREADS + threadIdx.x) * VEC);
     if (VEC == 4) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(p), "r"(inside ? 16 : 0) : "memory");
     else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to), "l"(p), "r"(inside ? 4 : 0) : "memory");
   }
   static __device__ __forceinline__ void arrive() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-  __device__ __forceinline__ Unit<VEC> unit(int k) const {
+  __device__ __forceinline__ Unit<VEC> at(uint32_t i) const {        // unit i of the CTA
     Unit<VEC> u;
     if (VEC == 4) {
-      const float4 f = *reinterpret_cast<const float4*>(&v[k][threadIdx.x * VEC]);
+      const float4 f = *reinterpret_cast<const float4*>(v + i * VEC);
       u.v[0] = f.x; u.v[1 % VEC] = f.y; u.v[2 % VEC] = f.z; u.v[3 % VEC] = f.w;
     } else {
-      u.v[0] = v[k][threadIdx.x];
+      u.v[0] = v[i];
     }
     return u;
   }
+  __device__ __forceinline__ Unit<VEC> unit(int k) const { return at(k * THREADS + threadIdx.x); }
 };
 
 template <int VEC>
@@ -106,29 +106,32 @@ __device__ __forceinline__ void cluster_sum(float (&v)[C], Table<C>& table, cg::
 // values and then their deviations from it (they are in registers); count, mean and deviations of all warps are merged after ONE exchange, so
 // that neither a common offset nor an outlier costs precision.  With the mean exchanged first and the deviations after it, 64x256x14x14
 // took 7.65 us (batch norm forward) and 16x512x32x32 in 32 groups 16.7 (group norm forward); now 7.24 and 15.3.
-template <int VEC, int N>
-__device__ __forceinline__ float2 row_moments(const Unit<VEC> (&in)[N], uint32_t u0, uint32_t end, float origin, float count, Table<3>& table,
+template <int VEC, int UNROLL, typename F>     // unit(k) for k < n: the thread's units
+__device__ __forceinline__ float2 row_moments(const F& unit, int n, uint32_t u0, uint32_t end, float origin, float count, Table<3>& table,
                                               cg::cluster_group& cluster) {
   const int ranks = (int)cluster.num_blocks(), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float s[4] = {0.f, 0.f, 0.f, 0.f};
   uint32_t mine = 0;
-#pragma unroll
-  for (int k = 0; k < N; ++k) {
+#pragma unroll UNROLL
+  for (int k = 0; k < n; ++k) {
     const bool inside = u0 + k * THREADS < end;
     mine += inside ? VEC : 0;
+    const Unit<VEC> in = unit(k);
 #pragma unroll
-    for (int j = 0; j < VEC; ++j) s[(k * VEC + j) & 3] += inside ? in[k].v[j] - origin : 0.f;
+    for (int j = 0; j < VEC; ++j) s[(k * VEC + j) & 3] += inside ? in.v[j] - origin : 0.f;
   }
   const float held = (float)__reduce_add_sync(0xffffffffu, mine);     // values of this warp
   const float own = held > 0.f ? warp_total((s[0] + s[1]) + (s[2] + s[3])) / held : 0.f;
   s[0] = s[1] = s[2] = s[3] = 0.f;
-#pragma unroll
-  for (int k = 0; k < N; ++k)
+#pragma unroll UNROLL
+  for (int k = 0; k < n; ++k) {
+    const Unit<VEC> in = unit(k);
 #pragma unroll
     for (int j = 0; j < VEC; ++j) {
-      const float d = u0 + k * THREADS < end ? (in[k].v[j] - origin) - own : 0.f;
+      const float d = u0 + k * THREADS < end ? (in.v[j] - origin) - own : 0.f;
       s[(k * VEC + j) & 3] = fmaf(d, d, s[(k * VEC + j) & 3]);
     }
+  }
   const float own_m2 = warp_total((s[0] + s[1]) + (s[2] + s[3]));
   cluster_wait_started();
   if (lane < ranks) {
@@ -158,10 +161,11 @@ inline Rows make_rows(int planes, int plane, int vec, long long plane_stride, in
 
 // grid (rows, ranks), clusters of `ranks` along y
 template <typename... P, typename... A>
-int launch(void (*kernel)(P...), unsigned rows, int ranks, cudaStream_t st, A... args) {
+int launch(void (*kernel)(P...), unsigned rows, int ranks, size_t smem, cudaStream_t st, A... args) {
+  if (smem) B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PLAN_STAGED_BYTES));
   if (ranks > 8) B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(rows, (unsigned)ranks); cfg.blockDim = dim3(THREADS); cfg.stream = st;
+  cfg.gridDim = dim3(rows, (unsigned)ranks); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = st;
   cudaLaunchAttribute attr[2] = {};
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = (unsigned)ranks; attr[0].val.clusterDim.z = 1;

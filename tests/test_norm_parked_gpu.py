@@ -28,16 +28,23 @@ def test_batch_norm(shape):
             assert oracle.rel_l2(got, e) <= 5 * GATE
 
 
-# (n, c, h, w), groups: nine ranks of four units, the widest row of four and of six units and the first beyond it, one wave with two thirds of the ranks
-GN = [((3, 9, 64, 64), 1), ((1, 64, 32, 32), 1), ((1, 65, 32, 32), 1), ((1, 24, 64, 64), 1), ((1, 48, 128, 64), 2), ((1, 49, 32, 64), 1), ((2, 14, 81, 84), 2),
-      ((20, 96, 22, 66), 32)]
+# (n, c, h, w), groups.  Registers hold 65536 values of a row forward and backward 65536 (planes of whole 16-byte pieces; half of them are the gradient's);
+# beyond that, shared memory: four CTAs to an SM, sixteen CTAs with two to an SM, the widest row and the first beyond it.  Nine ranks, one wave with two
+# thirds of the ranks; planes cut by ranks and by parts of a warp, a group of 64 planes and of 65.
+GN = [((3, 9, 64, 64), 1), ((20, 96, 22, 66), 32), ((1, 64, 32, 32), 1), ((1, 65, 32, 32), 1), ((1, 24, 64, 64), 1), ((1, 48, 128, 64), 2), ((1, 33, 64, 64), 1),
+      ((2, 14, 81, 84), 2), ((1, 2, 300, 340), 1), ((1, 51, 64, 64), 1), ((1, 100, 64, 64), 1), ((1, 101, 64, 64), 1), ((1, 66, 31, 33), 1), ((3, 16, 137, 63), 2),
+      ((1, 4, 227, 225), 1), ((1, 64, 81, 79), 2), ((1, 63, 51, 127), 1), ((1, 64, 51, 127), 1), ((2, 5, 1, 1023 * 20), 1)]
 
 
 @pytest.mark.parametrize("shape,groups", GN, ids=lambda v: "x".join(map(str, v)) if isinstance(v, tuple) else f"g{v}")
 def test_group_norm(shape, groups):
     rng = np.random.default_rng(sum(shape) + groups)
-    x, g = rng.standard_normal(shape, dtype=np.float32) + np.float32(3), rng.standard_normal(shape, dtype=np.float32)
+    x, g = rng.standard_normal(shape, dtype=np.float32) + np.float32(30), rng.standard_normal(shape, dtype=np.float32)
     w, b = rng.standard_normal(shape[1]).astype(np.float32), rng.standard_normal(shape[1]).astype(np.float32)
     y, mean, rstd = b200conv.group_norm_forward(x, groups, w, b, 1e-5)
+    wy, wmean, wrstd = gn.forward(x, groups, w, b, 1e-5, dtype=np.float64)
+    assert oracle.rel_l2(y, wy) <= 2 * GATE
+    np.testing.assert_allclose(mean, wmean, rtol=2e-6, atol=2e-6)
+    np.testing.assert_allclose(rstd, wrstd, rtol=1e-5)
     for got, e in zip(b200conv.group_norm_backward(g, x, mean, rstd, groups, w), gn.backward(g, x, mean, rstd, groups, w, dtype=np.float64)):
         assert oracle.rel_l2(got, e) <= 5 * GATE
