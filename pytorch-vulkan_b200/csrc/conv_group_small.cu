@@ -56,8 +56,7 @@ __device__ __forceinline__ unsigned long long both(float v) {
 // of all the group's output channels.
 // Bound by the FP32 multiply-adds, and before them by everything that does not run beside them:
 //   * the tile's copies are issued at once and waited for two input channels at a time, so the arithmetic starts when the first two have landed;
-//   * two rows a thread share the input rows between them, the columns beside a strip come from the neighbouring lanes: 64 shared-memory
-//     passes for 288 paired multiply-adds of a warp and channel, where one row and four-way conflicts on the two edge columns took 108;
+//   * two rows a thread share the input rows between them: three reads of an input row feed up to 96 paired multiply-adds;
 //   * tiles of 16 rows leave at most seven on an SM where tiles of 32 left four of 3.5 on average;
 //   * every product of an input value follows one doubling of it, and the copies walk rows and channels by additions.
 // 256 channels of 16 images of 32x32 in 32 groups: 28.1 us from a sliced view and 19.3 from a dense one, now 19.6 and 17.3 (the multiply-adds
