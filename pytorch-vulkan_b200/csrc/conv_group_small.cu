@@ -5,8 +5,8 @@
 // contraction per output is 36 or 72 long: the layers move 8 bytes per 9 to 18 FLOP, so their roofline is HBM, and
 // an implicit-GEMM tile of 64 rows per group (conv_simt.cu) would spend nine tenths of its multiply-adds on padding.
 // Here the tile follows the group instead: a thread block owns (image, group, 16 rows x 64 columns), brings the
-// group's input tile (with its one-pixel halo) into shared memory once, and every thread keeps a 1 x 4 pixel strip
-// of ALL the group's output channels in registers, so an input value is loaded once for up to 3 x 8 multiply-adds.
+// group's input tile (with its one-pixel halo) into shared memory once, and every thread keeps a 2 x 4 pixel strip
+// of all the group's output channels (or half of them) in registers, so an input value is loaded once for up to 3 x 8 multiply-adds.
 //   forward / dInput   one kernel; dInput runs it on dy with the filter rotated by 180 degrees and its channel roles
 //                      exchanged (prepared in shared memory while the tile loads)
 //   dWeight            each thread accumulates a 4 x 2 block of channel pairs with their nine taps over its pixel strips in
@@ -59,12 +59,16 @@ __device__ __forceinline__ unsigned long long both(float v) {
 //   * two rows a thread share the input rows between them: three reads of an input row feed up to 96 paired multiply-adds;
 //   * tiles of 16 rows leave at most seven on an SM where tiles of 32 left four of 3.5 on average;
 //   * every product of an input value follows one doubling of it, and the copies walk rows and channels by additions.
-// 256 channels of 16 images of 32x32 in 32 groups: 28.1 us from a sliced view and 19.3 from a dense one, now 19.6 and 17.3 (the multiply-adds
-// alone are 8.3).
-template <int CPG, int SX>
-__global__ void __launch_bounds__(8 * SX, SX == 8 ? 8 : 4) gconv_fwd_kernel(const GArgs a) {
+// 256 channels of 16 images of 32x32 in 32 groups: 28.1 us from a sliced view and 19.3 from a dense one, now 19.5 and 17.3 (the multiply-adds
+// alone are 8.3), and with
+//   * where all tiles run at once a thread keeps half of the group's eight channels (CO): twice the warps hide the latency of the one wave.
+//     256 channels of 16 images of 32x32: 19.5 -> 18.8 and 17.3 -> 16.9.  Beyond a wave, and for the tiles of wide images, the doubled reads of
+//     the input cost more than that (60 images of 20x20 51.2 -> 56.1, 33 of 43x43 87 -> 103).
+template <int CPG, int SX, int CO>
+__global__ void __launch_bounds__(8 * SX * (CPG / CO), CPG != CO ? 7 : SX == 8 ? 8 : 4) gconv_fwd_kernel(const GArgs a) {
   wait_previous();
-  constexpr int NT = 8 * SX, WARPS = NT / 32;              // threads: SX strips x 8 row pairs
+  constexpr int STRIPS = 8 * SX;                           // SX strips x 8 row pairs
+  constexpr int NT = STRIPS * (CPG / CO), WARPS = NT / 32;
   constexpr int TWK = 4 * SX, THK = 16;                    // tile extent
   constexpr int IWK = TWK + 8, IHK = THK + 2;              // with halo; image column x0 + c at c + 4, so that 16-byte pieces stay aligned
   constexpr int STAGES = CPG / 2;                          // of two input channels
@@ -135,12 +139,12 @@ __global__ void __launch_bounds__(8 * SX, SX == 8 ? 8 : 4) gconv_fwd_kernel(cons
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
 
-  const int tx = tid % SX, ty = tid / SX;   // rows 2*ty and 2*ty + 1, columns 4*tx .. 4*tx+3
-  unsigned long long pair[2][CPG / 2][4];   // output channels 2q and 2q + 1 of four pixels in two rows
+  const int tx = tid % SX, ty = tid % STRIPS / SX, co0 = tid / STRIPS * CO;   // rows 2*ty and 2*ty + 1, columns 4*tx .. 4*tx+3
+  unsigned long long pair[2][CO / 2][4];    // output channels co0 + 2q and co0 + 2q + 1 of four pixels in two rows
 #pragma unroll
   for (int r = 0; r < 2; ++r)
 #pragma unroll
-    for (int q = 0; q < CPG / 2; ++q)
+    for (int q = 0; q < CO / 2; ++q)
 #pragma unroll
       for (int j = 0; j < 4; ++j) pair[r][q][j] = 0ull;
 #pragma unroll 1
@@ -161,12 +165,12 @@ __global__ void __launch_bounds__(8 * SX, SX == 8 ? 8 : 4) gconv_fwd_kernel(cons
       for (int out = 0; out < 2; ++out) {   // input row 2*ty - 1 + r is tap ky of output row 2*ty + out
         const int ky = r - out;
         if (ky < 0 || ky > 2) continue;
-        unsigned long long wv[3][CPG / 2];
+        unsigned long long wv[3][CO / 2];
 #pragma unroll
         for (int kx = 0; kx < 3; ++kx)
 #pragma unroll
-          for (int q = 0; q < CPG / 4; ++q) {
-            const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(&s_w[ci][ky][kx][4 * q]);
+          for (int q = 0; q < CO / 4; ++q) {
+            const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(&s_w[ci][ky][kx][co0 + 4 * q]);
             wv[kx][2 * q] = t.x; wv[kx][2 * q + 1] = t.y;
           }
 #pragma unroll
@@ -176,7 +180,7 @@ __global__ void __launch_bounds__(8 * SX, SX == 8 ? 8 : 4) gconv_fwd_kernel(cons
           for (int kx = 0; kx < 3; ++kx)
             if (i - kx >= 0 && i - kx < 4) {
 #pragma unroll
-              for (int q = 0; q < CPG / 2; ++q) pair[out][q][i - kx] = fma2(vv, wv[kx][q], pair[out][q][i - kx]);
+              for (int q = 0; q < CO / 2; ++q) pair[out][q][i - kx] = fma2(vv, wv[kx][q], pair[out][q][i - kx]);
             }
         }
       }
@@ -191,13 +195,13 @@ __global__ void __launch_bounds__(8 * SX, SX == 8 ? 8 : 4) gconv_fwd_kernel(cons
     float* out = a.out + (n * (long long)a.c + chan0) * plane + (long long)y * a.w_ + x;
     const bool vec = x + 3 < a.w_ && ((reinterpret_cast<uintptr_t>(out) & 15) == 0) && (plane % 4 == 0);
 #pragma unroll
-    for (int q = 0; q < CPG / 2; ++q) {
+    for (int q = 0; q < CO / 2; ++q) {
       float acc[2][4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) asm("mov.b64 {%0, %1}, %2;" : "=f"(acc[0][j]), "=f"(acc[1][j]) : "l"(pair[r][q][j]));
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        const int co = 2 * q + i;
+        const int co = co0 + 2 * q + i;
         const float bv = a.bias ? __ldg(a.bias + (chan0 + co) * a.bias_stride) : 0.f;
         float* p = out + co * plane;
         if (vec) {
@@ -464,11 +468,12 @@ int group_small_conv(const ConvGeom& g, bool is_dx, View4 in, View4 w, const flo
   if (blocks > 2147483647ll) return fail(B200_ERANGE, "grouped convolution: grid exceeds launch limits");
   const unsigned nb = (unsigned)blocks;
   if (g.cig == 4) {
-    if (narrow) launch_next(gcs::gconv_fwd_kernel<4, 8>, nb, 64, 0, st, a);
-    else launch_next(gcs::gconv_fwd_kernel<4, 16>, nb, 128, 0, st, a);
+    if (narrow) launch_next(gcs::gconv_fwd_kernel<4, 8, 4>, nb, 64, 0, st, a);
+    else launch_next(gcs::gconv_fwd_kernel<4, 16, 4>, nb, 128, 0, st, a);
   } else {
-    if (narrow) launch_next(gcs::gconv_fwd_kernel<8, 8>, nb, 64, 0, st, a);
-    else launch_next(gcs::gconv_fwd_kernel<8, 16>, nb, 128, 0, st, a);
+    if (narrow && blocks <= 7ll * sm_count()) launch_next(gcs::gconv_fwd_kernel<8, 8, 4>, nb, 128, 0, st, a);   // one wave: seven CTAs fit an SM
+    else if (narrow) launch_next(gcs::gconv_fwd_kernel<8, 8, 8>, nb, 64, 0, st, a);
+    else launch_next(gcs::gconv_fwd_kernel<8, 16, 8>, nb, 128, 0, st, a);
   }
   count_launch();
   return launch_check("gconv_fwd_kernel");

@@ -61,3 +61,18 @@ def test_other_grouped_shapes_keep_the_general_kernels():
         assert b200conv.last_kernel() != "group_small_forward"
         want = oracle.torch_conv_all(x, w, None, np.zeros_like(y), kw.get("stride", (1, 1)), kw["padding"], (1, 1), 4)[0]
         assert oracle.rel_l2(y, want) <= GATE
+
+
+@pytest.mark.parametrize("n", [16, 17])     # 1024 and 1088 tiles: within and beyond one wave of seven CTAs on 148 SMs, where a thread keeps four and eight channels
+def test_both_splits_of_eight_channels_agree(n):
+    rng = np.random.default_rng(n)
+    x, go = rng.standard_normal((n, 256, 31, 31), dtype=np.float32), rng.standard_normal((n, 256, 31, 31), dtype=np.float32)
+    wt = (rng.standard_normal((256, 8, 3, 3), dtype=np.float32) / np.sqrt(72)).astype(np.float32)
+    b = rng.standard_normal(256, dtype=np.float32)
+    kw = dict(padding=(1, 1), groups=32)
+    y, dx = b200conv.conv2d_forward(x, wt, b, **kw), b200conv.conv2d_backward(go, x, wt, **kw)[0]
+    want = oracle.torch_conv_all(x, wt, b, go, (1, 1), (1, 1), (1, 1), 32)
+    assert max(oracle.rel_l2(y, want[0]), oracle.rel_l2(dx, want[1])) <= GATE
+    # every sum runs over the same products in the same order
+    assert np.array_equal(y[-1:], b200conv.conv2d_forward(x[-1:], wt, b, **kw))
+    assert np.array_equal(dx[-1:], b200conv.conv2d_backward(go[-1:], x[-1:], wt, **kw)[0])
