@@ -515,10 +515,11 @@ nres::StagedPlan forward_staged(const GnShape& sh, int vec) {
   return nres::plan_staged(units, 4 * vec, kStagedForward);
 }
 
-// The backward kernel's form.  Parked where four units of each tensor do not hold the row, need nine ranks or more and most of a wave, or take more
+// The backward kernel's form.  Parked where four units of each tensor do not hold the row, need eleven ranks or more and most of a wave, or take more
 // than one wave while six are one wave of two thirds as many ranks.  Measured on 150 random layers, the gain over what took them before: rows that
-// only the parked form holds 1.20 to 3.38, median 1.5, over the streaming kernel (32 rows of 74420 values 30.6 -> 9.1 us); rows of nine ranks or more
-// .98 to 1.27, median 1.06 (half a wave and less .90); two thirds as many ranks in one wave 1.15 to 1.29; elsewhere .87 to .98.
+// only the parked form holds 1.20 to 3.38, median 1.5, over the streaming kernel (32 rows of 74420 values 30.6 -> 9.1 us); rows of eleven ranks or
+// more .98 to 1.27, median 1.08 (half a wave and less .90, 1.4 to 1.5 waves of which the parked form leaves 1.0
+// to 1.1 .94 to 1.00; nine and ten ranks .95 to 1.00); two thirds as many ranks in one wave 1.15 to 1.29; elsewhere .87 to .98.
 // Rows beyond both, up to 204800 values, wait in shared memory altogether: 1.1 to 2.6 times as fast as the kernel with a CTA for a row (32 rows of
 // 154652 values 67.4 -> 25.9 us; single values 64 of 136367 123 -> 56, 416 of 103968 212 -> 195).  Where six units hold a row they are the faster form: 32
 // rows of 82944 values 9.3 against 12.5.  With two CTAs to an SM and many rows the other kernel is level: 288 rows of 148104 values 158 -> 165, 96 of
@@ -534,8 +535,10 @@ BackwardPlan backward_plan(const GnShape& sh, int blocks, int vec) {
   p.ranks = block_ranks(sh, blocks, vec, vec == 4 ? kUnitsBwd : kUnits1, true);
   const int parked = vec == 4 ? block_ranks(sh, blocks, vec, kUnitsParked, true) : 0;
   const long long slots = 4ll * sm_count();
-  p.park = parked && (p.ranks == 0 || (p.ranks >= 9 && 10ll * blocks * p.ranks > 7 * slots) ||
-                      ((long long)blocks * p.ranks > slots && (long long)blocks * parked <= slots && parked * 3 <= p.ranks * 2));
+  const long long ctas = (long long)blocks * p.ranks, parked_ctas = (long long)blocks * parked;
+  const bool wide = p.ranks >= 11 && 10 * ctas > 7 * slots && (10 * parked_ctas <= 9 * slots || 4 * ctas > 7 * slots);
+  const bool one_wave = ctas > slots && parked_ctas <= slots && parked * 3 <= p.ranks * 2;
+  p.park = parked && (p.ranks == 0 || wide || (one_wave && p.ranks < 11));
   if (p.park) p.ranks = parked;
   if (p.ranks == 0) p.staged = nres::plan_staged((long long)sh.cpg * sh.hw / vec, 8 * vec, kStagedBackward);
   if (vec == 4 && p.staged.units > 8 && blocks > 256) p.staged = {};

@@ -29,9 +29,9 @@ def test_batch_norm(shape):
 
 
 # (n, c, h, w), groups.  Registers hold 65536 values of a row forward and backward 65536 (planes of whole 16-byte pieces; half of them are the gradient's);
-# beyond that, shared memory: four CTAs to an SM, sixteen CTAs with two to an SM, the widest row and the first beyond it.  Nine ranks, one wave with two
+# beyond that, shared memory: four CTAs to an SM, sixteen CTAs with two to an SM, the widest row and the first beyond it.  Eleven ranks, one wave with two
 # thirds of the ranks; planes cut by ranks and by parts of a warp, a group of 64 planes and of 65.
-GN = [((3, 9, 64, 64), 1), ((20, 96, 22, 66), 32), ((1, 64, 32, 32), 1), ((1, 65, 32, 32), 1), ((1, 24, 64, 64), 1), ((1, 48, 128, 64), 2), ((1, 33, 64, 64), 1),
+GN = [((3, 9, 64, 64), 1), ((40, 11, 64, 64), 1), ((20, 96, 22, 66), 32), ((1, 64, 32, 32), 1), ((1, 65, 32, 32), 1), ((1, 24, 64, 64), 1), ((1, 48, 128, 64), 2), ((1, 33, 64, 64), 1),
       ((2, 14, 81, 84), 2), ((1, 2, 300, 340), 1), ((1, 51, 64, 64), 1), ((1, 100, 64, 64), 1), ((1, 101, 64, 64), 1), ((1, 66, 31, 33), 1), ((3, 16, 137, 63), 2),
       ((1, 4, 227, 225), 1), ((1, 64, 81, 79), 2), ((1, 63, 51, 127), 1), ((1, 64, 51, 127), 1), ((2, 5, 1, 1023 * 20), 1)]
 
