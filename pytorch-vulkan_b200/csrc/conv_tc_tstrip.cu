@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(tstrip_threads(AW), 1) conv_tstrip_kernel(cons
     const int chunks = (a.strip_rows + 31) / 32;
     const bool vec_layout = a.act.s1 == 1 && a.kc % 4 == 0 && ((reinterpret_cast<uintptr_t>(a.act.ptr) & 15) == 0) &&
                             (a.act.s0 % 4 == 0) && (a.act.s2 % 4 == 0) && (a.act.s3 % 4 == 0);
-    const int s1 = (int)a.act.s1;
+    const long long s1 = a.act.s1;   // 64-bit: views that 32-bit element offsets do not address come here
     const int total_jobs = my_tiles * a.cblocks * chunks;  // below 2^31 (checked by the host)
     // consecutive jobs of a warp stay within a_stages stages of each other (a waiter that skipped a whole
     // phase of a stage's mbarrier would see the parity of an older phase and run ahead)
@@ -348,8 +348,9 @@ __global__ void __launch_bounds__(tstrip_threads(AW), 1) conv_tstrip_kernel(cons
           v[4 * i] = f.x; v[4 * i + 1] = f.y; v[4 * i + 2] = f.z; v[4 * i + 3] = f.w;
         }
       } else {
+        const float* p = src;
 #pragma unroll
-        for (int j = 0; j < KB; ++j) v[j] = (src && j < nvalid) ? __ldg(src + j * s1) : 0.f;
+        for (int j = 0; j < KB; ++j, p += s1) v[j] = (src && j < nvalid) ? __ldg(p) : 0.f;
       }
       if (!mbar_wait(smem_u32(&ctrl->a_empty[as]), (a_round & 1) ^ 1, abort_flag, a.status, STATUS_TIMEOUT_EMPTY)) break;
       const uint32_t p_hi = tiles_base + as * a_stage_bytes, p_cr = p_hi + a_plane;
