@@ -102,7 +102,8 @@ struct TArgs {
 #endif
 #define TPROF(slot, stmt) do { if (B200_ROLE_PROFILE && a.prof && blockIdx.x == 0) { const long long t0__ = clock64(); stmt; atomicAdd(a.prof + (slot), (unsigned long long)(clock64() - t0__)); } else { stmt; } } while (0)
 
-// Second tap of a stack (filter column, NO_TAP: none) where 64 or fewer output channels leave half of the filter rows to it
+// Second tap of a stack (filter column) where 64 or fewer output channels leave half of the filter rows to it.  NO_TAP, there or for a first tap:
+// weights of zero.
 constexpr unsigned char NO_TAP = 255;
 struct Stacked {
   int delta = 0;
@@ -551,26 +552,30 @@ struct TPlan {
 // shared-memory operand read (4 KB of filter + 32 B per pixel) about 96 bytes per clock.
 static double mma_clocks(int pn) { return std::max(pn / 2.0, (4096.0 + 32.0 * pn) / 96.0); }
 
-// The pixel tile is the free parameter: wide tiles use the tensor pipe best, but the tile count should fill whole
-// waves of SMs.  Modelled time = waves x (MMAs of a tile x clocks(pn) + a fixed cost per tile).
-// Taps in stacks of two: neighbouring filter columns of one row and phase, the one that reads further on second.  False where the filter
-// does not gain by it (fewer than a quarter of the steps saved) or its taps lie too far apart.
+// Taps in stacks of two: neighbouring filter columns of one row and phase, the one that reads further on second.  The last of an odd number
+// shares a stack with its neighbour once more, whose weights are zero there: zeros must not meet pixels that the filter does not reach, where an
+// infinity or NaN would become one of the result.  False where a row of a phase has one tap only (every other column of a 3-wide filter at stride
+// 2), where the filter does not gain by it (fewer than a quarter of the steps saved) or its taps lie too far apart.
 static bool stack_taps(TapTable& tt, bool is_dx, Stacked& s) {
   TapTable out = tt;
   out.taps_total = 0;
   s.delta = 0;
   for (int ph = 0; ph < tt.n_phase; ++ph) {
     for (int t = tt.start[ph]; t < tt.start[ph + 1];) {
-      const bool two = t + 1 < tt.start[ph + 1] && tt.ky[t + 1] == tt.ky[t];
-      const int first = two && is_dx ? t + 1 : t, second = two ? (is_dx ? t : t + 1) : -1, i = out.taps_total++;
-      out.ky[i] = tt.ky[first]; out.kx[i] = tt.kx[first]; out.shift[i] = tt.shift[first];
-      s.kx[i] = two ? tt.kx[second] : NO_TAP;
-      if (two) {
+      int end = t + 1;
+      while (end < tt.start[ph + 1] && tt.ky[end] == tt.ky[t]) ++end;
+      if (end - t < 2) return false;
+      for (; t < end; t += 2) {
+        const bool again = t + 1 == end;            // the row's last tap, and taps t - 1 and t of which the first has had its turn
+        const int a = again ? t - 1 : t, first = is_dx ? a + 1 : a, second = is_dx ? a : a + 1, i = out.taps_total++;
+        out.ky[i] = tt.ky[a]; out.shift[i] = tt.shift[first];
+        out.kx[i] = again && first == a ? NO_TAP : tt.kx[first];
+        s.kx[i] = again && second == a ? NO_TAP : tt.kx[second];
         const int d = tt.shift[second] - tt.shift[first];
         if (d < 1 || d > 16 || (s.delta && d != s.delta)) return false;
         s.delta = d;
       }
-      t += two ? 2 : 1;
+      t = end;
     }
     out.start[ph + 1] = (unsigned char)out.taps_total;
   }
@@ -579,6 +584,8 @@ static bool stack_taps(TapTable& tt, bool is_dx, Stacked& s) {
   return true;
 }
 
+// The pixel tile is the free parameter: wide tiles use the tensor pipe best, but the tile count should fill whole
+// waves of SMs.  Modelled time = waves x (MMAs of a tile x clocks(pn) + a fixed cost per tile).
 static TPlan make_plan(const ConvGeom& g, bool is_dx) {
   TPlan p;
   p.geo = tcs::plan_strip_geometry(g, is_dx);

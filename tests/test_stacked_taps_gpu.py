@@ -39,3 +39,30 @@ def test_forward_and_dinput(case, layout, monkeypatch):
     assert b200conv.last_kernel() == "tc_strip_forward" and b200conv.device_status() == 0 and oracle.rel_l2(y, y64) <= 1e-5
     dx = b200conv.conv2d_backward(lay(go), lay(x), w, mask=(True, False, False), **kw)[0]
     assert b200conv.last_kernel() == "tc_strip_dinput" and b200conv.device_status() == 0 and oracle.rel_l2(dx, dx64) <= 1e-5
+
+
+@pytest.mark.parametrize("case", [*CASES[:8], CASES[9], ((2, 32, 13, 21), 32, (3, 5), dict(padding=(1, 2), stride=(1, 2)))],
+                         ids=lambda c: "x".join(map(str, c[0])) + f"-co{c[1]}-k{c[2][0]}x{c[2][1]}")
+def test_values_that_are_not_finite_stay_where_the_filter_reaches(case, monkeypatch):
+    monkeypatch.setenv("B200_CONV_TC_VARIANT", "stacked")
+    xshape, cout, kernel, kw = case
+    rng = np.random.default_rng(sum(xshape) + cout)
+    g = oracle.geometry(xshape, cout, kernel, **kw)
+    x, go = rng.standard_normal(g.x_shape, dtype=np.float32), rng.standard_normal(g.y_shape, dtype=np.float32)
+    w = (rng.standard_normal(g.w_shape, dtype=np.float32) / np.sqrt(np.prod(g.w_shape[1:]))).astype(np.float32)
+    args = (kw.get("stride", (1, 1)), kw.get("padding", (0, 0)), kw.get("dilation", (1, 1)), kw.get("groups", 1))
+    where = {}
+    for name, a in (("x", x), ("go", go)):      # a corner, the ends of a row and of the next, and an interior pixel of the last image
+        h, wd = a.shape[2:]
+        marks = np.zeros_like(a)
+        for i, (y0, x0) in enumerate([(0, 0), (h // 2, wd - 1), (h // 2 + 1, 0), (h - 1, wd // 2), (h // 3, wd // 3)]):
+            marks[-1, i % a.shape[1], y0, x0] = 1
+        where[name] = marks
+    reached = oracle.torch_conv_all(where["x"], np.ones_like(w), None, where["go"], *args)[:2]
+    want = oracle.torch_conv_all(np.where(where["x"] > 0, 0, x), w, None, np.where(where["go"] > 0, 0, go), *args)[:2]
+    for value in (np.inf, np.nan):
+        xv, gv = np.where(where["x"] > 0, np.float32(value), x), np.where(where["go"] > 0, np.float32(value), go)
+        got = b200conv.conv2d_forward(xv, w, None, **kw), b200conv.conv2d_backward(gv, xv, w, mask=(True, False, False), **kw)[0]
+        for a, r, e in zip(got, reached, want):
+            assert np.array_equal(np.isfinite(a), r < 0.5)
+            assert oracle.rel_l2(np.where(r < 0.5, a, 0), np.where(r < 0.5, e, 0)) <= 1e-5
