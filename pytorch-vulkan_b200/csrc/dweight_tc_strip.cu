@@ -658,8 +658,8 @@ bool dweight_strip_supported(const ConvGeom& g) {
 // The tensor-memory kernel gives a CTA of up to 64 output channels all vertical taps of an input block, where this one has a CTA for each
 // tap.  That pays while the splits fill the machine; where they cannot (little or no scratch, few pixels) its CTAs are a third as many and
 // do a third more per K block.  Per K block and for the rest of a CTA, measured: 0.74 us (six slots; 0.31 per strip of a strided input) and
-// 6 against 0.51 (0.60 in four blocks) + 4.  (1x1 filters always gain by the tensor-memory kernel's idle warps: 432 -> 64 channels of 5x 7x7
-// 10.8 us here, 7.8 there.)  16 -> 62 channels of 7x 21x21, stride 2, no scratch: 45.6 and 25.3 us;
+// 6 against 0.51 (0.60 in four blocks) + 4.  (1x1 filters always gain by the tensor-memory kernel's idle warps, and run in three TF32
+// passes there as here: 432 -> 64 channels of 5x 7x7 11.9 us here, 8.2 there.)  16 -> 62 channels of 7x 21x21, stride 2, no scratch: 45.6 and 25.3 us;
 // 38 -> 32 of 5x 46x46, no scratch: 265 and 181; 16 -> 64 of 61x61 x 14 with all the scratch it wants: 27.4 and 28.9.
 static bool strip_is_faster(const ConvGeom& g, const tcdt::PlanInfo& t, const tcdw::DwStripPlan& s) {
   if (!s.ok || g.cig * g.kh * g.kw < 32) return false;   // few products: short chains, which only the tensor-memory kernel has

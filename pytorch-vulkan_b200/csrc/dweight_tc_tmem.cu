@@ -37,6 +37,11 @@
 // quarters stage input, and four sets of two warps stage dY: a dY block is a load from memory, a conversion and a store in one warp, so
 // the number of warps that have one on its way sets the pace.  3 -> 64 channels, 7x7, stride 2, 64x224x224: 186 us, now 144.
 //
+// THREE (1x1 filters with 64 or fewer output channels): the cross terms are two TF32 products instead of one BF16 pass, in accumulator columns of
+// their own.  dweight_tc_strip.cu, which takes these layers otherwise, runs three passes too, and the multipliers are idle here in any case: 432 -> 64
+// channels of 5x 7x7 8.1 us and an error of 1.46e-6 against FP64 with the BF16 pass, 8.2 and 6.2e-7 with three (there 11.9 and 1.23e-6); 45 layers
+// 0.99 of the BF16 form's time and 0.2 to 0.5 of its error.
+//
 // Replaces csrc/shaders/conv2d_backward_weight_tiled_body.glsl:42-70 of the reference for these geometries.
 #include "common.cuh"
 #include "plan_cache.cuh"
@@ -107,8 +112,8 @@ struct Args {
   Slot slots[MAX_SLOTS];
   int fold_kh, fold_sh, fold_dh, fold_ph, fold_h;   // FOLD: the real filter height and what places its rows (g describes the folded layer)
   int* status;
+  int three;                  // THREE: as many accumulator columns again for the cross terms
 };
-
 
 struct Ctrl {
   unsigned long long x_full[MAX_RING], x_empty[MAX_RING], a_full[MAX_A], a_empty[MAX_A], accum, drained;
@@ -132,7 +137,7 @@ __device__ __forceinline__ uint64_t desc64(uint32_t lo, uint32_t hi) {
 
 // NG groups of NB N-blocks each where the plan has that shape (0: as the arguments say): with the loop bounds and the step width
 // known, the issuing warp needs 175 clocks less per K block of a 3x3 filter.
-template <int NG, int NB, bool FOLD>
+template <int NG, int NB, bool FOLD, bool THREE>
 __global__ void __launch_bounds__(THREADS, 1) dweight_tmem_kernel(const Args a) {
   wait_previous();
   constexpr int GROUPS = NG ? NG : MAX_GROUPS;
@@ -175,7 +180,7 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_tmem_kernel(const Args a) 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&ctrl->tmem_base);
-  const uint32_t a_cols = tmem + (uint32_t)a.n_slots * 32u;      // dY stages of 64 columns behind the accumulators
+  const uint32_t acc_cols = (uint32_t)a.n_slots * 32u, a_cols = tmem + (THREE ? 2u : 1u) * acc_cols;   // dY stages of 64 columns behind the accumulators
 
   // ---- which piece of dW this CTA owns ----
   int id = blockIdx.x;
@@ -201,7 +206,7 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_tmem_kernel(const Args a) 
     // parameters are indexed with constants, and the next K block's barriers are polled before the last group of the current one.
     const uint32_t idesc = make_idesc_tf32(128, 0) | (1u << 16), idesc16 = make_idesc_bf16(128, 0) | (1u << 16);
     const uint64_t hi_tmpl = tcdw::make_mn_desc(base, 0), b16_tmpl = tcdw::make_mn_desc16(base + ring_rows * 128u, 0);
-    const uint32_t hi_top = (uint32_t)(hi_tmpl >> 32), b16_top = (uint32_t)(b16_tmpl >> 32), l16_d = (ring_rows * 64u) >> 4;
+    const uint32_t hi_top = (uint32_t)(hi_tmpl >> 32), b16_top = (uint32_t)(b16_tmpl >> 32), l16_d = (ring_rows * 64u) >> 4, lo_d = (ring_rows * 128u) >> 4;
     uint32_t lo_h[GROUPS], lo_16[GROUPS], pos[GROUPS];   // low descriptor words and ring position of every group
 #pragma unroll
     for (int i = 0; i < GROUPS; ++i) {
@@ -243,10 +248,17 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_tmem_kernel(const Args a) 
         if (leader) {
 #pragma unroll
           for (int k = 0; k < 4; ++k) umma_tf32_ts(acc, ta + 8 * k, desc64(lo_h[i] + 64 * k, hi_top), idesc | n, (uint32_t)((in_chunk | k) != 0));
+          if (THREE) {
 #pragma unroll
-          for (int k = 0; k < 2; ++k) umma_bf16_ts(acc, ta + 32 + 8 * k, desc64(lo_16[i] + l16_d + 64 * k, b16_top), idesc16 | n, 1);
+            for (int k = 0; k < 4; ++k) umma_tf32_ts(acc + acc_cols, ta + 8 * k, desc64(lo_h[i] + lo_d + 64 * k, hi_top), idesc | n, (uint32_t)((in_chunk | k) != 0));
 #pragma unroll
-          for (int k = 0; k < 2; ++k) umma_bf16_ts(acc, ta + 48 + 8 * k, desc64(lo_16[i] + 64 * k, b16_top), idesc16 | n, 1);
+            for (int k = 0; k < 4; ++k) umma_tf32_ts(acc + acc_cols, ta + 32 + 8 * k, desc64(lo_h[i] + 64 * k, hi_top), idesc | n, 1);
+          } else {
+#pragma unroll
+            for (int k = 0; k < 2; ++k) umma_bf16_ts(acc, ta + 32 + 8 * k, desc64(lo_16[i] + l16_d + 64 * k, b16_top), idesc16 | n, 1);
+#pragma unroll
+            for (int k = 0; k < 2; ++k) umma_bf16_ts(acc, ta + 48 + 8 * k, desc64(lo_16[i] + 64 * k, b16_top), idesc16 | n, 1);
+          }
           if (last) {
             umma_commit(a_done);
             umma_commit(x_done);
@@ -326,15 +338,14 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_tmem_kernel(const Args a) 
       if (!warp_wait(smem_u32(&ctrl->x_empty[slot]), (round & 1u) ^ 1u, abort_flag, a.status, STATUS_TIMEOUT_EMPTY)) break;
       BlockPlanes pl;
       pl.hi = base + (uint32_t)strip * strip_bytes;
-      pl.lo = 0;
-      pl.h16 = pl.hi + ring_rows * 128u;
+      pl.lo = pl.h16 = pl.hi + ring_rows * 128u;
       pl.l16 = pl.h16 + ring_rows * 64u;
       const int copies = slot * KP < MIRROR ? 2 : 1;        // the first rows of the ring once more behind its end
 #pragma unroll 1
       for (int i = 0; i < copies; ++i) {
         const int row0 = slot * KP + i * (int)ring_pixels, rows = i ? min(KP, MIRROR - slot * KP) : KP;
-        if (chunked) tcdw::store_block_chunks<true>(val, rows, row0, pl, lane);
-        else tcdw::store_block<true>(val, rows, row0, pl, lane, FOLD ? g.cig - ci0 - a.strips[strip].cblk * 32 : 32);
+        if (chunked) tcdw::store_block_chunks<!THREE>(val, rows, row0, pl, lane);
+        else tcdw::store_block<!THREE>(val, rows, row0, pl, lane, FOLD ? g.cig - ci0 - a.strips[strip].cblk * 32 : 32);
       }
       fence_proxy_async();
       __syncwarp();
@@ -420,10 +431,15 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_tmem_kernel(const Args a) 
           split_tf32_fast(w[j], h[j], l[j]);
           hi[4 * i + j] = __float_as_uint(h[j]);
         }
-        cr[2 * i] = pack_bf16x2(h[0], h[1]);
-        cr[2 * i + 1] = pack_bf16x2(h[2], h[3]);
-        cr[16 + 2 * i] = pack_bf16x2(l[0], l[1]);
-        cr[17 + 2 * i] = pack_bf16x2(l[2], l[3]);
+        if (THREE) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) cr[4 * i + j] = __float_as_uint(l[j]);
+        } else {
+          cr[2 * i] = pack_bf16x2(h[0], h[1]);
+          cr[2 * i + 1] = pack_bf16x2(h[2], h[3]);
+          cr[16 + 2 * i] = pack_bf16x2(l[0], l[1]);
+          cr[17 + 2 * i] = pack_bf16x2(l[2], l[3]);
+        }
       }
       tmem_st32(ta, hi);
       tmem_st32(ta + 32, cr);
@@ -459,7 +475,9 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_tmem_kernel(const Args a) 
       for (int i = set; i < a.n_slots; i += a.dy_sets) {
         const Slot sl = a.slots[i];
         float v[32];
-        tmem_ld32(tmem + (uint32_t)(i * 32) + lane_base, v);
+        const uint32_t at = tmem + (uint32_t)(i * 32) + lane_base;
+        if (THREE) tmem_ld32_sum(at, at + acc_cols, v);
+        else tmem_ld32(at, v);
         __syncwarp();
 #pragma unroll
         for (int j = 0; j < 32; ++j) scratch[lane * 33 + j] = v[j];
@@ -605,6 +623,8 @@ static Plan make_plan(const ConvGeom& real, size_t budget) {
   // 64 x 56x56 42 and 53: the line is at five million input values, or one block of input channels.
   // Fewer than 64 input channels leave that kernel's rows half empty, with one value to a load in the ragged block: where wide outputs repeat it,
   // this one is faster at any size (48 -> 256 of 33 x 92x92 233 and 125 us, 61 -> 400 of 20 x 88x88 211 and 138; 64 -> 192 of 27 x 77x77 69 and 73).
+  // Its BF16 cross terms cost them nothing: such sums are long, and that kernel's chains are as long with more steps to a K block (the same layers
+  // 1.31e-5 and 8.9e-6 off, 1.46e-5 and 9.9e-6).
   if (!fold && g.kh * g.kw == 1 && g.cig > 32 && !(g.cig < 64 && g.cog > 128) && q_total * g.cig > (5ll << 20)) return best;
   const int row_pitch = gw + pc;
   // shift mode: vertical taps m apart lie a whole number of grid rows apart
@@ -624,6 +644,8 @@ static Plan make_plan(const ConvGeom& real, size_t budget) {
         ++n_list;
       }
   }
+  // 32 and more (input channel, tap) pairs, as with CHUNK_KB_FP32: below, chains of four K blocks
+  const bool three = !fold && g.kh * g.kw == 1 && g.cog <= 64 && g.cig >= 32;
   const int q_first = -((shift_rows + KP - 1) / KP * KP);
   const int cib = (g.cig + 31) / 32;
   const size_t dw_bytes = sizeof(float) * (size_t)g.cout * g.cig * g.kh * g.kw;
@@ -641,7 +663,9 @@ static Plan make_plan(const ConvGeom& real, size_t budget) {
       if (nky > 8) continue;
       for (int i = 0; i < nky; ++i) { list[i] = shift ? ky_list[i] : i; up[i] = shift ? upper[i] : -1; }
       if (layout(g, nci, nky, all ? list : nullptr, up, row_pitch, a) < 0) continue;
-      a.a_stages = std::min(MAX_A, (512 - 32 * a.n_slots) / 64);
+      a.three = three;
+      if ((three ? 64 : 32) * a.n_slots > ACC_COLS) continue;
+      a.a_stages = std::min(MAX_A, (512 - (three ? 64 : 32) * a.n_slots) / 64);
       // dY sets against input warps: whichever split lets the slower side keep up best
       a.dy_sets = 1;
       auto slower = [&](int sets) { return std::max(1.0 / sets, (double)a.n_strips / (MMA_WARP - 4 * sets)); };
@@ -662,7 +686,7 @@ static Plan make_plan(const ConvGeom& real, size_t budget) {
       // them beside the staging warps costs), the bytes pulled from L2 (about 22 per clock and SM), the work
       // of the staging warps (about 2400 clocks per job and warp)
       const int dy_jobs = shift ? 2 * std::min(2, (g.cog + 31) / 32) : std::min(4, (g.cog + 31) / 32);
-      const double mma = 128.0 * a.n_slots + 100.0 + 60.0 * a.n_groups + 30.0 * (a.n_strips + dy_jobs);
+      const double mma = (three ? 192.0 : 128.0) * a.n_slots + 100.0 + 60.0 * a.n_groups + 30.0 * (a.n_strips + dy_jobs);
       const double kb_clk = std::max({mma, 4096.0 * (a.n_strips + dy_jobs) / 22.0,
                                       2400.0 * (a.narrow ? std::max(1.0 / a.dy_sets, (double)a.n_strips / NARROW_X_WARPS) : slower(a.dy_sets))});
       for (int w = 0; w <= 3; ++w) {
@@ -712,13 +736,13 @@ bool plan_info(const ConvGeom& g, size_t budget, PlanInfo* info) {
   return p.ok;
 }
 
-template <int NG, int NB, bool FOLD = false>
+template <int NG, int NB, bool FOLD = false, bool THREE = false>
 static int launch(const Args& a, const Plan& p, cudaStream_t st) {
   static std::once_flag once;
   static cudaError_t opt_in = cudaSuccess;
-  std::call_once(once, [] { opt_in = cudaFuncSetAttribute(dweight_tmem_kernel<NG, NB, FOLD>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448); });
+  std::call_once(once, [] { opt_in = cudaFuncSetAttribute(dweight_tmem_kernel<NG, NB, FOLD, THREE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448); });
   B200_CUDA(opt_in);
-  launch_next(dweight_tmem_kernel<NG, NB, FOLD>, dim3((unsigned)p.tiles, (unsigned)a.splits), THREADS, (size_t)p.smem, st, a);
+  launch_next(dweight_tmem_kernel<NG, NB, FOLD, THREE>, dim3((unsigned)p.tiles, (unsigned)a.splits), THREADS, (size_t)p.smem, st, a);
   count_launch();
   return launch_check("dweight_tmem_kernel");
 }
@@ -744,7 +768,7 @@ int run(const ConvGeom& g, View4 x, View4 dy, float* dw, void* ws, size_t ws_byt
       if (a.groups[i].n_bits != 3u << 19) return false;
     return true;
   }();
-  const int rc = a.fold_kh ? (a.n_groups == 2 ? launch<2, 0, true>(a, p, st) : a.n_groups == 1 ? launch<1, 0, true>(a, p, st) : launch<0, 0, true>(a, p, st)) : threes && a.n_groups == 3 ? launch<3, 3>(a, p, st) : threes && a.n_groups == 4 ? launch<4, 3>(a, p, st)
+  const int rc = a.three ? launch<1, 0, false, true>(a, p, st) : a.fold_kh ? (a.n_groups == 2 ? launch<2, 0, true>(a, p, st) : a.n_groups == 1 ? launch<1, 0, true>(a, p, st) : launch<0, 0, true>(a, p, st)) : threes && a.n_groups == 3 ? launch<3, 3>(a, p, st) : threes && a.n_groups == 4 ? launch<4, 3>(a, p, st)
                : a.n_groups == 1 ? launch<1, 0>(a, p, st) : a.n_groups == 6 ? launch<6, 0>(a, p, st) : launch<0, 0>(a, p, st);
   if (rc) return rc;
   if (a.splits > 1) return tcdw::finalize_partials((const float*)ws, dw, a.g, a.splits, st);
