@@ -377,8 +377,9 @@ struct DwTcArgs {
   int tiles_m, tiles_n;
   int* status;
 };
+constexpr long long NO_ROW = -(1ll << 62);   // a channel offset that no view has (strides may be negative)
 struct DwRow {
-  long long chan_off;  // (g*cig + ci) * x.s1, or -1 for a padding row
+  long long chan_off;  // (g*cig + ci) * x.s1, or NO_ROW for a padding row
   int ydelta, xdelta;  // ky*dh - ph, kx*dw - pw
 };
 constexpr int DW_TABLE_BYTES = BLOCK_M * (int)sizeof(DwRow);
@@ -406,7 +407,7 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_tc_kernel(const DwTcArgs a
   if (threadIdx.x < BLOCK_M) {
     const int m = m0 + threadIdx.x;
     DwRow r;
-    r.chan_off = -1; r.ydelta = 0; r.xdelta = 0;
+    r.chan_off = NO_ROW; r.ydelta = 0; r.xdelta = 0;
     if (m < a.m_total) {
       const int tap = m / g.cig, ci = m - tap * g.cig;
       r.chan_off = ((long long)group * g.cig + ci) * a.x.s1;
@@ -451,7 +452,7 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_tc_kernel(const DwTcArgs a
           const bool is_a = rb < 4;
           const int r = (is_a ? rb : rb - 4) * 32 + lane;
           DwRow row;
-          row.chan_off = -1; row.ydelta = 0; row.xdelta = 0;
+          row.chan_off = NO_ROW; row.ydelta = 0; row.xdelta = 0;
           if (is_a) row = rows[r];
           const long long ychan = ((long long)group * g.cog + n0 + r) * a.dy.s1;
           const bool brow_ok = r < cols_valid;
@@ -468,7 +469,7 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_tc_kernel(const DwTcArgs a
               float val = 0.f;
               if (is_a) {
                 const int iy = kiy + row.ydelta, ix = kix + row.xdelta;
-                if (kok && row.chan_off >= 0 && iy >= 0 && iy < g.h && ix >= 0 && ix < g.w)
+                if (kok && row.chan_off != NO_ROW && iy >= 0 && iy < g.h && ix >= 0 && ix < g.w)
                   val = __ldg(a.x.ptr + kxb + row.chan_off + (long long)iy * a.x.s2 + (long long)ix * a.x.s3);
               } else if (kok && brow_ok) {
                 val = __ldg(a.dy.ptr + kyb + ychan);
@@ -498,7 +499,7 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_tc_kernel(const DwTcArgs a
         for (int j = 0; j < 8; ++j) {
           const DwRow row = rows[wi * 16 + r0 + j];
           const int iy = iy0 + row.ydelta, ix = ix0 + row.xdelta;
-          const bool in = ok && row.chan_off >= 0 && iy >= 0 && iy < g.h && ix >= 0 && ix < g.w;
+          const bool in = ok && row.chan_off != NO_ROW && iy >= 0 && iy < g.h && ix >= 0 && ix < g.w;
           v[j] = in ? __ldg(a.x.ptr + xb + row.chan_off + (long long)iy * a.x.s2 + (long long)ix * a.x.s3) : 0.f;
         }
 #pragma unroll
