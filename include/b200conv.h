@@ -415,6 +415,9 @@ uint64_t b200_launch_count(void);
 /* Name of the kernel family the last conv/gemm call on this thread launched
  * (e.g. "tc_igemm_fwd", "simt_igemm_dweight+finalize"). */
 const char* b200_last_kernel(void);
+/* Where the rows of the last normalisation call waited between its sums and its result: "registers", "parked" (one tensor of two in
+ * shared memory), "staged" (shared memory), or "" (every other kernel). */
+const char* b200_last_form(void);
 
 #ifdef __cplusplus
 }

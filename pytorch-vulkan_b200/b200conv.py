@@ -135,6 +135,7 @@ SIGNATURES = {
     "b200_device_status": (c_int, [POINTER(c_int), c_int]),
     "b200_launch_count": (c_uint64, []),
     "b200_last_kernel": (c_char_p, []),
+    "b200_last_form": (c_char_p, []),
 }
 
 _lib = None
@@ -178,6 +179,10 @@ def launch_count():
 
 def last_kernel():
     return lib().b200_last_kernel().decode()
+
+
+def last_form():
+    return lib().b200_last_form().decode()
 
 
 def comm_unique_id() -> bytes:

@@ -771,7 +771,6 @@ __global__ void __launch_bounds__(nres::THREADS, PARK ? 6 : 4) bn_backward_chann
   }
 }
 
-// Ranks per channel for the kernels above, or 0: the streaming kernels take the call.
 // Where the parked form (bn_backward_channel_kernel) is the faster one: beyond one wave of the other, if fewer ranks hold a channel or everything runs
 // at once.  Measured, gain over the other form on 60 random layers: 1.00 to 1.38, median 1.08, within the line (but 8 -> 7 ranks .93, and .97 to 1.03
 // where the second wave is up to a fifth full); .89 to 1.06, median .95, where the ranks stay and a wave does not hold all.
@@ -781,6 +780,7 @@ bool parks(const BnShape& sh, int ranks, int parked_ranks) {
   return waves <= 1.0 || (waves >= 1.2 && parked_ranks * 7 <= ranks * 6);
 }
 
+// Ranks per channel for the kernels above, or 0: the streaming kernels take the call.
 int channel_ranks(const BnShape& sh, int layout, int vec, int most, bool backward) {
   if (layout != B200_BN_PLANAR || sh.inner / vec >= (1 << 30) / sh.outer) return 0;
   const nres::RankPlan p = nres::plan_ranks((long long)sh.outer * (sh.inner / vec), sh.c, most, sm_count());
@@ -1002,10 +1002,10 @@ int b200_batch_norm_backward(int64_t n, int64_t c, int64_t s, int layout, const 
   if (has_sums) {
     const int vec = sh.inner % 4 == 0 && aligned16(x) && aligned16(grad) && aligned16(dx) ? 4 : 1;
     if (int ranks = channel_ranks(sh, layout, vec, vec == 4 ? kUnitsBwd : kUnits1, true)) {
-      note_kernel("bn_backward_channel");
       const int parked_ranks = channel_ranks(sh, layout, vec, kUnitsParked, true);
       const bool park = vec == 4 && parks(sh, ranks, parked_ranks);
       if (park) ranks = parked_ranks;
+      note_kernel("bn_backward_channel", park ? "parked" : "registers");
       const nres::Rows rows = nres::make_rows(sh.outer, sh.inner, vec, (long long)sh.c * sh.inner, ranks);
       return nres::launch(vec == 1 ? bn_backward_channel_kernel<1, kUnits1, false>
                           : park   ? bn_backward_channel_kernel<4, kUnitsParked, true>

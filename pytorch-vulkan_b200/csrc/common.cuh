@@ -26,7 +26,7 @@ int ensure_init();
 bool library_is_initialised();  // true once b200_init has bound a device
 int sm_count();
 extern std::atomic<uint64_t> g_launches;
-void note_kernel(const char* name);
+void note_kernel(const char* name, const char* form = "");   // what b200_last_kernel() and b200_last_form() answer
 inline void count_launch(int n = 1) { g_launches.fetch_add((uint64_t)n, std::memory_order_relaxed); }
 
 // Checks the launch of the kernel named `what`; to be used right after <<<>>>.

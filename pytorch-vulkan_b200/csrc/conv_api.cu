@@ -210,7 +210,7 @@ int b200_conv2d_forward(const b200_conv_params* p, b200_view4 x, b200_view4 w, c
   cudaStream_t st = (cudaStream_t)stream;
   if (!bias) bias_stride = 0;
   if (takes_one_launch(g, false, algo, chosen, workspace)) {
-    note_kernel("tc_strip_forward");
+    note_kernel("tc_small_forward");
     return conv_small(g, false, to_view(x), to_view(w), bias, bias_stride, nullptr, y, st);
   }
   switch (chosen) {
@@ -251,9 +251,11 @@ int b200_conv2d_forward_fused(const b200_conv_params* p, b200_view4 x, b200_view
   post.relu = relu;
   // the strip kernel applies everything in its epilogue and can write [pixel][channel] rows
   if (chosen == B200_ALGO_TC && strip_supported(g, B200_PHASE_FORWARD)) {
-    note_kernel("tc_strip_forward_fused");
-    if (!y_channels_last && takes_one_launch(g, false, algo, chosen, workspace, true))
+    if (!y_channels_last && takes_one_launch(g, false, algo, chosen, workspace, true)) {
+      note_kernel("tc_small_forward_fused");
       return conv_small(g, false, to_view(x), to_view(w), bias, bias_stride, &post, y, st);
+    }
+    note_kernel("tc_strip_forward_fused");
     if (const int slices = y_channels_last || !strip_view_addressable(g, false, to_view(x), nullptr) ? 1 : conv_slices(g, false, false);
         slices > 1 && workspace && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0 && conv_slices_workspace(g, false, slices, false) <= workspace_bytes)
       return conv_sliced(g, false, slices, false, to_view(x), to_view(w), bias, bias_stride, &post, y, workspace, st);
@@ -291,7 +293,7 @@ static int dinput_with_bias(const b200_conv_params* p, b200_view4 dy, b200_view4
       break;
     case B200_ALGO_TC:
       if (takes_one_launch(g, true, algo, chosen, workspace)) {
-        note_kernel("tc_strip_dinput");
+        note_kernel("tc_small_dinput");
         rc = conv_small(g, true, to_view(dy), to_view(w), bias, bias_stride, nullptr, dx, st);
         bias_applied = true;
         break;

@@ -740,7 +740,7 @@ int tc_forward(const ConvGeom& g, View4 x, View4 w, const float* bias, long long
   }
   int route = tc_route(g, false, x);
   if (automatic && route != 3 && ws && (reinterpret_cast<uintptr_t>(ws) & 15) == 0 && tstrip_stacks(g, false) && tstrip_workspace(g, B200_PHASE_FORWARD) <= ws_bytes) {
-    note_kernel("tc_strip_forward");
+    note_kernel("tc_stacked_forward");
     return tstrip_conv(g, false, x, w, bias, bias_stride, y, ws, ws_bytes, st);
   }
   if (route == 3 || route == 0)
@@ -773,7 +773,7 @@ int tc_dinput(const ConvGeom& g, View4 dy, View4 w, const float* bias, long long
   if (bias_applied) *bias_applied = bias != nullptr;
   int route = tc_route(g, true, dy);
   if (automatic && route != 3 && ws && (reinterpret_cast<uintptr_t>(ws) & 15) == 0 && tstrip_stacks(g, true) && tstrip_workspace(g, B200_PHASE_DINPUT) <= ws_bytes) {
-    note_kernel("tc_strip_dinput");
+    note_kernel("tc_stacked_dinput");
     return tstrip_conv(g, true, dy, w, bias, bias_stride, dx, ws, ws_bytes, st);
   }
   if (route == 3 || route == 0)

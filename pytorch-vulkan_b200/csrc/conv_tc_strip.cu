@@ -971,6 +971,7 @@ int strip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* b
       tiles_n == 1 && 4 * nc >= (plan.bn == 256 ? 3 : 2) * plan.bn && (long long)cpp * plan.bn * 256 <= gt::PLANES_B && act.s3 == 1 && (act.s2 == a.W || a.H == 1) && act.s1 % 4 == 0 && act.s0 % 4 == 0 &&
       (reinterpret_cast<uintptr_t>(act.ptr) & 15) == 0 && pixels >= 512 && (long long)g.n * ((pixels + 127) / 128) >= 2ll * sm_count() &&
       !getenv("B200_CONV_TC_VARIANT")) {
+    note_kernel(is_dx ? "tc_planes_dinput" : "tc_planes_forward");
     gt::GemmArgs m{};
     m.planes = 1;
     m.A = act.ptr; m.a_m = 1; m.a_k = act.s1; m.a_group = act.s0;

@@ -625,15 +625,19 @@ int b200_group_norm_forward(int64_t n, int64_t c, int64_t hw, int64_t groups, co
     count_launch();
     return launch_check("gn_forward_bulk_kernel");
   }
-  note_kernel("gn_forward");
   const int vec = sh.hw % 4 == 0 && aligned ? 4 : 1;
-  if (const int ranks = block_ranks(sh, blocks, vec, vec == 4 ? kUnits : kUnits1, false))
+  if (const int ranks = block_ranks(sh, blocks, vec, vec == 4 ? kUnits : kUnits1, false)) {
+    note_kernel("gn_forward", "registers");
     return nres::launch(vec == 4 ? gn_forward_cluster_kernel<4, kUnits> : gn_forward_cluster_kernel<1, kUnits1>, (unsigned)blocks, ranks, 0, st, x, weight,
                         bias, sh, nres::make_rows(sh.cpg, sh.hw, vec, sh.hw, ranks), eps, y, mean, rstd);
-  if (const nres::StagedPlan staged = forward_staged(sh, vec); staged.ranks)
+  }
+  if (const nres::StagedPlan staged = forward_staged(sh, vec); staged.ranks) {
+    note_kernel("gn_forward", "staged");
     return nres::launch(vec == 4 ? nres::gn_forward_staged_kernel<4> : nres::gn_forward_staged_kernel<1>, (unsigned)blocks, staged.ranks,
                         (size_t)staged.units * nres::THREADS * 4 * vec, st, x, weight, bias, group_shape(sh), nres::make_rows(sh.cpg, sh.hw, vec, sh.hw, staged.ranks),
                         staged.units, eps, y, mean, rstd);
+  }
+  note_kernel("gn_forward");
   launch_next(gn_forward_kernel, (unsigned)(n * groups), kThreads, 0, st, x, weight, bias, sh, eps, y, mean, rstd);
   count_launch();
   return launch_check("gn_forward_kernel");
@@ -652,11 +656,11 @@ int b200_group_norm_backward(int64_t n, int64_t c, int64_t hw, int64_t groups, c
     return fail(B200_EWORKSPACE, "native_group_norm_backward: workspace missing, unaligned or smaller than b200_group_norm_workspace()");
   cudaStream_t st = (cudaStream_t)stream;
   float* plane_sums = affine ? (float*)workspace : nullptr;
-  note_kernel(affine ? "gn_backward+affine" : "gn_backward");
   const bool aligned = ((reinterpret_cast<uintptr_t>(grad) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dx)) & 15) == 0;
   const int vec = sh.hw % 4 == 0 && aligned ? 4 : 1, blocks = (int)(n * groups);
   const BackwardPlan plan = backward_plan(sh, blocks, vec);
   const int ranks = plan.ranks;
+  note_kernel(affine ? "gn_backward+affine" : "gn_backward", plan.park ? "parked" : ranks ? "registers" : plan.staged.ranks ? "staged" : "");
   if (ranks) {
     const nres::Rows rows = nres::make_rows(sh.cpg, sh.hw, vec, sh.hw, ranks);
     if (int rc = nres::launch(vec == 1    ? gn_backward_cluster_kernel<1, kUnits1, false>

@@ -21,7 +21,7 @@
 namespace b200 {
 
 static thread_local std::string t_error;
-static thread_local const char* t_kernel = "";
+static thread_local const char *t_kernel = "", *t_form = "";
 std::atomic<uint64_t> g_launches{0};
 
 void set_error(const char* fmt, ...) {
@@ -44,7 +44,7 @@ int fail(int code, const char* fmt, ...) {
 int cuda_fail(cudaError_t e, const char* what) {
   return fail(B200_ECUDA, "CUDA error %d (%s) in %s", (int)e, cudaGetErrorString(e), what);
 }
-void note_kernel(const char* name) { t_kernel = name; }
+void note_kernel(const char* name, const char* form) { t_kernel = name; t_form = form; }
 int launch_check(const char* what) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(B200_ECUDA, "launch of %s failed: %s", what, cudaGetErrorString(e));
@@ -163,6 +163,7 @@ const char* b200_device_name(void) { return ensure_init() == B200_OK ? g_name : 
 int b200_device_sm_count(void) { return ensure_init() == B200_OK ? g_sms : 0; }
 uint64_t b200_launch_count(void) { return g_launches.load(); }
 const char* b200_last_kernel(void) { return t_kernel; }
+const char* b200_last_form(void) { return t_form; }
 
 int b200_malloc(void** ptr, size_t bytes, void* stream) {
   if (!ptr) return fail(B200_EINVAL, "b200_malloc: null out pointer");

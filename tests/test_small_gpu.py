@@ -45,15 +45,15 @@ def test_forward_fused_and_dinput(case, layout):
     b, res = rng.standard_normal(cout, dtype=np.float32), rng.standard_normal(g.y_shape, dtype=np.float32)
     y64, dx64 = oracle.torch_conv_all(x, w, b, go, (1, 1), kw.get("padding", (0, 0)), kw.get("dilation", (1, 1)), 1)[:2]
 
-    def one_launch(call):
+    def one_launch(kernel, call):
         before = b200conv.launch_count()
         out = call()
-        assert b200conv.launch_count() == before + 1 and b200conv.last_kernel().startswith("tc_strip") and b200conv.device_status() == 0
+        assert b200conv.launch_count() == before + 1 and b200conv.last_kernel() == kernel and b200conv.device_status() == 0
         return out
-    y = one_launch(lambda: b200conv.conv2d_forward(_lay(x, layout), w, b, **kw))
+    y = one_launch("tc_small_forward", lambda: b200conv.conv2d_forward(_lay(x, layout), w, b, **kw))
     assert oracle.rel_l2(y, y64) <= 1e-5
-    fused = one_launch(lambda: b200conv.conv2d_forward_fused(_lay(x, layout), w, b, residual=_lay(res, layout), relu=True, **kw))
+    fused = one_launch("tc_small_forward_fused", lambda: b200conv.conv2d_forward_fused(_lay(x, layout), w, b, residual=_lay(res, layout), relu=True, **kw))
     assert oracle.rel_l2(fused, np.maximum(y64 + res, 0)) <= 1e-5
     w_turned = np.ascontiguousarray(w.transpose(1, 0, 2, 3)).transpose(1, 0, 2, 3)      # the filter through other strides
-    dx = one_launch(lambda: b200conv.conv2d_backward(_lay(go, layout), x, w_turned, mask=(True, False, False), **kw)[0])
+    dx = one_launch("tc_small_dinput", lambda: b200conv.conv2d_backward(_lay(go, layout), x, w_turned, mask=(True, False, False), **kw)[0])
     assert oracle.rel_l2(dx, dx64) <= 1e-5
