@@ -656,9 +656,11 @@ bool tstrip_supported(const ConvGeom& g, int phase) {
 // comes here: a forced candidate stays on the strip kernel, whose sums are those of the fused forward pass bit for bit.
 bool tstrip_stacks(const ConvGeom& g, bool is_dx) {
   const int nc = is_dx ? g.cig : g.cog;
-  if (nc > tst::TM / 2 || !tst::plan_tstrip(g, is_dx).ok) return false;
-  if (const char* v = getenv("B200_CONV_TC_VARIANT")) return !strcmp(v, "stacked");   // testing aid
-  return tstrip_time(g, is_dx, nullptr) < 0.9 * conv_slices_time(g, is_dx);
+  if (nc > tst::TM / 2) return false;
+  if (const char* v = getenv("B200_CONV_TC_VARIANT")) return !strcmp(v, "stacked") && tst::plan_tstrip(g, is_dx).ok;   // testing aid
+  // Every call asks twice, and the other kernel's time is that of its best slices: kept, as conv_slices() keeps theirs.
+  thread_local PlanCache<int> cache;
+  return cache.get(g, is_dx, [&] { return tstrip_time(g, is_dx, nullptr) < 0.9 * conv_slices_time(g, is_dx) ? 1 : 0; }) != 0;
 }
 double tstrip_time(const ConvGeom& g, bool is_dx, long long* tiles) {
   const tst::TPlan& p = tst::plan_tstrip(g, is_dx);
