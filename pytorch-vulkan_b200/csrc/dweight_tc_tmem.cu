@@ -372,7 +372,7 @@ __global__ void __launch_bounds__(THREADS, 1) dweight_tmem_kernel(const Args a) 
     const float* src = a.dy.ptr + chan_off;
     // lane = pixel (channels apart in memory) or lane = channel (channels adjacent)
     auto load = [&](int k, float (&v)[32]) {
-      int off = NO_PIXEL;                          // element offset of this lane's pixel, -1 where the contraction has nothing
+      int off = NO_PIXEL;                          // element offset of this lane's pixel, NO_PIXEL where the contraction has nothing
       {
         const int qx = k_begin + k * KP + lane, q = qx + dq;
         if (qx < k_end && q >= 0 && q < a.q_total) {

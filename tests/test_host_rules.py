@@ -54,7 +54,7 @@ int main() {
     assert int(out.split()[1]) == 0
 
 
-CLUSTER_SOURCES = ("reduce.cu", "batch_norm.cu", "group_norm.cu", "norm_resident.cuh")
+CLUSTER_SOURCES = ("reduce.cu", "batch_norm.cu", "group_norm.cu", "norm_resident.cuh", "conv_tc_small.cu")
 
 
 def _functions(name):
@@ -74,7 +74,7 @@ def test_clusters_wait_until_every_cta_has_started():
     checked = 0
     for name in CLUSTER_SOURCES:
         for function, kernel, body in _functions(name):
-            stores = [body.find(w) for w in ("map_shared_rank", "cluster_sum(", "row_moments<") if w in body]
+            stores = [body.find(w) for w in ("map_shared_rank", "cluster_sum(", "row_moments<", "st_remote(") if w in body]
             if not stores or function == "cluster_sum":
                 continue
             waited, first = body.find("cluster_wait_started()"), min(stores)
@@ -84,7 +84,7 @@ def test_clusters_wait_until_every_cta_has_started():
                 announced = body.find("cluster_announce()")
                 assert 0 <= announced < body.find("wait_previous()"), f"{name}: {function} does not announce itself first"
                 checked += 1
-    assert checked == 6
+    assert checked == 7
 
 
 def test_norm_rank_plans_hold_their_rows(tmp_path):
