@@ -80,7 +80,8 @@ struct TArgs {
   int cb_per_phase, cblocks, images_per_tile;
   int tiles_m, tiles_p, tiles_total;
   int pn;                 // pixels per tile: a multiple of 16, at most 256
-  int delta, step;        // stacked taps: grid pixels between the two taps of a stack (0: off); pixels that a tile completes, pn - delta
+  int delta, step;        // Stacked::delta; pixels that a tile completes, pn - delta
+  unsigned long long lone;
   int q_total;
   FastDiv img_div, row_div, div_tiles_p, div_tiles_m, div_tiles_pp, div_chunks, div_cblocks, div_cbpp, div_a_stages;
   int halo, strip_rows;   // rows staged before a tile's first pixel; rows per stage (a multiple of 8)
@@ -102,12 +103,14 @@ struct TArgs {
 #endif
 #define TPROF(slot, stmt) do { if (B200_ROLE_PROFILE && a.prof && blockIdx.x == 0) { const long long t0__ = clock64(); stmt; atomicAdd(a.prof + (slot), (unsigned long long)(clock64() - t0__)); } else { stmt; } } while (0)
 
-// Second tap of a stack (filter column) where 64 or fewer output channels leave half of the filter rows to it.  NO_TAP, there or for a first tap:
-// weights of zero.
+// Stacked taps: 64 or fewer output channels leave half of the filter rows to a second tap of the same filter row.  In every 32 rows the first tap of
+// channels 16w .. 16w+15 is followed by their second one; a tap without a second runs as 64 rows, which the tensor core places on lanes 0-15 of every
+// 32.  So no weights of zero meet pixels that the filter does not reach, where an infinity or NaN would become one of the result.
 constexpr unsigned char NO_TAP = 255;
 struct Stacked {
-  int delta = 0;
-  unsigned char kx[MAX_TAPS];
+  int delta = 0;                   // grid pixels between the two taps of a stack (0: no stacks)
+  unsigned long long lone = 0;     // taps without a second
+  unsigned char kx[MAX_TAPS];      // filter column of the second tap, or NO_TAP
 };
 
 struct Ctrl {
@@ -121,14 +124,6 @@ struct Ctrl {
 // byte offset of 16-byte chunk `c` (0..3) of row `row` in a plane of 64-byte rows, SWIZZLE_64B
 __device__ __host__ __forceinline__ uint32_t sw64_chunk(int row, int c) {
   return (uint32_t)(row * ROWB + ((c ^ ((row >> 1) & 3)) << 4));
-}
-// barrier of the epilogue warps; with a predicate, true for all where it is true for each
-__device__ __forceinline__ void epilogue_sync() { asm volatile("barrier.cta.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory"); }
-__device__ __forceinline__ bool epilogue_all(bool mine) {
-  int all;
-  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbarrier.cta.red.and.pred q, 1, %2, p;\n\tselp.b32 %0, 1, 0, q;\n\t}"
-               : "=r"(all) : "r"((int)mine), "n"(EPI_WARPS * 32) : "memory");
-  return all != 0;
 }
 // K-major operand descriptor for a plane of 64-byte rows, SWIZZLE_64B: 8-row groups 512 bytes apart
 __device__ __forceinline__ uint64_t make_kmajor_sw64_desc(uint32_t smem_addr) {
@@ -155,7 +150,7 @@ __device__ __forceinline__ TileCoord tile_coord(const TArgs& a, int tile) {
   return c;
 }
 
-template <int AW>
+template <int AW, bool STACKED>
 __global__ void __launch_bounds__(tstrip_threads(AW), 1) conv_tstrip_kernel(const TArgs a) {
   constexpr int A_WARPS = AW, W_WARP = EPI_WARPS + AW, MMA_WARP = W_WARP + 1;
   extern __shared__ unsigned char smem_raw[];
@@ -209,6 +204,7 @@ __global__ void __launch_bounds__(tstrip_threads(AW), 1) conv_tstrip_kernel(cons
     // tensor-pipe idle time of 43 %) was what bounded the kernel.
     // D[128 filter rows][pn pixels] += W[128 x 8] * X[pn x 8]^T, both operands K-major
     const uint32_t idesc = make_idesc_tf32(TM, a.pn), idesc_cross = make_idesc_bf16(TM, a.pn);
+    constexpr uint32_t HALF = (uint32_t)(TM / 2 >> 4) << 24;     // from a descriptor of 128 rows to one of 64
     const uint64_t dx_base = make_kmajor_sw64_desc(tiles_base + (uint32_t)a.halo * ROWB);
     const uint64_t dw_base = make_kmajor_sw64_desc(w_base);
     const uint32_t a_stage_d = a_stage_bytes >> 4, a_plane_d = a_plane >> 4;
@@ -236,16 +232,17 @@ __global__ void __launch_bounds__(tstrip_threads(AW), 1) conv_tstrip_kernel(cons
           if (!warp_wait(smem_u32(&ctrl->w_full[ws]), w_par, abort_flag, a.status, STATUS_TIMEOUT_FULL)) { alive = false; break; }
           const uint64_t x0 = dx_strip + (uint64_t)(long long)(sh0 * (ROWB / 16)), x1 = dx_strip + (uint64_t)(long long)(sh1 * (ROWB / 16));
           const uint64_t w0 = dw_base + ws * w_ring_d, w1 = w0 + w_stage_d;
+          const uint32_t h0 = STACKED && (a.lone >> tap & 1) ? HALF : 0u, h1 = STACKED && (a.lone >> (tap + 1) & 1) ? HALF : 0u;
           if (leader) {
-            umma_tf32(tmem_acc, w0, x0, idesc, accumulate);
-            umma_tf32(tmem_acc, w0 + 2, x0 + 2, idesc, 1);
-            umma_bf16(tmem_acc, w0 + w_plane_d, x0 + a_plane_d, idesc_cross, 1);
-            umma_bf16(tmem_acc, w0 + w_plane_d + 2, x0 + a_plane_d + 2, idesc_cross, 1);
+            umma_tf32(tmem_acc, w0, x0, idesc - h0, accumulate);
+            umma_tf32(tmem_acc, w0 + 2, x0 + 2, idesc - h0, 1);
+            umma_bf16(tmem_acc, w0 + w_plane_d, x0 + a_plane_d, idesc_cross - h0, 1);
+            umma_bf16(tmem_acc, w0 + w_plane_d + 2, x0 + a_plane_d + 2, idesc_cross - h0, 1);
             if (two) {
-              umma_tf32(tmem_acc, w1, x1, idesc, 1);
-              umma_tf32(tmem_acc, w1 + 2, x1 + 2, idesc, 1);
-              umma_bf16(tmem_acc, w1 + w_plane_d, x1 + a_plane_d, idesc_cross, 1);
-              umma_bf16(tmem_acc, w1 + w_plane_d + 2, x1 + a_plane_d + 2, idesc_cross, 1);
+              umma_tf32(tmem_acc, w1, x1, idesc - h1, 1);
+              umma_tf32(tmem_acc, w1 + 2, x1 + 2, idesc - h1, 1);
+              umma_bf16(tmem_acc, w1 + w_plane_d, x1 + a_plane_d, idesc_cross - h1, 1);
+              umma_bf16(tmem_acc, w1 + w_plane_d + 2, x1 + a_plane_d + 2, idesc_cross - h1, 1);
             }
             umma_commit(smem_u32(&ctrl->w_empty[ws]));
           }
@@ -395,25 +392,21 @@ __global__ void __launch_bounds__(tstrip_threads(AW), 1) conv_tstrip_kernel(cons
     // Warp w owns accumulator lanes 32w .. 32w+31 (output channels).  tcgen05.ld hands thread = channel its 32
     // consecutive pixels; a 32x33 shared-memory tile turns that into thread = pixel, so that each store
     // instruction writes 32 consecutive pixels of one channel plane.
-    // Stacked taps: the lanes of warps 2 and 3 hold what the second taps add, `delta` pixels further on; every warp then adds and stores
-    // half of the channels of a pair of tiles.
-    float* tiles = reinterpret_cast<float*>(smem_raw + (tbuf_base - raw));
-    float* tb = tiles + warp * (32 * 33);
-    const int pair = a.delta ? warp & 1 : warp;
+    // Stacked taps: lanes 16-31 hold what the second taps add to the channels of lanes 0-15, `delta` pixels further on.
+    constexpr int CH = STACKED ? 16 : 32;    // channels of a warp
+    float* tb = reinterpret_cast<float*>(smem_raw + (tbuf_base - raw)) + warp * (32 * 33);
     for (int t = 0; t < my_tiles; ++t) {
       const TileCoord tc_ = tile_coord(a, (int)blockIdx.x + t * (int)gridDim.x);
       const int phase_m = a.phase_on_m ? (int)a.div_tiles_pp.div((uint32_t)tc_.m_tile) : 0;
-      const int c0 = (tc_.m_tile - phase_m * a.tiles_pp) * TM + pair * 32;   // first channel (within the group) of this warp
-      const int nch = min(32, a.nc - c0);                                       // channels of this warp that exist (may be <= 0)
+      const int c0 = (tc_.m_tile - phase_m * a.tiles_pp) * TM + warp * CH;   // first channel (within the group) of this warp
+      const int nch = min(CH, a.nc - c0);                                       // channels of this warp that exist (may be <= 0)
       const uint32_t ab = (uint32_t)t & 1u;
       const bool has_taps = !a.phase_on_m || ctrl->tap_start[phase_m + 1] > ctrl->tap_start[phase_m];
       float bv = 0.f;  // lane j holds the bias of channel c0 + j
       if (a.bias && lane < nch) bv = __ldg(a.bias + ((long long)tc_.group * a.nc + c0 + lane) * a.bias_stride);
-      bool complete = mbar_wait(smem_u32(&ctrl->acc_full[ab]), ((uint32_t)t >> 1) & 1u, abort_flag, a.status, STATUS_TIMEOUT_ACCUM);
-      if (a.delta) complete = epilogue_all(complete);   // the warps meet below: all of them go on, or none
-      if (!complete) break;
+      if (!mbar_wait(smem_u32(&ctrl->acc_full[ab]), ((uint32_t)t >> 1) & 1u, abort_flag, a.status, STATUS_TIMEOUT_ACCUM)) break;
       tc_fence_after();
-      const uint32_t tmem_acc = tmem_base + ab * ACC_COLS + ((uint32_t)(warp * 32) << 16) + (uint32_t)(warp >= 2 ? a.delta : 0);
+      const uint32_t tmem_acc = tmem_base + ab * ACC_COLS + ((uint32_t)(warp * 32) << 16);
       const int q_tile = tc_.p_tile * a.step;
       const int cols = min(a.step, a.q_total - q_tile);
       const int nchunks = (cols + 31) / 32;
@@ -424,11 +417,20 @@ __global__ void __launch_bounds__(tstrip_threads(AW), 1) conv_tstrip_kernel(cons
       for (int ch = 0; ch < nchunks; ++ch) {
         float v[32];
         tmem_ld32(tmem_acc + (uint32_t)(ch * 32), v);
+        if (STACKED) {
+#pragma unroll
+          for (int h = 0; h < 32; h += 16) {
+            float second[16];
+            tmem_ld16(tmem_acc + (uint32_t)(ch * 32 + h + a.delta), second);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[h + j] = lane < CH ? v[h + j] : second[j];
+          }
+        }
         if (ch + 1 == nchunks) {  // last read of this accumulator: hand it back
           tc_fence_before();
           mbar_arrive(smem_u32(&ctrl->acc_empty[ab]));
         }
-        if (nch <= 0 && !a.delta) continue;
+        if (nch <= 0) continue;
         // this lane's pixel of the chunk
         const int q = q_tile + ch * 32 + lane;
         bool ok = ch * 32 + lane < cols;
@@ -442,28 +444,19 @@ __global__ void __launch_bounds__(tstrip_threads(AW), 1) conv_tstrip_kernel(cons
           ok = ok && y < a.out_h && x < a.out_w;
           obase = ((n * a.out_channels + (long long)tc_.group * a.nc + c0) * a.out_h + y) * a.out_w + x;
         }
-        if (a.delta) {
-          epilogue_sync();   // the previous chunk's reads of the tiles are done
-#pragma unroll
-          for (int j = 0; j < 32; ++j) tb[lane * 33 + j] = v[j];
-          epilogue_sync();
-          const int first = (warp >> 1) * 16;
-          const float *lower = tiles + pair * (32 * 33) + first * 33 + lane, *upper = lower + 2 * 32 * 33;
-          float* p = a.out + obase + first * plane;
-#pragma unroll
-          for (int c = 0; c < 16; ++c, p += plane) {
-            const float val = lower[c * 33] + upper[c * 33] + __shfl_sync(0xffffffffu, bv, first + c);
-            if (ok && first + c < nch) *p = val;
-          }
-          continue;
-        }
         __syncwarp();   // the previous chunk's reads of the tile are done
 #pragma unroll
         for (int j = 0; j < 32; ++j) tb[lane * 33 + j] = has_taps ? v[j] : 0.f;   // [channel][pixel]
         __syncwarp();
         // every lane takes part in the shuffles (a pixel on padding only skips its stores)
         float* p = a.out + obase;
-        if (nch == 32) {
+        if (STACKED) {
+#pragma unroll
+          for (int c = 0; c < CH; ++c, p += plane) {
+            const float val = tb[c * 33 + lane] + tb[(CH + c) % 32 * 33 + lane] + __shfl_sync(0xffffffffu, bv, c);
+            if (ok && c < nch) *p = val;
+          }
+        } else if (nch == 32) {
 #pragma unroll
           for (int c = 0; c < 32; ++c, p += plane) {
             const float val = tb[c * 33 + lane] + __shfl_sync(0xffffffffu, bv, c);
@@ -495,7 +488,8 @@ __global__ void __launch_bounds__(tstrip_threads(AW), 1) conv_tstrip_kernel(cons
 // main loop consumes them: forward [group][channel tile][phase][channel block][tap of the phase], dInput
 // [group][phase][channel tile of the phase][channel block][tap of the phase].  A thread takes four channels of one row and
 // `per_thread` taps (stage_weights_kernel in conv_tc_strip.cu says why).
-// Stacked taps: rows 64 to 127 are those of the second tap of each stack.
+// Stacked taps: the rows of a stack as Stacked says; a lone tap has its channels in rows 0 to 63, and no one reads the others.
+template <bool STACKED>
 __global__ void __launch_bounds__(256) stage_filter16_kernel(ConvGeom g, View4 w, int is_dx, int tiles_pp, TapTable tt, Stacked stacked,
                                                              unsigned char* __restrict__ out, long long total, long long w_group_extra,
                                                              int rows_first, int per_thread) {
@@ -509,11 +503,9 @@ __global__ void __launch_bounds__(256) stage_filter16_kernel(ConvGeom g, View4 w
   const int piece = rows_first ? in_block >> 3 & 3 : in_block % 4, k = piece * 4;
   const int row = rows_first ? (in_block & 7) | in_block >> 5 << 3 : in_block / 4;
   const int tile_of_all = block / cpp, cbl = block - tile_of_all * cpp, grp = tile_of_all / tiles_pp, m_tile = tile_of_all - grp * tiles_pp;
-  const bool second = stacked.delta && row >= 64;
-  const int r = m_tile * TM + (second ? row - 64 : row), c = cbl * KB + k;
-  const int valid = r < nc ? min(4, kc - c) : 0;
-  const long long step = is_dx ? w.s0 : w.s1;
-  const float* src = w.ptr + ((long long)grp * g.cog + (is_dx ? c : r)) * w.s0 + (long long)(is_dx ? r : c) * w.s1 + grp * w_group_extra;
+  const int c = cbl * KB + k;
+  const long long step = is_dx ? w.s0 : w.s1, row_step = is_dx ? w.s1 : w.s0;
+  const float* src_c = w.ptr + (long long)grp * g.cog * w.s0 + c * step + grp * w_group_extra;
   const int t0 = blockIdx.y * per_thread, t1 = min(tt.taps_total, t0 + per_thread);
   int phase = 0;
 #pragma unroll 3
@@ -522,8 +514,9 @@ __global__ void __launch_bounds__(256) stage_filter16_kernel(ConvGeom g, View4 w
     const int ntap = tt.start[phase + 1] - tt.start[phase], rel = tap - tt.start[phase];
     const long long image = is_dx ? (long long)(grp * tt.taps_total + tt.start[phase]) * tiles_pp * cpp + ((long long)m_tile * cpp + cbl) * ntap + rel
                                   : ((long long)tile_of_all * tt.taps_total + tt.start[phase]) * cpp + cbl * ntap + rel;
-    const int kx = second ? stacked.kx[tap] : tt.kx[tap], here = kx == NO_TAP ? 0 : valid;
-    const float* p = src + tt.ky[tap] * w.s2 + kx * w.s3;
+    const bool stack = STACKED && stacked.kx[tap] != NO_TAP, second = stack && (row & 16);
+    const int r = m_tile * TM + (stack ? (row >> 5) * 16 + (row & 15) : row), here = r < nc ? min(4, kc - c) : 0;
+    const float* p = src_c + r * row_step + tt.ky[tap] * w.s2 + (second ? stacked.kx[tap] : tt.kx[tap]) * w.s3;
     float v[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) v[j] = j < here ? __ldg(p + j * step) : 0.f;
@@ -552,34 +545,43 @@ struct TPlan {
 // shared-memory operand read (4 KB of filter + 32 B per pixel) about 96 bytes per clock.
 static double mma_clocks(int pn) { return std::max(pn / 2.0, (4096.0 + 32.0 * pn) / 96.0); }
 
-// Taps in stacks of two: neighbouring filter columns of one row and phase, the one that reads further on second.  The last of an odd number
-// shares a stack with its neighbour once more, whose weights are zero there: zeros must not meet pixels that the filter does not reach, where an
-// infinity or NaN would become one of the result.  False where a row of a phase has one tap only (every other column of a 3-wide filter at stride
-// 2), where the filter does not gain by it (fewer than a quarter of the steps saved) or its taps lie too far apart.
+// Taps in stacks of two: neighbouring filter columns of one row and phase, the one that reads further on second.  A tile begins with a stack, which sets all
+// lanes of its accumulator: phases that have stacks go first, and their stacks before their lone taps.  False where the filter does not gain by it
+// (fewer than a quarter of the steps saved) or its taps lie too far apart.
 static bool stack_taps(TapTable& tt, bool is_dx, Stacked& s) {
   TapTable out = tt;
   out.taps_total = 0;
   s.delta = 0;
-  for (int ph = 0; ph < tt.n_phase; ++ph) {
-    for (int t = tt.start[ph]; t < tt.start[ph + 1];) {
-      int end = t + 1;
-      while (end < tt.start[ph + 1] && tt.ky[end] == tt.ky[t]) ++end;
-      if (end - t < 2) return false;
-      for (; t < end; t += 2) {
-        const bool again = t + 1 == end;            // the row's last tap, and taps t - 1 and t of which the first has had its turn
-        const int a = again ? t - 1 : t, first = is_dx ? a + 1 : a, second = is_dx ? a : a + 1, i = out.taps_total++;
-        out.ky[i] = tt.ky[a]; out.shift[i] = tt.shift[first];
-        out.kx[i] = again && first == a ? NO_TAP : tt.kx[first];
-        s.kx[i] = again && second == a ? NO_TAP : tt.kx[second];
-        const int d = tt.shift[second] - tt.shift[first];
-        if (d < 1 || d > 16 || (s.delta && d != s.delta)) return false;
-        s.delta = d;
-      }
-      t = end;
+  s.lone = 0;
+  auto pairs = [&](int t, int end) { return t + 1 < end && tt.ky[t + 1] == tt.ky[t]; };
+  auto has_stacks = [&](int ph) {
+    for (int t = tt.start[ph]; t < tt.start[ph + 1]; ++t)
+      if (pairs(t, tt.start[ph + 1])) return true;
+    return false;
+  };
+  int phase = 0;
+  for (bool stacks : {true, false})
+    for (int ph = 0; ph < tt.n_phase; ++ph) {
+      if (has_stacks(ph) != stacks) continue;
+      const int end = tt.start[ph + 1];
+      for (bool lone : {false, true})
+        for (int t = tt.start[ph]; t < end;) {
+          const bool two = pairs(t, end);
+          if (two != lone) {
+            const int first = two && is_dx ? t + 1 : t, second = is_dx ? t : t + 1, i = out.taps_total++;
+            out.ky[i] = tt.ky[first]; out.kx[i] = tt.kx[first]; out.shift[i] = tt.shift[first];
+            s.kx[i] = two ? tt.kx[second] : NO_TAP;
+            if (lone) s.lone |= 1ull << i;
+            const int d = two ? tt.shift[second] - tt.shift[first] : s.delta;
+            if (d < 1 || d > 16 || (s.delta && d != s.delta)) return false;
+            s.delta = d;
+          }
+          t += two ? 2 : 1;
+        }
+      out.a[phase] = tt.a[ph]; out.b[phase] = tt.b[ph];
+      out.start[++phase] = (unsigned char)out.taps_total;
     }
-    out.start[ph + 1] = (unsigned char)out.taps_total;
-  }
-  if (!s.delta || 4 * out.taps_total > 3 * tt.taps_total) return false;
+  if (4 * out.taps_total > 3 * tt.taps_total) return false;
   tt = out;
   return true;
 }
@@ -649,9 +651,9 @@ bool tstrip_supported(const ConvGeom& g, int phase) {
   }
   return tst::plan_tstrip(g, is_dx).ok;
 }
-// 64 or fewer output channels: half of the filter rows would multiply padding, so two taps share a tile (rows 0-63 one, 64-127 its
-// neighbour); a step then costs what it does at 128 channels and there are two thirds as many for a 3-wide filter.
-// 64 -> 64 channels of 8x 56x56: forward 18.6 us in the strip kernel, 15.9 here, dInput 17.9 and 15.5; 40 random 3x3 layers with 64 channels or
+// 64 or fewer output channels: half of the filter rows would multiply padding, so two taps share a tile (Stacked); a step
+// then costs what it does at 128 channels and there are two thirds as many for a 3-wide filter.
+// 64 -> 64 channels of 8x 56x56: forward 17.7 us in the strip kernel, 15.2 here, dInput 17.7 and 15.0; 464 -> 32 of 14x 94x94 at stride 2, forward 210 and 101; 40 random 3x3 layers with 64 channels or
 // fewer on a side, forward 0.86 and dInput 0.85 of the time (worst 1.03, a layer that keeps its kernel).  The line is where the models of both meet.  Only the automatic choice
 // comes here: a forced candidate stays on the strip kernel, whose sums are those of the fused forward pass bit for bit.
 bool tstrip_stacks(const ConvGeom& g, bool is_dx) {
@@ -684,7 +686,7 @@ int tstrip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* 
   const int taps = plan.geo.tt.taps_total;
   const long long threads = plan.images / taps * TM * 4;
   const int per_thread = tcs::staged_taps(threads, taps);
-  launch_next(stage_filter16_kernel, dim3((unsigned)div_up64(threads, 256), (unsigned)((taps + per_thread - 1) / per_thread)), 256, 0, st, 
+  launch_next(plan.stacked.delta ? stage_filter16_kernel<true> : stage_filter16_kernel<false>, dim3((unsigned)div_up64(threads, 256), (unsigned)((taps + per_thread - 1) / per_thread)), 256, 0, st, 
       g, w, is_dx ? 1 : 0, plan.tiles_pp, plan.geo.tt, plan.stacked, (unsigned char*)ws, threads, w_group_extra,
       std::llabs(is_dx ? w.s1 : w.s0) < std::llabs(is_dx ? w.s0 : w.s1) ? 1 : 0, per_thread);
   count_launch();
@@ -706,7 +708,7 @@ int tstrip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* 
   a.images_per_tile = plan.cpp * plan.geo.tt.taps_total;
   a.tiles_m = plan.tiles_m; a.tiles_p = plan.tiles_p;
   a.tiles_total = plan.tiles_p * plan.tiles_m * g.groups;
-  a.pn = plan.pn; a.delta = plan.stacked.delta; a.step = plan.pn - plan.stacked.delta;
+  a.pn = plan.pn; a.delta = plan.stacked.delta; a.step = plan.pn - plan.stacked.delta; a.lone = plan.stacked.lone;
   a.q_total = (int)((long long)g.n * (a.H + a.pr) * (a.W + a.pc));
   a.img_div = FastDiv((uint32_t)((a.H + a.pr) * (a.W + a.pc)));
   a.row_div = FastDiv((uint32_t)(a.W + a.pc));
@@ -731,8 +733,8 @@ int tstrip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* 
   static std::once_flag once;
   static cudaError_t opt_in = cudaSuccess;
   std::call_once(once, [] {
-    opt_in = cudaFuncSetAttribute(conv_tstrip_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
-    if (opt_in == cudaSuccess) opt_in = cudaFuncSetAttribute(conv_tstrip_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
+    for (auto kernel : {conv_tstrip_kernel<8, false>, conv_tstrip_kernel<16, false>, conv_tstrip_kernel<8, true>, conv_tstrip_kernel<16, true>})
+      if (opt_in == cudaSuccess) opt_in = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
   });
   B200_CUDA(opt_in);
   // A strided forward pass stages one strip per input phase and gets only one to four taps of MMAs out of it (a
@@ -746,8 +748,8 @@ int tstrip_conv(const ConvGeom& g, bool is_dx, View4 act, View4 w, const float* 
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr; cfg.numAttrs = 1;
-  if (wide) B200_CUDA(cudaLaunchKernelEx(&cfg, conv_tstrip_kernel<16>, a));
-  else B200_CUDA(cudaLaunchKernelEx(&cfg, conv_tstrip_kernel<8>, a));
+  auto kernel = a.delta ? (wide ? conv_tstrip_kernel<16, true> : conv_tstrip_kernel<8, true>) : (wide ? conv_tstrip_kernel<16, false> : conv_tstrip_kernel<8, false>);
+  B200_CUDA(cudaLaunchKernelEx(&cfg, kernel, a));
   count_launch();
   if (profiling) {
     unsigned long long h[16];

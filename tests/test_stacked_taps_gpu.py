@@ -1,6 +1,6 @@
 """Forward and dInput with 64 or fewer result channels in the transposed strip kernel, two filter taps to a tile: odd and even filter widths,
-dilations (the stacked taps lie that far apart), strides (neighbours within a phase; one tap to a row of a phase stays in the strip kernel), ragged channel
-blocks, images smaller than a tile and tiles that end inside one, groups, against PyTorch CPU FP64."""
+dilations (the stacked taps lie that far apart), strides (neighbours within a phase, and phases without any), ragged channel blocks, images smaller
+than a tile and tiles that end inside one, groups, against PyTorch CPU FP64."""
 import numpy as np
 import pytest
 
@@ -15,19 +15,20 @@ CASES = [  # (xshape, cout, kernel, conv arguments)
     ((3, 40, 23, 17), 33, (3, 3), dict(padding=(2, 2), dilation=(2, 2))),
     ((2, 48, 9, 31), 50, (2, 2), dict(padding=(0, 1))),
     ((1, 32, 19, 100), 32, (5, 5), dict(padding=(2, 2))),          # (four rows of 102 pixels beside a tile still fit shared memory)
-    ((2, 33, 31, 30), 64, (3, 3), dict(stride=(2, 2), padding=(1, 1))),    # columns 0 and 2 in one phase, 1 alone in the other: not stacked
+    ((2, 33, 31, 30), 64, (3, 3), dict(stride=(2, 2), padding=(1, 1))),    # columns 0 and 2 in one phase, 1 alone in the other
     ((1, 32, 40, 41), 64, (1, 7), dict(padding=(0, 3))),
     ((2, 96, 14, 15), 96, (3, 3), dict(padding=(1, 1), groups=3)),
     ((9, 64, 56, 56), 64, (3, 3), dict(padding=(1, 1))),
     ((1, 64, 12, 40), 48, (3, 3), dict(padding=(0, 16), dilation=(1, 16))),
     ((2, 32, 13, 21), 32, (3, 5), dict(padding=(1, 2), stride=(1, 2))),       # columns 0, 2, 4 and 1, 3
+    ((1, 20, 21, 23), 17, (1, 3), dict(padding=(0, 1))),                      # a stack and a lone tap; one channel on the second warp
+    ((3, 50, 25, 28), 48, (3, 3), dict(padding=(1, 1), stride=(2, 1))),
 ]
 
 
 def _kernels(case):
-    """The kernels of forward and dInput: every phase of a strided forward pass needs two taps in a row, and dInput has to have one phase."""
-    kernel, stride = case[2], case[3].get("stride", (1, 1))
-    return "tc_stacked_forward" if kernel[1] >= 2 * stride[1] else "tc_strip_forward", "tc_stacked_dinput" if stride == (1, 1) else "tc_strip_dinput"
+    """The kernels of forward and dInput, which is not stacked in several phases."""
+    return "tc_stacked_forward", "tc_stacked_dinput" if case[3].get("stride", (1, 1)) == (1, 1) else "tc_strip_dinput"
 
 
 @pytest.mark.parametrize("layout", ["nchw", "nhwc"])
